@@ -14,31 +14,64 @@ struct Acc {
     float fx, fy, fz, ffi, fpsi, fth, tx, ty, tz;
 };
 
+// The force arithmetic below is written with explicitly rounded operations
+// wherever a product meets a sum, so that every kernel it is inlined into
+// (per-step, persistent, forces only) gives the same bits.
+
 // Adds a pair term with radial factor dUdr = U'(r)/r along d = site_j - site_i
 // and its torque dUdr * (w_i x d) about the bead centre.
+__device__ __forceinline__ float cross1(float a, float b, float c, float d) {   // a b - c d
+    return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
 __device__ __forceinline__ void acc_pair(Acc &A, float dUdr, float3 d, float3 wi) {
-    A.fx += dUdr * d.x;
-    A.fy += dUdr * d.y;
-    A.fz += dUdr * d.z;
-    A.tx += dUdr * (wi.y * d.z - wi.z * d.y);
-    A.ty += dUdr * (wi.z * d.x - wi.x * d.z);
-    A.tz += dUdr * (wi.x * d.y - wi.y * d.x);
+    A.fx = __fmaf_rn(dUdr, d.x, A.fx);
+    A.fy = __fmaf_rn(dUdr, d.y, A.fy);
+    A.fz = __fmaf_rn(dUdr, d.z, A.fz);
+    A.tx = __fmaf_rn(dUdr, cross1(wi.y, d.z, wi.z, d.y), A.tx);
+    A.ty = __fmaf_rn(dUdr, cross1(wi.z, d.x, wi.x, d.z), A.ty);
+    A.tz = __fmaf_rn(dUdr, cross1(wi.x, d.y, wi.y, d.x), A.tz);
+}
+
+// sin(x) without the library's large-argument code in line: x = k pi + r, two
+// fused steps with pi in two parts, then an odd polynomial fitted to sin on
+// [-pi/2, pi/2] (minimax in the relative error: 6e-9 before rounding,
+// 1.2e-7 with it), and the sign of (-1)^k.  Angles past 1000 rad, where the
+// second part of pi runs out of bits, go to sinf.
+static __device__ __noinline__ float sin_far(float x) { return sinf(x); }
+__device__ __forceinline__ float sin_fit(float x) {
+    if (!(fabsf(x) < 1000.0f)) return sin_far(x);
+    const float t = __fmaf_rn(x, 0.318309886f, 12582912.0f), k = __fsub_rn(t, 12582912.0f);
+    const float r = __fmaf_rn(k, 8.74227766e-8f, __fmaf_rn(k, -3.14159274f, x)), u = __fmul_rn(r, r);
+    float p = __fmaf_rn(2.605780537e-6f, u, -1.980960224e-4f);
+    p = __fmaf_rn(p, u, 8.333066478e-3f);
+    p = __fmaf_rn(p, u, -1.666665971e-1f);
+    const float s = __fmaf_rn(__fmul_rn(r, u), p, r);
+    return __int_as_float(__float_as_int(s) ^ (__float_as_int(t) << 31));
 }
 
 // Bending terms of a harmonic/longitudinal partner (src/compute_cuda.cu:142-180,
 // :265-298): sign by the site side, theta0 chosen by the caller.
 __device__ __forceinline__ void acc_bend(const KParams &P, Acc &A, float rmon, float dpsi, float dfi, float dth,
                                          float th0) {
-    if (rmon > 0.0f) {
-        A.fpsi += P.B_psi * sinf(dpsi - P.psi_0);
-        A.ffi += P.B_fi * sinf(dfi - P.fi_0);
-        A.fth += P.B_theta * sinf(dth - th0);
-    } else {
-        A.fpsi -= P.B_psi * sinf(-dpsi - P.psi_0);
-        A.ffi -= P.B_fi * sinf(-dfi - P.fi_0);
-        A.fth -= P.B_theta * sinf(-dth - th0);
-    }
+    // rmon > 0: + B sin(d - d0); rmon < 0: - B sin(-d - d0)
+    const float sg = rmon > 0.0f ? 1.0f : -1.0f;
+    A.fpsi = __fmaf_rn(__fmul_rn(sg, P.B_psi), sin_fit(__fmaf_rn(sg, dpsi, -P.psi_0)), A.fpsi);
+    A.ffi = __fmaf_rn(__fmul_rn(sg, P.B_fi), sin_fit(__fmaf_rn(sg, dfi, -P.fi_0)), A.ffi);
+    A.fth = __fmaf_rn(__fmul_rn(sg, P.B_theta), sin_fit(__fmaf_rn(sg, dth, -th0)), A.fth);
 }
+
+// U'(r)/r of a Morse bond plus, with BARR, the Gaussian barrier, from r^2.  r
+// and 1/r come from the hardware reciprocal square root (2e-7 relative, below
+// the rounding of the site vectors that d = site_j - site_i carries).  Sites
+// closer than 1e-15 nm count as touching (no force), as r = 0 does.
+__device__ __forceinline__ float dmorse_over_r(float D, float a, float r, float rinv) {
+    const float e = expf(__fmul_rn(-a, r));
+    return __fmul_rn(__fmul_rn(__fmul_rn(2.0f * a, D), __fmul_rn(__fsub_rn(1.0f, e), e)), rinv);
+}
+__device__ __forceinline__ float norm2(float3 d) {
+    return __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
+}
+constexpr float kTouch2 = 1.0e-30f;
 
 // Where a bead's neighbours' frames and flags are read: plane k of local bead
 // j at fr[k * stride + base + j], its flags at fl[base + j].  The per-step
@@ -50,16 +83,70 @@ struct NbrView {
     const int *fl;
     int stride, base;
 };
-__device__ __forceinline__ NbrView global_view(const KParams &P, const DevBuffers &B, int traj) {
-    return {B.frame_in, B.flags, P.nb, B.off[traj]};
+
+// What a bead's force loops start from, requested together at the head of a
+// kernel so that no list's chain count -> entry -> neighbour waits for
+// another's (entries past a count are in bounds and ignored).
+struct ListHead {
+    int nl, nt, nlj;
+    int e_h0, e_l0, e_t0;
+    int jj[4];
+};
+__device__ __forceinline__ ListHead list_head(const KParams &P, const DevBuffers &B, int g) {
+    ListHead H;
+    H.nl = P.maxLong > 0 ? B.lonc[g] : 0;
+    H.nt = P.maxLat > 0 ? B.latc[g] : 0;
+    H.nlj = P.lj_on ? B.ljc[g] : 0;
+    H.e_h0 = B.harm[g * P.maxH];
+    H.e_l0 = P.maxLong > 0 ? B.lon[g] : 0;
+    H.e_t0 = P.maxLat > 0 ? B.lat[g] : 0;
+#pragma unroll
+    for (int u = 0; u < 4; u++) H.jj[u] = (P.lj_on && u < P.maxLJ) ? B.lj[u * P.nb + g] : 0;
+    return H;
 }
 
-// Generalised force on bead g (compute_kernel, src/compute_cuda.cu:32-525):
-// harmonic + bending, Morse longitudinal + bending, Morse lateral with seam
-// coefficient, barriers, LJ inside 6 nm, walls.  out = (fx, fy, fz, ffi,
-// ftheta, fpsi).
-__device__ __forceinline__ void bead_forces(const KParams &P, const DevBuffers &B, const NbrView &V, int g, int traj,
-                                            int flags, const Frame &Fi, float out[6]) {
+// LJ r^-6 repulsion with the hard 6 nm force cutoff (src/compute_cuda.cu:470-495):
+// 6 pref / r^8 along the difference.  Four neighbours a round; while a round is
+// summed, the indices of the next are in flight.
+// Even and odd list entries have sums of their own, added at the end.
+__device__ __forceinline__ float3 lj_force(const KParams &P, const DevBuffers &B, const NbrView &V, int g,
+                                           float4 p0, const ListHead &H) {
+    const int nb = P.nb;
+    const float4 *fr = V.fr + V.base;
+    float3 s[2] = {make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f)};
+    int jj[4] = {H.jj[0], H.jj[1], H.jj[2], H.jj[3]};
+    const int *next = B.lj + g;
+    const float c = 6.0f * P.lj_pref;
+#pragma unroll 1
+    for (int k0 = 0; k0 < H.nlj; k0 += 4) {
+        float4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = k0 + u < H.nlj ? fr[jj[u]] : make_float4(3.0e18f, 0.f, 0.f, 0.f);
+        next += 4 * nb;
+        if (k0 + 4 < H.nlj) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) jj[u] = k0 + 4 + u < P.maxLJ ? next[u * nb] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float dx = __fsub_rn(p0.x, q[u].x), dy = __fsub_rn(p0.y, q[u].y), dz = __fsub_rn(p0.z, q[u].z);
+            const float r2 = norm2(make_float3(dx, dy, dz));
+            if (r2 < 36.0f) {
+                const float i2 = rcp_hw(r2), i4 = __fmul_rn(i2, i2), f = __fmul_rn(c, __fmul_rn(i4, i4));
+                float3 &S = s[u & 1];
+                S.x = __fmaf_rn(f, dx, S.x);
+                S.y = __fmaf_rn(f, dy, S.y);
+                S.z = __fmaf_rn(f, dz, S.z);
+            }
+        }
+    }
+    return make_float3(__fadd_rn(s[0].x, s[1].x), __fadd_rn(s[0].y, s[1].y), __fadd_rn(s[0].z, s[1].z));
+}
+
+// Bonds of bead g (src/compute_cuda.cu:69-467): harmonic + bending, Morse
+// longitudinal + bending, Morse lateral with seam coefficient, barriers.
+__device__ __forceinline__ Acc bond_force(const KParams &P, const DevBuffers &B, const NbrView &V, int g, int flags,
+                                          const Frame &Fi, const ListHead &H) {
     const int nb = P.nb;          // list layout (k-major over all beads)
     const int ps = V.stride;      // plane stride of the neighbour frames
     const int base = V.base;
@@ -67,136 +154,105 @@ __device__ __forceinline__ void bead_forces(const KParams &P, const DevBuffers &
     Acc A = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float3 uzi = f3(Fi.p1);
     const bool off_tub = (flags & kFlagOnTubule) == 0;
-
-    // Every list count and the first entries of every list are requested
-    // before any is used (entries past a count are in bounds and ignored):
-    // the dependent chain index -> neighbour state starts for all lists at once.
+    // harmonic bond inside the dimer (:69-182), then Morse longitudinal
+    // (:187-301): one loop over both, the bonds along the protofilament axis
     const int hc = (flags >> kHarmShift) & 7;
-    const int nl = P.maxLong > 0 ? B.lonc[g] : 0;
-    const int nt = P.maxLat > 0 ? B.latc[g] : 0;
-    const int nlj = P.lj_on ? B.ljc[g] : 0;
-    const int e_h0 = B.harm[g * P.maxH];
-    const int e_l0 = P.maxLong > 0 ? B.lon[g] : 0;
-    const int e_t0 = P.maxLat > 0 ? B.lat[g] : 0;
-    int jj0[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) jj0[u] = (P.lj_on && u < P.maxLJ) ? B.lj[u * nb + g] : 0;
-
-    // harmonic bond inside the dimer (:69-182)
-    for (int k = 0; k < hc; k++) {
-        const int e = k == 0 ? e_h0 : B.harm[g * P.maxH + k];
+#pragma unroll 1
+    for (int k = 0; k < hc + H.nl; k++) {
+        const bool harm = k < hc;
+        int e;
+        if (harm)
+            e = k == 0 ? H.e_h0 : B.harm[g * P.maxH + k];
+        else
+            e = k == hc ? H.e_l0 : B.lon[(k - hc) * nb + g];
         const float rmon = e < 0 ? 2.0f : -2.0f;
         const int pj = base + (e < 0 ? -e : e);
         const float4 rj = fr[pj], uj = fr[ps + pj];
+        const float thj = fr[2 * ps + pj].w;
+        const int fj = V.fl[pj];
         const float3 wi = make_float3(uzi.x * rmon, uzi.y * rmon, uzi.z * rmon);
         const float3 wj = make_float3(-uj.x * rmon, -uj.y * rmon, -uj.z * rmon);
         const float3 d = site_delta(Fi.p0, rj, wi, wj);
-        const float dr = norm3_rn(d);
-        acc_pair(A, P.C, d, wi);
-        if (dr < 1.0f) {
-            const float thj = fr[2 * ps + pj].w;
-            acc_bend(P, A, rmon, uj.w - Fi.p1.w, rj.w - Fi.p0.w, thj - Fi.p2.w,
-                     (flags & kFlagGtp) ? P.th0_gtp : P.th0_gdp);
-        }
-    }
-    // Morse longitudinal (:187-301)
-    for (int k = 0; k < nl; k++) {
-        const int e = k == 0 ? e_l0 : B.lon[k * nb + g];
-        const float rmon = e < 0 ? 2.0f : -2.0f;
-        const int pj = base + (e < 0 ? -e : e);
-        const float4 rj = fr[pj], uj = fr[ps + pj];
-        const float3 wi = make_float3(uzi.x * rmon, uzi.y * rmon, uzi.z * rmon);
-        const float3 wj = make_float3(-uj.x * rmon, -uj.y * rmon, -uj.z * rmon);
-        const float3 d = site_delta(Fi.p0, rj, wi, wj);
-        const float dr = norm3_rn(d);
-        float dUdr = dr == 0.0f ? 0.0f : dmorse(P.D_long, P.A_long, dr) / dr;
-        int fj = -1;
-        if (P.barrier) {
-            fj = V.fl[pj];
-            if (off_tub && (fj & kFlagOnTubule) == 0 && dr != 0.0f) dUdr += dbarr(P.a_bl, P.r_bl, P.w_bl, dr) / dr;
+        const float r2 = norm2(d);
+        float dUdr = P.C;
+        int gl = flags;   // whose nucleotide sets theta0: the bead's own, or (longitudinal) the
+                          // bead's nearer the plus end (:282-283)
+        if (!harm) {
+            const float rinv = rsqrt_hw(r2), r = __fmul_rn(r2, rinv);
+            dUdr = dmorse_over_r(P.D_long, P.A_long, r, rinv);
+            if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
+                dUdr = __fmaf_rn(dbarr(P.a_bl, P.r_bl, P.w_bl, r), rinv, dUdr);
+            if (r2 < kTouch2) dUdr = 0.f;
+            if (!(Fi.p0.z > rj.z)) gl = fj;
         }
         acc_pair(A, dUdr, d, wi);
-        if (dr < 1.0f) {
-            // theta0 of the bead nearer the plus end (:282-283)
-            int glast = flags;
-            if (!(Fi.p0.z > rj.z)) glast = fj >= 0 ? fj : V.fl[pj];
-            const float thj = fr[2 * ps + pj].w;
+        if (r2 < 1.0f)
             acc_bend(P, A, rmon, uj.w - Fi.p1.w, rj.w - Fi.p0.w, thj - Fi.p2.w,
-                     (glast & kFlagGtp) ? P.th0_gtp : P.th0_gdp);
-        }
+                     (gl & kFlagGtp) ? P.th0_gtp : P.th0_gdp);
     }
     // Morse lateral (:303-467)
-    for (int k = 0; k < nt; k++) {
-        const int e = k == 0 ? e_t0 : B.lat[k * nb + g];
+#pragma unroll 1
+    for (int k = 0; k < H.nt; k++) {
+        const int e = k == 0 ? H.e_t0 : B.lat[k * nb + g];
         const bool neg = e <= 0;
         int j = e < 0 ? -e : e;
         if (j == kZeroCode) j = 0;
         const int pj = base + j;
         const float4 rj = fr[pj];
         const float4 sj = neg ? fr[3 * ps + pj] : fr[2 * ps + pj];
+        const int fj = V.fl[pj];
         const float3 wi = neg ? f3(Fi.p2) : f3(Fi.p3);
         const float3 d = site_delta(Fi.p0, rj, wi, f3(sj));
-        const float dr = norm3_rn(d);
-        const int fj = V.fl[pj];
-        const float D = ((flags ^ fj) & kFlagBeta) ? P.D_lat_seam : P.D_lat;
-        float dUdr = dr == 0.0f ? 0.0f : dmorse(D, P.A_lat, dr) / dr;
-        if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0 && dr != 0.0f)
-            dUdr += dbarr(P.a_bt, P.r_bt, P.w_bt, dr) / dr;
+        const float r2 = norm2(d), rinv = rsqrt_hw(r2), r = __fmul_rn(r2, rinv);
+        float dUdr = dmorse_over_r(((flags ^ fj) & kFlagBeta) ? P.D_lat_seam : P.D_lat, P.A_lat, r, rinv);
+        if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
+            dUdr = __fmaf_rn(dbarr(P.a_bt, P.r_bt, P.w_bt, r), rinv, dUdr);
+        if (r2 < kTouch2) dUdr = 0.f;
         acc_pair(A, dUdr, d, wi);
     }
-    // LJ r^-6 repulsion with the hard 6 nm force cutoff (:470-495)
-    if (P.lj_on) {
-        // four neighbours per round: their indices, then their positions, are
-        // all in flight before the first is used
-        for (int k0 = 0; k0 < nlj; k0 += 4) {
-            int jj[4];
-            float4 rj[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                jj[u] = k0 + u < nlj ? (k0 == 0 ? jj0[u] : B.lj[(k0 + u) * nb + g]) : -1;
-#pragma unroll
-            for (int u = 0; u < 4; u++) rj[u] = jj[u] >= 0 ? fr[base + jj[u]] : Fi.p0;
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (jj[u] < 0) continue;
-                const float dx = Fi.p0.x - rj[u].x, dy = Fi.p0.y - rj[u].y, dz = Fi.p0.z - rj[u].z;
-                const float dr = sqrtf(dx * dx + dy * dy + dz * dz);
-                if (dr < 6.0f) {
-                    const float dr2 = dr * dr, dr4 = dr2 * dr2;
-                    const float s = P.lj_pref * (6.0f / (dr4 * dr4));
-                    A.fx += s * dx;
-                    A.fy += s * dy;
-                    A.fz += s * dz;
-                }
-            }
-        }
-    }
-    // cylindrical walls (:497-517)
+    return A;
+}
+
+// The generalised force from its parts: bonds + LJ, the cylindrical walls
+// (src/compute_cuda.cu:497-517), and the bending terms plus the torque
+// projected on the Euler axes (psi about z, theta about Rz(psi) y, fi about
+// R x).  out = (fx, fy, fz, ffi, ftheta, fpsi).
+__device__ __forceinline__ void force_out(const KParams &P, const Acc &A, float3 L, const float *zs, float4 p0,
+                                          float psi, float theta, float out[6]) {
+    float fx = __fadd_rn(A.fx, L.x), fy = __fadd_rn(A.fy, L.y), fz = __fadd_rn(A.fz, L.z);
     if (P.is_wall) {
-        const float z = Fi.p0.z, top = B.zs[traj] + P.lb;
+        const float z = p0.z, top = __fadd_rn(*zs, P.lb);
         if (z < P.lb)
-            A.fz += P.rep_eps * fabsf(z - P.lb);
+            fz = __fmaf_rn(P.rep_eps, fabsf(z - P.lb), fz);
         else if (z > top)
-            A.fz += -P.rep_eps * fabsf(z - top);
-        const float rad2 = Fi.p0.x * Fi.p0.x + Fi.p0.y * Fi.p0.y;
+            fz = __fmaf_rn(-P.rep_eps, fabsf(z - top), fz);
+        const float rad2 = __fmaf_rn(p0.x, p0.x, __fmul_rn(p0.y, p0.y));
         if (rad2 > P.rep_r * P.rep_r) {
-            const float rad = sqrtf(rad2);
-            const float coeff = -P.rep_eps * (rad - P.rep_r);
-            A.fx += Fi.p0.x / rad * coeff;
-            A.fy += Fi.p0.y / rad * coeff;
+            const float rad = __fsqrt_rn(rad2);
+            const float coeff = __fdiv_rn(__fmul_rn(-P.rep_eps, __fsub_rn(rad, P.rep_r)), rad);
+            fx = __fmaf_rn(p0.x, coeff, fx);
+            fy = __fmaf_rn(p0.y, coeff, fy);
         }
     }
-    // generalised forces = bending terms + torque projected on the Euler axes:
-    // psi about z, theta about Rz(psi) y, fi about R x.
     float sp, cp, st, ct;
-    sincosf(Fi.p1.w, &sp, &cp);
-    sincosf(Fi.p2.w, &st, &ct);
-    out[0] = A.fx;
-    out[1] = A.fy;
-    out[2] = A.fz;
-    out[3] = A.ffi + (cp * ct * A.tx + sp * ct * A.ty - st * A.tz);
-    out[4] = A.fth + (-sp * A.tx + cp * A.ty);
-    out[5] = A.fpsi + A.tz;
+    sincosf(psi, &sp, &cp);
+    sincosf(theta, &st, &ct);
+    out[0] = fx;
+    out[1] = fy;
+    out[2] = fz;
+    const float tf = __fmaf_rn(__fmul_rn(cp, ct), A.tx, __fmaf_rn(__fmul_rn(sp, ct), A.ty, -__fmul_rn(st, A.tz)));
+    out[3] = __fadd_rn(A.ffi, tf);
+    out[4] = __fadd_rn(A.fth, __fmaf_rn(cp, A.ty, -__fmul_rn(sp, A.tx)));
+    out[5] = __fadd_rn(A.fpsi, A.tz);
+}
+
+// Generalised force on bead g (compute_kernel, src/compute_cuda.cu:32-525).
+__device__ __forceinline__ void bead_forces(const KParams &P, const DevBuffers &B, const NbrView &V, int g,
+                                            const float *zs, int flags, const Frame &Fi, const ListHead &H,
+                                            float out[6]) {
+    const float3 L = lj_force(P, B, V, g, Fi.p0, H);
+    const Acc A = bond_force(P, B, V, g, flags, Fi, H);
+    force_out(P, A, L, zs, Fi.p0, Fi.p1.w, Fi.p2.w, out);
 }
 
 __device__ __forceinline__ Frame load_frame(const float4 *planes, int nb, int g) {
@@ -225,26 +281,34 @@ __device__ __forceinline__ Frame em_update(const KParams &P, const Frame &Fi, co
     return make_frame(P, x, y, z, fi, th, psi);
 }
 
+// One MD step of one bead per thread.  Bound by the latency of the chain list
+// entry -> neighbour frame -> force, so everything that does not depend on
+// another bead (list heads, noise states) is requested first and the noise is
+// drawn while the neighbours are on their way.
 template <bool KEEP_FORCES>
 __global__ void __launch_bounds__(256) k_step_plain(KParams P, DevBuffers B) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P.nb) return;
     const int nb = P.nb;
     const int flags = B.flags[g];
+    const NbrView V = {B.frame_in, B.flags, nb, B.base[g]};
     Frame Fi = load_frame(B.frame_in, nb, g);
     float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (!(flags & kFlagExtra)) {
         const bool moving = !(flags & kFlagFixed);
         if (moving || KEEP_FORCES) {
-            const int traj = B.traj[g];
-            bead_forces(P, B, global_view(P, B, traj), g, traj, flags, Fi, f);
-        }
-        if (moving) {
-            uint4 s1 = B.seeds[g], s2 = B.seeds[nb + g];
-            const float4 gx = gauss4(s1), ga = gauss4(s2);
-            B.seeds[g] = s1;
-            B.seeds[nb + g] = s2;
-            Fi = em_update(P, Fi, f, gx, ga);
+            const ListHead H = list_head(P, B, g);
+            float4 gx, ga;
+            if (moving) {
+                uint4 s1 = B.seeds[g], s2 = B.seeds[nb + g];
+                gx = gauss4(s1);
+                ga = gauss4(s2);
+                B.seeds[g] = s1;
+                B.seeds[nb + g] = s2;
+            }
+            const float *zs = P.is_wall ? B.zs + B.traj[g] : B.zs;
+            bead_forces(P, B, V, g, zs, flags, Fi, H, f);
+            if (moving) Fi = em_update(P, Fi, f, gx, ga);
         }
     }
     store_frame(B.frame_out, nb, g, Fi);
@@ -331,7 +395,7 @@ __global__ void __launch_bounds__(kPeriodThreads, 2) k_step_period(KParams P, De
                     Fi.p1 = sf[n + j];
                     Fi.p2 = sf[2 * n + j];
                     Fi.p3 = sf[3 * n + j];
-                    bead_forces(P, B, V, base + j, traj, fl, Fi, f[q]);
+                    bead_forces(P, B, V, base + j, B.zs + traj, fl, Fi, list_head(P, B, base + j), f[q]);
                 }
             }
         }
@@ -385,9 +449,10 @@ __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
     const int flags = B.flags[g];
     float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (!(flags & kFlagExtra)) {
+        const NbrView V = {B.frame_in, B.flags, nb, B.base[g]};
+        const ListHead H = list_head(P, B, g);
         const Frame Fi = load_frame(B.frame_in, nb, g);
-        const int traj = B.traj[g];
-        bead_forces(P, B, global_view(P, B, traj), g, traj, flags, Fi, f);
+        bead_forces(P, B, V, g, P.is_wall ? B.zs + B.traj[g] : B.zs, flags, Fi, H, f);
     }
     B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
     B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);

@@ -445,9 +445,12 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     e->kp = make_kparams(*p, nb, nt, maxH, maxLong, maxLat, maxLJ);
 
     // host-side per-bead tables
-    std::vector<int> traj(nb), flags(nb), harm((size_t)maxH * nb);
+    std::vector<int> traj(nb), tbead(nb), flags(nb), harm((size_t)maxH * nb);
     for (int tr = 0; tr < nt; tr++)
-        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g++) traj[g] = tr;
+        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g++) {
+            traj[g] = tr;
+            tbead[g] = t->offsets[tr];
+        }
     for (int g = 0; g < nb; g++) {
         const int hc = t->harmonicCount[g];
         if (hc < 0 || hc > maxH) {
@@ -511,6 +514,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     }
     ALLOC(e->off, nt + 1);
     ALLOC(e->traj, nb);
+    ALLOC(e->base, nb);
     ALLOC(e->flags, nb);
     ALLOC(e->harm, (size_t)maxH * nb);
     ALLOC(e->zs, nt);
@@ -572,6 +576,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     std::vector<float> zs(nt, 0.f);
     if (t->zs) zs.assign(t->zs, t->zs + nt);
     if ((rc = upload(e->off, t->offsets, sizeof(int) * (nt + 1), s)) || (rc = upload(e->traj, traj.data(), sizeof(int) * nb, s)) ||
+        (rc = upload(e->base, tbead.data(), sizeof(int) * nb, s)) ||
         (rc = upload(e->flags, flags.data(), sizeof(int) * nb, s)) ||
         (rc = upload(e->harm, harm.data(), sizeof(int) * harm.size(), s)) ||
         (rc = upload(e->zs, zs.data(), sizeof(float) * nt, s)) ||
@@ -693,7 +698,7 @@ int mtg_destroy(mtg_engine *e) {
     mtg_internal_close_output(e);
     destroy_graphs(e);
     mtg_internal_ff_free(e);
-    void *ptrs[] = {e->off, e->traj, e->flags, e->harm, e->zs, e->frame[0], e->frame[1], e->force, e->seeds,
+    void *ptrs[] = {e->off, e->traj, e->base, e->flags, e->harm, e->zs, e->frame[0], e->frame[1], e->force, e->seeds,
                     e->ljc, e->lj, e->lonc, e->lon, e->latc, e->lat, e->err, e->work, e->work_first,
                     e->en_partials, e->en_traj, e->en_bead, e->tea_r, e->tea_ci, e->tea_eps, e->tea_beta,
                     e->tea_eps_t, e->stage, e->stage_u8, e->stage_i, e->cell_tbase, e->cell_tmask,

@@ -23,7 +23,7 @@ struct mtg_engine {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     std::vector<int> h_off;
     // device
-    int *off = nullptr, *traj = nullptr, *flags = nullptr, *harm = nullptr;
+    int *off = nullptr, *traj = nullptr, *base = nullptr, *flags = nullptr, *harm = nullptr;
     float *zs = nullptr;
     float4 *frame[2] = {nullptr, nullptr};
     float4 *force = nullptr;
@@ -124,6 +124,7 @@ struct mtg_engine {
         DevBuffers b{};
         b.off = off;
         b.traj = traj;
+        b.base = base;
         b.flags = flags;
         b.harm = harm;
         b.zs = zs;

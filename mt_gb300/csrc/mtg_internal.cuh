@@ -70,6 +70,7 @@ struct KParams {
 struct DevBuffers {
     const int *off;        // [nt+1]
     const int *traj;       // [nb]
+    const int *base;       // [nb] first bead of the bead's trajectory
     const int *flags;      // [nb]
     const int *harm;       // [nb*maxH]
     const float *zs;       // [nt]
@@ -173,17 +174,14 @@ __device__ __forceinline__ void store_frame(float4 *planes, int nb, int g, const
 }
 
 // ------------------------------------------------------------ potentials
-// Morse derivative / energy and Gaussian barrier (src/compute_cuda.cu:16-30).
-__device__ __forceinline__ float dmorse(float D, float a, float x) {
-    const float e = expf(-a * x);
-    return 2.0f * a * D * (1.0f - e) * e;
-}
+// Morse energy and Gaussian barrier (src/compute_cuda.cu:16-30).
 __device__ __forceinline__ float morse_en(float D, float a, float x) {
     const float e = expf(-a * x);
     return D * (1.0f - e) * (1.0f - e) - D;
 }
 __device__ __forceinline__ float dbarr(float a, float r, float w, float x) {
-    return -a * expf(-(x - r) * (x - r) / (2.0f * w * w)) * (x - r) / (w * w);
+    const float d = __fsub_rn(x, r), w2 = __fmul_rn(w, w);
+    return __fdiv_rn(__fmul_rn(__fmul_rn(-a, expf(__fdiv_rn(-__fmul_rn(d, d), __fmul_rn(2.0f, w2)))), d), w2);
 }
 __device__ __forceinline__ float barr(float a, float r, float w, float x) {
     return a * expf(-(x - r) * (x - r) / (2.0f * w * w));
@@ -303,6 +301,13 @@ __device__ __forceinline__ void list_append(const KParams &P, const DevBuffers &
 __device__ __forceinline__ float rsqrt_hw(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// 1/x as the single hardware approximation instruction (1 ulp).
+__device__ __forceinline__ float rcp_hw(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
