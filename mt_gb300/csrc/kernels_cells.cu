@@ -14,6 +14,8 @@
 //      list is in ascending j (orientation 0 before 1 for the lateral list),
 //      exactly the order of the reference's j loops
 //      (src/compute_cuda.cu:564-661, :927-936).
+#include <cmath>
+
 #include "mtg_internal.cuh"
 
 namespace mtg {
@@ -392,6 +394,313 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
     if (overflow) atomicOr(B.err, kErrOverflow);
 }
 
+// ---------------------------------------------- the whole rebuild in one CTA
+// Trajectories of up to kSmemBeads beads, LJ on and either no assembly lists or
+// every assembly candidate inside the LJ cutoff: one launch, one CTA per
+// (trajectory, kListThreads beads).  Each CTA bins its whole trajectory into
+// shared memory, so a candidate costs a shared-memory load instead of a
+// dependent L2 one, and the beads of a chunk then walk their cells.
+//   * The bucket of cell (cx, cy, cz) is (row hash of (cy, cz) + cx) mod M, so
+//     the three cells of a row are neighbouring buckets: 9 contiguous ranges a
+//     bead instead of 27 buckets, and no search for repeated buckets.  Rows that
+//     share buckets only add candidates; a hit counts in the row that is its
+//     own, so it counts once.  M >= 2 n keeps such extra candidates few (about one
+//     a row).
+//   * The bucket table holds 16-bit counts, then starts, then (after the fill)
+//     ends.
+//   * Distances are compared squared, against the largest square whose root is
+//     below the cutoff (sq_below), which is the same decision.
+//   * A hit is a 16-bit key: index * 8 + which site tests can succeed (the
+//     partner's centre within 4.51 nm of the bead's own site: sites are at most
+//     2 nm from a centre and bonds at most 2.5 nm long).  Keys are sorted in
+//     registers (Batcher's odd-even merge network, up to 16), so the lists come out in
+//     ascending j; only the site planes that a test needs are then gathered.
+// 256 x 1520 beads: 203 us for the general path's six launches (the 27-bucket
+// walk ran 7600 instructions a warp, half of them on repeated buckets), 77 us here;
+// 1024 uneven trajectories of up to 3560 beads 775 -> 308 us, one of 156 beads 45 (tiles) -> 18 us.
+constexpr int kSmemKeys = 32;      // keys a bead can keep; more take the slow path below
+constexpr int kSmemBeads = 8192;   // 13 bits of a key
+
+__host__ __device__ inline int smem_buckets(int n) {
+    int m = 64;
+    while (m < 2 * n) m <<= 1;
+    return m;
+}
+size_t smem_list_bytes(int nmax) {
+    return sizeof(float4) * (size_t)nmax + sizeof(uint16_t) * ((size_t)smem_buckets(nmax) + kSmemKeys * kListThreads);
+}
+
+__device__ __forceinline__ float dist2_rn(float4 a, float4 b) {
+    const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+
+// Batcher's odd-even merge sort of N keys in registers, ascending.
+template <int N>
+__device__ __forceinline__ void sort_network(unsigned (&k)[N]) {
+#pragma unroll
+    for (int p = 1; p < N; p *= 2)
+#pragma unroll
+        for (int q = p; q >= 1; q /= 2)
+#pragma unroll
+            for (int j = q % p; j + q < N; j += 2 * q)
+#pragma unroll
+                for (int i = 0; i < q; i++)
+                    if (i + j + q < N && (i + j) / (2 * p) == (i + j + q) / (2 * p)) {
+                        const unsigned a = k[i + j], b = k[i + j + q];
+                        k[i + j] = min(a, b);
+                        k[i + j + q] = max(a, b);
+                    }
+}
+template <int N>
+__device__ __forceinline__ void sort_keys(uint16_t (*s_key)[kListThreads], int n) {
+    unsigned k[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) k[i] = i < n ? s_key[i][threadIdx.x] : 0xffffu;
+    sort_network<N>(k);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < n) s_key[i][threadIdx.x] = (uint16_t)k[i];
+}
+
+// A trajectory's beads in bucket order, in shared memory.
+struct SmemCells {
+    const float4 *pos;    // w = index in the trajectory
+    const uint16_t *end;  // end of each bucket's range (a range starts where the one before ends)
+    int n, m;
+    float inv;
+};
+__device__ __forceinline__ uint32_t row_hash(int cy, int cz) {
+    return ((uint32_t)cy * 19349663u) ^ ((uint32_t)cz * 83492791u);
+}
+// Calls hit(slot) for every bead of the trajectory in the cells around p that
+// is closer than the root of t2, in no particular order; once for every row whose
+// buckets hold it, so a bead whose own row shares them can come twice.
+// Four candidates an iteration (two left the loop overhead as large as the tests).
+template <class F>
+__device__ __forceinline__ void smem_candidates(const SmemCells &C, float4 p, float t2, F &&hit) {
+    const int cx = cell_coord(p.x, C.inv), cy = cell_coord(p.y, C.inv), cz = cell_coord(p.z, C.inv);
+#pragma unroll 1
+    for (int dz = -1; dz <= 1; dz++)
+#pragma unroll 1
+        for (int dy = -1; dy <= 1; dy++) {
+            const int b0 = (int)((row_hash(cy + dy, cz + dz) + (uint32_t)(cx - 1)) & (uint32_t)(C.m - 1)), b2 = b0 + 2;
+            int s = b0 > 0 ? C.end[b0 - 1] : 0, e = C.end[min(b2, C.m - 1)];
+            int e2 = b2 >= C.m ? C.end[b2 - C.m] : 0;   // a range that wraps round the table has a second part
+            while (true) {
+#pragma unroll 1
+                for (; s < e; s += 4) {
+                    float r2[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) r2[u] = dist2_rn(p, C.pos[min(s + u, e - 1)]);
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (r2[u] < t2 && s + u < e) hit(s + u);
+                }
+                if (e2 == 0) break;
+                s = 0;
+                e = e2;
+                e2 = 0;
+            }
+        }
+}
+
+// The lists of one bead as its keys come in ascending order.
+struct ListWriter {
+    int nlj, nlo, nla;
+    bool overflow;
+};
+__device__ __forceinline__ void lj_append(const KParams &P, const DevBuffers &B, int g, int jl, ListWriter &W) {
+    if (W.nlj < P.maxLJ)
+        B.lj[W.nlj * P.nb + g] = jl;
+    else
+        W.overflow = true;
+    W.nlj++;
+}
+// The site tests of pairs_kernel (src/compute_cuda.cu:527-674) for one key:
+// the planes they need are requested together, then decided as list_bits does.
+struct PairPlanes {
+    float4 p, u, l1, l2;
+    int flags;
+};
+__device__ __forceinline__ PairPlanes pair_load(const DevBuffers &B, int nb, int jg, unsigned bits) {
+    const float4 *fr = B.frame_in;
+    PairPlanes J;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    J.p = bits ? fr[jg] : z;
+    J.u = (bits & 1u) ? fr[nb + jg] : z;
+    J.flags = (bits & 1u) ? B.flags[jg] : 0;
+    J.l2 = (bits & 2u) ? fr[3 * nb + jg] : z;
+    J.l1 = (bits & 4u) ? fr[2 * nb + jg] : z;
+    return J;
+}
+__device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &B, int g, const ListSite &I, int jl,
+                                            unsigned bits, const PairPlanes &J, float t_site, ListWriter &W) {
+    unsigned got = 0;
+    if ((bits & 1u) && ((I.flags ^ J.flags) & kFlagBeta)) {
+        const float3 wj = make_float3(-J.u.x * I.rmon, -J.u.y * I.rmon, -J.u.z * I.rmon);
+        if (norm2_rn(site_delta(I.p, J.p, I.wi, wj)) < t_site) got |= 2u;
+    }
+    if ((bits & 2u) && norm2_rn(site_delta(I.p, J.p, f3(I.l1), f3(J.l2))) < t_site) got |= 4u;
+    if ((bits & 4u) && norm2_rn(site_delta(I.p, J.p, f3(I.l2), f3(J.l1))) < t_site) got |= 8u;
+    if (got == 0) return;
+    list_append(P, B, g, I, got, jl, W.nlj, W.nlo, W.nla, W.overflow);
+}
+
+__global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int2 *work, int nmax,
+                                                                  float inv, float t_lj, float t_pair, float t_site) {
+    extern __shared__ float4 s_dyn[];
+    const int2 w = work[blockIdx.x];
+    const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
+    const int m = smem_buckets(n), t = threadIdx.x;
+    const float4 *fr = B.frame_in;
+    float4 *s_pos = s_dyn;
+    unsigned *s_tab = reinterpret_cast<unsigned *>(s_dyn + nmax);             // two 16-bit buckets a word
+    uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab);
+    uint16_t (*s_key)[kListThreads] = reinterpret_cast<uint16_t (*)[kListThreads]>(s_end + smem_buckets(nmax));
+    __shared__ unsigned s_warp[kListThreads / 32];
+
+    // the beads in bucket order
+    for (int k = t; k < m / 2; k += kListThreads) s_tab[k] = 0;
+    __syncthreads();
+    auto bucket = [&](float4 p) {
+        return (int)((row_hash(cell_coord(p.y, inv), cell_coord(p.z, inv)) + (uint32_t)cell_coord(p.x, inv)) &
+                     (uint32_t)(m - 1));
+    };
+    for (int j = t; j < n; j += kListThreads) {
+        const int b = bucket(fr[base + j]);
+        atomicAdd(&s_tab[b >> 1], 1u << (16 * (b & 1)));
+    }
+    __syncthreads();
+    {   // exclusive scan of the counts, whole words a thread
+        const int per = (m / 2 + kListThreads - 1) / kListThreads, lo = min(m / 2, t * per), hi = min(m / 2, lo + per);
+        unsigned sum = 0;
+        for (int k = lo; k < hi; k++) sum += (s_tab[k] & 0xffffu) + (s_tab[k] >> 16);
+        const int lane = t & 31, wid = t >> 5;
+        unsigned v = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) s_warp[wid] = v;
+        __syncthreads();
+        unsigned run = v - sum;
+        for (int k = 0; k < wid; k++) run += s_warp[k];
+        for (int k = lo; k < hi; k++) {
+            const unsigned c = s_tab[k], c0 = c & 0xffffu;
+            s_tab[k] = run | ((run + c0) << 16);
+            run += c0 + (c >> 16);
+        }
+    }
+    __syncthreads();
+    for (int j = t; j < n; j += kListThreads) {
+        float4 p = fr[base + j];
+        const int b = bucket(p), sh = 16 * (b & 1);
+        const unsigned slot = (atomicAdd(&s_tab[b >> 1], 1u << sh) >> sh) & 0xffffu;
+        p.w = __int_as_float(j);
+        s_pos[slot] = p;
+    }
+    __syncthreads();
+
+    const int il = w.y - base + t;
+    if (il >= n) return;   // no barrier after this point
+    const int g = base + il;
+    const ListSite I = list_site(P, fr[g], fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], B.flags[g], il,
+                                 B.harm[g * P.maxH]);
+    ListWriter W = {0, 0, 0, false};
+    if (I.do_lj) {
+        const SmemCells C = {s_pos, s_end, n, m, inv};
+        // where the bead's own sites are: a bond needs the partner's centre within
+        // 2.5 + 2 nm of one (0.01 nm over the rounding)
+        const float kSite2 = 4.51f * 4.51f;
+        const float4 a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
+        const float4 a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
+        const float4 a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);
+        auto make_key = [&](int slot) {
+            const float4 q = s_pos[slot];
+            const float r2 = dist2_rn(I.p, q);
+            const int jl = __float_as_int(q.w);
+            unsigned bits = 0;
+            if (I.do_pairs && r2 < t_pair && jl != I.hpart)
+                bits = (dist2_rn(a0, q) < kSite2 ? 1u : 0u) | (dist2_rn(a1, q) < kSite2 ? 2u : 0u) |
+                       (dist2_rn(a2, q) < kSite2 ? 4u : 0u);
+            return ((unsigned)jl << 3) | bits;
+        };
+        int nk = 0;
+        smem_candidates(C, I.p, t_lj, [&](int slot) {
+            if (nk < kSmemKeys) s_key[nk][t] = (uint16_t)slot;
+            nk++;
+        });
+        if (nk <= kSmemKeys) {
+            for (int k = 0; k < nk; k++) s_key[k][t] = (uint16_t)make_key(s_key[k][t]);
+            if (nk <= 8) {
+                sort_keys<8>(s_key, nk);
+            } else if (nk <= 16) {
+                sort_keys<16>(s_key, nk);
+            } else {
+                for (int i = 1; i < nk; i++) {
+                    const uint16_t v = s_key[i][t];
+                    int j = i - 1;
+                    while (j >= 0 && s_key[j][t] > v) {
+                        s_key[j + 1][t] = s_key[j][t];
+                        j--;
+                    }
+                    s_key[j + 1][t] = v;
+                }
+            }
+            // the LJ list; the keys with a site test close up in place
+            int np = 0;
+            unsigned before = 0x10000u;   // no key
+            for (int k = 0; k < nk; k++) {
+                const unsigned key = s_key[k][t];
+                if (key == before || (key >> 3) == (unsigned)il) continue;   // found from two rows; the bead itself
+                before = key;
+                lj_append(P, B, g, (int)(key >> 3), W);
+                if (key & 7u) s_key[np++][t] = (uint16_t)key;
+            }
+            for (int k = 0; k < np; k += 2) {   // two partners in flight
+                const unsigned k0 = s_key[k][t], k1 = k + 1 < np ? s_key[k + 1][t] : 0u;
+                const PairPlanes J0 = pair_load(B, nb, base + (int)(k0 >> 3), k0 & 7u);
+                const PairPlanes J1 = pair_load(B, nb, base + (int)(k1 >> 3), k1 & 7u);
+                pair_decide(P, B, g, I, (int)(k0 >> 3), k0 & 7u, J0, t_site, W);
+                pair_decide(P, B, g, I, (int)(k1 >> 3), k1 & 7u, J1, t_site, W);
+            }
+        } else {
+            // more neighbours than hard spheres of this size allow: the next larger
+            // key is looked up again and again
+            int last = -1;
+            while (true) {
+                unsigned best = 0x7fffffffu;
+                smem_candidates(C, I.p, t_lj, [&](int slot) {
+                    const unsigned key = make_key(slot);
+                    if ((int)(key >> 3) != il && (int)key > last) best = min(best, key);
+                });
+                if (best == 0x7fffffffu) break;
+                last = (int)best;
+                lj_append(P, B, g, (int)(best >> 3), W);
+                const PairPlanes J = pair_load(B, nb, base + (int)(best >> 3), best & 7u);
+                pair_decide(P, B, g, I, (int)(best >> 3), best & 7u, J, t_site, W);
+            }
+        }
+    }
+    B.ljc[g] = min(W.nlj, P.maxLJ);
+    if (P.is_assembly) {
+        B.lonc[g] = min(W.nlo, P.maxLong);
+        B.latc[g] = min(W.nla, P.maxLat);
+    }
+    if (W.overflow) atomicOr(B.err, kErrOverflow);
+}
+
+// The smallest float whose rounded square root is not below c, so that
+// r2 < sq_below(c) decides as sqrt(r2) < c does.
+float sq_below(float c) {
+    if (!(c > 0.0f)) return 0.0f;
+    float t = c * c;
+    while (std::sqrt(t) >= c && t > 0.0f) t = std::nextafter(t, 0.0f);
+    while (std::sqrt(t) < c) t = std::nextafter(t, INFINITY);
+    return t;
+}
+
 inline int nblk(int n, int t) { return (n + t - 1) / t; }
 
 }  // namespace
@@ -410,6 +719,22 @@ float bin_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, flo
         k_cell_sort<<<dim3(P.nt, (C.max_buckets + 127) / 128), 128, 0, s>>>(B.off, C.tbase, C.tmask, C.start, C.cnt,
                                                                             C.cell_bead, C.cell_pos);
     return inv;
+}
+
+bool smem_lists_apply(const KParams &P, int nmax) {
+    return P.lj_on && P.ljcut > 0.0f && (!P.is_assembly || P.ljcut >= kPairReach) && nmax <= kSmemBeads;
+}
+int smem_lists_prepare() {   // the limit of the largest trajectory, whatever this engine's, as engines share the kernel
+    return cudaFuncSetAttribute(k_cell_lists_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem_list_bytes(kSmemBeads)) == cudaSuccess
+               ? 0
+               : -1;
+}
+void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
+                         cudaStream_t s) {
+    const float inv = 1.0f / (P.ljcut * 1.001f + 1e-3f);   // the cells of bin_beads
+    k_cell_lists_smem<<<nwork, kListThreads, smem_list_bytes(nmax), s>>>(P, B, work, nmax, inv, sq_below(P.ljcut),
+                                                                         sq_below(kPairReach), sq_below(2.5f));
 }
 
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,

@@ -226,7 +226,9 @@ long long count_kernel_nodes(cudaGraph_t g) {
 
 // The list rebuild with the engine's method.
 void launch_lists(mtg_engine *e) {
-    if (e->use_cells)
+    if (e->use_cells && smem_lists_apply(e->kp, e->max_traj_beads))
+        launch_rebuild_smem(e->kp, e->bufs(), e->list_work, e->list_nwork, e->max_traj_beads, e->stream);
+    else if (e->use_cells)
         launch_rebuild_cells(e->kp, e->bufs(), e->cells(), e->work, e->nwork, e->stream);
     else
         launch_rebuild(e->kp, e->bufs(), e->work, e->nwork, e->stream);
@@ -239,7 +241,9 @@ void choose_list_method(mtg_engine *e) {
     else if (e->list_method == 2)
         e->use_cells = true;
     else
-        e->use_cells = e->max_traj_beads >= 512;
+        // the one-launch cell rebuild beats the tiles at every size it takes
+        // (156 beads: 45 against 18 us); the six-launch one from 512 beads on
+        e->use_cells = e->max_traj_beads >= 512 || smem_lists_apply(e->kp, e->max_traj_beads);
 }
 
 // Event slot for one timed launch (created outside any stream capture).
@@ -485,6 +489,10 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     }
     work_first[nt] = (int)work.size();
     e->nwork = (int)work.size();
+    std::vector<int2> list_work;
+    for (int tr = 0; tr < nt; tr++)
+        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kListThreads) list_work.push_back(make_int2(tr, g));
+    e->list_nwork = (int)list_work.size();
     std::vector<int2> tea_work;
     for (int tr = 0; tr < nt; tr++)
         for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) tea_work.push_back(make_int2(tr, g));
@@ -531,6 +539,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     ALLOC(e->err, 1);
     ALLOC(e->work, e->nwork);
     ALLOC(e->work_first, nt + 1);
+    ALLOC(e->list_work, e->list_nwork);
     ALLOC(e->en_partials, 7 * (size_t)e->nwork);
     ALLOC(e->en_traj, 7 * (size_t)nt);
     ALLOC(e->stage, 7 * (size_t)nb);
@@ -572,6 +581,10 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         mtg_destroy(e);
         return rc;
     }
+    if (smem_lists_prepare() != 0) {
+        mtg_destroy(e);
+        return fail(MTG_E_CUDA, "the list kernel could not reserve its shared memory");
+    }
     choose_list_method(e);
     std::vector<float> zs(nt, 0.f);
     if (t->zs) zs.assign(t->zs, t->zs + nt);
@@ -581,6 +594,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         (rc = upload(e->harm, harm.data(), sizeof(int) * harm.size(), s)) ||
         (rc = upload(e->zs, zs.data(), sizeof(float) * nt, s)) ||
         (rc = upload(e->work, work.data(), sizeof(int2) * work.size(), s)) ||
+        (rc = upload(e->list_work, list_work.data(), sizeof(int2) * list_work.size(), s)) ||
         (rc = upload(e->work_first, work_first.data(), sizeof(int) * (nt + 1), s))) {
         mtg_destroy(e);
         return rc;
@@ -699,7 +713,7 @@ int mtg_destroy(mtg_engine *e) {
     destroy_graphs(e);
     mtg_internal_ff_free(e);
     void *ptrs[] = {e->off, e->traj, e->base, e->flags, e->harm, e->zs, e->frame[0], e->frame[1], e->force, e->seeds,
-                    e->ljc, e->lj, e->lonc, e->lon, e->latc, e->lat, e->err, e->work, e->work_first,
+                    e->ljc, e->lj, e->lonc, e->lon, e->latc, e->lat, e->err, e->work, e->work_first, e->list_work,
                     e->en_partials, e->en_traj, e->en_bead, e->tea_r, e->tea_ci, e->tea_eps, e->tea_beta,
                     e->tea_eps_t, e->stage, e->stage_u8, e->stage_i, e->cell_tbase, e->cell_tmask,
                     e->cell_key, e->cell_bead, e->cell_pos, e->cell_cnt, e->cell_start, e->cell_cursor, e->tea_work,

@@ -200,9 +200,10 @@ __device__ __forceinline__ float3 site_delta(float4 ri, float4 rj, float3 wi, fl
                        __fsub_rn(__fadd_rn(__fsub_rn(rj.y, ri.y), wj.y), wi.y),
                        __fsub_rn(__fadd_rn(__fsub_rn(rj.z, ri.z), wj.z), wi.z));
 }
-__device__ __forceinline__ float norm3_rn(float3 d) {
-    return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(d.x, d.x), __fmul_rn(d.y, d.y)), __fmul_rn(d.z, d.z)));
+__device__ __forceinline__ float norm2_rn(float3 d) {
+    return __fadd_rn(__fadd_rn(__fmul_rn(d.x, d.x), __fmul_rn(d.y, d.y)), __fmul_rn(d.z, d.z));
 }
+__device__ __forceinline__ float norm3_rn(float3 d) { return __fsqrt_rn(norm2_rn(d)); }
 
 // --------------------------------------------------------- list decisions
 // Site offsets are at most |p1| ~ 2 nm from the centre, so a site distance
@@ -352,6 +353,13 @@ void launch_forces_to_coords(const KParams &P, const float4 *force, float *coord
 void launch_rebuild(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,
                           cudaStream_t s);
+// The cell-list rebuild in one launch, each CTA binning its trajectory in
+// shared memory; work = chunks of kListThreads beads, nmax the largest trajectory.
+constexpr int kListThreads = 512;
+bool smem_lists_apply(const KParams &P, int nmax);
+int smem_lists_prepare();                         // opts the kernel into its shared memory (outside captures)
+void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
+                         cudaStream_t s);
 // Bins the current positions into the per-trajectory spatial hash with cells
 // just larger than `reach`; returns 1/edge for the consumers' cell lookups.
 // `ordered` sorts every bucket by bead index (for sums that must not depend
