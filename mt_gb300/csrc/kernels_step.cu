@@ -143,19 +143,16 @@ __device__ __forceinline__ float3 lj_force(const KParams &P, const DevBuffers &B
     return make_float3(__fadd_rn(s[0].x, s[1].x), __fadd_rn(s[0].y, s[1].y), __fadd_rn(s[0].z, s[1].z));
 }
 
-// Bonds of bead g (src/compute_cuda.cu:69-467): harmonic + bending, Morse
-// longitudinal + bending, Morse lateral with seam coefficient, barriers.
-__device__ __forceinline__ Acc bond_force(const KParams &P, const DevBuffers &B, const NbrView &V, int g, int flags,
-                                          const Frame &Fi, const ListHead &H) {
+// Bonds along the protofilament axis of bead g (src/compute_cuda.cu:69-301):
+// harmonic + bending inside the dimer, then Morse longitudinal + bending and
+// barrier, in one loop.  (Force, bending and torque sums from zero.)
+__device__ __forceinline__ Acc axial_force(const KParams &P, const DevBuffers &B, const NbrView &V, int g, int flags,
+                                           float4 p0, float4 p1, float theta, const ListHead &H) {
     const int nb = P.nb;          // list layout (k-major over all beads)
     const int ps = V.stride;      // plane stride of the neighbour frames
-    const int base = V.base;
-    const float4 *fr = V.fr;
+    const float4 *fr = V.fr + V.base;
     Acc A = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float3 uzi = f3(Fi.p1);
     const bool off_tub = (flags & kFlagOnTubule) == 0;
-    // harmonic bond inside the dimer (:69-182), then Morse longitudinal
-    // (:187-301): one loop over both, the bonds along the protofilament axis
     const int hc = (flags >> kHarmShift) & 7;
 #pragma unroll 1
     for (int k = 0; k < hc + H.nl; k++) {
@@ -166,13 +163,13 @@ __device__ __forceinline__ Acc bond_force(const KParams &P, const DevBuffers &B,
         else
             e = k == hc ? H.e_l0 : B.lon[(k - hc) * nb + g];
         const float rmon = e < 0 ? 2.0f : -2.0f;
-        const int pj = base + (e < 0 ? -e : e);
+        const int pj = e < 0 ? -e : e;
         const float4 rj = fr[pj], uj = fr[ps + pj];
         const float thj = fr[2 * ps + pj].w;
-        const int fj = V.fl[pj];
-        const float3 wi = make_float3(uzi.x * rmon, uzi.y * rmon, uzi.z * rmon);
+        const int fj = V.fl[V.base + pj];
+        const float3 wi = make_float3(p1.x * rmon, p1.y * rmon, p1.z * rmon);
         const float3 wj = make_float3(-uj.x * rmon, -uj.y * rmon, -uj.z * rmon);
-        const float3 d = site_delta(Fi.p0, rj, wi, wj);
+        const float3 d = site_delta(p0, rj, wi, wj);
         const float r2 = norm2(d);
         float dUdr = P.C;
         int gl = flags;   // whose nucleotide sets theta0: the bead's own, or (longitudinal) the
@@ -183,26 +180,34 @@ __device__ __forceinline__ Acc bond_force(const KParams &P, const DevBuffers &B,
             if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
                 dUdr = __fmaf_rn(dbarr(P.a_bl, P.r_bl, P.w_bl, r), rinv, dUdr);
             if (r2 < kTouch2) dUdr = 0.f;
-            if (!(Fi.p0.z > rj.z)) gl = fj;
+            if (!(p0.z > rj.z)) gl = fj;
         }
         acc_pair(A, dUdr, d, wi);
         if (r2 < 1.0f)
-            acc_bend(P, A, rmon, uj.w - Fi.p1.w, rj.w - Fi.p0.w, thj - Fi.p2.w,
-                     (gl & kFlagGtp) ? P.th0_gtp : P.th0_gdp);
+            acc_bend(P, A, rmon, uj.w - p1.w, rj.w - p0.w, thj - theta, (gl & kFlagGtp) ? P.th0_gtp : P.th0_gdp);
     }
-    // Morse lateral (:303-467)
+    return A;
+}
+
+// Morse lateral bonds of bead g (src/compute_cuda.cu:303-467) with seam
+// coefficient and barrier; l1, l2: the bead's own sites.
+__device__ __forceinline__ Acc lateral_force(const KParams &P, const DevBuffers &B, const NbrView &V, int g, int flags,
+                                             float4 p0, float3 l1, float3 l2, const ListHead &H) {
+    const int nb = P.nb, ps = V.stride;
+    const float4 *fr = V.fr + V.base;
+    Acc A = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const bool off_tub = (flags & kFlagOnTubule) == 0;
 #pragma unroll 1
     for (int k = 0; k < H.nt; k++) {
         const int e = k == 0 ? H.e_t0 : B.lat[k * nb + g];
         const bool neg = e <= 0;
-        int j = e < 0 ? -e : e;
-        if (j == kZeroCode) j = 0;
-        const int pj = base + j;
+        int pj = e < 0 ? -e : e;
+        if (pj == kZeroCode) pj = 0;
         const float4 rj = fr[pj];
         const float4 sj = neg ? fr[3 * ps + pj] : fr[2 * ps + pj];
-        const int fj = V.fl[pj];
-        const float3 wi = neg ? f3(Fi.p2) : f3(Fi.p3);
-        const float3 d = site_delta(Fi.p0, rj, wi, f3(sj));
+        const int fj = V.fl[V.base + pj];
+        const float3 wi = neg ? l1 : l2;
+        const float3 d = site_delta(p0, rj, wi, f3(sj));
         const float r2 = norm2(d), rinv = rsqrt_hw(r2), r = __fmul_rn(r2, rinv);
         float dUdr = dmorse_over_r(((flags ^ fj) & kFlagBeta) ? P.D_lat_seam : P.D_lat, P.A_lat, r, rinv);
         if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
@@ -213,13 +218,26 @@ __device__ __forceinline__ Acc bond_force(const KParams &P, const DevBuffers &B,
     return A;
 }
 
-// The generalised force from its parts: bonds + LJ, the cylindrical walls
-// (src/compute_cuda.cu:497-517), and the bending terms plus the torque
+// sin and cos of psi and theta: the Euler axes of the torque.
+struct Euler {
+    float sp, cp, st, ct;
+};
+__device__ __forceinline__ Euler euler(float psi, float theta) {
+    Euler E;
+    sincosf(psi, &E.sp, &E.cp);
+    sincosf(theta, &E.st, &E.ct);
+    return E;
+}
+// The generalised force from its parts, which are summed in this order in
+// every kernel: axial bonds A, lateral bonds T, LJ L; then the cylindrical
+// walls (src/compute_cuda.cu:497-517), and the bending terms plus the torque
 // projected on the Euler axes (psi about z, theta about Rz(psi) y, fi about
 // R x).  out = (fx, fy, fz, ffi, ftheta, fpsi).
-__device__ __forceinline__ void force_out(const KParams &P, const Acc &A, float3 L, const float *zs, float4 p0,
-                                          float psi, float theta, float out[6]) {
-    float fx = __fadd_rn(A.fx, L.x), fy = __fadd_rn(A.fy, L.y), fz = __fadd_rn(A.fz, L.z);
+__device__ __forceinline__ void force_out(const KParams &P, const Acc &A, const Acc &T, float3 L, const float *zs,
+                                          float4 p0, const Euler &E, float out[6]) {
+    float fx = __fadd_rn(__fadd_rn(A.fx, T.fx), L.x), fy = __fadd_rn(__fadd_rn(A.fy, T.fy), L.y),
+          fz = __fadd_rn(__fadd_rn(A.fz, T.fz), L.z);
+    const float tx = __fadd_rn(A.tx, T.tx), ty = __fadd_rn(A.ty, T.ty), tz = __fadd_rn(A.tz, T.tz);
     if (P.is_wall) {
         const float z = p0.z, top = __fadd_rn(*zs, P.lb);
         if (z < P.lb)
@@ -234,16 +252,14 @@ __device__ __forceinline__ void force_out(const KParams &P, const Acc &A, float3
             fy = __fmaf_rn(p0.y, coeff, fy);
         }
     }
-    float sp, cp, st, ct;
-    sincosf(psi, &sp, &cp);
-    sincosf(theta, &st, &ct);
     out[0] = fx;
     out[1] = fy;
     out[2] = fz;
-    const float tf = __fmaf_rn(__fmul_rn(cp, ct), A.tx, __fmaf_rn(__fmul_rn(sp, ct), A.ty, -__fmul_rn(st, A.tz)));
+    const float tf =
+        __fmaf_rn(__fmul_rn(E.cp, E.ct), tx, __fmaf_rn(__fmul_rn(E.sp, E.ct), ty, -__fmul_rn(E.st, tz)));
     out[3] = __fadd_rn(A.ffi, tf);
-    out[4] = __fadd_rn(A.fth, __fmaf_rn(cp, A.ty, -__fmul_rn(sp, A.tx)));
-    out[5] = __fadd_rn(A.fpsi, A.tz);
+    out[4] = __fadd_rn(A.fth, __fmaf_rn(E.cp, ty, -__fmul_rn(E.sp, tx)));
+    out[5] = __fadd_rn(A.fpsi, tz);
 }
 
 // Generalised force on bead g (compute_kernel, src/compute_cuda.cu:32-525).
@@ -251,8 +267,9 @@ __device__ __forceinline__ void bead_forces(const KParams &P, const DevBuffers &
                                             const float *zs, int flags, const Frame &Fi, const ListHead &H,
                                             float out[6]) {
     const float3 L = lj_force(P, B, V, g, Fi.p0, H);
-    const Acc A = bond_force(P, B, V, g, flags, Fi, H);
-    force_out(P, A, L, zs, Fi.p0, Fi.p1.w, Fi.p2.w, out);
+    const Acc T = lateral_force(P, B, V, g, flags, Fi.p0, f3(Fi.p2), f3(Fi.p3), H);
+    const Acc A = axial_force(P, B, V, g, flags, Fi.p0, Fi.p1, Fi.p2.w, H);
+    force_out(P, A, T, L, zs, Fi.p0, euler(Fi.p1.w, Fi.p2.w), out);
 }
 
 __device__ __forceinline__ Frame load_frame(const float4 *planes, int nb, int g) {
@@ -286,7 +303,7 @@ __device__ __forceinline__ Frame em_update(const KParams &P, const Frame &Fi, co
 // another bead (list heads, noise states) is requested first and the noise is
 // drawn while the neighbours are on their way.
 template <bool KEEP_FORCES>
-__global__ void __launch_bounds__(256) k_step_plain(KParams P, DevBuffers B) {
+__global__ void __launch_bounds__(256, 4) k_step_plain(KParams P, DevBuffers B) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P.nb) return;
     const int nb = P.nb;
@@ -438,9 +455,20 @@ __global__ void __launch_bounds__(kPeriodThreads, 2) k_step_period(KParams P, De
     }
 }
 
-// Forces only (for output and the TEA path).  With TEA_PREPARE it also draws
-// the random force of every bead from stream g scaled by sqrt(2 kB T gammaR /
+// The random force of bead g for TEA from stream g, scaled by sqrt(2 kB T gammaR /
 // dt) (integrateTea_prepare, src/bdhitea_kernel.cu:16-36).
+__device__ __forceinline__ void tea_random(const KParams &P, const DevBuffers &B, int g) {
+    uint4 s = B.seeds[g];
+    float4 r = gauss4(s);
+    B.seeds[g] = s;
+    r.x *= P.tea_var;
+    r.y *= P.tea_var;
+    r.z *= P.tea_var;
+    B.tea_r[g] = r;
+}
+
+// Forces only (for output and the TEA path).  With TEA_PREPARE it also draws
+// the random force of every bead.
 template <bool TEA_PREPARE>
 __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -456,14 +484,92 @@ __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
     }
     B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
     B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);
-    if (TEA_PREPARE) {
-        uint4 s = B.seeds[g];
-        float4 r = gauss4(s);
-        B.seeds[g] = s;
-        r.x *= P.tea_var;
-        r.y *= P.tea_var;
-        r.z *= P.tea_var;
-        B.tea_r[g] = r;
+    if (TEA_PREPARE) tea_random(P, B, g);
+}
+
+// ------------------------------------------------ four warps for 32 beads
+// k_step_plain and k_forces for batches that leave most of the GPU idle, where a
+// step lasts as long as one bead's serial chain: a CTA of four warps serves 32
+// beads, warp 0 their axial bonds, warp 1 the lateral bonds, warp 2 the LJ
+// neighbours, warp 3 the noise and the Euler axes; the parts meet in shared
+// memory and warp 3 sums them (force_out) and moves the beads.  The same
+// functions and order of sums as the one-thread form: the same bits.
+constexpr int kSplitBeads = 32, kSplitThreads = 128;
+enum { kPartA = 0, kPartT = 9, kPartL = 15, kParts = 18 };
+__device__ __forceinline__ void put_axial(float (*s)[kSplitBeads], int l, const Acc &A) {
+    const float v[9] = {A.fx, A.fy, A.fz, A.ffi, A.fpsi, A.fth, A.tx, A.ty, A.tz};
+#pragma unroll
+    for (int c = 0; c < 9; c++) s[kPartA + c][l] = v[c];
+}
+__device__ __forceinline__ void put_lateral(float (*s)[kSplitBeads], int l, const Acc &T) {
+    const float v[6] = {T.fx, T.fy, T.fz, T.tx, T.ty, T.tz};
+#pragma unroll
+    for (int c = 0; c < 6; c++) s[kPartT + c][l] = v[c];
+}
+__device__ __forceinline__ void get_parts(float (*s)[kSplitBeads], int l, Acc &A, Acc &T, float3 &L) {
+    A = {s[0][l], s[1][l], s[2][l], s[3][l], s[4][l], s[5][l], s[6][l], s[7][l], s[8][l]};
+    T = {s[9][l], s[10][l], s[11][l], 0.f, 0.f, 0.f, s[12][l], s[13][l], s[14][l]};
+    L = make_float3(s[15][l], s[16][l], s[17][l]);
+}
+// STEP: the Euler-Maruyama step of k_step_plain; otherwise the forces (TEA:
+// with the random force of every bead).
+template <bool STEP, bool KEEP_FORCES, bool TEA>
+__global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B) {
+    __shared__ float s_part[kParts][kSplitBeads];
+    const int role = threadIdx.x >> 5, l = threadIdx.x & 31, g = blockIdx.x * kSplitBeads + l;
+    const int nb = P.nb;
+    const bool valid = g < nb;
+    const int flags = valid ? B.flags[g] : kFlagExtra;
+    const bool moving = !(flags & (kFlagExtra | kFlagFixed));
+    const bool work = STEP && !KEEP_FORCES ? moving : !(flags & kFlagExtra);
+    float4 gx, ga;
+    Frame Fi;
+    Euler E;
+    if (role < 3) {
+        if (work) {
+            const NbrView V = {B.frame_in, B.flags, nb, B.base[g]};
+            const ListHead H = list_head(P, B, g);
+            const float4 p0 = B.frame_in[g];
+            if (role == 0) {
+                put_axial(s_part, l, axial_force(P, B, V, g, flags, p0, B.frame_in[nb + g], B.frame_in[2 * nb + g].w, H));
+            } else if (role == 1) {
+                put_lateral(s_part, l,
+                            lateral_force(P, B, V, g, flags, p0, f3(B.frame_in[2 * nb + g]), f3(B.frame_in[3 * nb + g]), H));
+            } else {
+                const float3 L = lj_force(P, B, V, g, p0, H);
+                s_part[kPartL][l] = L.x;
+                s_part[kPartL + 1][l] = L.y;
+                s_part[kPartL + 2][l] = L.z;
+            }
+        }
+    } else if (valid) {
+        Fi = load_frame(B.frame_in, nb, g);
+        if (STEP && moving) {
+            uint4 s1 = B.seeds[g], s2 = B.seeds[nb + g];
+            gx = gauss4(s1);
+            ga = gauss4(s2);
+            B.seeds[g] = s1;
+            B.seeds[nb + g] = s2;
+        }
+        if (TEA) tea_random(P, B, g);
+        if (work) E = euler(Fi.p1.w, Fi.p2.w);
+    }
+    __syncthreads();
+    if (role < 3 || !valid) return;
+    float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (work) {
+        Acc A, T;
+        float3 L;
+        get_parts(s_part, l, A, T, L);
+        force_out(P, A, T, L, P.is_wall ? B.zs + B.traj[g] : B.zs, Fi.p0, E, f);
+    }
+    if (STEP) {
+        if (moving) Fi = em_update(P, Fi, f, gx, ga);
+        store_frame(B.frame_out, nb, g, Fi);
+    }
+    if (!STEP || KEEP_FORCES) {
+        B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
+        B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);
     }
 }
 
@@ -638,7 +744,20 @@ void launch_coords_from_frames(const KParams &P, const float4 *frame, float *c7,
 void launch_forces_to_coords(const KParams &P, const float4 *force, float *c7, cudaStream_t s) {
     k_forces_to_coords<<<blocks(P.nb, 256), 256, 0, s>>>(P.nb, force, c7);
 }
+// Beads up to which the four-warp form is used.  It wins while its four times as
+// many warps stay within about one and a half fillings of the GPU: a step of one
+// 1520-bead trajectory took 6.8 us with one thread a bead and 4.6 us so, forces
+// of 52,800 beads 11.5 and 11.0 us, but a step of 78,780 beads 12.2 and 14.5 us.
+constexpr int kSplitMaxBeads = 55000;
 void launch_step_plain(const KParams &P, const DevBuffers &B, bool keep_forces, cudaStream_t s) {
+    if (P.nb <= kSplitMaxBeads) {
+        const int n = blocks(P.nb, kSplitBeads);
+        if (keep_forces)
+            k_split<true, true, false><<<n, kSplitThreads, 0, s>>>(P, B);
+        else
+            k_split<true, false, false><<<n, kSplitThreads, 0, s>>>(P, B);
+        return;
+    }
     const int t = P.step_block > 0 ? P.step_block : 128;
     if (keep_forces)
         k_step_plain<true><<<blocks(P.nb, t), t, 0, s>>>(P, B);
@@ -670,6 +789,14 @@ void launch_step_period(const KParams &P, const DevBuffers &B, bool keep_forces,
 }
 
 void launch_forces(const KParams &P, const DevBuffers &B, bool tea_prepare, cudaStream_t s) {
+    if (P.nb <= kSplitMaxBeads) {
+        const int n = blocks(P.nb, kSplitBeads);
+        if (tea_prepare)
+            k_split<false, false, true><<<n, kSplitThreads, 0, s>>>(P, B);
+        else
+            k_split<false, false, false><<<n, kSplitThreads, 0, s>>>(P, B);
+        return;
+    }
     if (tea_prepare)
         k_forces<true><<<blocks(P.nb, 128), 128, 0, s>>>(P, B);
     else

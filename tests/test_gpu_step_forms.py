@@ -1,0 +1,72 @@
+"""The forms of the plain step and of the force pass (four warps for 32 beads in
+small batches, one thread a bead in large ones) give the same bits, and the
+bending sine holds for angles of any size."""
+import numpy as np
+import pytest
+
+from mt_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("over", [dict(), dict(barrier=1, is_wall=1, rep_r=20.0)], ids=str)
+@pytest.mark.parametrize("keep", [False, True])
+def test_small_batches_equal_a_large_one(over, keep):
+    """60 trajectories of 1018 and one of 33 beads: above the size of the small form
+    together, below it in three parts."""
+    from mt_gb300 import engine
+    p = synth.default_params(seed=71, **over)
+    a = synth.make_trajectory(18, 784, seed=71, radius=8.12, psi_mode="make_mt", cube=90.0, thermal=0.05)
+    c = synth.make_trajectory(1, 20, seed=72, radius=8.12, psi_mode="make_mt", cube=40.0, thermal=0.05)
+    trajs = [a] * 30 + [c] + [a] * 30
+    b = synth.batch_from_trajectories(p, trajs)
+    b.extra[5:6000:97] = 1
+    assert b.nbeads > 60000
+    with engine.Engine(b) as e, engine.ShardedEngine(b, [0, 0, 0]) as s:
+        e.upload_state(b.coords)
+        s.upload_state(b.coords)
+        for k in [e] + s.engines:
+            k.set_keep_forces(keep)
+            k.rebuild_pairs()
+        f = e.compute_forces()
+        assert np.array_equal(f, np.concatenate([k.compute_forces() for k in s.engines]))
+        assert np.abs(f[b.extra == 1]).max() == 0 and np.isfinite(f).all()
+        e.step(0, 13)
+        s.step(0, 13)
+        assert np.array_equal(e.download_state(), s.download_state())
+        assert np.array_equal(e.download_rng(), s.download_rng())
+        if keep:
+            assert np.array_equal(e.download_state(forces=True)[1],
+                                  np.concatenate([k.download_state(forces=True)[1] for k in s.engines]))
+
+
+@pytest.mark.parametrize("turns", [3, 150, 170, 4000])
+def test_bending_of_large_angles(turns):
+    """Angle differences of many turns, on both sides of the 1000 rad where the sine
+    goes to the library: the psi force of the dimers' harmonic bonds (no lists are
+    built) in FP64 from the same FP32 angles.  Allowed: the FP32 rounding of the
+    site vectors (2 nm, at most 8 units each, on the 2 nm arm of the bond C) and of
+    the sine's argument and value (4 units)."""
+    from mt_gb300 import engine
+    b = synth.uniform_batch(synth.default_params(seed=73, lj_on=0), 1, 8, 0, seed=73, radius=8.12,
+                            psi_mode="make_mt", thermal=0.05)
+    rng = np.random.default_rng(turns)
+    b.coords[:, 3:6] += (2 * np.pi * rng.integers(-turns, turns + 1, (b.nbeads, 3))).astype(np.float32)
+    p = b.params
+    with engine.Engine(b) as e:
+        e.upload_state(b.coords)
+        f = e.compute_forces().astype(np.float64)
+    c, j = b.coords.astype(np.float64), np.abs(b.harmonic)
+    sg = np.where(b.harmonic < 0, 1.0, -1.0)
+    cs, sn = np.cos(c[:, 3:6]), np.sin(c[:, 3:6])
+    uz = np.stack([cs[:, 2] * sn[:, 1] * cs[:, 0] + sn[:, 2] * sn[:, 0],
+                   sn[:, 2] * sn[:, 1] * cs[:, 0] - cs[:, 2] * sn[:, 0], cs[:, 1] * cs[:, 0]], 1)
+    w = 2.0 * sg[:, None] * uz
+    d = c[j, :3] - 2.0 * sg[:, None] * uz[j] - c[:, :3] - w
+    dpsi = c[j, 5] - c[:, 5]
+    near = np.linalg.norm(d, axis=1) < 0.99
+    assert near.sum() > 20
+    want = p.B_psi * sg * np.sin(sg * dpsi - p.psi_0) + p.C * np.cross(w, d)[:, 2]
+    ulp = np.spacing(np.abs(dpsi).astype(np.float32)).astype(np.float64)
+    tol = p.C * 2.0 * 8 * 2.0 ** -22 + p.B_psi * (ulp + 4 * 2.0 ** -24)
+    assert (np.abs(f[:, 5] - want)[near] <= tol[near]).all()
