@@ -429,11 +429,9 @@ int mtg_tea_effective_forces(mtg_engine *e, float *feff_exact, float *feff_ff, f
 /* Launch shapes of the engine's kernels.  list_method as
  * mtg_set_list_method (1 tiles, 2 cells); step_block: threads per CTA of the
  * fused plain step (64, 128, 256); tea_slices: threads per bead in the
- * all-pairs TEA kernels (1, 2, 4, 8); tea_jparts: parts the j range of a
- * work item is split into (1, 2, 3, 4).  With more than one part, the items
- * of the last one to two waves of a launch (all items of a launch shorter
- * than two waves) run as that many shorter CTAs, so the last waves are
- * fuller; the parts' sums meet in a second kernel.  plain_persistent: 1 runs
+ * near-pair kernel of learned TEA (1, 2, 4, 8); tea_jparts (1, 2, 3, 4): kept
+ * for saved tunings, without effect (the all-pairs kernels divide their work
+ * over the GPU themselves); plain_persistent: 1 runs
  * the plain (no-HI) steps between two pair-list rebuilds as one launch with
  * one CTA per trajectory and the trajectory's frames in shared memory (for
  * batches whose largest trajectory has at most 2048 beads), 0 one launch

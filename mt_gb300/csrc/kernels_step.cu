@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kPeriodThreads, 2) k_step_period(KParams P, De
 
 // The random force of bead g for TEA from stream g, scaled by sqrt(2 kB T gammaR /
 // dt) (integrateTea_prepare, src/bdhitea_kernel.cu:16-36).
-__device__ __forceinline__ void tea_random(const KParams &P, const DevBuffers &B, int g) {
+__device__ __forceinline__ float4 tea_random(const KParams &P, const DevBuffers &B, int g) {
     uint4 s = B.seeds[g];
     float4 r = gauss4(s);
     B.seeds[g] = s;
@@ -465,10 +465,11 @@ __device__ __forceinline__ void tea_random(const KParams &P, const DevBuffers &B
     r.y *= P.tea_var;
     r.z *= P.tea_var;
     B.tea_r[g] = r;
+    return r;
 }
 
 // Forces only (for output and the TEA path).  With TEA_PREPARE it also draws
-// the random force of every bead.
+// the random force of every bead and lays the bead out for the all-pairs pass.
 template <bool TEA_PREPARE>
 __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -476,15 +477,18 @@ __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
     const int nb = P.nb;
     const int flags = B.flags[g];
     float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const Frame Fi = load_frame(B.frame_in, nb, g);
     if (!(flags & kFlagExtra)) {
         const NbrView V = {B.frame_in, B.flags, nb, B.base[g]};
         const ListHead H = list_head(P, B, g);
-        const Frame Fi = load_frame(B.frame_in, nb, g);
         bead_forces(P, B, V, g, P.is_wall ? B.zs + B.traj[g] : B.zs, flags, Fi, H, f);
     }
     B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
     B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);
-    if (TEA_PREPARE) tea_random(P, B, g);
+    if (TEA_PREPARE) {
+        const float4 r = tea_random(P, B, g);
+        tea_pack_bead(B, g, (flags & kFlagExtra) != 0, Fi.p0, f[0], f[1], f[2], r);
+    }
 }
 
 // ------------------------------------------------ four warps for 32 beads
@@ -522,7 +526,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
     const int flags = valid ? B.flags[g] : kFlagExtra;
     const bool moving = !(flags & (kFlagExtra | kFlagFixed));
     const bool work = STEP && !KEEP_FORCES ? moving : !(flags & kFlagExtra);
-    float4 gx, ga;
+    float4 gx, ga, rt;
     Frame Fi;
     Euler E;
     if (role < 3) {
@@ -551,7 +555,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
             B.seeds[g] = s1;
             B.seeds[nb + g] = s2;
         }
-        if (TEA) tea_random(P, B, g);
+        if (TEA) rt = tea_random(P, B, g);
         if (work) E = euler(Fi.p1.w, Fi.p2.w);
     }
     __syncthreads();
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
         B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
         B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);
     }
+    if (TEA) tea_pack_bead(B, g, (flags & kFlagExtra) != 0, Fi.p0, f[0], f[1], f[2], rt);
 }
 
 // ------------------------------------------------------------- energies

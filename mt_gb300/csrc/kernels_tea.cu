@@ -1,75 +1,59 @@
 // kernels_tea.cu - TEA hydrodynamics (Geyer & Winter 2009): the all-pairs
 // epsilon / C_i pass, the FP64 epsilon -> beta reduction, and the all-pairs
-// RPY mobility product fused with the position update.
+// RPY mobility product fused with the position update; below them the far
+// field of the learned mode.
 //
-// Both O(N^2) kernels run one CTA per (trajectory, chunk of kTeaChunk beads)
-// and stream the trajectory through shared memory in tiles of kTeaTile
-// beads j.  A thread serves kTeaNI beads i (lanes il, il + 32, ...) as packed
-// FP32x2 pairs; `tea_slices` threads share each bead i and take interleaved
-// j of every tile, so small batches still fill the GPU, and the partial sums
-// meet in shared memory.  The tile holds every value of bead j twice (both
-// lanes of a packed operand, two operands per 16-byte word), so broadcast
-// loads feed the packed pairs of beads i directly.  Away from the CTA's own
-// beads the far-field formula runs for every pair; the few overlapping pairs
-// (r <= 2a) are found through running minima of r^2, one per quarter of a
-// thread's j values, and only a quarter that holds one is rescanned with the
-// near-field formula.  With tea_jparts > 1 the work items of the last waves
-// are split over parts of their j range (see tea_item).  In the tile that holds
-// the CTA's own beads the self pairs get r^2 = 1e30: their terms are then
-// far below the rounding of the sums, and the correction skips them.
-// Sums are kept in units of 0.75 a (T' = T / (0.75 a)).  The kernels are
-// bound by the FP32 pipe (about 45 FLOP per ordered pair).
+// Both O(N^2) passes are one kernel template, k_tea_pass.  They are bound by
+// the FP32 pipe (about 45 FLOP per ordered pair: 24 packed FP32x2 operations
+// for two pairs), so everything else is arranged to stay off its way:
+//   * The beads j come from B.tea_pack, where the force kernel of the step has
+//     laid every trajectory out in blocks of 32 beads = 16 pairs in the order the
+//     loop reads them: the two lanes of a packed operation are two beads j, one
+//     16-byte shared-memory broadcast feeds two operands of both.  A tile of
+//     kTeaTileBlocks blocks is copied by cp.async two tiles ahead, one barrier a
+//     tile.  Extra beads and padding sit at 1e18 nm with zero F and R: every term they give is zero or
+//     below the rounding of the sums.
+//   * A CTA of four warps serves 128 beads i, one a thread: 56 registers and nine
+//     CTAs an SM (two beads a thread load half as many words but leave six CTAs:
+//     1.82 against 1.76 ms).
+//   * The work of a launch is the list of units (128 beads i) x (one block of
+//     j), cut into equal contiguous runs, one CTA each, as many as the GPU holds
+//     at once: no last wave is partly filled, whatever the sizes.  A run
+//     that does not hold all units of its 128 beads leaves its partial sums, and the CTA
+//     that comes last (an atomic count; nothing waits) adds them in run order and
+//     finishes the beads, so the result does not depend on the timing.
+// The far-field formula runs for every pair; the few overlapping pairs
+// (r <= 2a) are found through a running minimum of r^2 per block; in a block
+// that holds one their distances are taken once more and only they get the near-field formula.  In
+// the block that holds a bead itself its own pair gets r^2 = 1e30: its term is
+// then far below the rounding of the sums, and the correction skips it.
+// Sums are kept in units of 0.75 a (T' = T / (0.75 a)).
+// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.72 ms (52 TFLOP/s of the measured 80;
+// the FMA pipe is 72% active), 16 x 3300 205 -> 168 us, one trajectory of 299 25 -> 14 us (before: a tile stored twice by
+// every CTA, whole 128-bead items in 3.7 waves or a second kernel for split ones).
 #include "mtg_internal.cuh"
 
 namespace mtg {
 
-constexpr int kTeaNI = 4;                   // beads i per thread
-constexpr int kTeaPairsI = kTeaNI / 2;      // packed pairs of them
-constexpr int kTeaLanes = 32;               // threads per slice
-constexpr int kTeaSeg = 4;                  // segments of a thread's j values, each with its own r^2 minimum
+constexpr int kTeaThreads = 128;
 constexpr int kTeaI = kTeaChunk;            // beads i per CTA
-static_assert(kTeaI == kTeaLanes * kTeaNI, "chunk = lanes x beads per thread");
-constexpr int kTeaTile = 128;               // beads j per tile
-constexpr float kFarAway = 1.0e18f;         // position of padding and extra beads j
+static_assert(kTeaI == kTeaThreads, "one bead a thread");
+constexpr int kTeaTileBlocks = 4;           // blocks of a tile
+constexpr int kTeaStages = 3;               // tiles in shared memory
+constexpr float kFarAway = kTeaFarAway;     // position of padding and extra beads j
 
-// Tile of the all-pairs kernels, every value duplicated into both lanes of
-// a packed pair and two pairs per 16-byte word, so that a bead j takes five
-// shared-memory loads (two without F and R).  Beads past the trajectory's end
-// and extra beads sit far away with zero F and R: every term they give is
-// zero or below the rounding of the sums.
-struct TeaTile {
-    float4 xy[kTeaTile];   // x x y y
-    float4 zf[kTeaTile];   // z z Fx Fx
-    float4 fyz[kTeaTile];  // Fy Fy Fz Fz
-    float4 rxy[kTeaTile];  // Rx Rx Ry Ry
-    float2 rz[kTeaTile];   // Rz Rz
-};
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 
-template <bool WITH_FR>
-__device__ __forceinline__ void tea_tile_load(TeaTile &T, const DevBuffers &B, int j0, int end) {
-    for (int k = threadIdx.x; k < kTeaTile; k += blockDim.x) {
-        const int jg = j0 + k;
-        float4 p = make_float4(kFarAway, kFarAway, kFarAway, 0.f), F = make_float4(0.f, 0.f, 0.f, 0.f), R = F;
-        if (jg < end && !(B.flags[jg] & kFlagExtra)) {
-            p = B.frame_in[jg];
-            if (WITH_FR) {
-                F = B.force[jg];
-                R = B.tea_r[jg];
-            }
-        }
-        T.xy[k] = make_float4(p.x, p.x, p.y, p.y);
-        T.zf[k] = make_float4(p.z, p.z, F.x, F.x);
-        if (WITH_FR) {
-            T.fyz[k] = make_float4(F.y, F.y, F.z, F.z);
-            T.rxy[k] = make_float4(R.x, R.x, R.y, R.y);
-            T.rz[k] = f2(R.z);
-        }
-    }
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Scaled RPY coefficients (integrateTea_RPY, src/bdhitea_kernel.cu:38-58:
 // T = cii I + crr u u^T, ra = r/a; ra > 2: cii = 0.75/ra (1 + 2/(3 ra^2)),
@@ -89,7 +73,6 @@ __device__ __forceinline__ void rpy_near(const TeaConst &K, float r2, float rinv
     crr = (3.0f / 32.0f) * ra * K.inv_c075a;
 }
 
-// ------------------------------------------------------------ epsilon pass
 // Scaled epsilon terms of one pair from cii', crr', q: the row sums of
 // squares minus cii'^2 (Bc d_c^2 with Bc = (2 cii' + crr') crr' q), cii'^2, and
 // the sum of all nine entries 3 cii' + crr' q (d_x + d_y + d_z)^2.
@@ -103,37 +86,6 @@ __device__ __forceinline__ EpsTerms eps_terms(float dx, float dy, float dz, floa
     return {bc * dx * dx, bc * dy * dy, bc * dz * dz, cii * cii, fmaf(crq * us, us, 3.0f * cii)};
 }
 
-// Range of beads j of part `part` of `parts` of a trajectory [base, end):
-// whole tiles, the parts as equal as the tile count allows.
-__device__ __forceinline__ void tea_jrange(int base, int end, int part, int parts, int &jb, int &je) {
-    const int ntiles = (end - base + kTeaTile - 1) / kTeaTile;
-    const int per = (ntiles + parts - 1) / parts;
-    jb = min(end, base + part * per * kTeaTile);
-    je = min(end, base + (part + 1) * per * kTeaTile);
-}
-
-// Work item and j part of this CTA.  The first P.tea_nhead items run whole;
-// with SPLIT every later item runs as P.tea_jparts CTAs over parts of its j
-// range, so that the last waves of a launch are made of short CTAs.
-template <bool SPLIT>
-__device__ __forceinline__ void tea_item(const KParams &P, int &item, int &part, int &parts) {
-    item = (int)blockIdx.x;
-    part = 0;
-    parts = 1;
-    if (SPLIT && item >= P.tea_nhead) {
-        const int k = item - P.tea_nhead;
-        item = P.tea_nhead + k / P.tea_jparts;
-        part = k % P.tea_jparts;
-        parts = P.tea_jparts;
-    }
-}
-// Bead of a finish kernel (one CTA of kTeaChunk threads per split item), or -1.
-__device__ __forceinline__ int tea_tail_bead(const KParams &P, const DevBuffers &B, const int2 *work) {
-    const int2 w = work[P.tea_nhead + blockIdx.x];
-    const int g = w.y + (int)threadIdx.x;
-    return g < B.off[w.x + 1] ? g : -1;
-}
-
 // Stores the epsilon-pass result of bead g from its scaled sums
 // (x, y, z: row sums of squares; w: sum of all entries).
 __device__ __forceinline__ void eps_store(const KParams &P, const DevBuffers &B, int g, bool active, float4 acc,
@@ -144,201 +96,6 @@ __device__ __forceinline__ void eps_store(const KParams &P, const DevBuffers &B,
     B.tea_eps[g] = acc.w * K.c075a;
 }
 
-// The packed pass of one tile of the epsilon pass (self pairs pushed to
-// r^2 = 1e30 when SELF), running minimum of r^2 per bead pair.
-template <int SLICES, bool SELF>
-__device__ __forceinline__ void tea_eps_tile(const TeaTile &T, int sl, int self_t, const float2 (&nx)[kTeaPairsI],
-                                             const float2 (&ny)[kTeaPairsI], const float2 (&nz)[kTeaPairsI],
-                                             float2 vkap, float2 vn2a2, float2 two, float2 three,
-                                             float2 (&sx)[kTeaPairsI], float2 (&sy)[kTeaPairsI],
-                                             float2 (&sz)[kTeaPairsI], float2 (&sa)[kTeaPairsI],
-                                             float2 (&sw)[kTeaPairsI], float (&rmin)[kTeaPairsI][kTeaSeg]) {
-    constexpr int kLen = kTeaTile / SLICES / kTeaSeg;
-#pragma unroll
-    for (int sg = 0; sg < kTeaSeg; sg++) {
-#pragma unroll 2
-        for (int k = 0; k < kLen; k++) {
-            const int t = sl + (sg * kLen + k) * SLICES;
-            const float4 a = T.xy[t];
-            const float2 xj = lo2(a), yj = hi2(a), zj = lo2(T.zf[t]);
-#pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++) {
-                const float2 dx = __fadd2_rn(xj, nx[p]), dy = __fadd2_rn(yj, ny[p]), dz = __fadd2_rn(zj, nz[p]);
-                float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                if (SELF) {
-                    if (t == self_t + kTeaLanes * 2 * p) r2.x = 1e30f;
-                    if (t == self_t + kTeaLanes * (2 * p + 1)) r2.y = 1e30f;
-                }
-                rmin[p][sg] = fmin3(rmin[p][sg], r2.x, r2.y);
-                const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
-                const float2 q = __fmul2_rn(rinv, rinv);
-                const float2 tq = __fmul2_rn(q, rinv);
-                const float2 cii = __ffma2_rn(vkap, tq, rinv);
-                const float2 crr = __ffma2_rn(vn2a2, tq, rinv);
-                const float2 crq = __fmul2_rn(crr, q);
-                const float2 bc = __fmul2_rn(__ffma2_rn(two, cii, crr), crq);
-                sa[p] = __ffma2_rn(cii, cii, sa[p]);
-                sx[p] = __ffma2_rn(__fmul2_rn(bc, dx), dx, sx[p]);
-                sy[p] = __ffma2_rn(__fmul2_rn(bc, dy), dy, sy[p]);
-                sz[p] = __ffma2_rn(__fmul2_rn(bc, dz), dz, sz[p]);
-                const float2 us = __fadd2_rn(__fadd2_rn(dx, dy), dz);
-                sw[p] = __ffma2_rn(__fmul2_rn(crq, us), us, __ffma2_rn(three, cii, sw[p]));
-            }
-        }
-    }
-}
-
-// integrateTea_epsilon_unlisted (src/bdhitea_kernel.cu:84-101): per bead i,
-// sum over non-extra j != i of the row sums of squared entries (-> tea_ci)
-// and of all nine entries (-> tea_eps).  With T = cii I + crr u u^T the row
-// sums of squares are cii^2 + (2 cii + crr) crr u_c^2 and the sum of all
-// entries is 3 cii + crr (u_x + u_y + u_z)^2.
-template <int SLICES, bool SPLIT>
-__global__ void __launch_bounds__(kTeaLanes *SLICES, 20 / SLICES) k_tea_eps(KParams P, DevBuffers B, const int2 *work,
-                                                                const int *gate, int run_if) {
-    if (gate && *gate != run_if) return;
-    int item, part, parts;
-    tea_item<SPLIT>(P, item, part, parts);
-    const int2 w = work[item];
-    const int traj = w.x, base = B.off[traj], end = B.off[traj + 1];
-    int jb, je;
-    tea_jrange(base, end, part, parts, jb, je);
-    const int il = threadIdx.x % kTeaLanes, sl = threadIdx.x / kTeaLanes;
-    __shared__ TeaTile T;
-    __shared__ float4 s_red[kTeaI * SLICES];
-    int gi[kTeaNI];
-    bool act[kTeaNI];
-    float4 pi[kTeaNI];
-    float2 nx[kTeaPairsI], ny[kTeaPairsI], nz[kTeaPairsI];
-    float2 sx[kTeaPairsI], sy[kTeaPairsI], sz[kTeaPairsI], sa[kTeaPairsI], sw[kTeaPairsI];
-    bool any_act = false;
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        gi[h] = w.y + il + h * kTeaLanes;
-        act[h] = false;
-        pi[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gi[h] < end) {
-            pi[h] = B.frame_in[gi[h]];
-            act[h] = (B.flags[gi[h]] & kFlagExtra) == 0;
-        }
-        any_act |= act[h];
-    }
-#pragma unroll
-    for (int p = 0; p < kTeaPairsI; p++) {
-        nx[p] = make_float2(-pi[2 * p].x, -pi[2 * p + 1].x);
-        ny[p] = make_float2(-pi[2 * p].y, -pi[2 * p + 1].y);
-        nz[p] = make_float2(-pi[2 * p].z, -pi[2 * p + 1].z);
-        sx[p] = sy[p] = sz[p] = sa[p] = sw[p] = f2(0.f);
-    }
-    const TeaConst K = tea_const(P.tea_a);
-    const float2 vkap = f2(K.kap), vn2a2 = f2(-K.two_a2), two = f2(2.0f), three = f2(3.0f);
-    for (int j0 = jb; j0 < je; j0 += kTeaTile) {
-        tea_tile_load<false>(T, B, j0, end);
-        __syncthreads();
-        if (any_act) {
-            // self pairs: as in k_tea_step
-            const bool self_tile = (w.y < j0 + kTeaTile) && (w.y + kTeaI > j0);
-            const int self_t = self_tile ? w.y - j0 + il : -(1 << 30);
-            float rmin[kTeaPairsI][kTeaSeg];
-#pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++)
-#pragma unroll
-                for (int sg = 0; sg < kTeaSeg; sg++) rmin[p][sg] = 3.4e38f;
-            if (self_tile)
-                tea_eps_tile<SLICES, true>(T, sl, self_t, nx, ny, nz, vkap, vn2a2, two, three, sx, sy, sz, sa, sw,
-                                           rmin);
-            else
-                tea_eps_tile<SLICES, false>(T, sl, self_t, nx, ny, nz, vkap, vn2a2, two, three, sx, sy, sz, sa, sw,
-                                            rmin);
-            // overlapping pairs (r <= 2a): replace the far-field terms by the near ones
-#pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++) {
-                unsigned segs = 0;
-#pragma unroll
-                for (int sg = 0; sg < kTeaSeg; sg++) segs |= (rmin[p][sg] <= K.four_a2 ? 1u : 0u) << sg;
-                constexpr int kLen = kTeaTile / SLICES / kTeaSeg;
-                while (segs) {  // the segments that hold an overlapping pair
-                    const int sg = __ffs(segs) - 1;
-                    segs &= segs - 1;
-                    for (int k = 0; k < kLen; k++) {
-                        const int t = sl + (sg * kLen + k) * SLICES;
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            if (t == self_t + kTeaLanes * (2 * p + e)) continue;
-                            const float ax = e ? nx[p].y : nx[p].x, ay = e ? ny[p].y : ny[p].x,
-                                        az = e ? nz[p].y : nz[p].x;
-                            const float dx = T.xy[t].x + ax, dy = T.xy[t].z + ay, dz = T.zf[t].x + az;
-                            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            if (!(r2 <= K.four_a2)) continue;
-                            const float rinv = rsqrt_hw(r2), q = rinv * rinv, tq = q * rinv;
-                            const EpsTerms f = eps_terms(dx, dy, dz, fmaf(K.kap, tq, rinv), fmaf(-K.two_a2, tq, rinv), q);
-                            float cn, rn;
-                            rpy_near(K, r2, rinv, cn, rn);
-                            const EpsTerms n = eps_terms(dx, dy, dz, cn, rn, q);
-                            if (e) {
-                                sx[p].y += n.bx - f.bx;
-                                sy[p].y += n.by - f.by;
-                                sz[p].y += n.bz - f.bz;
-                                sa[p].y += n.a2 - f.a2;
-                                sw[p].y += n.w - f.w;
-                            } else {
-                                sx[p].x += n.bx - f.bx;
-                                sy[p].x += n.by - f.by;
-                                sz[p].x += n.bz - f.bz;
-                                sa[p].x += n.a2 - f.a2;
-                                sw[p].x += n.w - f.w;
-                            }
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        const int p = h >> 1;
-        const bool hi = h & 1;
-        const float A = hi ? sa[p].y : sa[p].x;
-        s_red[(sl * kTeaNI + h) * kTeaLanes + il] =
-            make_float4((hi ? sx[p].y : sx[p].x) + A, (hi ? sy[p].y : sy[p].x) + A, (hi ? sz[p].y : sz[p].x) + A,
-                        hi ? sw[p].y : sw[p].x);
-    }
-    __syncthreads();
-    if (sl != 0) return;
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        if (gi[h] >= end) continue;
-        float4 acc = s_red[h * kTeaLanes + il];
-        for (int k = 1; k < SLICES; k++) {
-            const float4 v = s_red[(k * kTeaNI + h) * kTeaLanes + il];
-            acc.x += v.x;
-            acc.y += v.y;
-            acc.z += v.z;
-            acc.w += v.w;
-        }
-        if (SPLIT && parts > 1)
-            B.tea_part[(size_t)part * P.nb + gi[h]] = acc;
-        else
-            eps_store(P, B, gi[h], act[h], acc, K);
-    }
-}
-
-// Sums of the parts of a split epsilon pass.
-__global__ void k_tea_eps_finish(KParams P, DevBuffers B, const int2 *work, const int *gate, int run_if) {
-    if (gate && *gate != run_if) return;
-    const int g = tea_tail_bead(P, B, work);
-    if (g < 0) return;
-    float4 acc = B.tea_part[g];
-    for (int k = 1; k < P.tea_jparts; k++) {
-        const float4 v = B.tea_part[(size_t)k * P.nb + g];
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-    }
-    eps_store(P, B, g, (B.flags[g] & kFlagExtra) == 0, acc, tea_const(P.tea_a));
-}
 
 // updateTea's reduction (src/bdhitea.cu:75-116), in FP64 on the device: one
 // CTA per trajectory sums the bead epsilons and counts the non-extra beads N',
@@ -396,7 +153,6 @@ __global__ void __launch_bounds__(256) k_tea_beta(KParams P, DevBuffers B, int c
     }
 }
 
-// ------------------------------------------------------- mobility product
 // Scaled far-field term of one pair in scalar arithmetic, the operations of
 // one lane of the packed loop in the same order.
 __device__ __forceinline__ float3 tea_far1(const TeaConst &K, float dx, float dy, float dz, float gx, float gy,
@@ -422,50 +178,6 @@ __device__ __forceinline__ float3 tea_pair1(const TeaConst &K, float dx, float d
     }
     const float s = cr * fmaf(dx, gx, fmaf(dy, gy, dz * gz));
     return make_float3(fmaf(cii, gx, s * dx), fmaf(cii, gy, s * dy), fmaf(cii, gz, s * dz));
-}
-
-// The packed pass of one tile: far-field terms of every pair (self pairs
-// pushed to r^2 = 1e30 when SELF), running minimum of r^2 per bead pair.
-template <int SLICES, bool SELF>
-__device__ __forceinline__ void tea_step_tile(const TeaTile &T, int sl, int self_t, const float2 (&nx)[kTeaPairsI],
-                                              const float2 (&ny)[kTeaPairsI], const float2 (&nz)[kTeaPairsI],
-                                              const float2 (&cbx)[kTeaPairsI], const float2 (&cby)[kTeaPairsI],
-                                              const float2 (&cbz)[kTeaPairsI], float2 vkap, float2 vn2a2,
-                                              float2 one, float2 (&ax)[kTeaPairsI], float2 (&ay)[kTeaPairsI],
-                                              float2 (&az)[kTeaPairsI], float (&rmin)[kTeaPairsI][kTeaSeg]) {
-    constexpr int kLen = kTeaTile / SLICES / kTeaSeg;
-#pragma unroll
-    for (int sg = 0; sg < kTeaSeg; sg++) {
-#pragma unroll(kLen <= 8 ? kLen : 2)
-        for (int k = 0; k < kLen; k++) {
-            const int t = sl + (sg * kLen + k) * SLICES;
-            const float4 a = T.xy[t], b = T.zf[t], c = T.fyz[t], d = T.rxy[t];
-            const float2 xj = lo2(a), yj = hi2(a), zj = lo2(b);
-            const float2 fxj = hi2(b), fyj = lo2(c), fzj = hi2(c);
-            const float2 rxj = lo2(d), ryj = hi2(d), rzj = T.rz[t];
-#pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++) {
-                const float2 dx = __fadd2_rn(xj, nx[p]), dy = __fadd2_rn(yj, ny[p]), dz = __fadd2_rn(zj, nz[p]);
-                const float2 gx = __ffma2_rn(rxj, cbx[p], fxj), gy = __ffma2_rn(ryj, cby[p], fyj),
-                             gz = __ffma2_rn(rzj, cbz[p], fzj);
-                float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                if (SELF) {
-                    if (t == self_t + kTeaLanes * 2 * p) r2.x = 1e30f;
-                    if (t == self_t + kTeaLanes * (2 * p + 1)) r2.y = 1e30f;
-                }
-                rmin[p][sg] = fmin3(rmin[p][sg], r2.x, r2.y);
-                const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
-                const float2 q = __fmul2_rn(rinv, rinv);
-                const float2 tq = __fmul2_rn(q, rinv);
-                const float2 cii = __ffma2_rn(vkap, tq, rinv);
-                const float2 cr = __fmul2_rn(tq, __ffma2_rn(vn2a2, q, one));
-                const float2 s = __fmul2_rn(cr, __ffma2_rn(dx, gx, __ffma2_rn(dy, gy, __fmul2_rn(dz, gz))));
-                ax[p] = __ffma2_rn(cii, gx, __ffma2_rn(s, dx, ax[p]));
-                ay[p] = __ffma2_rn(cii, gy, __ffma2_rn(s, dy, ay[p]));
-                az[p] = __ffma2_rn(cii, gz, __ffma2_rn(s, dz, az[p]));
-            }
-        }
-    }
 }
 
 // The update of bead g from its scaled mobility sums (sx, sy, sz): back to
@@ -502,201 +214,329 @@ __device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffe
     store_frame(B.frame_out, nb, g, Fr);
 }
 
-// integrateTea_kernel_unlisted + integrateTea_force (src/bdhitea_kernel.cu:104-213):
-// f_i = F_i + C_i o R_i + sum_{j != i, non-extra} T_ij (F_j + beta C_i o R_j),
-// x_i += dt/gammaR f_i; angles by Euler-Maruyama from stream i + nb, which is
-// drawn for every bead.  Reads the current frame, writes the next one.  With
-// FEFF the kernel stores f_i instead and moves nothing.
-template <int SLICES, bool FEFF, bool SPLIT>
-__global__ void __launch_bounds__(kTeaLanes *SLICES, 20 / SLICES) k_tea_step(KParams P, DevBuffers B, const int2 *work,
-                                                                 float4 *feff, const int *gate) {
-    if (FEFF && gate && *gate != 0) return;
-    if (!FEFF && gate && *gate == 0) return;   // the gated update runs after a fall-back only
-    int item, part, parts;
-    tea_item<SPLIT>(P, item, part, parts);
-    const int2 w = work[item];
-    const int traj = w.x, base = B.off[traj], end = B.off[traj + 1];
-    int jb, je;
-    tea_jrange(base, end, part, parts, jb, je);
-    const int il = threadIdx.x % kTeaLanes, sl = threadIdx.x / kTeaLanes;
-    const int nb = P.nb;
-    __shared__ TeaTile T;
-    __shared__ float4 s_red[kTeaI * SLICES];
 
-    // per packed pair p of beads i (2p, 2p+1): -position, beta C_i, sums
-    float2 nx[kTeaPairsI], ny[kTeaPairsI], nz[kTeaPairsI], cbx[kTeaPairsI], cby[kTeaPairsI], cbz[kTeaPairsI];
-    float2 ax[kTeaPairsI], ay[kTeaPairsI], az[kTeaPairsI];
-    bool any_act = false;
-    const float beta = B.tea_beta[traj], b2 = beta * beta;
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        const int g = w.y + il + h * kTeaLanes;
-        float4 p = make_float4(0.f, 0.f, 0.f, 0.f), c = p;
-        if (g < end) {
-            p = B.frame_in[g];
-            any_act |= (B.flags[g] & kFlagExtra) == 0;
+// ------------------------------------------------------- the all-pairs pass
+// One block of beads j for the epsilon pass (integrateTea_epsilon_unlisted,
+// src/bdhitea_kernel.cu:84-101): per bead i, sums over non-extra j != i of the
+// row sums of squared entries and of all nine entries.  With T = cii I + crr u u^T
+// the row sums of squares are cii^2 + (2 cii + crr) crr u_c^2 and the sum of
+// all entries is 3 cii + crr (u_x + u_y + u_z)^2.
+struct EpsOp {
+    static constexpr int kWords = 2 * kTeaPairSlots;   // float4 of a block that it reads: positions
+    float2 nx, ny, nz;
+    float2 sx, sy, sz, sa, sw;
+    __device__ __forceinline__ void start(const KParams &, const DevBuffers &, int, float4 p, int, bool) {
+        nx = f2(-p.x);
+        ny = f2(-p.y);
+        nz = f2(-p.z);
+        sx = sy = sz = sa = sw = f2(0.f);
+    }
+    template <bool SELF>
+    __device__ __forceinline__ void pair(const TeaConst &K, const float4 *blk, int t, int sp, int se,
+                                         float &rm) {
+        const float2 vkap = f2(K.kap), vn2a2 = f2(-K.two_a2), two = f2(2.0f), three = f2(3.0f);
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t];
+        const float2 dx = __fadd2_rn(lo2(a), nx), dy = __fadd2_rn(hi2(a), ny), dz = __fadd2_rn(lo2(b), nz);
+        const float2 x2 = __fmul2_rn(dx, dx), y2 = __fmul2_rn(dy, dy), z2 = __fmul2_rn(dz, dz);
+        float2 r2 = __fadd2_rn(x2, __fadd2_rn(y2, z2));
+        if (SELF && t == sp) {
+            if (se)
+                r2.y = 1e30f;
+            else
+                r2.x = 1e30f;
+        }
+        rm = fmin3(rm, r2.x, r2.y);
+        const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+        const float2 q = __fmul2_rn(rinv, rinv);
+        const float2 tq = __fmul2_rn(q, rinv);
+        const float2 cii = __ffma2_rn(vkap, tq, rinv);
+        const float2 crr = __ffma2_rn(vn2a2, tq, rinv);
+        const float2 crq = __fmul2_rn(crr, q);
+        const float2 bc = __fmul2_rn(__ffma2_rn(two, cii, crr), crq);
+        sa = __ffma2_rn(cii, cii, sa);
+        sx = __ffma2_rn(bc, x2, sx);
+        sy = __ffma2_rn(bc, y2, sy);
+        sz = __ffma2_rn(bc, z2, sz);
+        const float2 us = __fadd2_rn(__fadd2_rn(dx, dy), dz);
+        sw = __ffma2_rn(__fmul2_rn(crq, us), us, __ffma2_rn(three, cii, sw));
+    }
+    __device__ __forceinline__ float2 dist2(const float4 *blk, int t) const {
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t];
+        const float2 dx = __fadd2_rn(lo2(a), nx), dy = __fadd2_rn(hi2(a), ny), dz = __fadd2_rn(lo2(b), nz);
+        return __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    }
+    // one overlapping pair: the far-field terms are replaced by the near ones
+    __device__ __forceinline__ void near(const TeaConst &K, const float4 *blk, int t, int e) {
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t];
+        const float dx = (e ? a.y : a.x) + nx.x, dy = (e ? a.w : a.z) + ny.x, dz = (e ? b.y : b.x) + nz.x;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float rinv = rsqrt_hw(r2), q = rinv * rinv, tq = q * rinv;
+        const EpsTerms f = eps_terms(dx, dy, dz, fmaf(K.kap, tq, rinv), fmaf(-K.two_a2, tq, rinv), q);
+        float cn, rn;
+        rpy_near(K, r2, rinv, cn, rn);
+        const EpsTerms n = eps_terms(dx, dy, dz, cn, rn, q);
+        sx.x += n.bx - f.bx;
+        sy.x += n.by - f.by;
+        sz.x += n.bz - f.bz;
+        sa.x += n.a2 - f.a2;
+        sw.x += n.w - f.w;
+    }
+    __device__ __forceinline__ float4 sum() const {
+        const float A = sa.x + sa.y;
+        return make_float4(sx.x + sx.y + A, sy.x + sy.y + A, sz.x + sz.y + A, sw.x + sw.y);
+    }
+    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, int, float4 acc,
+                                           const TeaConst &K, float4 *) const {
+        eps_store(P, B, g, (B.flags[g] & kFlagExtra) == 0, acc, K);
+    }
+};
+
+// The mobility product (integrateTea_kernel_unlisted + integrateTea_force,
+// src/bdhitea_kernel.cu:104-213): f_i = F_i + C_i o R_i + sum_{j != i, non-extra}
+// T_ij (F_j + beta C_i o R_j), x_i += dt/gammaR f_i; angles by
+// Euler-Maruyama from stream i + nb, which is drawn for every bead.  Reads the
+// current frame, writes the next one.  With FEFF it stores f_i instead and moves nothing.
+template <bool FEFF>
+struct StepOp {
+    static constexpr int kWords = kTeaBlockF4;
+    float2 nx, ny, nz, cbx, cby, cbz;
+    float2 ax, ay, az;
+    __device__ __forceinline__ void start(const KParams &P, const DevBuffers &B, int traj, float4 p, int g,
+                                          bool valid) {
+        nx = f2(-p.x);
+        ny = f2(-p.y);
+        nz = f2(-p.z);
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid) {
+            const float beta = B.tea_beta[traj], b2 = beta * beta;
             const float4 ci = B.tea_ci[g];
             c = make_float4(beta / sqrtf(1.0f + b2 * ci.x), beta / sqrtf(1.0f + b2 * ci.y),
                             beta / sqrtf(1.0f + b2 * ci.z), 0.f);
         }
-        float2 *v[6] = {&nx[h >> 1], &ny[h >> 1], &nz[h >> 1], &cbx[h >> 1], &cby[h >> 1], &cbz[h >> 1]};
-        const float val[6] = {-p.x, -p.y, -p.z, c.x, c.y, c.z};
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            if (h & 1)
-                v[k]->y = val[k];
-            else
-                v[k]->x = val[k];
-        }
+        cbx = f2(c.x);
+        cby = f2(c.y);
+        cbz = f2(c.z);
+        ax = ay = az = f2(0.f);
     }
-#pragma unroll
-    for (int p = 0; p < kTeaPairsI; p++) ax[p] = ay[p] = az[p] = f2(0.f);
-    const TeaConst K = tea_const(P.tea_a);
-    const float2 vkap = f2(K.kap), vn2a2 = f2(-K.two_a2), one = f2(1.0f);
-    for (int j0 = jb; j0 < je; j0 += kTeaTile) {
-        tea_tile_load<true>(T, B, j0, end);
-        __syncthreads();
-        if (any_act) {
-            // the tile that holds this CTA's beads: bead h of this thread sits
-            // at tile index self_t + 32 h, and its self pair gets r^2 = 1e30
-            // (a far-away term that is below the rounding of the sums)
-            const bool self_tile = (w.y < j0 + kTeaTile) && (w.y + kTeaI > j0);
-            const int self_t = self_tile ? w.y - j0 + il : -(1 << 30);
-            float rmin[kTeaPairsI][kTeaSeg];
-#pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++)
-#pragma unroll
-                for (int sg = 0; sg < kTeaSeg; sg++) rmin[p][sg] = 3.4e38f;
-            if (self_tile)
-                tea_step_tile<SLICES, true>(T, sl, self_t, nx, ny, nz, cbx, cby, cbz, vkap, vn2a2, one, ax, ay, az,
-                                            rmin);
+    template <bool SELF>
+    __device__ __forceinline__ void pair(const TeaConst &K, const float4 *blk, int t, int sp, int se,
+                                         float &rm) {
+        const float2 vkap = f2(K.kap), vn2a2 = f2(-K.two_a2), one = f2(1.0f);
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t], c = blk[2 * kTeaPairSlots + t], d = blk[3 * kTeaPairSlots + t];
+        const float2 rz = reinterpret_cast<const float2 *>(blk + 4 * kTeaPairSlots)[t];
+        const float2 dx = __fadd2_rn(lo2(a), nx), dy = __fadd2_rn(hi2(a), ny), dz = __fadd2_rn(lo2(b), nz);
+        const float2 gx = __ffma2_rn(lo2(d), cbx, hi2(b)), gy = __ffma2_rn(hi2(d), cby, lo2(c)),
+                     gz = __ffma2_rn(rz, cbz, hi2(c));
+        float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        if (SELF && t == sp) {
+            if (se)
+                r2.y = 1e30f;
             else
-                tea_step_tile<SLICES, false>(T, sl, self_t, nx, ny, nz, cbx, cby, cbz, vkap, vn2a2, one, ax, ay, az,
-                                             rmin);
-            // overlapping pairs (r <= 2a): replace the far-field term by the near one
+                r2.x = 1e30f;
+        }
+        rm = fmin3(rm, r2.x, r2.y);
+        const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+        const float2 q = __fmul2_rn(rinv, rinv);
+        const float2 tq = __fmul2_rn(q, rinv);
+        const float2 cii = __ffma2_rn(vkap, tq, rinv);
+        const float2 cr = __fmul2_rn(tq, __ffma2_rn(vn2a2, q, one));
+        const float2 s = __fmul2_rn(cr, __ffma2_rn(dx, gx, __ffma2_rn(dy, gy, __fmul2_rn(dz, gz))));
+        ax = __ffma2_rn(cii, gx, __ffma2_rn(s, dx, ax));
+        ay = __ffma2_rn(cii, gy, __ffma2_rn(s, dy, ay));
+        az = __ffma2_rn(cii, gz, __ffma2_rn(s, dz, az));
+    }
+    __device__ __forceinline__ float2 dist2(const float4 *blk, int t) const {
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t];
+        const float2 dx = __fadd2_rn(lo2(a), nx), dy = __fadd2_rn(hi2(a), ny), dz = __fadd2_rn(lo2(b), nz);
+        return __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    }
+    __device__ __forceinline__ void near(const TeaConst &K, const float4 *blk, int t, int e) {
+        const float4 a = blk[t], b = blk[kTeaPairSlots + t], c = blk[2 * kTeaPairSlots + t], d = blk[3 * kTeaPairSlots + t];
+        const float2 rz = reinterpret_cast<const float2 *>(blk + 4 * kTeaPairSlots)[t];
+        const float dx = (e ? a.y : a.x) + nx.x, dy = (e ? a.w : a.z) + ny.x, dz = (e ? b.y : b.x) + nz.x;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float gx = fmaf(e ? d.y : d.x, cbx.x, e ? b.w : b.z), gy = fmaf(e ? d.w : d.z, cby.x, e ? c.y : c.x),
+                    gz = fmaf(e ? rz.y : rz.x, cbz.x, e ? c.w : c.z);
+        const float3 fa = tea_far1(K, dx, dy, dz, gx, gy, gz);
+        const float3 nr = tea_pair1(K, dx, dy, dz, gx, gy, gz);
+        ax.x += nr.x - fa.x;
+        ay.x += nr.y - fa.y;
+        az.x += nr.z - fa.z;
+    }
+    __device__ __forceinline__ float4 sum() const {
+        return make_float4(ax.x + ax.y, ay.x + ay.y, az.x + az.y, 0.f);
+    }
+    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, int traj, float4 acc,
+                                           const TeaConst &K, float4 *feff) const {
+        const float beta = B.tea_beta[traj];
+        tea_bead_update<FEFF>(P, B, g, acc.x, acc.y, acc.z, beta * beta, K, feff);
+    }
+};
+
+// Run k of a launch: units [k U / G, (k + 1) U / G).
+__device__ __forceinline__ long long tea_run_start(long long units, int runs, int k) { return k * units / runs; }
+
+// The item that holds unit u: the last of unit0[0 .. nwork - 1] that is <= u, by a
+// 32-way search (each round is one dependent load instead of five).
+__device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, long long u) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, n = nwork;
+    while (n > 1) {
+        const int step = (n + 31) / 32, k = lo + lane * step;
+        const bool le = lane * step < n && unit0[k] <= u;
+        const int last = 31 - __clz((int)__ballot_sync(0xffffffffu, le));   // lane 0 always is
+        n = min(step, n - last * step);
+        lo += last * step;
+    }
+    return lo;
+}
+
+// Runs while gate is null or *gate == run_if.
+template <class Op>
+__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
+                                                             float4 *feff, const int *gate, int run_if) {
+    if (gate && *gate != run_if) return;
+    constexpr int kW = Op::kWords;
+    __shared__ float4 s_tile[kTeaStages][kTeaTileBlocks * kW];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long U = P.tea_units;
+    const int G = gridDim.x;
+    long long u = tea_run_start(U, G, blockIdx.x);
+    const long long u_end = tea_run_start(U, G, blockIdx.x + 1);
+    int item = tea_find_item(B.tea_unit0, nwork, u);
+    const TeaConst K = tea_const(P.tea_a);
+    while (u < u_end) {
+        const long long first = B.tea_unit0[item];
+        const int nblk = (int)(B.tea_unit0[item + 1] - first);
+        const int b0 = (int)(u - first), b1 = (int)min((long long)nblk, u_end - first);
+        const int2 w = work[item];
+        const int traj = w.x, g = w.y + tid;
+        const float4 *pack = B.tea_pack + (size_t)B.tea_blk0[traj] * kTeaBlockF4;
+        auto issue = [&](int tile) {
+            const int q0 = b0 + tile * kTeaTileBlocks, nq = min(kTeaTileBlocks, b1 - q0);
+            float4 *dst = s_tile[tile % kTeaStages];
+            for (int c = tid; c < nq * kW; c += kTeaThreads)
+                cp_async16(dst + c, pack + (size_t)(q0 + c / kW) * kTeaBlockF4 + c % kW);
+        };
+        const int ntiles = (b1 - b0 + kTeaTileBlocks - 1) / kTeaTileBlocks;
 #pragma unroll
-            for (int p = 0; p < kTeaPairsI; p++) {
-                unsigned segs = 0;
-#pragma unroll
-                for (int sg = 0; sg < kTeaSeg; sg++) segs |= (rmin[p][sg] <= K.four_a2 ? 1u : 0u) << sg;
-                constexpr int kLen = kTeaTile / SLICES / kTeaSeg;
-                while (segs) {  // the segments that hold an overlapping pair
-                    const int sg = __ffs(segs) - 1;
-                    segs &= segs - 1;
-                    for (int k = 0; k < kLen; k++) {
-                        const int t = sl + (sg * kLen + k) * SLICES;
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            if (t == self_t + kTeaLanes * (2 * p + e)) continue;
-                            const float dx = T.xy[t].x + (e ? nx[p].y : nx[p].x),
-                                        dy = T.xy[t].z + (e ? ny[p].y : ny[p].x),
-                                        dz = T.zf[t].x + (e ? nz[p].y : nz[p].x);
-                            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            if (!(r2 <= K.four_a2)) continue;
-                            const float gx = fmaf(T.rxy[t].x, e ? cbx[p].y : cbx[p].x, T.zf[t].z),
-                                        gy = fmaf(T.rxy[t].z, e ? cby[p].y : cby[p].x, T.fyz[t].x),
-                                        gz = fmaf(T.rz[t].x, e ? cbz[p].y : cbz[p].x, T.fyz[t].z);
-                            const float3 fa = tea_far1(K, dx, dy, dz, gx, gy, gz);
-                            const float3 nr = tea_pair1(K, dx, dy, dz, gx, gy, gz);
-                            if (e) {
-                                ax[p].y += nr.x - fa.x;
-                                ay[p].y += nr.y - fa.y;
-                                az[p].y += nr.z - fa.z;
-                            } else {
-                                ax[p].x += nr.x - fa.x;
-                                ay[p].x += nr.y - fa.y;
-                                az[p].x += nr.z - fa.z;
-                            }
-                        }
+        for (int k = 0; k < kTeaStages - 1; k++) {
+            if (k < ntiles) issue(k);
+            cp_async_commit();
+        }
+        const bool valid = g < B.off[traj + 1];
+        const float4 p = valid ? B.frame_in[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool act = __any_sync(0xffffffffu, valid && !(B.flags[g] & kFlagExtra));
+        Op X;
+        X.start(P, B, traj, p, g, valid);
+        const int self = (w.y - B.off[traj]) / kTeaBlock + warp;   // the block that holds this warp's beads
+        for (int tile = 0; tile < ntiles; tile++) {
+            cp_async_wait<kTeaStages - 2>();
+            __syncthreads();
+            if (tile + kTeaStages - 1 < ntiles) issue(tile + kTeaStages - 1);
+            cp_async_commit();
+            if (!act) continue;
+            const int q0 = b0 + tile * kTeaTileBlocks, nq = min(kTeaTileBlocks, b1 - q0);
+            for (int q = 0; q < nq; q++) {
+                const float4 *blk = s_tile[tile % kTeaStages] + q * kW;
+                const bool own = q0 + q == self;
+                float rm = 3.4e38f;
+                if (own) {
+#pragma unroll 1
+                    for (int t = 0; t < kTeaPairSlots; t++) X.template pair<true>(K, blk, t, lane >> 1, lane & 1, rm);
+                } else {
+#pragma unroll 8
+                    for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
+                }
+                if (rm <= K.four_a2) {   // which beads of the block overlap, then their terms
+                    unsigned near = 0;
+#pragma unroll 4
+                    for (int t = 0; t < kTeaPairSlots; t++) {
+                        const float2 r2 = X.dist2(blk, t);
+                        near |= (r2.x <= K.four_a2 ? 1u : 0u) << (2 * t) | (r2.y <= K.four_a2 ? 2u : 0u) << (2 * t);
+                    }
+                    if (own) near &= ~(1u << lane);
+                    for (; near; near &= near - 1) {
+                        const int j = __ffs((int)near) - 1;
+                        X.near(K, blk, j >> 1, j & 1);
                     }
                 }
             }
         }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        const int p = h >> 1;
-        const bool hi = h & 1;
-        s_red[(sl * kTeaNI + h) * kTeaLanes + il] =
-            make_float4(hi ? ax[p].y : ax[p].x, hi ? ay[p].y : ay[p].x, hi ? az[p].y : az[p].x, 0.f);
-    }
-    __syncthreads();
-    if (sl != 0) return;
-#pragma unroll
-    for (int h = 0; h < kTeaNI; h++) {
-        const int g = w.y + il + h * kTeaLanes;
-        if (g >= end) continue;
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-        for (int k = 0; k < SLICES; k++) {
-            const float4 v = s_red[(k * kTeaNI + h) * kTeaLanes + il];
-            sx += v.x;
-            sy += v.y;
-            sz += v.z;
+        float4 acc = X.sum();
+        bool done = true;
+        __syncthreads();   // the tiles are free again (and s_last)
+        if (b0 > 0 || b1 < nblk) {
+            // part of the item: slot 0 of the run for an item begun before it, slot 1 for one it begins
+            B.tea_part[((size_t)blockIdx.x * 2 + (b0 > 0 ? 0 : 1)) * kTeaI + tid] = acc;
+            const int k0 = (int)(((first + 1) * G - 1) / U), k1 = (int)(((first + nblk) * G - 1) / U);
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(&B.tea_cnt[item], 1) == k1 - k0;
+            __syncthreads();
+            done = s_last;
+            if (done) {
+                __threadfence();
+                acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int k = k0; k <= k1; k++) {
+                    const int slot = tea_run_start(U, G, k) > first ? 0 : 1;
+                    const float4 q = __ldcg(&B.tea_part[((size_t)k * 2 + slot) * kTeaI + tid]);
+                    acc = make_float4(acc.x + q.x, acc.y + q.y, acc.z + q.z, acc.w + q.w);
+                }
+                if (tid == 0) B.tea_cnt[item] = 0;
+            }
         }
-        if (SPLIT && parts > 1)
-            B.tea_part[(size_t)part * nb + g] = make_float4(sx, sy, sz, 0.f);
-        else
-            tea_bead_update<FEFF>(P, B, g, sx, sy, sz, b2, K, feff);
+        if (done && valid) X.finish(P, B, g, traj, acc, K, feff);
+        u = first + b1;
+        item++;
     }
 }
 
-// Sums of the parts of a split mobility product, then the bead's update.
-template <bool FEFF>
-__global__ void k_tea_step_finish(KParams P, DevBuffers B, const int2 *work, float4 *feff, const int *gate) {
-    if (FEFF && gate && *gate != 0) return;
-    if (!FEFF && gate && *gate == 0) return;
-    const int g = tea_tail_bead(P, B, work);
-    if (g < 0) return;
-    float4 acc = B.tea_part[g];
-    for (int k = 1; k < P.tea_jparts; k++) {
-        const float4 v = B.tea_part[(size_t)k * P.nb + g];
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-    }
-    const float beta = B.tea_beta[B.traj[g]];
-    tea_bead_update<FEFF>(P, B, g, acc.x, acc.y, acc.z, beta * beta, tea_const(P.tea_a), feff);
+// Positions of every bead into the pack (the force kernel of a TEA step does
+// it with F and R; this one serves epsilon passes outside a step).
+__global__ void k_tea_pack(KParams P, DevBuffers B) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= P.nb) return;
+    const bool extra = (B.flags[g] & kFlagExtra) != 0;
+    const float4 p = B.frame_in[g];
+    tea_pack_position(B, g, extra ? make_float3(kTeaFarAway, kTeaFarAway, kTeaFarAway) : make_float3(p.x, p.y, p.z));
+}
+// An empty pack: every slot far away with zero F and R.
+__global__ void k_tea_pack_clear(float4 *pack, int nblocks) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nblocks * kTeaBlockF4) return;
+    const int w = k % kTeaBlockF4;
+    const float a = w < 2 * kTeaPairSlots ? kTeaFarAway : 0.f, b = w < kTeaPairSlots ? kTeaFarAway : 0.f;
+    pack[k] = make_float4(a, a, b, b);
 }
 
-// CTAs of kernel k that fit on the device at once.
-template <typename Kern>
-static int tea_slots(Kern k, int threads) {
+// Runs of a launch: one CTA each, as many as the device holds at once, but no
+// item cut into more than about 16 (their sums meet in one CTA).
+template <class Op>
+static int tea_runs(const KParams &P) {
     int dev = 0, sms = 1, occ = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, 0);
-    return (occ > 0 ? occ : 1) * sms;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tea_pass<Op>, kTeaThreads, 0);
+    const long long slots = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
+    const long long least = (P.tea_max_blocks + 15) / 16, runs = (P.tea_units + least - 1) / least;
+    return (int)(runs < slots ? runs : slots);
 }
-// Items run whole: all but the last one to two waves' worth; grid of the launch.
-static int tea_split_grid(KParams &Q, int nwork, int slots) {
-    const int full = nwork / slots;
-    Q.tea_nhead = full >= 2 ? (full - 1) * slots : 0;
-    return Q.tea_nhead + (nwork - Q.tea_nhead) * Q.tea_jparts;
+template <class Op>
+static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
+                       int run_if, cudaStream_t s) {
+    k_tea_pass<Op><<<tea_runs<Op>(P), kTeaThreads, 0, s>>>(P, B, work, nwork, feff, gate, run_if);
 }
-
-template <int SL>
-static void tea_eps_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
-                           int run_if, cudaStream_t s) {
-    const int t = kTeaLanes * SL;
-    KParams Q = P;
-    if (P.tea_jparts > 1) {
-        const int grid = tea_split_grid(Q, nwork, tea_slots(k_tea_eps<SL, true>, t));
-        k_tea_eps<SL, true><<<grid, t, 0, s>>>(Q, B, work, gate, run_if);
-        if (nwork > Q.tea_nhead) k_tea_eps_finish<<<nwork - Q.tea_nhead, kTeaChunk, 0, s>>>(Q, B, work, gate, run_if);
-        return;
-    }
-    Q.tea_nhead = nwork;
-    k_tea_eps<SL, false><<<nwork, t, 0, s>>>(Q, B, work, gate, run_if);
+void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
+    k_tea_pack<<<(P.nb + 127) / 128, 128, 0, s>>>(P, B);
+}
+void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s) {
+    k_tea_pack_clear<<<(int)(((size_t)nblocks * kTeaBlockF4 + 255) / 256), 256, 0, s>>>(pack, nblocks);
 }
 void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                           int run_if, cudaStream_t s) {
-    switch (P.tea_slices) {
-        case 1: tea_eps_launch<1>(P, B, work, nwork, gate, run_if, s); break;
-        case 2: tea_eps_launch<2>(P, B, work, nwork, gate, run_if, s); break;
-        case 4: tea_eps_launch<4>(P, B, work, nwork, gate, run_if, s); break;
-        default: tea_eps_launch<8>(P, B, work, nwork, gate, run_if, s); break;
-    }
+    tea_launch<EpsOp>(P, B, work, nwork, nullptr, gate, run_if, s);
 }
 void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
     launch_tea_eps_gated(P, B, work, nwork, nullptr, 0, s);
@@ -708,47 +548,22 @@ void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s) {
     launch_tea_beta_gated(P, B, capricious, epsmax, nullptr, 0, s);
 }
-template <int SL, bool FEFF>
-static void tea_step_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
-                            const int *gate, cudaStream_t s) {
-    const int t = kTeaLanes * SL;
-    KParams Q = P;
-    if (P.tea_jparts > 1) {
-        const int grid = tea_split_grid(Q, nwork, tea_slots(k_tea_step<SL, FEFF, true>, t));
-        k_tea_step<SL, FEFF, true><<<grid, t, 0, s>>>(Q, B, work, feff, gate);
-        if (nwork > Q.tea_nhead) k_tea_step_finish<FEFF><<<nwork - Q.tea_nhead, kTeaChunk, 0, s>>>(Q, B, work, feff, gate);
-        return;
-    }
-    Q.tea_nhead = nwork;
-    k_tea_step<SL, FEFF, false><<<nwork, t, 0, s>>>(Q, B, work, feff, gate);
-}
-template <bool FEFF>
-static void tea_step_dispatch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
-                              const int *gate, cudaStream_t s) {
-    switch (P.tea_slices) {
-        case 1: tea_step_launch<1, FEFF>(P, B, work, nwork, feff, gate, s); break;
-        case 2: tea_step_launch<2, FEFF>(P, B, work, nwork, feff, gate, s); break;
-        case 4: tea_step_launch<4, FEFF>(P, B, work, nwork, feff, gate, s); break;
-        default: tea_step_launch<8, FEFF>(P, B, work, nwork, feff, gate, s); break;
-    }
-}
 void launch_tea_step(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
-    tea_step_dispatch<false>(P, B, work, nwork, nullptr, nullptr, s);
+    tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, nullptr, 0, s);
 }
 void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                            cudaStream_t s) {
-    tea_step_dispatch<false>(P, B, work, nwork, nullptr, gate, s);
+    tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, gate, 1, s);
 }
 void launch_tea_feff(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
                      const int *gate, cudaStream_t s) {
-    tea_step_dispatch<true>(P, B, work, nwork, feff, gate, s);
+    tea_launch<StepOp<true>>(P, B, work, nwork, feff, gate, 0, s);
 }
 
 // ---------------------------------------------- far field of learned TEA
 // The learned mode's approximation of sum_j T_ij (F_j + beta C_i o R_j) on a
 // k-d tree per trajectory (tea_ff.cu): pairs of beads in near leaves are
-// summed exactly (the packed pair loop of k_tea_step, source beads in the two
-// lanes), and every far node J acts on a target node N through proxies: J's
+// summed exactly (the packed pair loop of the all-pairs pass), and every far node J acts on a target node N through proxies: J's
 // sources are spread onto the 8 points of a Chebyshev grid in its bounding box
 // (P2M, trilinear Lagrange weights at nodes +-h/sqrt(2)), the RPY far field
 // of those 8 charges is evaluated at the 8 grid points of N (M2L), brought
@@ -769,14 +584,6 @@ struct FFTile {
     float4 rxy[kFFTileSlots];  // Rxa Rxb Rya Ryb
     float2 rz[kFFTileSlots];   // Rza Rzb
 };
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Near-list entries a step CTA keeps in shared memory (longer lists are read
 // from global memory).

@@ -5,6 +5,7 @@
 // (one graph per pair-list period and frame-buffer parity), device error
 // words read back once per call instead of a device synchronisation after
 // every launch (the reference's checkCUDAError, src/Cuda.h:120-135).
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstdarg>
@@ -493,20 +494,32 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     for (int tr = 0; tr < nt; tr++)
         for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kListThreads) list_work.push_back(make_int2(tr, g));
     e->list_nwork = (int)list_work.size();
+    // all-pairs TEA kernels: chunks of kTeaChunk beads i, blocks of kTeaBlock
+    // beads j, a chunk's units = the blocks of its trajectory
     std::vector<int2> tea_work;
-    for (int tr = 0; tr < nt; tr++)
-        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) tea_work.push_back(make_int2(tr, g));
+    std::vector<int> tea_slot(nb), tea_blk0(nt + 1);
+    std::vector<long long> tea_unit0{0};
+    for (int tr = 0; tr < nt; tr++) {
+        const int n = t->offsets[tr + 1] - t->offsets[tr], nblk = (n + kTeaBlock - 1) / kTeaBlock;
+        tea_blk0[tr + 1] = tea_blk0[tr] + nblk;
+        e->kp.tea_max_blocks = std::max(e->kp.tea_max_blocks, nblk);
+        for (int i = 0; i < n; i++) tea_slot[t->offsets[tr] + i] = tea_blk0[tr] * kTeaBlock + i;
+        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) {
+            tea_work.push_back(make_int2(tr, g));
+            tea_unit0.push_back(tea_unit0.back() + nblk);
+        }
+    }
     e->tea_nwork = (int)tea_work.size();
-    // threads per bead in the all-pairs TEA kernels: enough to fill the GPU
+    e->kp.tea_units = tea_unit0.back();
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    // threads per bead in the near-pair kernel of learned TEA: enough to fill the GPU
     {
-        int dev = p->device, sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         // two beads per thread; aim for about two full waves at 64 registers
         const double target = (double)sms * 2048.0;
         int sl = 1;
         while (sl < 8 && (double)nb / 4 * sl < target) sl <<= 1;   // four beads per thread
         e->kp.tea_slices = sl;
-        e->kp.tea_jparts = 1;
     }
 
 #define ALLOC(ptr, n)                         \
@@ -552,7 +565,12 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         ALLOC(e->tea_eps, nb);
         ALLOC(e->tea_beta, nt);
         ALLOC(e->tea_eps_t, nt);
-        ALLOC(e->tea_part, (size_t)kTeaMaxParts * nb);
+        ALLOC(e->tea_pack, (size_t)kTeaBlockF4 * tea_blk0[nt]);
+        ALLOC(e->tea_slot, nb);
+        ALLOC(e->tea_blk0, nt + 1);
+        ALLOC(e->tea_unit0, e->tea_nwork + 1);
+        ALLOC(e->tea_part, (size_t)2 * kTeaChunk * std::min<long long>(e->kp.tea_units, (long long)kTeaMaxOcc * sms));
+        ALLOC(e->tea_cnt, e->tea_nwork);
     }
     // spatial-hash tables of the cell-list rebuild
     std::vector<int> tbase(nt + 1, 0), tmask(nt, 0);
@@ -605,10 +623,15 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     cudaMemsetAsync(e->latc, 0, sizeof(int) * nb, s);
     cudaMemsetAsync(e->force, 0, sizeof(float4) * 2 * nb, s);
     if (p->hdi_on) {
-        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int2) * tea_work.size(), s)) != 0) {
+        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int2) * tea_work.size(), s)) ||
+            (rc = upload(e->tea_slot, tea_slot.data(), sizeof(int) * nb, s)) ||
+            (rc = upload(e->tea_blk0, tea_blk0.data(), sizeof(int) * (nt + 1), s)) ||
+            (rc = upload(e->tea_unit0, tea_unit0.data(), sizeof(long long) * tea_unit0.size(), s))) {
             mtg_destroy(e);
             return rc;
         }
+        cudaMemsetAsync(e->tea_cnt, 0, sizeof(int) * e->tea_nwork, s);
+        launch_tea_pack_clear(e->tea_pack, tea_blk0[nt], s);
         cudaMemsetAsync(e->tea_ci, 0, sizeof(float4) * nb, s);
         cudaMemsetAsync(e->tea_beta, 0, sizeof(float) * nt, s);
     }
@@ -720,7 +743,7 @@ int mtg_destroy(mtg_engine *e) {
                     e->surr_desc, e->surr_pred, e->surr_stats, e->surr_gate, e->surr_err, e->surr_part,
                     e->tea_ci2, e->feff_a, e->feff_b, e->tea_eps2, e->tea_beta2, e->tea_eps_t2,
                     e->hydro_cand, e->hydro_rank, e->hydro_sums, e->hydro_counts, e->hydro_events,
-                    e->tea_part};
+                    e->tea_pack, e->tea_slot, e->tea_blk0, e->tea_unit0, e->tea_part, e->tea_cnt};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (e->stage_host) cudaFreeHost(e->stage_host);
@@ -1046,7 +1069,7 @@ int mtg_get_tuning(mtg_engine *e, mtg_tuning *t) {
     t->list_method = e->use_cells ? 2 : 1;
     t->step_block = e->kp.step_block;
     t->tea_slices = e->kp.tea_slices;
-    t->tea_jparts = e->kp.tea_jparts;
+    t->tea_jparts = e->tea_jparts;
     t->plain_persistent = e->persistent ? 1 : 0;
     return MTG_OK;
 }
@@ -1072,7 +1095,7 @@ int mtg_set_tuning(mtg_engine *e, const mtg_tuning *t) {
     e->persistent = t->plain_persistent != 0;
     e->kp.step_block = t->step_block;
     e->kp.tea_slices = t->tea_slices;
-    e->kp.tea_jparts = t->tea_jparts;
+    e->tea_jparts = t->tea_jparts;
     destroy_graphs(e);
     return MTG_OK;
 }
@@ -1098,8 +1121,12 @@ int mtg_autotune(mtg_engine *e, long long first_step, int trial_steps, mtg_tunin
         if (lm == 2 && (!cells_ok || !lists)) continue;
         if (lm == 1 && !lists && !cands.empty()) continue;
         if (e->p.hdi_on) {
-            for (int sl : {1, 2, 4, 8})
-                for (int jp = 1; jp <= kTeaMaxParts; jp++) cands.push_back({lm, orig.step_block, sl, jp, 0});
+            // the all-pairs kernels divide their work themselves; threads per bead
+            // matter to the near pairs of the learned mode alone
+            if (e->surr && e->ff_on)
+                for (int sl : {2, 4, 8}) cands.push_back({lm, orig.step_block, sl, orig.tea_jparts, 0});
+            else
+                cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 0});
         } else {
             for (int bs : {64, 128, 256}) cands.push_back({lm, bs, orig.tea_slices, orig.tea_jparts, 0});
             if (period_fits(e->max_traj_beads)) cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 1});
@@ -1205,6 +1232,7 @@ int mtg_tea_update(mtg_engine *e, double *eps_out, float *beta_out, float *ci_ou
     cudaSetDevice(e->device);
     if (!e->p.hdi_on) return fail(MTG_E_STATE, "engine created without hdi_on");
     if (!e->have_state) return fail(MTG_E_STATE, "no state uploaded");
+    launch_tea_pack(e->kp, e->bufs(), e->stream);
     launch_tea_eps(e->kp, e->bufs(), e->tea_work, e->tea_nwork, e->stream);
     launch_tea_beta(e->kp, e->bufs(), e->p.tea_capricious, e->p.tea_epsmax, e->stream);
     CK(cudaGetLastError());

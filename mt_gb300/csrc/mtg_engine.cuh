@@ -41,7 +41,10 @@ struct mtg_engine {
     float4 *tea_r = nullptr, *tea_ci = nullptr;
     float *tea_eps = nullptr, *tea_beta = nullptr;
     double *tea_eps_t = nullptr;
-    float4 *tea_part = nullptr;    // kTeaMaxParts * nb partial sums (split TEA kernels)
+    float4 *tea_pack = nullptr, *tea_part = nullptr;   // all-pairs TEA kernels, see DevBuffers
+    int *tea_slot = nullptr, *tea_blk0 = nullptr, *tea_cnt = nullptr;
+    long long *tea_unit0 = nullptr;
+    int tea_jparts = 1;            // as set (no effect any more)
     float *stage = nullptr;        // 7*nb floats for host <-> device Coord transfers
     void *stage_host = nullptr;    // pinned mirror of stage
     uint8_t *stage_u8 = nullptr;
@@ -141,7 +144,12 @@ struct mtg_engine {
         b.latc = latc;
         b.lat = lat;
         b.err = err;
+        b.tea_pack = tea_pack;
+        b.tea_slot = tea_slot;
+        b.tea_blk0 = tea_blk0;
+        b.tea_unit0 = tea_unit0;
         b.tea_part = tea_part;
+        b.tea_cnt = tea_cnt;
         b.tea_r = tea_r;
         b.tea_ci = tea_ci;
         b.tea_eps = tea_eps;

@@ -60,9 +60,9 @@ struct KParams {
     int maxH, maxLong, maxLat, maxLJ;
     // TEA
     float tea_a, tea_var;
-    int tea_slices;        // threads per bead i in the all-pairs TEA kernels (1, 2, 4 or 8)
-    int tea_jparts;        // parts of a split work item's j range (1..kTeaMaxParts), summed by a second kernel
-    int tea_nhead;         // work items run whole before the split tail (set by the TEA launchers)
+    int tea_slices;        // threads per bead in the near-pair kernel of learned TEA (1, 2, 4 or 8)
+    int tea_max_blocks;    // blocks of kTeaBlock beads of the largest trajectory
+    long long tea_units;   // (chunk of kTeaChunk beads) x (block) pairs of the all-pairs kernels
     int step_block;        // threads per CTA of the fused plain step (64, 128 or 256)
 };
 
@@ -86,7 +86,13 @@ struct DevBuffers {
     float *tea_eps;        // per-bead epsilon sums
     float *tea_beta;       // [nt]
     double *tea_eps_t;     // [nt]
-    float4 *tea_part;      // [kTeaMaxParts][nb] partial sums of the split all-pairs kernels
+    // all-pairs kernels (kernels_tea.cu)
+    float4 *tea_pack;      // every trajectory's beads in blocks, see tea_pack_bead
+    const int *tea_slot;   // [nb] slot of each bead in the pack (32 a block)
+    const int *tea_blk0;   // [nt] first block of each trajectory
+    const long long *tea_unit0;  // [work items + 1] first unit of each item
+    float4 *tea_part;      // partial sums: two slots of kTeaChunk beads per CTA of a launch
+    int *tea_cnt;          // [work items] CTAs of an item that have left their partial sums (0 between launches)
 };
 
 // ------------------------------------------------------------------ RNG
@@ -296,6 +302,44 @@ __device__ __forceinline__ void list_append(const KParams &P, const DevBuffers &
     }
 }
 
+// ------------------------------------------------------------- TEA pack
+// Beads of a trajectory in blocks of 32, the pairs (2p, 2p + 1) of a block in
+// the order the all-pairs loop reads them (float4 words, kTeaPairSlots each):
+//   xa xb ya yb | za zb Fxa Fxb | Fya Fyb Fza Fzb | Rxa Rxb Rya Ryb,
+// then Rza Rzb of two pairs a word.
+constexpr int kTeaBlock = 32;
+constexpr int kTeaPairSlots = kTeaBlock / 2;
+constexpr int kTeaBlockF4 = 4 * kTeaPairSlots + kTeaPairSlots / 2;
+constexpr float kTeaFarAway = 1.0e18f;     // where extra beads and padding are, with zero F and R
+__device__ __forceinline__ float *tea_pack_at(const DevBuffers &B, int g, int &p, int &odd) {
+    const int slot = B.tea_slot[g], l = slot % kTeaBlock;
+    p = l >> 1;
+    odd = l & 1;
+    return reinterpret_cast<float *>(B.tea_pack + (size_t)(slot / kTeaBlock) * kTeaBlockF4);
+}
+__device__ __forceinline__ void tea_pack_position(const DevBuffers &B, int g, float3 x) {
+    int p, odd;
+    float *b = tea_pack_at(B, g, p, odd);
+    b[4 * p + odd] = x.x;
+    b[4 * p + 2 + odd] = x.y;
+    b[4 * kTeaPairSlots + 4 * p + odd] = x.z;
+}
+__device__ __forceinline__ void tea_pack_bead(const DevBuffers &B, int g, bool extra, float4 pos, float fx, float fy,
+                                              float fz, float4 r) {
+    int p, odd;
+    float *b = tea_pack_at(B, g, p, odd) + 4 * p + odd;
+    constexpr int n = 4 * kTeaPairSlots;
+    b[0] = extra ? kTeaFarAway : pos.x;
+    b[2] = extra ? kTeaFarAway : pos.y;
+    b[n] = extra ? kTeaFarAway : pos.z;
+    b[n + 2] = extra ? 0.f : fx;
+    b[2 * n] = extra ? 0.f : fy;
+    b[2 * n + 2] = extra ? 0.f : fz;
+    b[3 * n] = extra ? 0.f : r.x;
+    b[3 * n + 2] = extra ? 0.f : r.y;
+    (b - 2 * p)[4 * n] = extra ? 0.f : r.z;
+}
+
 // 1/sqrt(x) as the single hardware approximation instruction (a few ulp);
 // pair distances are never subnormal, so the flush-to-zero form gives the
 // same value for them without a subnormal fix-up.
@@ -388,7 +432,11 @@ void launch_energy_totals(const KParams &P, const double *partials, const int *w
                           int *err, cudaStream_t s);
 // TEA kernels run over their own work list: chunks of kTeaChunk beads.
 constexpr int kTeaChunk = 128;
-constexpr int kTeaMaxParts = 4;
+constexpr int kTeaMaxParts = 4;      // largest mtg_tuning::tea_jparts that is accepted
+constexpr int kTeaMaxOcc = 12;       // CTAs of the all-pairs kernels per SM at most (sizes tea_part)
+// positions (F and R are zeroed once) into the pack, for epsilon passes outside a TEA step
+void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s);
+void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s);
 void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s);
 void launch_tea_step(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);

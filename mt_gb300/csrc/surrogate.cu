@@ -635,6 +635,7 @@ int mtg_tea_training_data(mtg_engine *e, float *X, float *T) {
     k_descriptors<<<e->nwork, kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv, e->surr_stats, e->surr_desc,
                                                      nullptr);
     if (T) {
+        launch_tea_pack(e->kp, B, e->stream);
         launch_tea_eps(e->kp, B, e->tea_work, e->tea_nwork, e->stream);
         launch_tea_beta(e->kp, B, e->p.tea_capricious, e->p.tea_epsmax, e->stream);
         k_tea_targets<<<(e->nb + 255) / 256, 256, 0, e->stream>>>(e->kp, B, e->surr_pred);
