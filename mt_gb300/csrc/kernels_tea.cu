@@ -17,8 +17,10 @@
 //     CTAs an SM (two beads a thread load half as many words but leave six CTAs:
 //     1.82 against 1.76 ms).
 //   * The work of a launch is the list of units (128 beads i) x (one block of
-//     j), cut into equal contiguous runs, one CTA each, as many as the GPU holds
-//     at once: no last wave is partly filled, whatever the sizes.  A run
+//     j), cut into equal contiguous runs, one CTA each, four for every CTA the
+//     GPU holds at once, so the last ones to finish are short whatever the
+//     sizes.  (One each: an SM's schedulers favour their older warps, which leave
+//     the younger ones alone at the end, 1.72 against 1.66 ms.)  A run
 //     that does not hold all units of its 128 beads leaves its partial sums, and the CTA
 //     that comes last (an atomic count; nothing waits) adds them in run order and
 //     finishes the beads, so the result does not depend on the timing.
@@ -28,8 +30,8 @@
 // the block that holds a bead itself its own pair gets r^2 = 1e30: its term is
 // then far below the rounding of the sums, and the correction skips it.
 // Sums are kept in units of 0.75 a (T' = T / (0.75 a)).
-// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.72 ms (52 TFLOP/s of the measured 80;
-// the FMA pipe is 72% active), 16 x 3300 205 -> 168 us, one trajectory of 299 25 -> 14 us (before: a tile stored twice by
+// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.66 ms (54 TFLOP/s of the measured 80;
+// the FMA pipe is 75% active), 16 x 3300 205 -> 168 us, one trajectory of 299 25 -> 14 us (before: a tile stored twice by
 // every CTA, whole 128-bead items in 3.7 waves or a second kernel for split ones).
 #include "mtg_internal.cuh"
 
@@ -373,6 +375,23 @@ struct StepOp {
     }
 };
 
+// The overlapping beads of a block (own: the bead of this lane is one of it, in
+// slot lane): which they are, then their terms.
+template <class Op>
+__device__ __forceinline__ void tea_near_block(Op &X, const TeaConst &K, const float4 *blk, bool own, int lane) {
+    unsigned near = 0;
+#pragma unroll 4
+    for (int t = 0; t < kTeaPairSlots; t++) {
+        const float2 r2 = X.dist2(blk, t);
+        near |= (r2.x <= K.four_a2 ? 1u : 0u) << (2 * t) | (r2.y <= K.four_a2 ? 2u : 0u) << (2 * t);
+    }
+    if (own) near &= ~(1u << lane);
+    for (; near; near &= near - 1) {
+        const int j = __ffs((int)near) - 1;
+        X.near(K, blk, j >> 1, j & 1);
+    }
+}
+
 // Run k of a launch: units [k U / G, (k + 1) U / G).
 __device__ __forceinline__ long long tea_run_start(long long units, int runs, int k) { return k * units / runs; }
 
@@ -449,19 +468,7 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
 #pragma unroll 8
                     for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
                 }
-                if (rm <= K.four_a2) {   // which beads of the block overlap, then their terms
-                    unsigned near = 0;
-#pragma unroll 4
-                    for (int t = 0; t < kTeaPairSlots; t++) {
-                        const float2 r2 = X.dist2(blk, t);
-                        near |= (r2.x <= K.four_a2 ? 1u : 0u) << (2 * t) | (r2.y <= K.four_a2 ? 2u : 0u) << (2 * t);
-                    }
-                    if (own) near &= ~(1u << lane);
-                    for (; near; near &= near - 1) {
-                        const int j = __ffs((int)near) - 1;
-                        X.near(K, blk, j >> 1, j & 1);
-                    }
-                }
+                if (rm <= K.four_a2) tea_near_block(X, K, blk, own, lane);
             }
         }
         float4 acc = X.sum();
@@ -511,22 +518,24 @@ __global__ void k_tea_pack_clear(float4 *pack, int nblocks) {
     pack[k] = make_float4(a, a, b, b);
 }
 
-// Runs of a launch: one CTA each, as many as the device holds at once, but no
-// item cut into more than about 16 (their sums meet in one CTA).
+// Runs of a launch, one CTA each: kTeaRunsPerSlot for every CTA that fits the device, but
+// no item cut into more than about 16 (their sums meet in one CTA).  rare: a
+// launch that mostly finds its gate closed, which should be short then.
 template <class Op>
-static int tea_runs(const KParams &P) {
+static int tea_runs(const KParams &P, bool rare) {
     int dev = 0, sms = 1, occ = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tea_pass<Op>, kTeaThreads, 0);
-    const long long slots = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
+    long long slots = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
+    if (!rare) slots *= kTeaRunsPerSlot;
     const long long least = (P.tea_max_blocks + 15) / 16, runs = (P.tea_units + least - 1) / least;
     return (int)(runs < slots ? runs : slots);
 }
 template <class Op>
 static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
                        int run_if, cudaStream_t s) {
-    k_tea_pass<Op><<<tea_runs<Op>(P), kTeaThreads, 0, s>>>(P, B, work, nwork, feff, gate, run_if);
+    k_tea_pass<Op><<<tea_runs<Op>(P, gate && run_if == 1), kTeaThreads, 0, s>>>(P, B, work, nwork, feff, gate, run_if);
 }
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
     k_tea_pack<<<(P.nb + 127) / 128, 128, 0, s>>>(P, B);
@@ -571,45 +580,6 @@ void launch_tea_feff(const KParams &P, const DevBuffers &B, const int2 *work, in
 // Because C_i weights R_j per component and per target, the proxies carry F
 // and R separately and the targets receive A = T Q_F and B_k = T e_k Q_R,k
 // (k = x, y, z); a bead adds A + sum_k beta C_ik B_k.
-
-// Tile of kFFTileLeaves source leaves (kFFPairSlots bead pairs each), in the
-// layout of FFBuffers::pack: the two lanes of a packed pair are two source
-// beads.  Filled from pack by asynchronous 16-byte copies.
-constexpr int kFFTileLeaves = 4;   // 128 beads; tiles of 8 leaves measured slower (0.288 against 0.246 ms)
-constexpr int kFFTileSlots = kFFPairSlots * kFFTileLeaves;
-struct FFTile {
-    float4 xy[kFFTileSlots];   // xa xb ya yb
-    float4 zf[kFFTileSlots];   // za zb Fxa Fxb
-    float4 fyz[kFFTileSlots];  // Fya Fyb Fza Fzb
-    float4 rxy[kFFTileSlots];  // Rxa Rxb Rya Ryb
-    float2 rz[kFFTileSlots];   // Rza Rzb
-};
-
-// Near-list entries a step CTA keeps in shared memory (longer lists are read
-// from global memory).
-constexpr int kFFNearSmem = 256;
-
-// Issues the copies of near-list entries e0 .. min(e0 + kFFTileLeaves, e1) - 1
-// (entries relative to the list's start) into tile T: each leaf is kFFPackF4
-// contiguous float4 of pack.
-__device__ __forceinline__ void ff_tile_issue(FFTile &T, const FFBuffers &F, const int *near, int e0, int e1) {
-    constexpr int kPer = kFFPackF4;
-    for (int c = threadIdx.x; c < kFFTileLeaves * kPer; c += blockDim.x) {
-        const int q = c / kPer, w = c % kPer;
-        const int e = e0 + q;
-        if (e >= e1) continue;   // past the list: the tile pass skips the slot
-        const int J = near[e];
-        const float4 *src = F.pack + (size_t)J * kPer + w;
-        float4 *dst;
-        if (w < 4 * kFFPairSlots) {
-            const int a = w / kFFPairSlots, k = q * kFFPairSlots + w % kFFPairSlots;
-            dst = a == 0 ? &T.xy[k] : a == 1 ? &T.zf[k] : a == 2 ? &T.fyz[k] : &T.rxy[k];
-        } else {
-            dst = reinterpret_cast<float4 *>(&T.rz[q * kFFPairSlots + 2 * (w - 4 * kFFPairSlots)]);
-        }
-        cp_async16(dst, src);
-    }
-}
 
 // Trilinear Lagrange weights of the 8 proxies (bit 0: x, bit 1: y, bit 2: z;
 // a clear bit is the node at -h/sqrt(2), a set bit the one at +h/sqrt(2)) at
@@ -878,230 +848,134 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
     }
 }
 
-// Targets of one thread of the far-field step: TPT beads of the leaf, each
-// with its negated position, its weights beta C_i (both duplicated into the
-// two lanes of a packed pair), its packed sums, its own pair slot and lane.
-template <int TPT>
-struct FFTargets {
-    float2 nx[TPT], ny[TPT], nz[TPT], cbx[TPT], cby[TPT], cbz[TPT];
-    float2 ax[TPT], ay[TPT], az[TPT];
-    int self_p[TPT], self_h[TPT];
-};
-
-// The packed pass of one tile: the thread's targets against the tile's bead
-// pairs; with SELF a target's own slot is pushed to r^2 = 1e30, with TRACK
-// the running minimum of r^2 per segment of the thread's pairs is kept.
-// A thread takes the pair slots sl, sl + SLICES, ... of every leaf of the
-// tile, leaf after leaf (so the order of its sums does not depend on the tile
-// size); the padding leaves of a list's last tile (q >= nleaves) are skipped.
-template <int SLICES, int TPT, bool SELF, bool TRACK>
-__device__ __forceinline__ void ff_step_tile(const FFTile &T, int sl, int nleaves, FFTargets<TPT> &X, float2 vkap,
-                                             float2 vn2a2, float2 one, float (&rmin)[kFFTileLeaves]) {
-    constexpr int kLen = kFFPairSlots / SLICES;
-#pragma unroll
-    for (int q = 0; q < kFFTileLeaves; q++) {
-        if (q >= nleaves) break;
-#pragma unroll(kLen <= 4 ? kLen : 4)
-        for (int k = 0; k < kLen; k++) {
-            const int t = q * kFFPairSlots + sl + k * SLICES;
-            const float4 a = T.xy[t], b = T.zf[t], c = T.fyz[t], d = T.rxy[t];
-            const float2 rz = T.rz[t];
-#pragma unroll
-            for (int h = 0; h < TPT; h++) {
-                const float2 dx = __fadd2_rn(lo2(a), X.nx[h]), dy = __fadd2_rn(hi2(a), X.ny[h]),
-                             dz = __fadd2_rn(lo2(b), X.nz[h]);
-                const float2 gx = __ffma2_rn(lo2(d), X.cbx[h], hi2(b)), gy = __ffma2_rn(hi2(d), X.cby[h], lo2(c)),
-                             gz = __ffma2_rn(rz, X.cbz[h], hi2(c));
-                float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                if (SELF && t == X.self_p[h]) {
-                    if (X.self_h[h])
-                        r2.y = 1e30f;
-                    else
-                        r2.x = 1e30f;
-                }
-                if (TRACK) rmin[q] = fmin3(rmin[q], r2.x, r2.y);
-                const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
-                const float2 q2 = __fmul2_rn(rinv, rinv);
-                const float2 tq = __fmul2_rn(q2, rinv);
-                const float2 cii = __ffma2_rn(vkap, tq, rinv);
-                const float2 cr = __fmul2_rn(tq, __ffma2_rn(vn2a2, q2, one));
-                const float2 s = __fmul2_rn(cr, __ffma2_rn(dx, gx, __ffma2_rn(dy, gy, __fmul2_rn(dz, gz))));
-                X.ax[h] = __ffma2_rn(cii, gx, __ffma2_rn(s, dx, X.ax[h]));
-                X.ay[h] = __ffma2_rn(cii, gy, __ffma2_rn(s, dy, X.ay[h]));
-                X.az[h] = __ffma2_rn(cii, gz, __ffma2_rn(s, dz, X.az[h]));
-            }
-        }
-    }
+// Near pairs.  The near lists of all leaves, one after another, are cut into
+// equal runs, one warp each, as many as the GPU holds at once; a warp goes through the
+// leaves its run touches, a bead a lane, with the near leaves' beads copied one
+// leaf at a time, two ahead, into its own ring in shared memory: no barrier, no
+// partly filled wave, and equal work for all four schedulers of an SM.  The pair loop
+// is that of the all-pairs pass (StepOp), and like it the kernel is bound by the FP32 pipe.
+// 64 x 5600 beads, 225 M pairs: 256 us with four warps a leaf on 128-bead tiles (2100 of
+// 3950 instructions a warp were not pair arithmetic), 268 us with a whole leaf
+// a warp (a third of the time was the last wave), 233 us so.
+// A leaf that one run holds goes to FFBuffers::nearsum; of a leaf that several
+// share each writes its part (slot 0 of the run for a leaf begun before it, slot 1 for
+// one it begins) and k_ff_far adds them in run order.
+// Overlapping pairs (r <= 2a): with LISTCORR the far-field term of the pair loop is
+// replaced while walking the bead's LJ list once, which holds every pair
+// that close (checked by the launcher), by the run that begins the leaf;
+// otherwise they are looked for in the leaves whose smallest r^2 shows one, as
+// the all-pairs pass does.
+constexpr int kFFStages = 3, kFFWarps = 4;
+constexpr int kFFRunsPerSlot = 2;   // runs for every warp that fits the device, see kTeaRunsPerSlot
+static_assert(kFFLeaf == kTeaBlock && kFFPackF4 == kTeaBlockF4, "leaves are blocks of the pair loop");
+// first near entry of run k of F.near_runs
+__device__ __forceinline__ int ff_run_start(const FFBuffers &F, int units, int k) {
+    return (int)((long long)k * units / F.near_runs);
 }
-
-// Near pairs: one CTA of (32 / TPT) x SLICES threads per target leaf; thread
-// lane il serves the leaf's beads il + h 32 / TPT (h < TPT), the SLICES
-// groups of lanes take interleaved bead pairs of every tile of near leaves
-// (kFFTileLeaves leaves per tile, copied asynchronously one tile ahead), the
-// two lanes of each packed operation being two source beads.  Overlapping
-// pairs (r <= 2a) get the near formula: with LISTCORR by walking the bead's
-// LJ list once (while the first tile is in flight), otherwise by rescanning
-// the tile segments whose running minimum of r^2 flags one, as in
-// k_tea_step.  The bead's sum goes to FFBuffers::nearsum (k_ff_far adds the
-// far field and moves it).
-template <int SLICES, int TPT, bool LISTCORR>
-__global__ void __launch_bounds__(32 / TPT * SLICES, 32 * TPT / SLICES) k_ff_near(KParams P, DevBuffers B,
-                                                                                FFBuffers F, const int *gate) {
+template <bool LISTCORR>
+__global__ void __launch_bounds__(32 * kFFWarps, 8) k_ff_near(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
     if (gate && *gate != 0) return;
-    constexpr int kLanes = 32 / TPT;
-    const int L = blockIdx.x;
-    const int il = threadIdx.x % kLanes, sl = threadIdx.x / kLanes;
-    const int s0 = F.leaf_start[L], n = F.leaf_start[L + 1] - s0;
-    const int traj = F.leaf_traj[L];
-    __shared__ FFTile T2[2];
-    __shared__ float4 s_red[SLICES * 32];
-    __shared__ float4 s_x[32], s_cb[32];       // the leaf's beads: position, beta C_i
-    __shared__ int s_near[kFFNearSmem];
-    const float beta = B.tea_beta[traj], b2 = beta * beta;
-    if (threadIdx.x < 32) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), cb = x;
-        if (threadIdx.x < n) {
-            const int g = F.leaf_bead[s0 + threadIdx.x];
-            x = B.frame_in[g];
-            const float4 ci = B.tea_ci[g];
-            cb = make_float4(beta / sqrtf(1.0f + b2 * ci.x), beta / sqrtf(1.0f + b2 * ci.y),
-                             beta / sqrtf(1.0f + b2 * ci.z), 0.f);
-        }
-        s_x[threadIdx.x] = x;
-        s_cb[threadIdx.x] = cb;
+    __shared__ float4 s_leaf[kFFWarps][kFFStages][kFFPackF4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, run = blockIdx.x * kFFWarps + warp;
+    if (run >= F.near_runs) return;
+    const int units = F.near_start[F.nleaf];
+    const int u0 = ff_run_start(F, units, run), u1 = ff_run_start(F, units, run + 1);
+    if (u0 >= u1) return;
+    int L = 0;   // the leaf whose list holds entry u0 (32-way search)
+    for (int n = F.nleaf; n > 1;) {
+        const int step = (n + 31) / 32;
+        const bool le = lane * step < n && F.near_start[L + lane * step] <= u0;
+        const int last = 31 - __clz((int)__ballot_sync(0xffffffffu, le));
+        n = min(step, n - last * step);
+        L += last * step;
     }
-    // near leaves in tiles of kFFTileLeaves, double-buffered: the copies of
-    // tile k + 1 are in flight while tile k is summed
-    const int e_beg = F.near_start[L], nnear = F.near_start[L + 1] - e_beg;
-    const int *near = F.near + e_beg;
-    const bool near_smem = nnear <= kFFNearSmem;
-    if (near_smem)
-        for (int k = threadIdx.x; k < nnear; k += blockDim.x) s_near[k] = near[k];
-    __syncthreads();
-    if (near_smem) near = s_near;
-    const TeaConst K = tea_const(P.tea_a);
-    const float2 vkap = f2(K.kap), vn2a2 = f2(-K.two_a2), one = f2(1.0f);
-    const int ntiles = (nnear + kFFTileLeaves - 1) / kFFTileLeaves;
-    ff_tile_issue(T2[0], F, near, 0, nnear);
-    cp_async_commit();
-    FFTargets<TPT> X;
-    float3 corr[TPT];
+    auto issue = [&](int u) {
+        if (u < u1) {
+            const float4 *src = F.pack + (size_t)F.near[u] * kFFPackF4;
+            float4 *dst = s_leaf[warp][(u - u0) % kFFStages];
 #pragma unroll
-    for (int h = 0; h < TPT; h++) {
-        const int bi = il + h * kLanes;
-        const float4 x = s_x[bi], cb = s_cb[bi];
-        X.nx[h] = f2(-x.x);
-        X.ny[h] = f2(-x.y);
-        X.nz[h] = f2(-x.z);
-        X.cbx[h] = f2(cb.x);
-        X.cby[h] = f2(cb.y);
-        X.cbz[h] = f2(cb.z);
-        X.ax[h] = X.ay[h] = X.az[h] = f2(0.f);
-        corr[h] = make_float3(0.f, 0.f, 0.f);
-        if (LISTCORR && bi < n) {
-            // overlapping pairs (r <= 2a): every one is within the LJ list
-            // cutoff (checked by the launcher), so the far-field term of the
-            // tile pass is replaced by the near one while walking the bead's
-            // list, the SLICES threads of a bead taking interleaved entries;
-            // done while the first tile is in flight
-            const int g = F.leaf_bead[s0 + bi];
+            for (int c = 0; c < kFFPackF4; c += 32)
+                if (c + lane < kFFPackF4) cp_async16(dst + c + lane, src + c + lane);
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int k = 0; k < kFFStages - 1; k++) issue(u0 + k);
+    const TeaConst K = tea_const(P.tea_a);
+    for (int u = u0; u < u1; L++) {
+        const int e0 = F.near_start[L], e1 = F.near_start[L + 1], stop = min(u1, e1);
+        const int s0 = F.leaf_start[L], n = F.leaf_start[L + 1] - s0, traj = F.leaf_traj[L];
+        const bool valid = lane < n;
+        const int g = valid ? F.leaf_bead[s0 + lane] : 0;
+        const float4 x = valid ? B.frame_in[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+        StepOp<false> X;
+        X.start(P, B, traj, x, g, valid);
+        float3 corr = make_float3(0.f, 0.f, 0.f);
+        if (LISTCORR && valid && u == e0) {
             const int base = B.off[traj], nb = P.nb;
             const int cnt = B.ljc[g];
-            for (int q = sl; q < cnt; q += SLICES) {
-                const int pj = base + B.lj[q * nb + g];
-                const float4 xj = B.frame_in[pj];
-                const float dx = xj.x - x.x, dy = xj.y - x.y, dz = xj.z - x.z;
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                if (!(r2 <= K.four_a2) || (B.flags[pj] & kFlagExtra)) continue;
-                const float4 Fj = B.force[pj], Rj = B.tea_r[pj];
-                const float gx = fmaf(Rj.x, cb.x, Fj.x), gy = fmaf(Rj.y, cb.y, Fj.y), gz = fmaf(Rj.z, cb.z, Fj.z);
-                const float3 fa = tea_far1(K, dx, dy, dz, gx, gy, gz);
-                const float3 nr = tea_pair1(K, dx, dy, dz, gx, gy, gz);
-                corr[h].x += nr.x - fa.x;
-                corr[h].y += nr.y - fa.y;
-                corr[h].z += nr.z - fa.z;
-            }
-        }
-    }
-    for (int it = 0; it < ntiles; it++) {
-        if (it + 1 < ntiles) ff_tile_issue(T2[(it + 1) & 1], F, near, (it + 1) * kFFTileLeaves, nnear);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const FFTile &T = T2[it & 1];
-        int self_q = -1;
+            for (int q0 = 0; q0 < cnt; q0 += 4) {   // four entries in flight
+                float4 xj[4];
+                int pj[4];
 #pragma unroll
-        for (int q = 0; q < kFFTileLeaves; q++) {
-            const int e = it * kFFTileLeaves + q;
-            if (e < nnear && near[e] == L) self_q = q;
-        }
-        float rmin[kFFTileLeaves];
+                for (int v = 0; v < 4; v++) pj[v] = q0 + v < cnt ? base + B.lj[(q0 + v) * nb + g] : -1;
 #pragma unroll
-        for (int q = 0; q < kFFTileLeaves; q++) rmin[q] = 3.4e38f;
-        const bool self = self_q >= 0;
+                for (int v = 0; v < 4; v++)
+                    xj[v] = pj[v] >= 0 ? B.frame_in[pj[v]] : make_float4(kFarAway, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int h = 0; h < TPT; h++) {
-            const int bi = il + h * kLanes;
-            X.self_p[h] = self_q * kFFPairSlots + (bi >> 1);
-            X.self_h[h] = bi & 1;
-        }
-        const int nleaves = min(kFFTileLeaves, nnear - it * kFFTileLeaves);
-        if (self)
-            ff_step_tile<SLICES, TPT, true, !LISTCORR>(T, sl, nleaves, X, vkap, vn2a2, one, rmin);
-        else
-            ff_step_tile<SLICES, TPT, false, !LISTCORR>(T, sl, nleaves, X, vkap, vn2a2, one, rmin);
-        if (!LISTCORR) {
-            constexpr int kLen = kFFPairSlots / SLICES;
-            unsigned segs = 0;
-#pragma unroll
-            for (int q = 0; q < kFFTileLeaves; q++) segs |= (rmin[q] <= K.four_a2 ? 1u : 0u) << q;
-            while (segs) {  // the tile leaves that hold an overlapping pair
-                const int sg = __ffs(segs) - 1;
-                segs &= segs - 1;
-                for (int k = 0; k < kLen; k++) {
-                    const int t = sg * kFFPairSlots + sl + k * SLICES;
-                    const float4 a = T.xy[t], b = T.zf[t], c = T.fyz[t], d = T.rxy[t];
-                    const float2 rz = T.rz[t];
-#pragma unroll
-                    for (int h = 0; h < TPT; h++)
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            if (self && t == X.self_p[h] && e == X.self_h[h]) continue;
-                            const float dx = (e ? a.y : a.x) + X.nx[h].x, dy = (e ? a.w : a.z) + X.ny[h].x,
-                                        dz = (e ? b.y : b.x) + X.nz[h].x;
-                            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            if (!(r2 <= K.four_a2)) continue;
-                            const float gx = fmaf(e ? d.y : d.x, X.cbx[h].x, e ? b.w : b.z),
-                                        gy = fmaf(e ? d.w : d.z, X.cby[h].x, e ? c.y : c.x),
-                                        gz = fmaf(e ? rz.y : rz.x, X.cbz[h].x, e ? c.w : c.z);
-                            const float3 fa = tea_far1(K, dx, dy, dz, gx, gy, gz);
-                            const float3 nr = tea_pair1(K, dx, dy, dz, gx, gy, gz);
-                            corr[h].x += nr.x - fa.x;
-                            corr[h].y += nr.y - fa.y;
-                            corr[h].z += nr.z - fa.z;
-                        }
+                for (int v = 0; v < 4; v++) {
+                    const float dx = xj[v].x - x.x, dy = xj[v].y - x.y, dz = xj[v].z - x.z;
+                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    if (!(r2 <= K.four_a2) || (B.flags[pj[v]] & kFlagExtra)) continue;
+                    const float4 Fj = B.force[pj[v]], Rj = B.tea_r[pj[v]];
+                    const float gx = fmaf(Rj.x, X.cbx.x, Fj.x), gy = fmaf(Rj.y, X.cby.x, Fj.y),
+                                gz = fmaf(Rj.z, X.cbz.x, Fj.z);
+                    const float3 fa = tea_far1(K, dx, dy, dz, gx, gy, gz);
+                    const float3 nr = tea_pair1(K, dx, dy, dz, gx, gy, gz);
+                    corr.x += nr.x - fa.x;
+                    corr.y += nr.y - fa.y;
+                    corr.z += nr.z - fa.z;
                 }
             }
         }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int h = 0; h < TPT; h++) {
-        const int bi = il + h * kLanes;
-        s_red[sl * 32 + bi] = make_float4(X.ax[h].x + X.ax[h].y + corr[h].x, X.ay[h].x + X.ay[h].y + corr[h].y,
-                                          X.az[h].x + X.az[h].y + corr[h].z, 0.f);
-    }
-    __syncthreads();
-    if (threadIdx.x < n) {
-        float4 v = s_red[threadIdx.x];
-        for (int k = 1; k < SLICES; k++) {
-            const float4 u = s_red[k * 32 + threadIdx.x];
-            v.x += u.x;
-            v.y += u.y;
-            v.z += u.z;
+        const bool whole = u == e0 && stop == e1;
+        const int slot = u == e0 ? 1 : 0;
+        for (; u < stop; u++) {
+            cp_async_wait<kFFStages - 2>();
+            __syncwarp();
+            const float4 *blk = s_leaf[warp][(u - u0) % kFFStages];
+            const bool own = F.near[u] == L;
+            issue(u + kFFStages - 1);
+            float rm = 3.4e38f;
+            if (own) {
+#pragma unroll 1
+                for (int t = 0; t < kTeaPairSlots; t++) X.template pair<true>(K, blk, t, lane >> 1, lane & 1, rm);
+            } else {
+#pragma unroll 8
+                for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
+            }
+            if (!LISTCORR && rm <= K.four_a2) tea_near_block(X, K, blk, own, lane);
         }
-        F.nearsum[s0 + threadIdx.x] = v;
+        const float4 sum = X.sum();
+        const float4 v = make_float4(sum.x + corr.x, sum.y + corr.y, sum.z + corr.z, 0.f);
+        if (!whole)
+            F.nearpart[((size_t)run * 2 + slot) * kFFLeaf + lane] = v;
+        else if (valid)
+            F.nearsum[s0 + lane] = v;
     }
+}
+// The near sum of bead `lane` of leaf L (leaf bead s0 + lane) from its runs.
+__device__ __forceinline__ float4 ff_near_sum(const FFBuffers &F, int L, int s0, int lane) {
+    const int units = F.near_start[F.nleaf], e0 = F.near_start[L], e1 = F.near_start[L + 1];
+    const int k0 = (int)(((long long)(e0 + 1) * F.near_runs - 1) / units),
+              k1 = (int)(((long long)e1 * F.near_runs - 1) / units);
+    if (k0 == k1) return F.nearsum[s0 + lane];
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = k0; k <= k1; k++) {
+        const float4 q = F.nearpart[((size_t)k * 2 + (ff_run_start(F, units, k) > e0 ? 0 : 1)) * kFFLeaf + lane];
+        v = make_float4(v.x + q.x, v.y + q.y, v.z + q.z, 0.f);
+    }
+    return v;
 }
 
 // Far field and update: one warp per leaf.  The far fields of the leaf and
@@ -1115,12 +989,10 @@ __global__ void __launch_bounds__(32) k_ff_far(KParams P, DevBuffers B, FFBuffer
     if (gate && *gate != 0) return;
     const int L = blockIdx.x, lane = threadIdx.x;
     const int s0 = F.leaf_start[L], n = F.leaf_start[L + 1] - s0;
-    // per ancestor: box (2) and potentials (24), then its far field at the
-    // leaf's proxies; sized for the tree's longest ancestor list (max_anc)
-    extern __shared__ float4 s_dyn[];
-    float4 *s_far = s_dyn;
-    float *s_l2l = reinterpret_cast<float *>(s_dyn + 26 * F.max_anc);
-    __shared__ float s_pl[8 * 12];             // the far field at the leaf's proxies
+    // per ancestor: box (2) and potentials (24); sized for the tree's longest
+    // ancestor list (max_anc)
+    extern __shared__ float4 s_far[];
+    __shared__ float4 s_pl[8 * 3];             // the far field at the leaf's proxies
     __shared__ float4 s_lbox[2];
     const int a0 = F.anc_start[L], na = min(F.anc_start[L + 1] - a0, F.max_anc);
     for (int k = lane; k < 26 * na; k += 32) {
@@ -1129,25 +1001,38 @@ __global__ void __launch_bounds__(32) k_ff_far(KParams P, DevBuffers B, FFBuffer
     }
     if (lane < 2) s_lbox[lane] = F.box[2 * L + lane];
     __syncwarp();
-    for (int t = lane; t < 8 * na; t += 32) {
-        const int A = t >> 3, pn = t & 7;
-        const float4 *fr = s_far + 26 * A;
-        const float *ph = reinterpret_cast<const float *>(fr + 2);
-        float w[8];
-        ff_weights(ff_proxy(s_lbox[0], s_lbox[1], pn), fr[0], fr[1], w);
+    {   // lane (A, pn): ancestors A, A + 4, ... at the leaf's proxy pn, the four
+        // groups of ancestors summed by shuffles
+        const int pn = lane & 7;
+        const float3 y = ff_proxy(s_lbox[0], s_lbox[1], pn);
+        float4 v[3];
 #pragma unroll
-        for (int c = 0; c < 12; c++) {
-            float v = 0.f;
+        for (int c = 0; c < 3; c++) v[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int A = lane >> 3; A < na; A += 4) {
+            const float4 *fr = s_far + 26 * A;
+            float w[8];
+            ff_weights(y, fr[0], fr[1], w);
 #pragma unroll
-            for (int m = 0; m < 8; m++) v = fmaf(w[m], ph[12 * m + c], v);
-            s_l2l[96 * A + 12 * pn + c] = v;
+            for (int m = 0; m < 8; m++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const float4 q = fr[2 + 3 * m + c];
+                    v[c] = make_float4(fmaf(w[m], q.x, v[c].x), fmaf(w[m], q.y, v[c].y), fmaf(w[m], q.z, v[c].z),
+                                       fmaf(w[m], q.w, v[c].w));
+                }
         }
-    }
-    __syncwarp();
-    for (int t = lane; t < 96; t += 32) {
-        float v = 0.f;
-        for (int A = 0; A < na; A++) v += s_l2l[96 * A + t];
-        s_pl[t] = v;
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                v[c].x += __shfl_xor_sync(0xffffffffu, v[c].x, o);
+                v[c].y += __shfl_xor_sync(0xffffffffu, v[c].y, o);
+                v[c].z += __shfl_xor_sync(0xffffffffu, v[c].z, o);
+                v[c].w += __shfl_xor_sync(0xffffffffu, v[c].w, o);
+            }
+        if (lane < 8)
+#pragma unroll
+            for (int c = 0; c < 3; c++) s_pl[3 * lane + c] = v[c];
     }
     __syncwarp();
     if (lane >= n) return;
@@ -1158,18 +1043,19 @@ __global__ void __launch_bounds__(32) k_ff_far(KParams P, DevBuffers B, FFBuffer
     const float4 ci = B.tea_ci[g];
     const float3 cbi = make_float3(beta / sqrtf(1.0f + b2 * ci.x), beta / sqrtf(1.0f + b2 * ci.y),
                                    beta / sqrtf(1.0f + b2 * ci.z));
-    const float4 ns = F.nearsum[s0 + lane];
+    const float4 ns = ff_near_sum(F, L, s0, lane);
     float sx = ns.x, sy = ns.y, sz = ns.z;
     if (na > 0) {   // L2P from the leaf's proxies
         float w[8];
         ff_weights(xi, s_lbox[0], s_lbox[1], w);
 #pragma unroll
         for (int m = 0; m < 8; m++) {
-            const float *p = s_pl + 12 * m;   // A.xyz, B_x.xyz, B_y.xyz, B_z.xyz
+            // A.xyz, B_x.xyz, B_y.xyz, B_z.xyz
+            const float4 p = s_pl[3 * m], q = s_pl[3 * m + 1], r = s_pl[3 * m + 2];
             // A + beta C_x B_x + beta C_y B_y + beta C_z B_z
-            const float ux = p[0] + cbi.x * p[3] + cbi.y * p[6] + cbi.z * p[9];
-            const float uy = p[1] + cbi.x * p[4] + cbi.y * p[7] + cbi.z * p[10];
-            const float uz = p[2] + cbi.x * p[5] + cbi.y * p[8] + cbi.z * p[11];
+            const float ux = p.x + cbi.x * p.w + cbi.y * q.z + cbi.z * r.y;
+            const float uy = p.y + cbi.x * q.x + cbi.y * q.w + cbi.z * r.z;
+            const float uz = p.z + cbi.x * q.y + cbi.y * r.x + cbi.z * r.w;
             sx = fmaf(w[m], ux, sx);
             sy = fmaf(w[m], uy, sy);
             sz = fmaf(w[m], uz, sz);
@@ -1207,35 +1093,31 @@ void launch_ff_proxies(const KParams &P, const DevBuffers &B, const FFBuffers &F
     launch_ff_m2l(P, F, gate, s);
 }
 
+// Runs of the near lists: a few for each warp the device holds at once, or one an entry.
+int ff_near_runs(int entries) {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int warps = sms * 8 * kFFWarps * kFFRunsPerSlot;
+    return entries < warps ? entries : warps;
+}
+
 // Overlapping pairs can be taken from the LJ list when it holds every pair
 // within 2a (plus 2 nm for the motion since its rebuild).
 static bool ff_list_corr(const KParams &P) { return P.lj_on && P.ljcut >= 2.0f * P.tea_a + 2.0f; }
 
-// target beads per thread of the near-pair kernel (two, with 16 lanes per
-// slice, measured slower)
-constexpr int kFFTPT = 1;
-template <int SL>
-static void ff_near_launch(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate,
-                           cudaStream_t s) {
-    constexpr int threads = 32 / kFFTPT * SL;
-    if (F.nleaf == 0) return;
-    if (ff_list_corr(P))
-        k_ff_near<SL, kFFTPT, true><<<F.nleaf, threads, 0, s>>>(P, B, F, gate);
-    else
-        k_ff_near<SL, kFFTPT, false><<<F.nleaf, threads, 0, s>>>(P, B, F, gate);
-}
 void launch_ff_near(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s) {
-    switch (P.tea_slices) {
-        case 1:
-        case 2: ff_near_launch<2>(P, B, F, gate, s); break;
-        case 4: ff_near_launch<4>(P, B, F, gate, s); break;
-        default: ff_near_launch<8>(P, B, F, gate, s); break;
-    }
+    if (F.nleaf == 0) return;
+    const int ctas = (F.near_runs + kFFWarps - 1) / kFFWarps;
+    if (ff_list_corr(P))
+        k_ff_near<true><<<ctas, 32 * kFFWarps, 0, s>>>(P, B, F, gate);
+    else
+        k_ff_near<false><<<ctas, 32 * kFFWarps, 0, s>>>(P, B, F, gate);
 }
 void launch_ff_far(const KParams &P, const DevBuffers &B, const FFBuffers &F, bool feff_only, float4 *feff,
                    const int *gate, cudaStream_t s) {
     if (F.nleaf > 0) {
-        const size_t smem = (size_t)F.max_anc * (26 * sizeof(float4) + 96 * sizeof(float));
+        const size_t smem = (size_t)F.max_anc * 26 * sizeof(float4);
         if (feff_only)
             k_ff_far<true><<<F.nleaf, 32, smem, s>>>(P, B, F, feff, gate);
         else

@@ -569,7 +569,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         ALLOC(e->tea_slot, nb);
         ALLOC(e->tea_blk0, nt + 1);
         ALLOC(e->tea_unit0, e->tea_nwork + 1);
-        ALLOC(e->tea_part, (size_t)2 * kTeaChunk * std::min<long long>(e->kp.tea_units, (long long)kTeaMaxOcc * sms));
+        ALLOC(e->tea_part, (size_t)2 * kTeaChunk * std::min<long long>(e->kp.tea_units, (long long)kTeaMaxOcc * kTeaRunsPerSlot * sms));
         ALLOC(e->tea_cnt, e->tea_nwork);
     }
     // spatial-hash tables of the cell-list rebuild

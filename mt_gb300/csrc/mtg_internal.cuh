@@ -433,6 +433,7 @@ void launch_energy_totals(const KParams &P, const double *partials, const int *w
 // TEA kernels run over their own work list: chunks of kTeaChunk beads.
 constexpr int kTeaChunk = 128;
 constexpr int kTeaMaxParts = 4;      // largest mtg_tuning::tea_jparts that is accepted
+constexpr int kTeaRunsPerSlot = 4;   // runs of an all-pairs launch for every CTA that fits the device
 constexpr int kTeaMaxOcc = 12;       // CTAs of the all-pairs kernels per SM at most (sizes tea_part)
 // positions (F and R are zeroed once) into the pack, for epsilon passes outside a TEA step
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s);
@@ -488,6 +489,8 @@ struct FFBuffers {
     float4 *phi;             // [24*nnode] target proxy n: (A.xyz, B0.x), (B0.yz, B1.xy), (B1.z, B2.xyz) at 24N+3n
     float4 *pack;            // [(nleaf+1)*kFFPackF4] each leaf's beads in the tile layout of the step kernel
                              // (leaf nleaf: padding, far away with zero F and R), written every step by P2M
+    int near_runs;           // warps the near lists are divided over (ff_near_runs)
+    float4 *nearpart;        // [2 * near_runs][kFFLeaf] parts of the near sums of leaves that runs share
     float4 *nearsum;         // [leaf beads] each bead's near-pair sum, in leaf bead order
 };
 // float4 per leaf of FFBuffers::pack, for the bead pairs (2p, 2p+1):
@@ -503,6 +506,7 @@ void launch_ff_p2m_leaves(const KParams &P, const DevBuffers &B, const FFBuffers
 void launch_ff_m2l(const KParams &P, const FFBuffers &F, const int *gate, cudaStream_t s);
 // both of the above
 void launch_ff_proxies(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s);
+int ff_near_runs(int entries);
 // near-pair sums; needs the leaf proxies' packed beads
 void launch_ff_near(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s);
 // far field + update (FEFF: effective forces into feff, no update); needs the near sums and M2L

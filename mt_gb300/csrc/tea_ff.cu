@@ -285,7 +285,9 @@ static int ff_build(mtg_engine *e) {
     size_t nints = 0;
     for (auto *v : parts) nints += v->size() + 1;
     const size_t nn1 = (size_t)std::max(nnode, 1);
-    const size_t nf4 = (size_t)(2 + 16 + 24) * nn1 + (size_t)kFFPackF4 * (nleaf + 1) + P.leaf_bead.size();
+    const int near_runs = ff_near_runs((int)P.near.size());
+    const size_t nf4 = (size_t)(2 + 16 + 24) * nn1 + (size_t)kFFPackF4 * (nleaf + 1) + P.leaf_bead.size() +
+                       (size_t)2 * near_runs * kFFLeaf;
     if (nints > e->ff_ints_cap) {
         if (e->ff_ints) cudaFree(e->ff_ints);
         e->ff_ints = nullptr;
@@ -335,6 +337,8 @@ static int ff_build(mtg_engine *e) {
     F.phi = e->ff_f4 + 18 * nn1;
     F.pack = e->ff_f4 + 42 * nn1;
     F.nearsum = F.pack + (size_t)kFFPackF4 * (nleaf + 1);
+    F.near_runs = near_runs;
+    F.nearpart = F.nearsum + P.leaf_bead.size();
     e->ff_near_pairs = P.near_pairs;
     e->ff_proxy_pairs = P.proxy_pairs;
     e->ff_sizes[0] = nleaf;
