@@ -430,11 +430,6 @@ size_t smem_list_bytes(int nmax) {
     return sizeof(float4) * (size_t)nmax + sizeof(uint16_t) * ((size_t)smem_buckets(nmax) + kSmemKeys * kListThreads);
 }
 
-__device__ __forceinline__ float dist2_rn(float4 a, float4 b) {
-    const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-
 // Batcher's odd-even merge sort of N keys in registers, ascending.
 template <int N>
 __device__ __forceinline__ void sort_network(unsigned (&k)[N]) {
@@ -548,7 +543,7 @@ __device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &
 }
 
 __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int2 *work, int nmax,
-                                                                  float inv, float t_lj, float t_pair, float t_site) {
+                                                                  float inv, ListCuts cut) {
     extern __shared__ float4 s_dyn[];
     const int2 w = work[blockIdx.x];
     const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
@@ -621,13 +616,13 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
             const float r2 = dist2_rn(I.p, q);
             const int jl = __float_as_int(q.w);
             unsigned bits = 0;
-            if (I.do_pairs && r2 < t_pair && jl != I.hpart)
+            if (I.do_pairs && r2 < cut.pair && jl != I.hpart)
                 bits = (dist2_rn(a0, q) < kSite2 ? 1u : 0u) | (dist2_rn(a1, q) < kSite2 ? 2u : 0u) |
                        (dist2_rn(a2, q) < kSite2 ? 4u : 0u);
             return ((unsigned)jl << 3) | bits;
         };
         int nk = 0;
-        smem_candidates(C, I.p, t_lj, [&](int slot) {
+        smem_candidates(C, I.p, cut.lj, [&](int slot) {
             if (nk < kSmemKeys) s_key[nk][t] = (uint16_t)slot;
             nk++;
         });
@@ -662,8 +657,8 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
                 const unsigned k0 = s_key[k][t], k1 = k + 1 < np ? s_key[k + 1][t] : 0u;
                 const PairPlanes J0 = pair_load(B, nb, base + (int)(k0 >> 3), k0 & 7u);
                 const PairPlanes J1 = pair_load(B, nb, base + (int)(k1 >> 3), k1 & 7u);
-                pair_decide(P, B, g, I, (int)(k0 >> 3), k0 & 7u, J0, t_site, W);
-                pair_decide(P, B, g, I, (int)(k1 >> 3), k1 & 7u, J1, t_site, W);
+                pair_decide(P, B, g, I, (int)(k0 >> 3), k0 & 7u, J0, cut.site, W);
+                pair_decide(P, B, g, I, (int)(k1 >> 3), k1 & 7u, J1, cut.site, W);
             }
         } else {
             // more neighbours than hard spheres of this size allow: the next larger
@@ -671,7 +666,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
             int last = -1;
             while (true) {
                 unsigned best = 0x7fffffffu;
-                smem_candidates(C, I.p, t_lj, [&](int slot) {
+                smem_candidates(C, I.p, cut.lj, [&](int slot) {
                     const unsigned key = make_key(slot);
                     if ((int)(key >> 3) != il && (int)key > last) best = min(best, key);
                 });
@@ -679,7 +674,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
                 last = (int)best;
                 lj_append(P, B, g, (int)(best >> 3), W);
                 const PairPlanes J = pair_load(B, nb, base + (int)(best >> 3), best & 7u);
-                pair_decide(P, B, g, I, (int)(best >> 3), best & 7u, J, t_site, W);
+                pair_decide(P, B, g, I, (int)(best >> 3), best & 7u, J, cut.site, W);
             }
         }
     }
@@ -689,16 +684,6 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         B.latc[g] = min(W.nla, P.maxLat);
     }
     if (W.overflow) atomicOr(B.err, kErrOverflow);
-}
-
-// The smallest float whose rounded square root is not below c, so that
-// r2 < sq_below(c) decides as sqrt(r2) < c does.
-float sq_below(float c) {
-    if (!(c > 0.0f)) return 0.0f;
-    float t = c * c;
-    while (std::sqrt(t) >= c && t > 0.0f) t = std::nextafter(t, 0.0f);
-    while (std::sqrt(t) < c) t = std::nextafter(t, INFINITY);
-    return t;
 }
 
 inline int nblk(int n, int t) { return (n + t - 1) / t; }
@@ -730,11 +715,21 @@ int smem_lists_prepare() {   // the limit of the largest trajectory, whatever th
                ? 0
                : -1;
 }
+// The smallest float whose rounded square root is not below c, so that
+// r2 < sq_below(c) decides as sqrt(r2) < c does.
+static float sq_below(float c) {
+    if (!(c > 0.0f)) return 0.0f;
+    float t = c * c;
+    while (std::sqrt(t) >= c && t > 0.0f) t = std::nextafter(t, 0.0f);
+    while (std::sqrt(t) < c) t = std::nextafter(t, INFINITY);
+    return t;
+}
+ListCuts list_cuts(const KParams &P) { return {sq_below(P.ljcut), sq_below(kPairReach), sq_below(2.5f)}; }
+
 void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
                          cudaStream_t s) {
     const float inv = 1.0f / (P.ljcut * 1.001f + 1e-3f);   // the cells of bin_beads
-    k_cell_lists_smem<<<nwork, kListThreads, smem_list_bytes(nmax), s>>>(P, B, work, nmax, inv, sq_below(P.ljcut),
-                                                                         sq_below(kPairReach), sq_below(2.5f));
+    k_cell_lists_smem<<<nwork, kListThreads, smem_list_bytes(nmax), s>>>(P, B, work, nmax, inv, list_cuts(P));
 }
 
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,

@@ -578,6 +578,185 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
     if (TEA) tea_pack_bead(B, g, (flags & kFlagExtra) != 0, Fi.p0, f[0], f[1], f[2], rt);
 }
 
+// --------------------------------------- persistent period, four warps a bead group
+// k_step_period for trajectories of up to kPeriodSplitBeads beads: the roles of
+// k_split inside one CTA per trajectory that keeps the frames (two buffers) in
+// shared memory across the steps.  A step is the serial chain of one bead, so it is
+// cut by role: three groups of warps take the axial bonds, the lateral bonds and
+// the LJ neighbours while the fourth takes the Euler axes; after a barrier the fourth sums
+// the parts and moves the beads while the lateral and LJ groups draw the noise of
+// the next step; list heads and noise states stay in registers.  The pair lists are rebuilt
+// first when due, a quarter of the trajectory for each of a bead's four threads.
+// The same functions, order of sums and list order as the other forms: the same bits.
+// One 156-bead seed: 7.1 us a step with one thread a bead, 3.1 us so (10 steps and
+// a rebuild a launch).
+constexpr int kPeriodSplitBeads = 192;   // 768 threads of 80 registers (256 beads would leave 64 and spill)
+struct PeriodSplitSmem {   // offsets in bytes; s: beads rounded up to a warp
+    int frames, noise, parts, flags, total;
+    __host__ __device__ explicit PeriodSplitSmem(int s) {
+        frames = 0;
+        noise = frames + 2 * 4 * 16 * s;
+        parts = noise + 2 * 2 * 16 * s;
+        flags = parts + kParts * 4 * s;
+        total = flags + 4 * s;
+    }
+};
+template <bool KEEP_FORCES>
+__global__ void __launch_bounds__(4 * kPeriodSplitBeads) k_period_split(KParams P, DevBuffers B, int nsteps,
+                                                                        int rebuild, ListCuts cut) {
+    extern __shared__ float4 s_dyn[];
+    char *smem = reinterpret_cast<char *>(s_dyn);
+    const int S = blockDim.x >> 2, role = threadIdx.x / S, l = threadIdx.x % S;
+    const PeriodSplitSmem at(S);
+    const int traj = blockIdx.x, base = B.off[traj], n = B.off[traj + 1] - base, nb = P.nb, g = base + l;
+    float4 *s_fr = reinterpret_cast<float4 *>(smem + at.frames);     // plane k of bead j of buffer b at [(4 b + k) S + j]
+    float4 *s_noise = reinterpret_cast<float4 *>(smem + at.noise);   // [2 parity + (xyz, angles)][S]
+    float *s_part = reinterpret_cast<float *>(smem + at.parts);      // [kParts][S]
+    int *s_fl = reinterpret_cast<int *>(smem + at.flags);
+    const bool valid = l < n;
+    if (valid) {   // role k copies plane k, into both buffers (beads that never move stay as they are)
+        const float4 p = B.frame_in[role * nb + g];
+        s_fr[role * S + l] = p;
+        s_fr[(4 + role) * S + l] = p;
+        if (role == 0) s_fl[l] = B.flags[g];
+    }
+    __syncthreads();
+    const int flags = valid ? s_fl[l] : kFlagExtra;
+    if (rebuild) {
+        // exact decisions on squared distances (sq_below): the near ones of a
+        // quarter first, as a mask, then their lists, four bits each
+        const int quarter = (n + 3) / 4, j0 = min(n, role * quarter), j1 = min(n, j0 + quarter);   // at most 48 beads
+        int *s_cnt = reinterpret_cast<int *>(s_part);   // [3][4][S]
+        ListSite I;
+        unsigned long long near = 0, got[3] = {0, 0, 0};
+        int c[3] = {0, 0, 0};
+        bool overflow = false;
+        if (valid) {
+            I = list_site(P, s_fr[l], s_fr[S + l], s_fr[2 * S + l], s_fr[3 * S + l], flags, l, B.harm[g * P.maxH]);
+            const float t_near = fmaxf(I.do_lj ? cut.lj : 0.f, I.do_pairs ? cut.pair : 0.f);
+            unsigned lo = 0, hi = 0;
+#pragma unroll 4
+            for (int j = j0; j < j1; j++) {
+                const unsigned bit = dist2_rn(I.p, s_fr[j]) < t_near ? 1u << ((j - j0) & 31) : 0u;
+                if (j - j0 < 32)
+                    lo |= bit;
+                else
+                    hi |= bit;
+            }
+            near = (unsigned long long)hi << 32 | lo;
+            int k = 0;
+            for (unsigned long long m = near; m; m &= m - 1, k++) {
+                const int j = j0 + __ffsll((long long)m) - 1;
+                const unsigned bits = list_bits_sq(I, j, s_fr[j], s_fr[S + j], s_fr[2 * S + j], s_fr[3 * S + j],
+                                                   s_fl[j], cut);
+                c[0] += bits & 1u;
+                c[1] += (bits >> 1) & 1u;
+                c[2] += ((bits >> 2) & 1u) + (bits >> 3);
+                const unsigned long long at16 = (unsigned long long)bits << (4 * (k & 15));
+                got[0] |= k < 16 ? at16 : 0;   // 48 beads, 16 a word
+                got[1] |= k >= 16 && k < 32 ? at16 : 0;
+                got[2] |= k >= 32 ? at16 : 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) s_cnt[(4 * k + role) * S + l] = c[k];
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            c[k] = 0;
+            for (int r = 0; r < role; r++) c[k] += s_cnt[(4 * k + r) * S + l];
+        }
+        if (valid) {
+            int k = 0;
+            for (unsigned long long m = near; m; m &= m - 1, k++) {
+                const unsigned bits = (unsigned)((k < 16 ? got[0] : k < 32 ? got[1] : got[2]) >> (4 * (k & 15))) & 15u;
+                list_append(P, B, g, I, bits, j0 + __ffsll((long long)m) - 1, c[0], c[1], c[2], overflow);
+            }
+            if (role == 3) {   // the last quarter ends with the totals
+                if (P.lj_on) B.ljc[g] = min(c[0], P.maxLJ);
+                if (P.is_assembly) {
+                    B.lonc[g] = min(c[1], P.maxLong);
+                    B.latc[g] = min(c[2], P.maxLat);
+                }
+            }
+            if (overflow) atomicOr(B.err, kErrOverflow);
+        }
+        __syncthreads();
+    }
+    const bool moving = !(flags & (kFlagExtra | kFlagFixed));
+    const bool work = KEEP_FORCES ? !(flags & kFlagExtra) : moving;
+    ListHead H = {};
+    if (role < 3 && work) H = list_head(P, B, g);
+    // the noise of the lateral (angles) and LJ (xyz) groups' beads
+    uint4 seed = make_uint4(0u, 0u, 0u, 0u);
+    const bool draws = (role == 1 || role == 2) && moving;
+    uint4 *my_seed = B.seeds + (role == 1 ? nb + g : g);
+    if (draws) {
+        seed = *my_seed;
+        s_noise[(role == 1 ? S : 0) + l] = gauss4(seed);
+    }
+    float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int step = 0; step < nsteps; step++) {
+        const float4 *fr = s_fr + 4 * S * (step & 1);
+        const NbrView V = {fr, s_fl, S, 0};
+        Euler E;
+        if (work) {
+            const float4 p0 = fr[l];
+            if (role == 0) {
+                const Acc A = axial_force(P, B, V, g, flags, p0, fr[S + l], fr[2 * S + l].w, H);
+                const float v[9] = {A.fx, A.fy, A.fz, A.ffi, A.fpsi, A.fth, A.tx, A.ty, A.tz};
+#pragma unroll
+                for (int k = 0; k < 9; k++) s_part[(kPartA + k) * S + l] = v[k];
+            } else if (role == 1) {
+                const Acc T = lateral_force(P, B, V, g, flags, p0, f3(fr[2 * S + l]), f3(fr[3 * S + l]), H);
+                const float v[6] = {T.fx, T.fy, T.fz, T.tx, T.ty, T.tz};
+#pragma unroll
+                for (int k = 0; k < 6; k++) s_part[(kPartT + k) * S + l] = v[k];
+            } else if (role == 2) {
+                const float3 L = lj_force(P, B, V, g, p0, H);
+                s_part[kPartL * S + l] = L.x;
+                s_part[(kPartL + 1) * S + l] = L.y;
+                s_part[(kPartL + 2) * S + l] = L.z;
+            } else {
+                E = euler(fr[S + l].w, fr[2 * S + l].w);
+            }
+        }
+        __syncthreads();
+        if (role == 3 && work) {
+            Frame Fi;
+            Fi.p0 = fr[l];
+            Fi.p1 = fr[S + l];
+            Fi.p2 = fr[2 * S + l];
+            float v[kParts];
+#pragma unroll
+            for (int k = 0; k < kParts; k++) v[k] = s_part[k * S + l];
+            const Acc A = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]};
+            const Acc T = {v[9], v[10], v[11], 0.f, 0.f, 0.f, v[12], v[13], v[14]};
+            force_out(P, A, T, make_float3(v[15], v[16], v[17]), B.zs + traj, Fi.p0, E, f);
+            if (moving) {
+                const float4 *noise = s_noise + 2 * S * (step & 1);
+                Fi = em_update(P, Fi, f, noise[l], noise[S + l]);
+                float4 *to = s_fr + 4 * S * ((step & 1) ^ 1);
+                to[l] = Fi.p0;
+                to[S + l] = Fi.p1;
+                to[2 * S + l] = Fi.p2;
+                to[3 * S + l] = Fi.p3;
+            }
+        } else if (draws && step + 1 < nsteps) {
+            s_noise[2 * S * ((step & 1) ^ 1) + (role == 1 ? S : 0) + l] = gauss4(seed);
+        }
+        __syncthreads();
+    }
+    if (draws) *my_seed = seed;
+    if (!valid) return;
+    float4 *out = (nsteps & 1) ? B.frame_out : B.frame_in;
+    out[role * nb + g] = s_fr[(4 * (nsteps & 1) + role) * S + l];
+    if (KEEP_FORCES && role == 3) {
+        B.force[g] = make_float4(f[0], f[1], f[2], 0.f);
+        B.force[nb + g] = make_float4(f[3], f[4], f[5], 0.f);
+    }
+}
+
 // ------------------------------------------------------------- energies
 // energy_kernel (src/compute_cuda.cu:676-911): per-bead FP32 terms, halved;
 // block partial sums in FP64 over one trajectory chunk.
@@ -773,11 +952,13 @@ size_t period_smem_bytes(int nmax) { return (size_t)nmax * (4 * sizeof(float4) +
 bool period_fits(int nmax) {
     return nmax > 0 && nmax <= kPeriodThreads * kPeriodBeads && period_smem_bytes(nmax) <= kPeriodMaxSmem;
 }
-int period_prepare(int nmax) {
-    const int bytes = (int)period_smem_bytes(nmax);
-    if (cudaFuncSetAttribute(k_step_period<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_step_period<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+int period_prepare(int) {   // the limits of the largest trajectory: engines share the kernels
+    const int whole = (int)kPeriodMaxSmem, split = PeriodSplitSmem(kPeriodSplitBeads).total;
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (cudaFuncSetAttribute(k_step_period<false>, attr, whole) != cudaSuccess ||
+        cudaFuncSetAttribute(k_step_period<true>, attr, whole) != cudaSuccess ||
+        cudaFuncSetAttribute(k_period_split<false>, attr, split) != cudaSuccess ||
+        cudaFuncSetAttribute(k_period_split<true>, attr, split) != cudaSuccess)
         return -1;
     return 0;
 }
@@ -785,6 +966,15 @@ bool period_rebuilds(int nmax) { return nmax <= kPeriodRebuildMax; }
 void launch_step_period(const KParams &P, const DevBuffers &B, bool keep_forces, int nsteps, int nmax, bool rebuild,
                         cudaStream_t s) {
     int t = ((nmax + 31) / 32) * 32;
+    if (t <= kPeriodSplitBeads) {
+        const size_t bytes = PeriodSplitSmem(t).total;
+        const ListCuts cut = list_cuts(P);
+        if (keep_forces)
+            k_period_split<true><<<P.nt, 4 * t, bytes, s>>>(P, B, nsteps, rebuild ? 1 : 0, cut);
+        else
+            k_period_split<false><<<P.nt, 4 * t, bytes, s>>>(P, B, nsteps, rebuild ? 1 : 0, cut);
+        return;
+    }
     if (t > kPeriodThreads) t = kPeriodThreads;
     const size_t bytes = period_smem_bytes(nmax);
     if (keep_forces)

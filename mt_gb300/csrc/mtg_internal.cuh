@@ -266,6 +266,31 @@ __device__ __forceinline__ unsigned list_bits(const KParams &P, const ListSite &
     }
     return bits;
 }
+// The same decisions on squared distances: each cutoff is the smallest float
+// whose rounded root is not below it (list_cuts), so r2 < cut is sqrt(r2) < cutoff.
+struct ListCuts {
+    float lj, pair, site;
+};
+__device__ __forceinline__ float dist2_rn(float4 a, float4 b) {
+    return norm2_rn(make_float3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z)));
+}
+__device__ __forceinline__ unsigned list_bits_sq(const ListSite &I, int jl, float4 q, float4 uj, float4 l1j, float4 l2j,
+                                                 int fj, const ListCuts &cut) {
+    unsigned bits = 0;
+    const float r2 = dist2_rn(I.p, q);
+    if (I.do_lj && jl != I.il && r2 < cut.lj) bits |= 1u;
+    if (I.do_pairs && r2 < cut.pair && jl != I.hpart) {
+        if (((I.flags ^ fj) & kFlagBeta) != 0) {
+            const float3 d = site_delta(I.p, q, I.wi, make_float3(-uj.x * I.rmon, -uj.y * I.rmon, -uj.z * I.rmon));
+            if (norm2_rn(d) < cut.site) bits |= 2u;
+        }
+        if (jl != I.il) {
+            if (norm2_rn(site_delta(I.p, q, f3(I.l1), f3(l2j))) < cut.site) bits |= 4u;
+            if (norm2_rn(site_delta(I.p, q, f3(I.l2), f3(l1j))) < cut.site) bits |= 8u;
+        }
+    }
+    return bits;
+}
 // Appends bead j's entries to bead g's lists (k-major, capacity-checked).
 __device__ __forceinline__ void list_append(const KParams &P, const DevBuffers &B, int g, const ListSite &I,
                                             unsigned bits, int jl, int &nlj, int &nlo, int &nla, bool &overflow) {
@@ -327,7 +352,8 @@ __device__ __forceinline__ void tea_pack_position(const DevBuffers &B, int g, fl
 __device__ __forceinline__ void tea_pack_bead(const DevBuffers &B, int g, bool extra, float4 pos, float fx, float fy,
                                               float fz, float4 r) {
     int p, odd;
-    float *b = tea_pack_at(B, g, p, odd) + 4 * p + odd;
+    float *b = tea_pack_at(B, g, p, odd);
+    b += 4 * p + odd;
     constexpr int n = 4 * kTeaPairSlots;
     b[0] = extra ? kTeaFarAway : pos.x;
     b[2] = extra ? kTeaFarAway : pos.y;
@@ -397,6 +423,7 @@ void launch_forces_to_coords(const KParams &P, const float4 *force, float *coord
 void launch_rebuild(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,
                           cudaStream_t s);
+ListCuts list_cuts(const KParams &P);
 // The cell-list rebuild in one launch, each CTA binning its trajectory in
 // shared memory; work = chunks of kListThreads beads, nmax the largest trajectory.
 constexpr int kListThreads = 512;

@@ -70,3 +70,36 @@ def test_bending_of_large_angles(turns):
     ulp = np.spacing(np.abs(dpsi).astype(np.float32)).astype(np.float64)
     tol = p.C * 2.0 * 8 * 2.0 ** -22 + p.B_psi * (ulp + 4 * 2.0 ** -24)
     assert (np.abs(f[:, 5] - want)[near] <= tol[near]).all()
+
+
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("sizes", [(2, 0), (12, 0), (1, 8), (14, 10), (2, 38), (14, 12)], ids=str)
+def test_persistent_seed_equals_per_step_kernels(sizes, keep):
+    """The persistent kernel of small trajectories (four threads a bead, lists rebuilt
+    inside) against the per-step kernels, bit for bit: 13 x sizes[0] lattice and
+    sizes[1] free beads, fixed and extra beads, barriers and walls, period ends inside a run."""
+    from mt_gb300 import engine
+    p = synth.default_params(seed=81, barrier=1, is_wall=1, rep_r=15.0)
+    trajs = [synth.make_trajectory(*sizes, seed=81 + k, radius=8.12, psi_mode="make_mt", cube=40.0, thermal=0.05)
+             for k in range(3)]
+    b = synth.batch_from_trajectories(p, trajs)
+    b.extra[7:b.nbeads:31] = 1
+    runs = []
+    for persistent in (0, 1):
+        with engine.Engine(b) as e:
+            e.upload_state(b.coords)
+            e.set_keep_forces(keep)
+            t = e.tuning()
+            t["plain_persistent"] = persistent
+            e.set_tuning(**t)
+            for first, n in ((0, 20), (20, 7), (27, 1), (28, 14)):
+                e.step(first, n)
+            runs.append((e.download_state(forces=True), e.download_rng(), e.lists()))
+    (x0, f0), r0, l0 = runs[0]
+    (x1, f1), r1, l1 = runs[1]
+    assert np.array_equal(x0, x1) and np.array_equal(r0, r1)
+    if keep:
+        assert np.array_equal(f0, f1)
+    for k in ("lj", "long", "lat"):
+        assert np.array_equal(l0[k][0], l1[k][0]) and np.array_equal(l0[k][1], l1[k][1])
+    assert l0["lj"][0].max() > 1
