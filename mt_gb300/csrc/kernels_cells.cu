@@ -544,6 +544,7 @@ __device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &
 
 __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int2 *work, int nmax,
                                                                   float inv, ListCuts cut) {
+    chain_wait();
     extern __shared__ float4 s_dyn[];
     const int2 w = work[blockIdx.x];
     const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
@@ -729,7 +730,8 @@ ListCuts list_cuts(const KParams &P) { return {sq_below(P.ljcut), sq_below(kPair
 void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
                          cudaStream_t s) {
     const float inv = 1.0f / (P.ljcut * 1.001f + 1e-3f);   // the cells of bin_beads
-    k_cell_lists_smem<<<nwork, kListThreads, smem_list_bytes(nmax), s>>>(P, B, work, nmax, inv, list_cuts(P));
+    launch_chained(P, k_cell_lists_smem, nwork, kListThreads, smem_list_bytes(nmax), s, P, B, work, nmax, inv,
+                   list_cuts(P));
 }
 
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,

@@ -304,6 +304,7 @@ __device__ __forceinline__ Frame em_update(const KParams &P, const Frame &Fi, co
 // drawn while the neighbours are on their way.
 template <bool KEEP_FORCES>
 __global__ void __launch_bounds__(256, 4) k_step_plain(KParams P, DevBuffers B) {
+    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P.nb) return;
     const int nb = P.nb;
@@ -472,6 +473,7 @@ __device__ __forceinline__ float4 tea_random(const KParams &P, const DevBuffers 
 // the random force of every bead and lays the bead out for the all-pairs pass.
 template <bool TEA_PREPARE>
 __global__ void __launch_bounds__(256) k_forces(KParams P, DevBuffers B) {
+    chain_wait();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P.nb) return;
     const int nb = P.nb;
@@ -519,6 +521,7 @@ __device__ __forceinline__ void get_parts(float (*s)[kSplitBeads], int l, Acc &A
 // with the random force of every bead).
 template <bool STEP, bool KEEP_FORCES, bool TEA>
 __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B) {
+    chain_wait();
     __shared__ float s_part[kParts][kSplitBeads];
     const int role = threadIdx.x >> 5, l = threadIdx.x & 31, g = blockIdx.x * kSplitBeads + l;
     const int nb = P.nb;
@@ -604,6 +607,7 @@ struct PeriodSplitSmem {   // offsets in bytes; s: beads rounded up to a warp
 template <bool KEEP_FORCES>
 __global__ void __launch_bounds__(4 * kPeriodSplitBeads) k_period_split(KParams P, DevBuffers B, int nsteps,
                                                                         int rebuild, ListCuts cut) {
+    chain_wait();
     extern __shared__ float4 s_dyn[];
     char *smem = reinterpret_cast<char *>(s_dyn);
     const int S = blockDim.x >> 2, role = threadIdx.x / S, l = threadIdx.x % S;
@@ -928,25 +932,20 @@ void launch_coords_from_frames(const KParams &P, const float4 *frame, float *c7,
 void launch_forces_to_coords(const KParams &P, const float4 *force, float *c7, cudaStream_t s) {
     k_forces_to_coords<<<blocks(P.nb, 256), 256, 0, s>>>(P.nb, force, c7);
 }
-// Beads up to which the four-warp form is used.  It wins while its four times as
-// many warps stay within about one and a half fillings of the GPU: a step of one
-// 1520-bead trajectory took 6.8 us with one thread a bead and 4.6 us so, forces
-// of 52,800 beads 11.5 and 11.0 us, but a step of 78,780 beads 12.2 and 14.5 us.
-constexpr int kSplitMaxBeads = 55000;
 void launch_step_plain(const KParams &P, const DevBuffers &B, bool keep_forces, cudaStream_t s) {
     if (P.nb <= kSplitMaxBeads) {
         const int n = blocks(P.nb, kSplitBeads);
         if (keep_forces)
-            k_split<true, true, false><<<n, kSplitThreads, 0, s>>>(P, B);
+            launch_chained(P, k_split<true, true, false>, n, kSplitThreads, 0, s, P, B);
         else
-            k_split<true, false, false><<<n, kSplitThreads, 0, s>>>(P, B);
+            launch_chained(P, k_split<true, false, false>, n, kSplitThreads, 0, s, P, B);
         return;
     }
     const int t = P.step_block > 0 ? P.step_block : 128;
     if (keep_forces)
-        k_step_plain<true><<<blocks(P.nb, t), t, 0, s>>>(P, B);
+        launch_chained(P, k_step_plain<true>, blocks(P.nb, t), t, 0, s, P, B);
     else
-        k_step_plain<false><<<blocks(P.nb, t), t, 0, s>>>(P, B);
+        launch_chained(P, k_step_plain<false>, blocks(P.nb, t), t, 0, s, P, B);
 }
 size_t period_smem_bytes(int nmax) { return (size_t)nmax * (4 * sizeof(float4) + sizeof(int)); }
 bool period_fits(int nmax) {
@@ -970,9 +969,9 @@ void launch_step_period(const KParams &P, const DevBuffers &B, bool keep_forces,
         const size_t bytes = PeriodSplitSmem(t).total;
         const ListCuts cut = list_cuts(P);
         if (keep_forces)
-            k_period_split<true><<<P.nt, 4 * t, bytes, s>>>(P, B, nsteps, rebuild ? 1 : 0, cut);
+            launch_chained(P, k_period_split<true>, P.nt, 4 * t, bytes, s, P, B, nsteps, rebuild ? 1 : 0, cut);
         else
-            k_period_split<false><<<P.nt, 4 * t, bytes, s>>>(P, B, nsteps, rebuild ? 1 : 0, cut);
+            launch_chained(P, k_period_split<false>, P.nt, 4 * t, bytes, s, P, B, nsteps, rebuild ? 1 : 0, cut);
         return;
     }
     if (t > kPeriodThreads) t = kPeriodThreads;
@@ -987,15 +986,15 @@ void launch_forces(const KParams &P, const DevBuffers &B, bool tea_prepare, cuda
     if (P.nb <= kSplitMaxBeads) {
         const int n = blocks(P.nb, kSplitBeads);
         if (tea_prepare)
-            k_split<false, false, true><<<n, kSplitThreads, 0, s>>>(P, B);
+            launch_chained(P, k_split<false, false, true>, n, kSplitThreads, 0, s, P, B);
         else
-            k_split<false, false, false><<<n, kSplitThreads, 0, s>>>(P, B);
+            launch_chained(P, k_split<false, false, false>, n, kSplitThreads, 0, s, P, B);
         return;
     }
     if (tea_prepare)
-        k_forces<true><<<blocks(P.nb, 128), 128, 0, s>>>(P, B);
+        launch_chained(P, k_forces<true>, blocks(P.nb, 128), 128, 0, s, P, B);
     else
-        k_forces<false><<<blocks(P.nb, 128), 128, 0, s>>>(P, B);
+        launch_chained(P, k_forces<false>, blocks(P.nb, 128), 128, 0, s, P, B);
 }
 void launch_energy(const KParams &P, const DevBuffers &B, double *per_bead, double *partials, const int2 *work,
                    int nwork, cudaStream_t s) {

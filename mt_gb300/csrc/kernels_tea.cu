@@ -106,6 +106,7 @@ __device__ __forceinline__ void eps_store(const KParams &P, const DevBuffers &B,
 // exits become the kErrTeaEps bit.
 __global__ void __launch_bounds__(256) k_tea_beta(KParams P, DevBuffers B, int capricious, float epsmax,
                                                   const int *gate, int run_if) {
+    chain_wait();
     if (gate && *gate != run_if) return;
     const int t = blockIdx.x;
     const int base = B.off[t], end = B.off[t + 1];
@@ -414,6 +415,7 @@ __device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, 
 template <class Op>
 __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
                                                              float4 *feff, const int *gate, int run_if) {
+    chain_wait();
     if (gate && *gate != run_if) return;
     constexpr int kW = Op::kWords;
     __shared__ float4 s_tile[kTeaStages][kTeaTileBlocks * kW];
@@ -535,7 +537,8 @@ static int tea_runs(const KParams &P, bool rare) {
 template <class Op>
 static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
                        int run_if, cudaStream_t s) {
-    k_tea_pass<Op><<<tea_runs<Op>(P, gate && run_if == 1), kTeaThreads, 0, s>>>(P, B, work, nwork, feff, gate, run_if);
+    launch_chained(P, k_tea_pass<Op>, tea_runs<Op>(P, gate && run_if == 1), kTeaThreads, 0, s, P, B, work, nwork, feff,
+                   gate, run_if);
 }
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
     k_tea_pack<<<(P.nb + 127) / 128, 128, 0, s>>>(P, B);
@@ -552,7 +555,7 @@ void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int
 }
 void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious, float epsmax, const int *gate,
                            int run_if, cudaStream_t s) {
-    k_tea_beta<<<P.nt, 256, 0, s>>>(P, B, capricious, epsmax, gate, run_if);
+    launch_chained(P, k_tea_beta, P.nt, 256, 0, s, P, B, capricious, epsmax, gate, run_if);
 }
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s) {
     launch_tea_beta_gated(P, B, capricious, epsmax, nullptr, 0, s);
@@ -691,6 +694,7 @@ __device__ __forceinline__ void ff_pack_warp(const FFBuffers &F, int N, float3 x
 // the proxy charges Q_m = sum_j w_m(x_j) (F_j, R_j), and the leaf's beads in
 // the step kernel's tile layout (leaf nleaf: the padding leaf's pack).
 __global__ void __launch_bounds__(32 * kP2MWarps) k_ff_p2m(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
+    chain_wait();
     if (gate && *gate != 0) return;
     const int N = blockIdx.x * kP2MWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (N > F.nleaf) return;
@@ -874,6 +878,7 @@ __device__ __forceinline__ int ff_run_start(const FFBuffers &F, int units, int k
 }
 template <bool LISTCORR>
 __global__ void __launch_bounds__(32 * kFFWarps, 8) k_ff_near(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
+    chain_wait();
     if (gate && *gate != 0) return;
     __shared__ float4 s_leaf[kFFWarps][kFFStages][kFFPackF4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, run = blockIdx.x * kFFWarps + warp;
@@ -1079,7 +1084,7 @@ __global__ void k_ff_rest(KParams P, DevBuffers B, FFBuffers F, float4 *feff, co
 void launch_ff_p2m_leaves(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate,
                           cudaStream_t s) {
     if (F.nleaf == 0) return;
-    k_ff_p2m<<<(F.nleaf + kP2MWarps) / kP2MWarps, 32 * kP2MWarps, 0, s>>>(P, B, F, gate);
+    launch_chained(P, k_ff_p2m, (F.nleaf + kP2MWarps) / kP2MWarps, 32 * kP2MWarps, 0, s, P, B, F, gate);
 }
 void launch_ff_m2l(const KParams &P, const FFBuffers &F, const int *gate, cudaStream_t s) {
     if (F.nleaf == 0) return;
@@ -1110,9 +1115,9 @@ void launch_ff_near(const KParams &P, const DevBuffers &B, const FFBuffers &F, c
     if (F.nleaf == 0) return;
     const int ctas = (F.near_runs + kFFWarps - 1) / kFFWarps;
     if (ff_list_corr(P))
-        k_ff_near<true><<<ctas, 32 * kFFWarps, 0, s>>>(P, B, F, gate);
+        launch_chained(P, k_ff_near<true>, ctas, 32 * kFFWarps, 0, s, P, B, F, gate);
     else
-        k_ff_near<false><<<ctas, 32 * kFFWarps, 0, s>>>(P, B, F, gate);
+        launch_chained(P, k_ff_near<false>, ctas, 32 * kFFWarps, 0, s, P, B, F, gate);
 }
 void launch_ff_far(const KParams &P, const DevBuffers &B, const FFBuffers &F, bool feff_only, float4 *feff,
                    const int *gate, cudaStream_t s) {

@@ -158,6 +158,7 @@ KParams make_kparams(const mtg_params &p, int nb, int nt, int maxH, int maxLong,
     k.maxLat = maxLat;
     k.maxLJ = maxLJ;
     k.step_block = 128;
+    k.chain = 1;
     k.tea_a = p.tea_a;
     k.tea_var = sqrtf(2.0f * 0.0019872041f * p.Temp * p.gammaR / p.dt);
     return k;
@@ -1170,6 +1171,7 @@ int mtg_set_kernel_timing(mtg_engine *e, int on) {
     cudaSetDevice(e->device);
     if (e->timing != (on != 0)) destroy_graphs(e);
     e->timing = on != 0;
+    e->kp.chain = e->timing ? 0 : 1;
     return MTG_OK;
 }
 

@@ -63,6 +63,7 @@ struct KParams {
     int tea_slices;        // threads per bead in the near-pair kernel of learned TEA (1, 2, 4 or 8)
     int tea_max_blocks;    // blocks of kTeaBlock beads of the largest trajectory
     long long tea_units;   // (chunk of kTeaChunk beads) x (block) pairs of the all-pairs kernels
+    int chain;             // launch the kernels of a step chained (launch_chained)
     int step_block;        // threads per CTA of the fused plain step (64, 128 or 256)
 };
 
@@ -413,6 +414,44 @@ __device__ __forceinline__ int cell_coord(float x, float inv) {
 }
 __device__ __forceinline__ uint32_t cell_hash(int cx, int cy, int cz) {
     return ((uint32_t)cx * 73856093u) ^ ((uint32_t)cy * 19349663u) ^ ((uint32_t)cz * 83492791u);
+}
+
+// Beads up to which the four-warp form is used.  It wins while its four times as
+// many warps stay within about one and a half fillings of the GPU: a step of one
+// 1520-bead trajectory took 6.8 us with one thread a bead and 4.6 us so, forces
+// of 52,800 beads 11.5 and 11.0 us, but a step of 78,780 beads 12.2 and 14.5 us.
+constexpr int kSplitMaxBeads = 55000;
+
+// ------------------------------------------------------- chained launches
+// The kernels of a step follow one another on one stream.  Chained (programmatic
+// dependent launch), the next kernel's CTAs are put on the SMs while the last
+// CTAs of the one before still run, and wait there: chain_wait() returns when
+// everything before on the stream is complete and visible.  Every kernel that may be
+// launched so calls it first of all, also where it then has nothing to do: a
+// kernel that ended without it could let its successor overtake its predecessor.
+// Batches of the four-warp form only: a launch there costs up to 1 us less (one
+// 1520-bead trajectory, 200 steps, 1.14 -> 1.06 ms), but the waiting CTAs slow a full
+// GPU down (1024 uneven trajectories, 50 steps, 6.85 -> 7.58 ms).
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// k<<<grid, block, smem, s>>>(args...), chained if P.chain (off while per-kernel
+// timing puts events between the launches).
+template <class... KA, class... A>
+inline void launch_chained(const KParams &P, void (*k)(KA...), int grid, int block, size_t smem, cudaStream_t s,
+                           const A &...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &attr;
+    c.numAttrs = P.chain && P.nb <= kSplitMaxBeads ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, KA(args)...);
 }
 
 // ------------------------------------------------------ host entry points
