@@ -421,13 +421,8 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 constexpr int kSmemKeys = 32;      // keys a bead can keep; more take the slow path below
 constexpr int kSmemBeads = 8192;   // 13 bits of a key
 
-__host__ __device__ inline int smem_buckets(int n) {
-    int m = 64;
-    while (m < 2 * n) m <<= 1;
-    return m;
-}
 size_t smem_list_bytes(int nmax) {
-    return sizeof(float4) * (size_t)nmax + sizeof(uint16_t) * ((size_t)smem_buckets(nmax) + kSmemKeys * kListThreads);
+    return sizeof(float4) * (size_t)nmax + sizeof(uint16_t) * ((size_t)row_buckets(nmax) + kSmemKeys * kListThreads);
 }
 
 // Batcher's odd-even merge sort of N keys in registers, ascending.
@@ -465,9 +460,6 @@ struct SmemCells {
     int n, m;
     float inv;
 };
-__device__ __forceinline__ uint32_t row_hash(int cy, int cz) {
-    return ((uint32_t)cy * 19349663u) ^ ((uint32_t)cz * 83492791u);
-}
 // Calls hit(slot) for every bead of the trajectory in the cells around p that
 // is closer than the root of t2, in no particular order; once for every row whose
 // buckets hold it, so a bead whose own row shares them can come twice.
@@ -548,12 +540,12 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     extern __shared__ float4 s_dyn[];
     const int2 w = work[blockIdx.x];
     const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
-    const int m = smem_buckets(n), t = threadIdx.x;
+    const int m = row_buckets(n), t = threadIdx.x;
     const float4 *fr = B.frame_in;
     float4 *s_pos = s_dyn;
     unsigned *s_tab = reinterpret_cast<unsigned *>(s_dyn + nmax);             // two 16-bit buckets a word
     uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab);
-    uint16_t (*s_key)[kListThreads] = reinterpret_cast<uint16_t (*)[kListThreads]>(s_end + smem_buckets(nmax));
+    uint16_t (*s_key)[kListThreads] = reinterpret_cast<uint16_t (*)[kListThreads]>(s_end + row_buckets(nmax));
     __shared__ unsigned s_warp[kListThreads / 32];
 
     // the beads in bucket order
@@ -687,6 +679,123 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     if (W.overflow) atomicOr(B.err, kErrOverflow);
 }
 
+// ------------------------------------------------ ordered binning in one CTA
+// bin_beads with ordered buckets, one CTA per trajectory of up to kOrderBeads
+// beads: counts, scan and fill in shared memory, then every bead's rank among the
+// beads of its bucket (ascending index, so that sums over a bucket are
+// reproducible) and its place in the ordered copy.  Also the trajectory's centroid
+// and non-extra count.  Before: five launches, the sort with one thread a bucket
+// in global memory; 64 x 5600 beads 138 us, 40 us so.
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderBeads = 16384;
+__host__ __device__ inline int order_buckets(int n) {   // the table sizes of CellBuffers
+    int m = 32;
+    while (m < n) m <<= 1;
+    return m;
+}
+inline size_t order_bytes(int nmax) { return sizeof(uint16_t) * ((size_t)order_buckets(nmax) + nmax); }
+
+// Sum in two floats (Knuth's two-sum): the accuracy a centroid needs without the FP64
+// pipe, which the additions of a CTA would fill.  A sum that has left the finite numbers is its
+// first float.
+struct Sum2 {
+    float s = 0.f, e = 0.f;
+    __device__ __forceinline__ void add(float x, float xe) {
+        const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+        e = __fadd_rn(e, __fadd_rn(xe, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z))));
+        s = t;
+    }
+    __device__ __forceinline__ double value() const { return isfinite(s) ? (double)s + (double)e : (double)s; }
+};
+
+__global__ void __launch_bounds__(kOrderThreads) k_cell_order(KParams P, DevBuffers B, CellBuffers C, float inv,
+                                                              float4 *stats) {
+    extern __shared__ unsigned s_tab[];                     // two 16-bit buckets a word, then the indices
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, traj = blockIdx.x;
+    const int base = B.off[traj], n = B.off[traj + 1] - base, tb = C.tbase[traj], m = C.tmask[traj] + 1;
+    uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab), *s_idx = s_end + m;
+    __shared__ Sum2 s_sum[kOrderThreads / 32][3];
+    __shared__ unsigned s_warp[kOrderThreads / 32], s_act[kOrderThreads / 32];
+    for (int k = t; k < m / 2; k += kOrderThreads) s_tab[k] = 0;
+    __syncthreads();
+    auto bucket = [&](float4 p) {
+        return (int)(cell_hash(cell_coord(p.x, inv), cell_coord(p.y, inv), cell_coord(p.z, inv)) & (uint32_t)(m - 1));
+    };
+    Sum2 c[3];
+    unsigned act = 0;
+    for (int j = t; j < n; j += kOrderThreads) {
+        const float4 p = B.frame_in[base + j];
+        const int b = bucket(p);
+        atomicAdd(&s_tab[b >> 1], 1u << (16 * (b & 1)));
+        if (B.flags[base + j] & kFlagExtra) continue;
+        c[0].add(p.x, 0.f);
+        c[1].add(p.y, 0.f);
+        c[2].add(p.z, 0.f);
+        act++;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+        for (int d = 0; d < 3; d++)
+            c[d].add(__shfl_xor_sync(0xffffffffu, c[d].s, o), __shfl_xor_sync(0xffffffffu, c[d].e, o));
+    act = __reduce_add_sync(0xffffffffu, act);
+    if (lane == 0) {
+        for (int d = 0; d < 3; d++) s_sum[wid][d] = c[d];
+        s_act[wid] = act;
+    }
+    __syncthreads();
+    {   // exclusive scan of the counts, whole words a thread
+        const int per = (m / 2 + kOrderThreads - 1) / kOrderThreads, lo = min(m / 2, t * per), hi = min(m / 2, lo + per);
+        unsigned sum = 0;
+        for (int k = lo; k < hi; k++) sum += (s_tab[k] & 0xffffu) + (s_tab[k] >> 16);
+        unsigned v = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) s_warp[wid] = v;
+        __syncthreads();
+        unsigned run = v - sum;
+        for (int k = 0; k < wid; k++) run += s_warp[k];
+        for (int k = lo; k < hi; k++) {
+            const unsigned both = s_tab[k], c0 = both & 0xffffu, c1 = both >> 16;
+            s_tab[k] = run | ((run + c0) << 16);
+            C.start[tb + 2 * k] = (int)run;
+            C.start[tb + 2 * k + 1] = (int)(run + c0);
+            C.cnt[tb + 2 * k] = (int)c0;
+            C.cnt[tb + 2 * k + 1] = (int)c1;
+            run += c0 + c1;
+        }
+    }
+    if (t == 0) {
+        unsigned count = 0;
+        for (int w = 0; w < kOrderThreads / 32; w++) {
+            count += s_act[w];
+            if (w > 0)
+                for (int d = 0; d < 3; d++) c[d].add(s_sum[w][d].s, s_sum[w][d].e);
+        }
+        const double inv_n = count > 0 ? 1.0 / count : 0.0;
+        stats[traj] = make_float4((float)(c[0].value() * inv_n), (float)(c[1].value() * inv_n),
+                                  (float)(c[2].value() * inv_n), (float)count);
+    }
+    __syncthreads();
+    for (int j = t; j < n; j += kOrderThreads) {
+        const int b = bucket(B.frame_in[base + j]), sh = 16 * (b & 1);
+        s_idx[(atomicAdd(&s_tab[b >> 1], 1u << sh) >> sh) & 0xffffu] = (uint16_t)j;
+    }
+    __syncthreads();
+    for (int j = t; j < n; j += kOrderThreads) {
+        const int g = base + j;
+        float4 p = B.frame_in[g];
+        const int b = bucket(p), e = s_end[b];
+        int slot = b > 0 ? s_end[b - 1] : 0;
+        int rank = 0;
+        for (int k = slot; k < e; k++) rank += s_idx[k] < j;
+        slot += rank;
+        C.cell_bead[base + slot] = g;
+        p.w = __int_as_float(g | ((B.flags[g] & kFlagExtra) ? kCellExtraBit : 0));
+        C.cell_pos[base + slot] = p;
+    }
+}
+
 inline int nblk(int n, int t) { return (n + t - 1) / t; }
 
 }  // namespace
@@ -704,6 +813,20 @@ float bin_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, flo
     if (ordered)
         k_cell_sort<<<dim3(P.nt, (C.max_buckets + 127) / 128), 128, 0, s>>>(B.off, C.tbase, C.tmask, C.start, C.cnt,
                                                                             C.cell_bead, C.cell_pos);
+    return inv;
+}
+
+bool order_beads_applies(int nmax) { return nmax <= kOrderBeads; }
+int order_beads_prepare() {   // the limit of the largest trajectory: engines share the kernel
+    return cudaFuncSetAttribute(k_cell_order, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)order_bytes(kOrderBeads)) == cudaSuccess
+               ? 0
+               : -1;
+}
+float order_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, float reach, int nmax, float4 *stats,
+                  cudaStream_t s) {
+    const float inv = 1.0f / (reach * 1.001f + 1e-3f);   // the cells of bin_beads
+    k_cell_order<<<P.nt, kOrderThreads, order_bytes(nmax), s>>>(P, B, C, inv, stats);
     return inv;
 }
 

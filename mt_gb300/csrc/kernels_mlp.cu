@@ -7,6 +7,9 @@
 //   k_mlp_adam      : reduces the per-CTA partial gradients, Adam step on
 //                     the FP32 masters, refreshes both BF16 copies (forward
 //                     [out][in] and transposed [in][out])
+//   k_mlp_grad_sum  : the gradient of one batch from the partial gradients
+//                     (summed on the host until now: 4.8 MB of parts came back
+//                     for 4096 samples instead of 0.15)
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -48,6 +51,21 @@ __global__ void k_mlp_loss_sum(const float *part, int nparts, float *out) {
         for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += w[k];
         *out = t;
     }
+}
+
+// Gradient of a batch: the per-CTA parts summed in FP64 in their order.
+__global__ void k_mlp_grad_sum(const float *G, int nparts, float *grad) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kParams) return;
+    double g = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < nparts; p++) g += (double)G[(size_t)p * kParams + i];
+    grad[i] = (float)g;
+}
+
+cudaError_t launch_grad_sum(const float *G, int nparts, float *grad, cudaStream_t s) {
+    k_mlp_grad_sum<<<(kParams + 127) / 128, 128, 0, s>>>(G, nparts, grad);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_adam(const Weights &W, const float *G, int nparts, float lr, int step, cudaStream_t s) {

@@ -422,6 +422,17 @@ __device__ __forceinline__ uint32_t cell_hash(int cx, int cy, int cz) {
 // of 52,800 beads 11.5 and 11.0 us, but a step of 78,780 beads 12.2 and 14.5 us.
 constexpr int kSplitMaxBeads = 55000;
 
+// Bucket of cell (cx, cy, cz) = (row_hash(cy, cz) + cx) mod a power of two: the
+// cells of a row along x are neighbouring buckets.
+__device__ __forceinline__ uint32_t row_hash(int cy, int cz) {
+    return ((uint32_t)cy * 19349663u) ^ ((uint32_t)cz * 83492791u);
+}
+__host__ __device__ inline int row_buckets(int n) {   // at least 2 n
+    int m = 64;
+    while (m < 2 * n) m <<= 1;
+    return m;
+}
+
 // ------------------------------------------------------- chained launches
 // The kernels of a step follow one another on one stream.  Chained (programmatic
 // dependent launch), the next kernel's CTAs are put on the SMs while the last
@@ -476,6 +487,12 @@ void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work
 // on the arrival order of the atomic fill).
 float bin_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, float reach, bool ordered,
                 cudaStream_t s);
+// bin_beads(ordered) in one launch, with the centroid and non-extra count of each
+// trajectory in stats (x, y, z, count), for trajectories order_beads_applies() to.
+bool order_beads_applies(int nmax);
+int order_beads_prepare();                        // opts the kernel into its shared memory (outside captures)
+float order_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, float reach, int nmax, float4 *stats,
+                  cudaStream_t s);
 void launch_step_plain(const KParams &P, const DevBuffers &B, bool keep_forces, cudaStream_t s);
 void launch_forces(const KParams &P, const DevBuffers &B, bool tea_prepare, cudaStream_t s);
 // Persistent run of nsteps plain steps (no rebuild inside), one CTA per

@@ -49,6 +49,7 @@ __device__ __forceinline__ void refresh_one(const Weights &W, int i, float w) {
 }
 
 cudaError_t launch_adam(const Weights &W, const float *G, int nparts, float lr, int step, cudaStream_t s);
+cudaError_t launch_grad_sum(const float *G, int nparts, float *grad, cudaStream_t s);
 cudaError_t launch_refresh(const Weights &W, cudaStream_t s);
 cudaError_t launch_loss_sum(const float *part, int nparts, float *out, cudaStream_t s);
 

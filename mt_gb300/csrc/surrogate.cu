@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <random>
 #include <vector>
@@ -319,6 +320,12 @@ struct mtg_surrogate {
     __nv_bfloat16 *bf = nullptr;  // all BF16 copies
     int *err = nullptr;            // device error word of the tensor-core inference
     int adam_step = 0;
+    // Device scratch of predict and loss_grad: one allocation, kept up to
+    // kScratchKeep bytes between calls (six cudaMalloc / cudaFree pairs cost more
+    // than the kernels of a 4096-sample batch), held by one call at a time.
+    std::mutex scratch_lock;
+    char *scratch = nullptr;
+    size_t scratch_bytes = 0;
     uint32_t spin = mlp::tc_default_spin();   // polls of the inference's waits for its MMAs
 };
 
@@ -336,6 +343,41 @@ int sfail(int code, const char *msg) {
         cudaError_t e_ = (call);                                                   \
         if (e_ != cudaSuccess) return sfail(MTG_E_CUDA, cudaGetErrorString(e_));   \
     } while (0)
+
+constexpr size_t kScratchKeep = 64u << 20;
+
+// The scratch for one call, cut into 256-byte aligned float arrays.  Released at
+// the end of the call (every call ends with its stream idle) when it is large.
+struct ScratchLease {
+    mtg_surrogate *s;
+    std::lock_guard<std::mutex> lock;
+    size_t used = 0;
+    explicit ScratchLease(mtg_surrogate *s_) : s(s_), lock(s_->scratch_lock) {}
+    ~ScratchLease() {
+        if (s->scratch_bytes > kScratchKeep) drop();
+    }
+    void drop() {
+        cudaFree(s->scratch);
+        s->scratch = nullptr;
+        s->scratch_bytes = 0;
+    }
+    static size_t room(size_t floats) { return (floats * sizeof(float) + 255) / 256 * 256; }
+    cudaError_t reserve(size_t bytes) {
+        if (bytes <= s->scratch_bytes) return cudaSuccess;
+        drop();
+        const cudaError_t e = cudaMalloc(&s->scratch, bytes);
+        if (e == cudaSuccess)
+            s->scratch_bytes = bytes;
+        else
+            s->scratch = nullptr;
+        return e;
+    }
+    float *take(size_t floats) {
+        float *p = reinterpret_cast<float *>(s->scratch + used);
+        used += room(floats);
+        return p;
+    }
+};
 
 int upload_norms(mtg_surrogate *s) {
     SCK(cudaMemcpyAsync(s->norm, s->h_norm, sizeof(s->h_norm), cudaMemcpyHostToDevice, s->stream));
@@ -401,6 +443,7 @@ int mtg_surrogate_destroy(mtg_surrogate *s) {
     if (!s) return MTG_OK;
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
+    cudaFree(s->scratch);
     cudaFree(s->W.master);
     cudaFree(s->bf);
     cudaFree(s->norm);
@@ -444,17 +487,16 @@ int mtg_surrogate_set_params(mtg_surrogate *s, const float *params, const float 
 int mtg_surrogate_predict(mtg_surrogate *s, const float *X, int n, float *Y) {
     if (!s || !X || !Y || n < 0) return sfail(MTG_E_CONFIG, "bad arguments");
     SCK(cudaSetDevice(s->device));
-    float *dX = nullptr, *dY = nullptr;
-    SCK(cudaMalloc(&dX, sizeof(float) * (size_t)n * mlp::kIn + 16));
-    SCK(cudaMalloc(&dY, sizeof(float) * (size_t)n * mlp::kOut + 16));
+    ScratchLease A(s);
+    const size_t nx = (size_t)n * mlp::kIn, ny = (size_t)n * mlp::kOut;
+    SCK(A.reserve(A.room(nx) + A.room(ny) + 256));
+    float *dX = A.take(nx), *dY = A.take(ny);
     SCK(cudaMemcpyAsync(dX, X, sizeof(float) * (size_t)n * mlp::kIn, cudaMemcpyHostToDevice, s->stream));
     SCK(mlp::launch_infer_tc(s->W, dX, n, s->norm, dY, s->err, s->stream, s->spin));
     int herr = 0;
     SCK(cudaMemcpyAsync(Y, dY, sizeof(float) * (size_t)n * mlp::kOut, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(&herr, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
-    cudaFree(dX);
-    cudaFree(dY);
     if (herr) {
         cudaMemsetAsync(s->err, 0, sizeof(int), s->stream);
         return sfail(MTG_E_TIMEOUT, "a bounded wait for the tensor cores ran out");
@@ -476,38 +518,30 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     for (int i = 0; i < n; i++)
         for (int k = 0; k < mlp::kOut; k++)
             Tn[(size_t)i * mlp::kOut + k] = (T[(size_t)i * mlp::kOut + k] - s->h_ynorm[k]) / s->h_ynorm[mlp::kOut + k];
-    float *dX, *dT, *dY, *dZ, *dG, *dL;
-    SCK(cudaMalloc(&dX, sizeof(float) * (size_t)n * mlp::kIn));
-    SCK(cudaMalloc(&dT, sizeof(float) * (size_t)n * mlp::kOut));
-    SCK(cudaMalloc(&dY, sizeof(float) * (size_t)n * mlp::kOut));
-    SCK(cudaMalloc(&dZ, sizeof(float) * (size_t)n * 3 * mlp::kHid));
-    SCK(cudaMalloc(&dG, sizeof(float) * (size_t)parts * mlp::kParams));
-    SCK(cudaMalloc(&dL, sizeof(float) * parts));
+    ScratchLease A(s);
+    const size_t nx = (size_t)n * mlp::kIn, ny = (size_t)n * mlp::kOut, nz = (size_t)n * 3 * mlp::kHid,
+                 ng = (size_t)parts * mlp::kParams;
+    SCK(A.reserve(A.room(nx) + 2 * A.room(ny) + A.room(nz) + A.room(ng) + A.room(mlp::kParams) + A.room(parts)));
+    float *dX = A.take(nx), *dT = A.take(ny), *dY = A.take(ny), *dZ = A.take(nz), *dG = A.take(ng),
+          *dSum = A.take(mlp::kParams), *dL = A.take(parts);
     SCK(cudaMemcpyAsync(dX, X, sizeof(float) * (size_t)n * mlp::kIn, cudaMemcpyHostToDevice, s->stream));
     SCK(cudaMemcpyAsync(dT, Tn.data(), sizeof(float) * Tn.size(), cudaMemcpyHostToDevice, s->stream));
     SCK(mlp::launch_forward_tc(s->W, dX, nullptr, n, s->norm, dY, dZ, s->err, s->stream));
     SCK(mlp::launch_backward_tc(s->W, dX, nullptr, s->norm, dT, n, dY, dZ, dG, dL, s->err, s->stream));
-    std::vector<float> G((size_t)parts * mlp::kParams), L(parts);
+    if (grad) SCK(mlp::launch_grad_sum(dG, parts, dSum, s->stream));
+    std::vector<float> L(parts);
     int herr = 0;
-    SCK(cudaMemcpyAsync(G.data(), dG, sizeof(float) * G.size(), cudaMemcpyDeviceToHost, s->stream));
+    if (grad) SCK(cudaMemcpyAsync(grad, dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(L.data(), dL, sizeof(float) * parts, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(&herr, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
     if (herr) {
-        for (float *p : {dX, dT, dY, dZ, dG, dL}) cudaFree(p);
         cudaMemsetAsync(s->err, 0, sizeof(int), s->stream);
         return sfail(MTG_E_TIMEOUT, "a bounded wait for the tensor cores ran out");
     }
-    for (float *p : {dX, dT, dY, dZ, dG, dL}) cudaFree(p);
     double l = 0.0;
     for (float v : L) l += v;
     if (loss) *loss = l / ((double)n * mlp::kOut);
-    if (grad)
-        for (int i = 0; i < mlp::kParams; i++) {
-            double g = 0.0;
-            for (int p = 0; p < parts; p++) g += G[(size_t)p * mlp::kParams + i];
-            grad[i] = (float)g;
-        }
     return MTG_OK;
 }
 
@@ -619,6 +653,23 @@ int mtg_surrogate_train(mtg_surrogate *s, const float *X, const float *T, int n,
     return MTG_OK;
 }
 
+}  // extern "C"
+
+// Descriptors of the current state into surr_desc.
+static void launch_descriptors(mtg_engine *e, const int *gate) {
+    const DevBuffers B = e->bufs();
+    float inv;
+    if (order_beads_applies(e->max_traj_beads)) {
+        inv = order_beads(e->kp, B, e->cells(), kDescCut, e->max_traj_beads, e->surr_stats, e->stream);
+    } else {
+        k_traj_stats<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_stats);
+        inv = bin_beads(e->kp, B, e->cells(), kDescCut, true, e->stream);
+    }
+    k_descriptors<<<e->nwork, kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv, e->surr_stats, e->surr_desc, gate);
+}
+
+extern "C" {
+
 // --------------------------------------------------- engine integration
 // Descriptors of the current state and, with TEA on, the exact targets
 // (an epsilon pass is run first).  X [nb*32], T [nb*4] (either may be NULL).
@@ -630,10 +681,7 @@ int mtg_tea_training_data(mtg_engine *e, float *X, float *T) {
     int rc = mtg_surrogate_buffers(e);
     if (rc) return rc;
     const DevBuffers B = e->bufs();
-    k_traj_stats<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_stats);
-    const float inv = bin_beads(e->kp, B, e->cells(), kDescCut, true, e->stream);
-    k_descriptors<<<e->nwork, kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv, e->surr_stats, e->surr_desc,
-                                                     nullptr);
+    launch_descriptors(e, nullptr);
     if (T) {
         launch_tea_pack(e->kp, B, e->stream);
         launch_tea_eps(e->kp, B, e->tea_work, e->tea_nwork, e->stream);
@@ -658,6 +706,8 @@ int mtg_surrogate_buffers(mtg_engine *e) {
     SCK(cudaMalloc(&e->surr_desc, sizeof(float) * nb * kF));
     SCK(cudaMalloc(&e->surr_pred, sizeof(float) * nb * mlp::kOut));
     SCK(cudaMalloc(&e->surr_stats, sizeof(float4) * e->nt));
+    if (order_beads_prepare() != 0)
+        return mtg_internal_fail(MTG_E_CUDA, "the binning kernel could not reserve its shared memory");
     SCK(cudaMalloc(&e->surr_gate, sizeof(int) * 3));
     SCK(cudaMalloc(&e->surr_err, sizeof(double)));
     SCK(cudaMalloc(&e->surr_part, sizeof(double) * 2 * kMobBlocks));
@@ -678,10 +728,7 @@ int mtg_surrogate_buffers(mtg_engine *e) {
 void enqueue_surrogate_eps(mtg_engine *e) {
     const DevBuffers B = e->bufs();
     const int *gate = e->surr_gate;
-    k_traj_stats<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_stats);
-    const float inv = bin_beads(e->kp, B, e->cells(), kDescCut, true, e->stream);
-    k_descriptors<<<e->nwork, kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv, e->surr_stats, e->surr_desc,
-                                                     gate);
+    launch_descriptors(e, gate);
     mlp::launch_infer_tc(e->surr->W, e->surr_desc, e->nb, e->surr->norm, e->surr_pred, e->err, e->stream,
                          e->surr->spin);
     k_surr_beta<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_pred, e->surr->ynorm, gate);
