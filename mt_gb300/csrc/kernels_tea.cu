@@ -869,15 +869,14 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
 // that close (checked by the launcher), by the run that begins the leaf;
 // otherwise they are looked for in the leaves whose smallest r^2 shows one, as
 // the all-pairs pass does.
-constexpr int kFFStages = 3, kFFWarps = 4;
-constexpr int kFFRunsPerSlot = 2;   // runs for every warp that fits the device, see kTeaRunsPerSlot
+constexpr int kFFStages = 3;
 static_assert(kFFLeaf == kTeaBlock && kFFPackF4 == kTeaBlockF4, "leaves are blocks of the pair loop");
 // first near entry of run k of F.near_runs
 __device__ __forceinline__ int ff_run_start(const FFBuffers &F, int units, int k) {
     return (int)((long long)k * units / F.near_runs);
 }
 template <bool LISTCORR>
-__global__ void __launch_bounds__(32 * kFFWarps, 8) k_ff_near(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
+__global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
     chain_wait();
     if (gate && *gate != 0) return;
     __shared__ float4 s_leaf[kFFWarps][kFFStages][kFFPackF4];
@@ -1096,15 +1095,6 @@ void launch_ff_m2l(const KParams &P, const FFBuffers &F, const int *gate, cudaSt
 void launch_ff_proxies(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s) {
     launch_ff_p2m_leaves(P, B, F, gate, s);
     launch_ff_m2l(P, F, gate, s);
-}
-
-// Runs of the near lists: a few for each warp the device holds at once, or one an entry.
-int ff_near_runs(int entries) {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int warps = sms * 8 * kFFWarps * kFFRunsPerSlot;
-    return entries < warps ? entries : warps;
 }
 
 // Overlapping pairs can be taken from the LJ list when it holds every pair

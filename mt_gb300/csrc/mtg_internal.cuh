@@ -549,6 +549,8 @@ constexpr int kTile = 128;   // beads per CTA tile of the O(N^2) kernels
 // of the nodes far from it, interpolated to each bead of the node.
 constexpr int kFFLeaf = 32;
 constexpr float kFFNode = 0.70710678f;
+constexpr int kFFWarps = 4, kFFCtas = 8;   // warps of a CTA of the near-pair kernel, CTAs an SM
+constexpr int kFFRunsPerSlot = 2;      // runs of the near lists for every warp that fits the device
 constexpr int kFFMaxAnc = 16;          // nodes with far fields on a leaf's path to the root (tree depth bound)
 struct FFBuffers {
     int nleaf, nnode, ntgt, ninner, nrest;
@@ -572,7 +574,7 @@ struct FFBuffers {
     float4 *phi;             // [24*nnode] target proxy n: (A.xyz, B0.x), (B0.yz, B1.xy), (B1.z, B2.xyz) at 24N+3n
     float4 *pack;            // [(nleaf+1)*kFFPackF4] each leaf's beads in the tile layout of the step kernel
                              // (leaf nleaf: padding, far away with zero F and R), written every step by P2M
-    int near_runs;           // warps the near lists are divided over (ff_near_runs)
+    int near_runs;           // warps the near lists are divided over
     float4 *nearpart;        // [2 * near_runs][kFFLeaf] parts of the near sums of leaves that runs share
     float4 *nearsum;         // [leaf beads] each bead's near-pair sum, in leaf bead order
 };
@@ -589,7 +591,6 @@ void launch_ff_p2m_leaves(const KParams &P, const DevBuffers &B, const FFBuffers
 void launch_ff_m2l(const KParams &P, const FFBuffers &F, const int *gate, cudaStream_t s);
 // both of the above
 void launch_ff_proxies(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s);
-int ff_near_runs(int entries);
 // near-pair sums; needs the leaf proxies' packed beads
 void launch_ff_near(const KParams &P, const DevBuffers &B, const FFBuffers &F, const int *gate, cudaStream_t s);
 // far field + update (FEFF: effective forces into feff, no update); needs the near sums and M2L
