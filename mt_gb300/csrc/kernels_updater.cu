@@ -29,10 +29,14 @@ constexpr float kMtRad = 8.12f + 2.0f * 8.0f;
 __device__ __forceinline__ int dimer_slots(const int *off, int t) { return (off[t + 1] - off[t]) / 2; }
 
 // rad = |(x, y)| < R_MT + R_THRES, rad > 1, cos(theta) > cos(ANG_THRES): the
-// bead is on the tubule (src/updater.cpp:166-168); counts per trajectory.
+// bead is on the tubule (src/updater.cpp:166-168); counts per trajectory.  The lanes
+// of a warp that hold beads of one trajectory add once: with an atomic for every
+// bead the adds to one address set the time (101 x 780 beads all on the tubule: 34 us,
+// 4.5 us so).
 __global__ void k_mt_length(int nb, const int *traj, const float4 *frame, int *flags, int save_prev, float cos_thres,
                             int *counts) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned warp = __ballot_sync(0xffffffffu, g < nb);
     if (g >= nb) return;
     const float4 p = frame[g];
     const float theta = frame[2 * nb + g].w;
@@ -42,7 +46,10 @@ __global__ void k_mt_length(int nb, const int *traj, const float4 *frame, int *f
     if (save_prev) f = (f & kFlagOnTubule) ? (f | kFlagOnTubPrev) : (f & ~kFlagOnTubPrev);
     f = on ? (f | kFlagOnTubule) : (f & ~kFlagOnTubule);
     flags[g] = f;
-    if (on) atomicAdd(&counts[traj[g]], 1);   // integer sums: order-independent
+    const int t = traj[g];
+    const unsigned same = __match_any_sync(warp, t);
+    const unsigned ons = __ballot_sync(warp, on) & same;
+    if (ons != 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&counts[t], __popc(ons));   // integer sums: order-independent
 }
 
 // Candidate dimers of the hydrolysis loop (src/updater.cpp:232-235): dimer k
