@@ -413,16 +413,19 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 //   * A hit is a 16-bit key: index * 8 + which site tests can succeed (the
 //     partner's centre within 4.51 nm of the bead's own site: sites are at most
 //     2 nm from a centre and bonds at most 2.5 nm long).  Keys are sorted in
-//     registers (Batcher's odd-even merge network, up to 16), so the lists come out in
+//     registers (Batcher's odd-even merge network, up to 24), so the lists come out in
 //     ascending j; only the site planes that a test needs are then gathered.
+// Bound by instruction issue and, in the walk, by shared-memory bandwidth.
 // 256 x 1520 beads: 203 us for the general path's six launches (the 27-bucket
-// walk ran 7600 instructions a warp, half of them on repeated buckets), 77 us here;
-// 1024 uneven trajectories of up to 3560 beads 775 -> 308 us, one of 156 beads 45 (tiles) -> 18 us.
-constexpr int kSmemKeys = 32;      // keys a bead can keep; more take the slow path below
+// walk ran 7600 instructions a warp, half of them on repeated buckets), 62 us here;
+// 1024 uneven trajectories of up to 3560 beads 775 -> 277 us, 101 lattices of 780 beads
+// 68 -> 29 us, one trajectory of 156 beads 45 (tiles) -> 12 us.
+constexpr int kSmemKeys = 32;      // slots for a bead's hits; beads with more than 28 take the slow path below
 constexpr int kSmemBeads = 8192;   // 13 bits of a key
+constexpr unsigned kNoKey = 0x10000u;
 
 size_t smem_list_bytes(int nmax) {
-    return sizeof(float4) * (size_t)nmax + sizeof(uint16_t) * ((size_t)row_buckets(nmax) + kSmemKeys * kListThreads);
+    return sizeof(float4) * ((size_t)nmax + 3) + sizeof(uint16_t) * ((size_t)row_buckets(nmax) + kSmemKeys * kListThreads);
 }
 
 // Batcher's odd-even merge sort of N keys in registers, ascending.
@@ -460,36 +463,93 @@ struct SmemCells {
     int n, m;
     float inv;
 };
+// The slots of the buckets of cells cx - 1 .. cx + 1 of a row: [s, e) and, of a range
+// that wraps round the table, [0, e2).
+__device__ __forceinline__ void row_range(const SmemCells &C, int cx, int cy, int cz, int &s, int &e, int &e2) {
+    const int b0 = (int)((row_hash(cy, cz) + (uint32_t)(cx - 1)) & (uint32_t)(C.m - 1)), b2 = b0 + 2;
+    s = b0 > 0 ? C.end[b0 - 1] : 0;
+    e = C.end[min(b2, C.m - 1)];
+    e2 = b2 >= C.m ? C.end[b2 - C.m] : 0;
+}
 // Calls hit(slot) for every bead of the trajectory in the cells around p that
 // is closer than the root of t2, in no particular order; once for every row whose
 // buckets hold it, so a bead whose own row shares them can come twice.
-// Four candidates an iteration (two left the loop overhead as large as the tests).
 template <class F>
 __device__ __forceinline__ void smem_candidates(const SmemCells &C, float4 p, float t2, F &&hit) {
     const int cx = cell_coord(p.x, C.inv), cy = cell_coord(p.y, C.inv), cz = cell_coord(p.z, C.inv);
 #pragma unroll 1
-    for (int dz = -1; dz <= 1; dz++)
+    for (int r = 0; r < 9; r++) {
+        int s, e, e2;
+        row_range(C, cx, cy + r % 3 - 1, cz + r / 3 - 1, s, e, e2);
 #pragma unroll 1
-        for (int dy = -1; dy <= 1; dy++) {
-            const int b0 = (int)((row_hash(cy + dy, cz + dz) + (uint32_t)(cx - 1)) & (uint32_t)(C.m - 1)), b2 = b0 + 2;
-            int s = b0 > 0 ? C.end[b0 - 1] : 0, e = C.end[min(b2, C.m - 1)];
-            int e2 = b2 >= C.m ? C.end[b2 - C.m] : 0;   // a range that wraps round the table has a second part
-            while (true) {
-#pragma unroll 1
-                for (; s < e; s += 4) {
-                    float r2[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) r2[u] = dist2_rn(p, C.pos[min(s + u, e - 1)]);
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        if (r2[u] < t2 && s + u < e) hit(s + u);
-                }
-                if (e2 == 0) break;
+        for (; s < e || e2 > 0; s++) {
+            if (s >= e) {
                 s = 0;
                 e = e2;
                 e2 = 0;
             }
+            if (dist2_rn(p, C.pos[s]) < t2) hit(s);
         }
+    }
+}
+// The same slots, and perhaps a few a rounding further off, written down one key row after
+// another; returns their number, or more than kSmemKeys - 4 if that many were met
+// (the walk ends there).  The ranges of the 32 beads of a warp differ in length, so the
+// loop over candidates runs for the longest (22 iterations of four a warp where a
+// bead has 30 candidates) and what an iteration costs is what counts: no branch
+// for a hit, the distance contracted, the ends of the next row requested ahead, and
+// no shared-memory wavefronts for lanes past their range (half of the time before).
+__device__ __forceinline__ int smem_slots(const SmemCells &C, float4 p, float t2, uint16_t *key) {
+    const int cx = cell_coord(p.x, C.inv), cy = cell_coord(p.y, C.inv), cz = cell_coord(p.z, C.inv);
+    const float loose = t2 * 1.00001f;   // over the difference between the two roundings
+    const unsigned k0 = (unsigned)__cvta_generic_to_shared(key), stride = sizeof(uint16_t) * kListThreads;
+    const unsigned full = k0 + (kSmemKeys - 4) * stride;
+    unsigned to = k0;   // where the next hit goes
+    const unsigned pos = (unsigned)__cvta_generic_to_shared(C.pos);
+    auto load = [&](int slot, int end) {   // a lane past its range takes no bandwidth
+        float4 q;
+        asm volatile("{ .reg .pred a;\n\t"
+                     "setp.lt.s32 a, %4, %5;\n\t"
+                     "@a ld.shared.v4.f32 {%0, %1, %2, %3}, [%6]; }"
+                     : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w)
+                     : "r"(slot), "r"(end), "r"(pos + 16u * (unsigned)slot)
+                     : "memory");
+        return q;
+    };
+    auto test = [&](float4 q, int slot, int end) {
+        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        asm volatile("{ .reg .pred a, b;\n\t"
+                     "setp.lt.s32 a, %1, %2;\n\t"
+                     "setp.lt.and.f32 b, %3, %4, a;\n\t"
+                     "@b st.shared.u16 [%0], %5;\n\t"
+                     "@b add.u32 %0, %0, %6; }"
+                     : "+r"(to)
+                     : "r"(slot), "r"(end), "f"(r2), "f"(loose), "h"((uint16_t)slot), "n"(sizeof(uint16_t) * kListThreads)
+                     : "memory");
+    };
+    int s, e, e2;
+    row_range(C, cx, cy - 1, cz - 1, s, e, e2);
+#pragma unroll 1
+    for (int r = 1; r <= 9; r++) {
+        int k = s, end = e, again = e2;
+        if (r < 9) row_range(C, cx, cy + r % 3 - 1, cz + r / 3 - 1, s, e, e2);   // the next one's, ahead
+        while (true) {
+#pragma unroll 1
+            for (; k < end && to <= full; k += 4) {
+                float4 q[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) q[u] = load(k + u, end);
+#pragma unroll
+                for (int u = 0; u < 4; u++) test(q[u], k + u, end);
+            }
+            if (again == 0) break;
+            k = 0;
+            end = again;
+            again = 0;
+        }
+    }
+    return (int)((to - k0) / stride);
 }
 
 // The lists of one bead as its keys come in ascending order.
@@ -543,7 +603,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     const int m = row_buckets(n), t = threadIdx.x;
     const float4 *fr = B.frame_in;
     float4 *s_pos = s_dyn;
-    unsigned *s_tab = reinterpret_cast<unsigned *>(s_dyn + nmax);             // two 16-bit buckets a word
+    unsigned *s_tab = reinterpret_cast<unsigned *>(s_dyn + nmax + 3);         // two 16-bit buckets a word
     uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab);
     uint16_t (*s_key)[kListThreads] = reinterpret_cast<uint16_t (*)[kListThreads]>(s_end + row_buckets(nmax));
     __shared__ unsigned s_warp[kListThreads / 32];
@@ -572,8 +632,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         }
         if (lane == 31) s_warp[wid] = v;
         __syncthreads();
-        unsigned run = v - sum;
-        for (int k = 0; k < wid; k++) run += s_warp[k];
+        unsigned run = v - sum + __reduce_add_sync(0xffffffffu, lane < wid ? s_warp[lane] : 0u);
         for (int k = lo; k < hi; k++) {
             const unsigned c = s_tab[k], c0 = c & 0xffffu;
             s_tab[k] = run | ((run + c0) << 16);
@@ -593,14 +652,21 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     const int il = w.y - base + t;
     if (il >= n) return;   // no barrier after this point
     const int g = base + il;
-    const ListSite I = list_site(P, fr[g], fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], B.flags[g], il,
-                                 B.harm[g * P.maxH]);
     ListWriter W = {0, 0, 0, false};
-    if (I.do_lj) {
+    const int flags = B.flags[g];
+    if (!(flags & kFlagExtra)) {
         const SmemCells C = {s_pos, s_end, n, m, inv};
+        const float4 p = fr[g];
+        const int met = smem_slots(C, p, cut.lj, &s_key[0][t]);
+        // the bead's other planes only now: the walk has no registers to spare
+        const ListSite I = list_site(P, p, fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], flags, il, B.harm[g * P.maxH]);
         // where the bead's own sites are: a bond needs the partner's centre within
         // 2.5 + 2 nm of one (0.01 nm over the rounding)
         const float kSite2 = 4.51f * 4.51f;
+        auto site2 = [](float4 a, float4 q) {   // a coarse test: contracted
+            const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
+            return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        };
         const float4 a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
         const float4 a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
         const float4 a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);
@@ -609,22 +675,28 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
             const float r2 = dist2_rn(I.p, q);
             const int jl = __float_as_int(q.w);
             unsigned bits = 0;
-            if (I.do_pairs && r2 < cut.pair && jl != I.hpart)
-                bits = (dist2_rn(a0, q) < kSite2 ? 1u : 0u) | (dist2_rn(a1, q) < kSite2 ? 2u : 0u) |
-                       (dist2_rn(a2, q) < kSite2 ? 4u : 0u);
-            return ((unsigned)jl << 3) | bits;
+            if (P.is_assembly) {
+                bits = (site2(a0, q) < kSite2 ? 1u : 0u) | (site2(a1, q) < kSite2 ? 2u : 0u) |
+                       (site2(a2, q) < kSite2 ? 4u : 0u);
+                if (!(r2 < cut.pair) || jl == I.hpart) bits = 0;
+            }
+            return r2 < cut.lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
         };
-        int nk = 0;
-        smem_candidates(C, I.p, cut.lj, [&](int slot) {
-            if (nk < kSmemKeys) s_key[nk][t] = (uint16_t)slot;
-            nk++;
-        });
-        if (nk <= kSmemKeys) {
-            for (int k = 0; k < nk; k++) s_key[k][t] = (uint16_t)make_key(s_key[k][t]);
-            if (nk <= 8) {
+        if (met <= kSmemKeys - 4) {
+            int nk = 0;
+            for (int k = 0; k < met; k++) {
+                const unsigned key = make_key(s_key[k][t]);
+                s_key[nk][t] = (uint16_t)key;   // nk <= k
+                nk += key != kNoKey;
+            }
+            // one way for the whole warp: a warp with both would run both
+            const unsigned warp = __activemask();
+            if (!__any_sync(warp, nk > 8)) {
                 sort_keys<8>(s_key, nk);
-            } else if (nk <= 16) {
+            } else if (!__any_sync(warp, nk > 16)) {
                 sort_keys<16>(s_key, nk);
+            } else if (!__any_sync(warp, nk > 24)) {
+                sort_keys<24>(s_key, nk);
             } else {
                 for (int i = 1; i < nk; i++) {
                     const uint16_t v = s_key[i][t];
@@ -638,14 +710,17 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
             }
             // the LJ list; the keys with a site test close up in place
             int np = 0;
-            unsigned before = 0x10000u;   // no key
+            unsigned before = kNoKey;
             for (int k = 0; k < nk; k++) {
                 const unsigned key = s_key[k][t];
-                if (key == before || (key >> 3) == (unsigned)il) continue;   // found from two rows; the bead itself
+                const bool keep = key != before;   // not found from two rows
                 before = key;
-                lj_append(P, B, g, (int)(key >> 3), W);
-                if (key & 7u) s_key[np++][t] = (uint16_t)key;
+                if (keep && W.nlj < P.maxLJ) B.lj[W.nlj * nb + g] = (int)(key >> 3);
+                W.nlj += keep;
+                s_key[np][t] = (uint16_t)key;   // np <= k
+                np += keep && (key & 7u) != 0;
             }
+            W.overflow = W.nlj > P.maxLJ;
             for (int k = 0; k < np; k += 2) {   // two partners in flight
                 const unsigned k0 = s_key[k][t], k1 = k + 1 < np ? s_key[k + 1][t] : 0u;
                 const PairPlanes J0 = pair_load(B, nb, base + (int)(k0 >> 3), k0 & 7u);
@@ -661,7 +736,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
                 unsigned best = 0x7fffffffu;
                 smem_candidates(C, I.p, cut.lj, [&](int slot) {
                     const unsigned key = make_key(slot);
-                    if ((int)(key >> 3) != il && (int)key > last) best = min(best, key);
+                    if (key != kNoKey && (int)key > last) best = min(best, key);
                 });
                 if (best == 0x7fffffffu) break;
                 last = (int)best;
