@@ -397,9 +397,11 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 // ---------------------------------------------- the whole rebuild in one CTA
 // Trajectories of up to kSmemBeads beads, LJ on and either no assembly lists or
 // every assembly candidate inside the LJ cutoff: one launch, one CTA per
-// (trajectory, kListThreads beads).  Each CTA bins its whole trajectory into
+// chunk of a trajectory's beads.  Each CTA bins its whole trajectory into
 // shared memory, so a candidate costs a shared-memory load instead of a
-// dependent L2 one, and the beads of a chunk then walk their cells.
+// dependent L2 one, and the beads of the chunk then walk their cells; of chunks
+// smaller than the CTA 2 or 4 threads share a bead's rows and keys, and the first sorts
+// and writes (small batches last as long as one bead's chain: 18 -> 11 us for 1520 beads).
 //   * The bucket of cell (cx, cy, cz) is (row hash of (cy, cz) + cx) mod M, so
 //     the three cells of a row are neighbouring buckets: 9 contiguous ranges a
 //     bead instead of 27 buckets, and no search for repeated buckets.  Rows that
@@ -419,13 +421,14 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 // 256 x 1520 beads: 203 us for the general path's six launches (the 27-bucket
 // walk ran 7600 instructions a warp, half of them on repeated buckets), 62 us here;
 // 1024 uneven trajectories of up to 3560 beads 775 -> 277 us, 101 lattices of 780 beads
-// 68 -> 29 us, one trajectory of 156 beads 45 (tiles) -> 12 us.
+// 66 -> 22 us, one trajectory of 156 beads 45 (tiles) -> 10 us.
 constexpr int kSmemKeys = 32;      // slots for a bead's hits; beads with more than 28 take the slow path below
 constexpr int kSmemBeads = 8192;   // 13 bits of a key
 constexpr unsigned kNoKey = 0x10000u;
 
 size_t smem_list_bytes(int nmax) {
-    return sizeof(float4) * ((size_t)nmax + 3) + sizeof(uint16_t) * ((size_t)row_buckets(nmax) + kSmemKeys * kListThreads);
+    return sizeof(float4) * ((size_t)nmax + 3) +
+           sizeof(uint16_t) * ((size_t)row_buckets(nmax) + kSmemKeys * kListThreads);
 }
 
 // Batcher's odd-even merge sort of N keys in registers, ascending.
@@ -499,7 +502,7 @@ __device__ __forceinline__ void smem_candidates(const SmemCells &C, float4 p, fl
 // bead has 30 candidates) and what an iteration costs is what counts: no branch
 // for a hit, the distance contracted, the ends of the next row requested ahead, and
 // no shared-memory wavefronts for lanes past their range (half of the time before).
-__device__ __forceinline__ int smem_slots(const SmemCells &C, float4 p, float t2, uint16_t *key) {
+__device__ __forceinline__ int smem_slots(const SmemCells &C, float4 p, float t2, int row, int last, uint16_t *key) {
     const int cx = cell_coord(p.x, C.inv), cy = cell_coord(p.y, C.inv), cz = cell_coord(p.z, C.inv);
     const float loose = t2 * 1.00001f;   // over the difference between the two roundings
     const unsigned k0 = (unsigned)__cvta_generic_to_shared(key), stride = sizeof(uint16_t) * kListThreads;
@@ -529,11 +532,11 @@ __device__ __forceinline__ int smem_slots(const SmemCells &C, float4 p, float t2
                      : "memory");
     };
     int s, e, e2;
-    row_range(C, cx, cy - 1, cz - 1, s, e, e2);
+    row_range(C, cx, cy + row % 3 - 1, cz + row / 3 - 1, s, e, e2);
 #pragma unroll 1
-    for (int r = 1; r <= 9; r++) {
+    for (int r = row + 1; r <= last; r++) {
         int k = s, end = e, again = e2;
-        if (r < 9) row_range(C, cx, cy + r % 3 - 1, cz + r / 3 - 1, s, e, e2);   // the next one's, ahead
+        if (r < last) row_range(C, cx, cy + r % 3 - 1, cz + r / 3 - 1, s, e, e2);   // the next one's, ahead
         while (true) {
 #pragma unroll 1
             for (; k < end && to <= full; k += 4) {
@@ -594,11 +597,12 @@ __device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &
     list_append(P, B, g, I, got, jl, W.nlj, W.nlo, W.nla, W.overflow);
 }
 
-__global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int2 *work, int nmax,
+template <int PARTS>
+__global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int4 *work, int nmax,
                                                                   float inv, ListCuts cut) {
     chain_wait();
     extern __shared__ float4 s_dyn[];
-    const int2 w = work[blockIdx.x];
+    const int4 w = work[blockIdx.x];   // trajectory, first bead, number of beads
     const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
     const int m = row_buckets(n), t = threadIdx.x;
     const float4 *fr = B.frame_in;
@@ -607,6 +611,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab);
     uint16_t (*s_key)[kListThreads] = reinterpret_cast<uint16_t (*)[kListThreads]>(s_end + row_buckets(nmax));
     __shared__ unsigned s_warp[kListThreads / 32];
+    __shared__ uint8_t s_count[kListThreads];
 
     // the beads in bucket order
     for (int k = t; k < m / 2; k += kListThreads) s_tab[k] = 0;
@@ -649,46 +654,67 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     }
     __syncthreads();
 
-    const int il = w.y - base + t;
-    if (il >= n) return;   // no barrier after this point
-    const int g = base + il;
-    ListWriter W = {0, 0, 0, false};
-    const int flags = B.flags[g];
-    if (!(flags & kFlagExtra)) {
-        const SmemCells C = {s_pos, s_end, n, m, inv};
+    // the bead of this thread, and which of the bead's threads it is
+    constexpr int cap = kListThreads / PARTS;
+    const int part = t / cap, il = w.y - base + t % cap, g = base + il;
+    const bool valid = t % cap < w.z;
+    if (PARTS == 1 && !valid) return;   // no barrier after this point
+    const int flags = valid ? B.flags[g] : kFlagExtra;
+    const bool live = !(flags & kFlagExtra);
+    const SmemCells C = {s_pos, s_end, n, m, inv};
+    // where the bead's own sites are: a bond needs the partner's centre within
+    // 2.5 + 2 nm of one (0.01 nm over the rounding)
+    const float kSite2 = 4.51f * 4.51f;
+    auto site2 = [](float4 a, float4 q) {   // a coarse test: contracted
+        const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
+        return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    };
+    ListSite I;
+    float4 a0, a1, a2;
+    auto make_key = [&](int slot) {
+        const float4 q = s_pos[slot];
+        const float r2 = dist2_rn(I.p, q);
+        const int jl = __float_as_int(q.w);
+        unsigned bits = 0;
+        if (P.is_assembly) {
+            bits = (site2(a0, q) < kSite2 ? 1u : 0u) | (site2(a1, q) < kSite2 ? 2u : 0u) |
+                   (site2(a2, q) < kSite2 ? 4u : 0u);
+            if (!(r2 < cut.pair) || jl == I.hpart) bits = 0;
+        }
+        return r2 < cut.lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
+    };
+    int nk = 0;
+    bool many = false;
+    if (live) {
         const float4 p = fr[g];
-        const int met = smem_slots(C, p, cut.lj, &s_key[0][t]);
+        const int met = smem_slots(C, p, cut.lj, part * 9 / PARTS, (part + 1) * 9 / PARTS, &s_key[0][t]);
         // the bead's other planes only now: the walk has no registers to spare
-        const ListSite I = list_site(P, p, fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], flags, il, B.harm[g * P.maxH]);
-        // where the bead's own sites are: a bond needs the partner's centre within
-        // 2.5 + 2 nm of one (0.01 nm over the rounding)
-        const float kSite2 = 4.51f * 4.51f;
-        auto site2 = [](float4 a, float4 q) {   // a coarse test: contracted
-            const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
-            return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        };
-        const float4 a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
-        const float4 a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
-        const float4 a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);
-        auto make_key = [&](int slot) {
-            const float4 q = s_pos[slot];
-            const float r2 = dist2_rn(I.p, q);
-            const int jl = __float_as_int(q.w);
-            unsigned bits = 0;
-            if (P.is_assembly) {
-                bits = (site2(a0, q) < kSite2 ? 1u : 0u) | (site2(a1, q) < kSite2 ? 2u : 0u) |
-                       (site2(a2, q) < kSite2 ? 4u : 0u);
-                if (!(r2 < cut.pair) || jl == I.hpart) bits = 0;
-            }
-            return r2 < cut.lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
-        };
-        if (met <= kSmemKeys - 4) {
-            int nk = 0;
+        I = list_site(P, p, fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], flags, il, B.harm[g * P.maxH]);
+        a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
+        a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
+        a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);
+        many = met > kSmemKeys - 4;
+        if (!many)
             for (int k = 0; k < met; k++) {
                 const unsigned key = make_key(s_key[k][t]);
                 s_key[nk][t] = (uint16_t)key;   // nk <= k
                 nk += key != kNoKey;
             }
+    }
+    if (PARTS > 1) {   // the keys of the bead's other threads join those of its first
+        s_count[t] = (uint8_t)(many ? 255 : nk);
+        __syncthreads();
+        if (part > 0) return;
+        for (int o = t + cap; o < kListThreads && live; o += cap) {
+            const int c = s_count[o];
+            many = many || nk + c > kSmemKeys;
+            for (int k = 0; k < c && !many; k++) s_key[nk++][t] = s_key[k][o];
+        }
+    }
+    if (!valid) return;
+    ListWriter W = {0, 0, 0, false};
+    if (live) {
+        if (!many) {
             // one way for the whole warp: a warp with both would run both
             const unsigned warp = __activemask();
             if (!__any_sync(warp, nk > 8)) {
@@ -908,9 +934,13 @@ float order_beads(const KParams &P, const DevBuffers &B, const CellBuffers &C, f
 bool smem_lists_apply(const KParams &P, int nmax) {
     return P.lj_on && P.ljcut > 0.0f && (!P.is_assembly || P.ljcut >= kPairReach) && nmax <= kSmemBeads;
 }
+int smem_lists_resident(int nmax) { return smem_list_bytes(nmax) <= 112 * 1024 ? 2 : 1; }
 int smem_lists_prepare() {   // the limit of the largest trajectory, whatever this engine's, as engines share the kernel
-    return cudaFuncSetAttribute(k_cell_lists_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_list_bytes(kSmemBeads)) == cudaSuccess
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int bytes = (int)smem_list_bytes(kSmemBeads);
+    return cudaFuncSetAttribute(k_cell_lists_smem<1>, attr, bytes) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_cell_lists_smem<2>, attr, bytes) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_cell_lists_smem<4>, attr, bytes) == cudaSuccess
                ? 0
                : -1;
 }
@@ -925,11 +955,11 @@ static float sq_below(float c) {
 }
 ListCuts list_cuts(const KParams &P) { return {sq_below(P.ljcut), sq_below(kPairReach), sq_below(2.5f)}; }
 
-void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
+void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, int parts, int nmax,
                          cudaStream_t s) {
     const float inv = 1.0f / (P.ljcut * 1.001f + 1e-3f);   // the cells of bin_beads
-    launch_chained(P, k_cell_lists_smem, nwork, kListThreads, smem_list_bytes(nmax), s, P, B, work, nmax, inv,
-                   list_cuts(P));
+    const auto kernel = parts == 4 ? k_cell_lists_smem<4> : parts == 2 ? k_cell_lists_smem<2> : k_cell_lists_smem<1>;
+    launch_chained(P, kernel, nwork, kListThreads, smem_list_bytes(nmax), s, P, B, work, nmax, inv, list_cuts(P));
 }
 
 void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffers &C, const int2 *work, int nwork,

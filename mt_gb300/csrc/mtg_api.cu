@@ -229,7 +229,7 @@ long long count_kernel_nodes(cudaGraph_t g) {
 // The list rebuild with the engine's method.
 void launch_lists(mtg_engine *e) {
     if (e->use_cells && smem_lists_apply(e->kp, e->max_traj_beads))
-        launch_rebuild_smem(e->kp, e->bufs(), e->list_work, e->list_nwork, e->max_traj_beads, e->stream);
+        launch_rebuild_smem(e->kp, e->bufs(), e->list_work, e->list_nwork, e->list_parts, e->max_traj_beads, e->stream);
     else if (e->use_cells)
         launch_rebuild_cells(e->kp, e->bufs(), e->cells(), e->work, e->nwork, e->stream);
     else
@@ -400,6 +400,35 @@ long long lcm_ll(long long a, long long b) {
     return a / x * b;
 }
 
+// The CTAs of the one-launch list rebuild: a trajectory's beads in equal chunks, as small as
+// still puts all CTAs on the GPU at once (each bins its whole trajectory, so
+// a second wave of small ones costs more than it gives), at least 128 beads, at most
+// one a thread; where a chunk leaves threads over, 2 or 4 share a bead's walk.
+// Lists of 1520 beads: 18 us with chunks of 512, 11 with 128 and four threads a bead (13 with
+// one); 101 x 780 beads 29 us with 2 CTAs a trajectory, 22 with 3 (303 of 304 places), 33
+// with 4; 256 x 1520 beads 62 us with 3 CTAs a trajectory, 84 with 6.
+std::vector<int4> plan_lists(int sms, int nt, const int *off, int *parts) {
+    int nmax = 0, chunk = kListThreads;
+    for (int t = 0; t < nt; t++) nmax = std::max(nmax, off[t + 1] - off[t]);
+    const long long places = (long long)sms * smem_lists_resident(nmax);
+    for (int c : {128, 192, 256, 384}) {
+        long long ctas = 0;
+        for (int t = 0; t < nt; t++) ctas += (off[t + 1] - off[t] + c - 1) / c;
+        if (ctas <= places) {
+            chunk = c;
+            break;
+        }
+    }
+    *parts = chunk <= 128 ? 4 : chunk <= 256 ? 2 : 1;
+    std::vector<int4> work;
+    for (int t = 0; t < nt; t++) {
+        const int n = off[t + 1] - off[t], chunks = (n + chunk - 1) / chunk;
+        const int size = chunks ? ((n + chunks - 1) / chunks + 31) / 32 * 32 : 0;
+        for (int k = 0; k < n; k += size) work.push_back(make_int4(t, off[t] + k, std::min(size, n - k), 0));
+    }
+    return work;
+}
+
 }  // namespace
 
 extern "C" {
@@ -491,10 +520,6 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     }
     work_first[nt] = (int)work.size();
     e->nwork = (int)work.size();
-    std::vector<int2> list_work;
-    for (int tr = 0; tr < nt; tr++)
-        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kListThreads) list_work.push_back(make_int2(tr, g));
-    e->list_nwork = (int)list_work.size();
     // all-pairs TEA kernels: chunks of kTeaChunk beads i, blocks of kTeaBlock
     // beads j, a chunk's units = the blocks of its trajectory
     std::vector<int2> tea_work;
@@ -514,6 +539,8 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     e->kp.tea_units = tea_unit0.back();
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    const std::vector<int4> list_work = plan_lists(sms, nt, t->offsets, &e->list_parts);
+    e->list_nwork = (int)list_work.size();
     // threads per bead in the near-pair kernel of learned TEA: enough to fill the GPU
     {
         // two beads per thread; aim for about two full waves at 64 registers
@@ -613,7 +640,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         (rc = upload(e->harm, harm.data(), sizeof(int) * harm.size(), s)) ||
         (rc = upload(e->zs, zs.data(), sizeof(float) * nt, s)) ||
         (rc = upload(e->work, work.data(), sizeof(int2) * work.size(), s)) ||
-        (rc = upload(e->list_work, list_work.data(), sizeof(int2) * list_work.size(), s)) ||
+        (rc = upload(e->list_work, list_work.data(), sizeof(int4) * list_work.size(), s)) ||
         (rc = upload(e->work_first, work_first.data(), sizeof(int) * (nt + 1), s))) {
         mtg_destroy(e);
         return rc;

@@ -32,8 +32,8 @@ struct mtg_engine {
     int *err = nullptr;
     int2 *work = nullptr;
     int nwork = 0;
-    int2 *list_work = nullptr;  // chunks of kListThreads beads for the one-launch list rebuild
-    int list_nwork = 0;
+    int4 *list_work = nullptr;  // CTAs of the one-launch list rebuild: trajectory, first bead, beads
+    int list_nwork = 0, list_parts = 1;
     int2 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels
     int tea_nwork = 0;
     int *work_first = nullptr;

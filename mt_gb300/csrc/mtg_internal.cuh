@@ -475,11 +475,13 @@ void launch_rebuild_cells(const KParams &P, const DevBuffers &B, const CellBuffe
                           cudaStream_t s);
 ListCuts list_cuts(const KParams &P);
 // The cell-list rebuild in one launch, each CTA binning its trajectory in
-// shared memory; work = chunks of kListThreads beads, nmax the largest trajectory.
+// shared memory; work = (trajectory, first bead, beads) of each CTA, at most
+// kListThreads / parts beads, nmax the largest trajectory.
 constexpr int kListThreads = 512;
 bool smem_lists_apply(const KParams &P, int nmax);
+int smem_lists_resident(int nmax);                // CTAs an SM holds
 int smem_lists_prepare();                         // opts the kernel into its shared memory (outside captures)
-void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, int nmax,
+void launch_rebuild_smem(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, int parts, int nmax,
                          cudaStream_t s);
 // Bins the current positions into the per-trajectory spatial hash with cells
 // just larger than `reach`; returns 1/edge for the consumers' cell lookups.

@@ -72,6 +72,14 @@ def test_many_hits(box):
     assert t["lj"][0].max() > (8, 16, 32)[(22.0, 14.0, 9.0).index(box)]
 
 
+@pytest.mark.parametrize("sizes,box", [((150, 31) * 85, 14.0), ((150, 31) * 85, 9.0), ((300, 257) * 100, 14.0),
+                                       ((600, 513) * 165, 22.0)], ids=["two", "two-many", "one", "full"])
+def test_threads_a_bead(sizes, box):
+    """Batches large enough for two threads a bead, one, and a thread for every bead of a CTA (the small ones have four)."""
+    t = same(cloud(sizes, seed=4, box=box, ljpairscutoff=7.0))
+    assert t["lj"][0].max() > 8
+
+
 @pytest.mark.parametrize("over", [dict(ljpairscutoff=6.6), dict(ljpairscutoff=13.7), dict(is_wall=1)], ids=str)
 def test_cutoffs(over):
     same(cloud((700, 300), seed=5, **over))
