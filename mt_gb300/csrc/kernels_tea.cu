@@ -3,7 +3,8 @@
 // RPY mobility product fused with the position update; below them the far
 // field of the learned mode.
 //
-// Both O(N^2) passes are one kernel template, k_tea_pass.  They are bound by
+// Both O(N^2) passes are one kernel template, k_tea_pass (k_tea_lanes for small
+// systems, which are bound by latency).  They are bound by
 // the FP32 pipe (about 45 FLOP per ordered pair: 24 packed FP32x2 operations
 // for two pairs), so everything else is arranged to stay off its way:
 //   * The beads j come from B.tea_pack, where the force kernel of the step has
@@ -31,7 +32,7 @@
 // then far below the rounding of the sums, and the correction skips it.
 // Sums are kept in units of 0.75 a (T' = T / (0.75 a)).
 // Measured (mobility product): 64 x 5600 beads 1.82 -> 1.66 ms (54 TFLOP/s of the measured 80;
-// the FMA pipe is 75% active), 16 x 3300 205 -> 168 us, one trajectory of 299 25 -> 14 us (before: a tile stored twice by
+// the FMA pipe is 75% active), 16 x 3300 205 -> 165 us (before: a tile stored twice by
 // every CTA, whole 128-bead items in 3.7 waves or a second kernel for split ones).
 #include "mtg_internal.cuh"
 
@@ -189,7 +190,7 @@ template <bool FEFF>
 __device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffers &B, int g, float sx, float sy,
                                                 float sz, float b2, const TeaConst &K, float4 *feff) {
     const int nb = P.nb;
-    const float4 ci = B.tea_ci[g], Fi = B.force[g], Ri = B.tea_r[g];
+    const float4 ci = B.tea_ci[g], Fi = B.force[g], Ri = B.tea_r[g], fa = B.force[nb + g];   // (ffi, ftheta, fpsi)
     sx = fmaf(K.c075a, sx, Fi.x + Ri.x * (1.0f / sqrtf(1.0f + b2 * ci.x)));
     sy = fmaf(K.c075a, sy, Fi.y + Ri.y * (1.0f / sqrtf(1.0f + b2 * ci.y)));
     sz = fmaf(K.c075a, sz, Fi.z + Ri.z * (1.0f / sqrtf(1.0f + b2 * ci.z)));
@@ -207,7 +208,6 @@ __device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffe
     const float4 ga = gauss4(s2);
     B.seeds[nb + g] = s2;
     if (!(flags & (kFlagExtra | kFlagFixed))) {
-        const float4 fa = B.force[nb + g];  // (ffi, ftheta, fpsi)
         const float x = Fr.p0.x + P.kr * sx, y = Fr.p0.y + P.kr * sy, z = Fr.p0.z + P.kr * sz;
         const float fi = Fr.p0.w + (P.kfi * fa.x + P.nfi * ga.x);
         const float psi = Fr.p1.w + (P.kfi * fa.z + P.nfi * ga.y);
@@ -394,7 +394,10 @@ __device__ __forceinline__ void tea_near_block(Op &X, const TeaConst &K, const f
 }
 
 // Run k of a launch: units [k U / G, (k + 1) U / G).
-__device__ __forceinline__ long long tea_run_start(long long units, int runs, int k) { return k * units / runs; }
+__device__ __forceinline__ long long tea_div(long long a, long long b) {   // 64-bit division only where needed
+    return ((a | b) >> 32) == 0 ? (long long)((unsigned)a / (unsigned)b) : a / b;
+}
+__device__ __forceinline__ long long tea_run_start(long long units, int runs, int k) { return tea_div(k * units, runs); }
 
 // The item that holds unit u: the last of unit0[0 .. nwork - 1] that is <= u, by a
 // 32-way search (each round is one dependent load instead of five).
@@ -413,7 +416,7 @@ __device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, 
 
 // Runs while gate is null or *gate == run_if.
 template <class Op>
-__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
+__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int4 *work, int nwork,
                                                              float4 *feff, const int *gate, int run_if) {
     chain_wait();
     if (gate && *gate != run_if) return;
@@ -431,9 +434,9 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
         const long long first = B.tea_unit0[item];
         const int nblk = (int)(B.tea_unit0[item + 1] - first);
         const int b0 = (int)(u - first), b1 = (int)min((long long)nblk, u_end - first);
-        const int2 w = work[item];
+        const int4 w = work[item];   // trajectory, first bead, end of the trajectory, its first block
         const int traj = w.x, g = w.y + tid;
-        const float4 *pack = B.tea_pack + (size_t)B.tea_blk0[traj] * kTeaBlockF4;
+        const float4 *pack = B.tea_pack + (size_t)w.w * kTeaBlockF4;
         auto issue = [&](int tile) {
             const int q0 = b0 + tile * kTeaTileBlocks, nq = min(kTeaTileBlocks, b1 - q0);
             float4 *dst = s_tile[tile % kTeaStages];
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
             if (k < ntiles) issue(k);
             cp_async_commit();
         }
-        const bool valid = g < B.off[traj + 1];
+        const bool valid = g < w.z;
         const float4 p = valid ? B.frame_in[g] : make_float4(0.f, 0.f, 0.f, 0.f);
         const bool act = __any_sync(0xffffffffu, valid && !(B.flags[g] & kFlagExtra));
         Op X;
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
         if (b0 > 0 || b1 < nblk) {
             // part of the item: slot 0 of the run for an item begun before it, slot 1 for one it begins
             B.tea_part[((size_t)blockIdx.x * 2 + (b0 > 0 ? 0 : 1)) * kTeaI + tid] = acc;
-            const int k0 = (int)(((first + 1) * G - 1) / U), k1 = (int)(((first + nblk) * G - 1) / U);
+            const int k0 = (int)tea_div((first + 1) * G - 1, U), k1 = (int)tea_div((first + nblk) * G - 1, U);
             __threadfence();
             __syncthreads();
             if (tid == 0) s_last = atomicAdd(&B.tea_cnt[item], 1) == k1 - k0;
@@ -488,10 +491,15 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
             if (done) {
                 __threadfence();
                 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = k0; k <= k1; k++) {
-                    const int slot = tea_run_start(U, G, k) > first ? 0 : 1;
-                    const float4 q = __ldcg(&B.tea_part[((size_t)k * 2 + slot) * kTeaI + tid]);
-                    acc = make_float4(acc.x + q.x, acc.y + q.y, acc.z + q.z, acc.w + q.w);
+                for (int k = k0; k <= k1; k += 4) {   // four requested at once; run k0 begins the item
+                    float4 q[4];
+#pragma unroll
+                    for (int v = 0; v < 4; v++)
+                        if (k + v <= k1)
+                            q[v] = __ldcg(&B.tea_part[((size_t)(k + v) * 2 + (k + v == k0 ? 1 : 0)) * kTeaI + tid]);
+#pragma unroll
+                    for (int v = 0; v < 4; v++)
+                        if (k + v <= k1) acc = make_float4(acc.x + q[v].x, acc.y + q[v].y, acc.z + q[v].z, acc.w + q[v].w);
                 }
                 if (tid == 0) B.tea_cnt[item] = 0;
             }
@@ -523,6 +531,67 @@ __global__ void k_tea_pack_clear(float4 *pack, int nblocks) {
 // Runs of a launch, one CTA each: kTeaRunsPerSlot for every CTA that fits the device, but
 // no item cut into more than about 16 (their sums meet in one CTA).  rare: a
 // launch that mostly finds its gate closed, which should be short then.
+// The same pass for systems too small to fill the GPU, where a pass lasts as long as its
+// chain of waits: a warp a bead, sixteen lanes for the slots of a block and two blocks at once,
+// adds up in registers and by shuffles, so no partial sum goes through memory and
+// no CTA waits for another's (in k_tea_pass the fence, the count and the parts of the runs
+// are half of the time there).  The blocks are read straight from L1 and L2.  Overlapping
+// beads are noted in a mask and come after each 32 pairs of blocks, so that the loop
+// has no branch and its loads overlap.
+constexpr int kTeaLanes = 32, kTeaLaneThreads = 128;
+template <class Op>
+__global__ void __launch_bounds__(kTeaLaneThreads) k_tea_lanes(KParams P, DevBuffers B, float4 *feff, const int *gate,
+                                                               int run_if) {
+    chain_wait();
+    if (gate && *gate != run_if) return;
+    constexpr int kGroups = kTeaLanes / kTeaPairSlots;   // blocks taken at once
+    const int g = blockIdx.x * (kTeaLaneThreads / kTeaLanes) + threadIdx.x / kTeaLanes, lane = threadIdx.x % kTeaLanes;
+    const int t = lane % kTeaPairSlots;
+    const bool valid = g < P.nb;
+    const int gc = valid ? g : P.nb - 1;
+    const int traj = B.traj[gc], base = B.off[traj], n = B.off[traj + 1] - base, slot = B.tea_slot[gc];
+    const float4 p = B.frame_in[gc];
+    const TeaConst K = tea_const(P.tea_a);
+    Op X;
+    X.start(P, B, traj, p, gc, valid);
+    const int self = (gc - base) / kTeaBlock, se = slot & 1;
+    const bool mine = (slot % kTeaBlock) >> 1 == t;
+    const float4 *pack = B.tea_pack + (size_t)(slot / kTeaBlock - self) * kTeaBlockF4;
+    const int nblk = (n + kTeaBlock - 1) / kTeaBlock;
+    for (int q0 = lane / kTeaPairSlots; q0 < nblk; q0 += 32 * kGroups) {
+        unsigned near = 0;   // of these blocks, the ones with an overlapping bead in this lane's slot
+        const int nq = min(32, (nblk - q0 + kGroups - 1) / kGroups);
+#pragma unroll 4
+        for (int k = 0; k < nq; k++) {
+            const int q = q0 + k * kGroups;
+            float rm = 3.4e38f;
+            X.template pair<true>(K, pack + (size_t)q * kTeaBlockF4, t, mine && q == self ? t : -1, se, rm);
+            near |= (rm <= K.four_a2 ? 1u : 0u) << k;
+        }
+        for (; near; near &= near - 1) {
+            const int q = q0 + (__ffs((int)near) - 1) * kGroups;
+            const float4 *blk = pack + (size_t)q * kTeaBlockF4;
+            const bool own = mine && q == self;
+            const float2 r2 = X.dist2(blk, t);
+            if (r2.x <= K.four_a2 && !(own && se == 0)) X.near(K, blk, t, 0);
+            if (r2.y <= K.four_a2 && !(own && se == 1)) X.near(K, blk, t, 1);
+        }
+    }
+    float4 acc = X.sum();
+#pragma unroll
+    for (int o = kTeaLanes / 2; o > 0; o >>= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+        acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+    }
+    if (valid && lane == 0) X.finish(P, B, g, traj, acc, K, feff);
+}
+// Up to these beads and units (32 x 128 pairs) the lanes form is used.  A step of 299 beads 13.9
+// us with k_tea_pass and 10.2 so, 16 x 299 beads 16.8 and 13.3, 1520 beads 18.8 and
+// 17.9, 3300 beads (2704 units) 31.6 and 30.8; but 2 x 3300 beads 46.7 and 50.0,
+// 5600 beads (7700 units) 57.6 and 73.9, 40 x 299 beads (1200 units) 21.7 and 22.3.
+constexpr int kTeaLaneBeads = 6500, kTeaLaneUnits = 2800;
 template <class Op>
 static int tea_runs(const KParams &P, bool rare) {
     int dev = 0, sms = 1, occ = 1;
@@ -535,8 +604,13 @@ static int tea_runs(const KParams &P, bool rare) {
     return (int)(runs < slots ? runs : slots);
 }
 template <class Op>
-static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
+static void tea_launch(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff, const int *gate,
                        int run_if, cudaStream_t s) {
+    if (P.nb <= kTeaLaneBeads && P.tea_units <= kTeaLaneUnits) {
+        const int beads = kTeaLaneThreads / kTeaLanes;
+        launch_chained(P, k_tea_lanes<Op>, (P.nb + beads - 1) / beads, kTeaLaneThreads, 0, s, P, B, feff, gate, run_if);
+        return;
+    }
     launch_chained(P, k_tea_pass<Op>, tea_runs<Op>(P, gate && run_if == 1), kTeaThreads, 0, s, P, B, work, nwork, feff,
                    gate, run_if);
 }
@@ -546,11 +620,11 @@ void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
 void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s) {
     k_tea_pack_clear<<<(int)(((size_t)nblocks * kTeaBlockF4 + 255) / 256), 256, 0, s>>>(pack, nblocks);
 }
-void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
+void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
                           int run_if, cudaStream_t s) {
     tea_launch<EpsOp>(P, B, work, nwork, nullptr, gate, run_if, s);
 }
-void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
+void launch_tea_eps(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s) {
     launch_tea_eps_gated(P, B, work, nwork, nullptr, 0, s);
 }
 void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious, float epsmax, const int *gate,
@@ -560,14 +634,14 @@ void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s) {
     launch_tea_beta_gated(P, B, capricious, epsmax, nullptr, 0, s);
 }
-void launch_tea_step(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
+void launch_tea_step(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s) {
     tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, nullptr, 0, s);
 }
-void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
+void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
                            cudaStream_t s) {
     tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, gate, 1, s);
 }
-void launch_tea_feff(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
+void launch_tea_feff(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff,
                      const int *gate, cudaStream_t s) {
     tea_launch<StepOp<true>>(P, B, work, nwork, feff, gate, 0, s);
 }

@@ -522,7 +522,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     e->nwork = (int)work.size();
     // all-pairs TEA kernels: chunks of kTeaChunk beads i, blocks of kTeaBlock
     // beads j, a chunk's units = the blocks of its trajectory
-    std::vector<int2> tea_work;
+    std::vector<int4> tea_work;
     std::vector<int> tea_slot(nb), tea_blk0(nt + 1);
     std::vector<long long> tea_unit0{0};
     for (int tr = 0; tr < nt; tr++) {
@@ -531,7 +531,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         e->kp.tea_max_blocks = std::max(e->kp.tea_max_blocks, nblk);
         for (int i = 0; i < n; i++) tea_slot[t->offsets[tr] + i] = tea_blk0[tr] * kTeaBlock + i;
         for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) {
-            tea_work.push_back(make_int2(tr, g));
+            tea_work.push_back(make_int4(tr, g, t->offsets[tr + 1], tea_blk0[tr]));
             tea_unit0.push_back(tea_unit0.back() + nblk);
         }
     }
@@ -595,7 +595,6 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         ALLOC(e->tea_eps_t, nt);
         ALLOC(e->tea_pack, (size_t)kTeaBlockF4 * tea_blk0[nt]);
         ALLOC(e->tea_slot, nb);
-        ALLOC(e->tea_blk0, nt + 1);
         ALLOC(e->tea_unit0, e->tea_nwork + 1);
         ALLOC(e->tea_part, (size_t)2 * kTeaChunk * std::min<long long>(e->kp.tea_units, (long long)kTeaMaxOcc * kTeaRunsPerSlot * sms));
         ALLOC(e->tea_cnt, e->tea_nwork);
@@ -651,9 +650,8 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     cudaMemsetAsync(e->latc, 0, sizeof(int) * nb, s);
     cudaMemsetAsync(e->force, 0, sizeof(float4) * 2 * nb, s);
     if (p->hdi_on) {
-        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int2) * tea_work.size(), s)) ||
+        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int4) * tea_work.size(), s)) ||
             (rc = upload(e->tea_slot, tea_slot.data(), sizeof(int) * nb, s)) ||
-            (rc = upload(e->tea_blk0, tea_blk0.data(), sizeof(int) * (nt + 1), s)) ||
             (rc = upload(e->tea_unit0, tea_unit0.data(), sizeof(long long) * tea_unit0.size(), s))) {
             mtg_destroy(e);
             return rc;
@@ -771,7 +769,7 @@ int mtg_destroy(mtg_engine *e) {
                     e->surr_desc, e->surr_pred, e->surr_stats, e->surr_gate, e->surr_err, e->surr_part,
                     e->tea_ci2, e->feff_a, e->feff_b, e->tea_eps2, e->tea_beta2, e->tea_eps_t2,
                     e->hydro_cand, e->hydro_rank, e->hydro_sums, e->hydro_counts, e->hydro_events,
-                    e->tea_pack, e->tea_slot, e->tea_blk0, e->tea_unit0, e->tea_part, e->tea_cnt};
+                    e->tea_pack, e->tea_slot, e->tea_unit0, e->tea_part, e->tea_cnt};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (e->stage_host) cudaFreeHost(e->stage_host);

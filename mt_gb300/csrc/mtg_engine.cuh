@@ -34,7 +34,7 @@ struct mtg_engine {
     int nwork = 0;
     int4 *list_work = nullptr;  // CTAs of the one-launch list rebuild: trajectory, first bead, beads
     int list_nwork = 0, list_parts = 1;
-    int2 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels
+    int4 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels: trajectory, first bead, its end, its first block
     int tea_nwork = 0;
     int *work_first = nullptr;
     double *en_partials = nullptr, *en_traj = nullptr, *en_bead = nullptr;
@@ -42,7 +42,7 @@ struct mtg_engine {
     float *tea_eps = nullptr, *tea_beta = nullptr;
     double *tea_eps_t = nullptr;
     float4 *tea_pack = nullptr, *tea_part = nullptr;   // all-pairs TEA kernels, see DevBuffers
-    int *tea_slot = nullptr, *tea_blk0 = nullptr, *tea_cnt = nullptr;
+    int *tea_slot = nullptr, *tea_cnt = nullptr;
     long long *tea_unit0 = nullptr;
     int tea_jparts = 1;            // as set (no effect any more)
     float *stage = nullptr;        // 7*nb floats for host <-> device Coord transfers
@@ -146,7 +146,6 @@ struct mtg_engine {
         b.err = err;
         b.tea_pack = tea_pack;
         b.tea_slot = tea_slot;
-        b.tea_blk0 = tea_blk0;
         b.tea_unit0 = tea_unit0;
         b.tea_part = tea_part;
         b.tea_cnt = tea_cnt;
