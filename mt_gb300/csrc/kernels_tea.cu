@@ -27,11 +27,13 @@
 //     finishes the beads, so the result does not depend on the timing.
 // The far-field formula runs for every pair; the few overlapping pairs
 // (r <= 2a) are found through a running minimum of r^2 per block; in a block
-// that holds one their distances are taken once more and only they get the near-field formula.  In
+// that holds one their distances are taken once more and only they get the near-field formula
+// in place of the far one.  That one takes r >= 2a, so what is replaced is never larger than the
+// sums (at r = 0.14 nm the row sums were 4e-3 off without it, 1e-7 so; 1% of the time).  In
 // the block that holds a bead itself its own pair gets r^2 = 1e30: its term is
 // then far below the rounding of the sums, and the correction skips it.
 // Sums are kept in units of 0.75 a (T' = T / (0.75 a)).
-// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.66 ms (54 TFLOP/s of the measured 80;
+// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.68 ms (54 TFLOP/s of the measured 80;
 // the FMA pipe is 75% active), 16 x 3300 205 -> 165 us (before: a tile stored twice by
 // every CTA, whole 128-bead items in 3.7 waves or a second kernel for split ones).
 #include "mtg_internal.cuh"
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(256) k_tea_beta(KParams P, DevBuffers B, int c
 __device__ __forceinline__ float3 tea_far1(const TeaConst &K, float dx, float dy, float dz, float gx, float gy,
                                            float gz) {
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float rinv = rsqrt_hw(r2), q = rinv * rinv, tq = q * rinv;
+    const float rinv = rsqrt_hw(fmaxf(r2, K.four_a2)), q = rinv * rinv, tq = q * rinv;
     const float cii = fmaf(K.kap, tq, rinv);
     const float cr = tq * fmaf(-K.two_a2, q, 1.0f);
     const float s = cr * fmaf(dx, gx, fmaf(dy, gy, dz * gz));
@@ -249,7 +251,7 @@ struct EpsOp {
                 r2.x = 1e30f;
         }
         rm = fmin3(rm, r2.x, r2.y);
-        const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+        const float2 rinv = make_float2(rsqrt_hw(fmaxf(r2.x, K.four_a2)), rsqrt_hw(fmaxf(r2.y, K.four_a2)));
         const float2 q = __fmul2_rn(rinv, rinv);
         const float2 tq = __fmul2_rn(q, rinv);
         const float2 cii = __ffma2_rn(vkap, tq, rinv);
@@ -273,11 +275,12 @@ struct EpsOp {
         const float4 a = blk[t], b = blk[kTeaPairSlots + t];
         const float dx = (e ? a.y : a.x) + nx.x, dy = (e ? a.w : a.z) + ny.x, dz = (e ? b.y : b.x) + nz.x;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        const float rinv = rsqrt_hw(r2), q = rinv * rinv, tq = q * rinv;
-        const EpsTerms f = eps_terms(dx, dy, dz, fmaf(K.kap, tq, rinv), fmaf(-K.two_a2, tq, rinv), q);
+        const float rc = rsqrt_hw(fmaxf(r2, K.four_a2)), qc = rc * rc, tq = qc * rc;
+        const EpsTerms f = eps_terms(dx, dy, dz, fmaf(K.kap, tq, rc), fmaf(-K.two_a2, tq, rc), qc);
+        const float rinv = rsqrt_hw(r2);
         float cn, rn;
         rpy_near(K, r2, rinv, cn, rn);
-        const EpsTerms n = eps_terms(dx, dy, dz, cn, rn, q);
+        const EpsTerms n = eps_terms(dx, dy, dz, cn, rn, rinv * rinv);
         sx.x += n.bx - f.bx;
         sy.x += n.by - f.by;
         sz.x += n.bz - f.bz;
@@ -338,7 +341,7 @@ struct StepOp {
                 r2.x = 1e30f;
         }
         rm = fmin3(rm, r2.x, r2.y);
-        const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+        const float2 rinv = make_float2(rsqrt_hw(fmaxf(r2.x, K.four_a2)), rsqrt_hw(fmaxf(r2.y, K.four_a2)));
         const float2 q = __fmul2_rn(rinv, rinv);
         const float2 tq = __fmul2_rn(q, rinv);
         const float2 cii = __ffma2_rn(vkap, tq, rinv);
@@ -885,7 +888,7 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
             const float3 y = ff_proxy(cJ, hJ, m);
             const float2 dx = __fadd2_rn(f2(y.x), nxx), dy = __fadd2_rn(f2(y.y), nxy), dz = __fadd2_rn(f2(y.z), nxz);
             const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-            const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+            const float2 rinv = make_float2(rsqrt_hw(fmaxf(r2.x, K.four_a2)), rsqrt_hw(fmaxf(r2.y, K.four_a2)));
             const float2 q2 = __fmul2_rn(rinv, rinv), tq = __fmul2_rn(q2, rinv);
             const float2 cii = __ffma2_rn(vkap, tq, rinv);
             const float2 cr = __fmul2_rn(tq, __ffma2_rn(vn2a2, q2, one));

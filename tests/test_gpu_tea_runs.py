@@ -43,7 +43,9 @@ def tensors(x, a):
     return T
 
 
-@pytest.mark.parametrize("sizes", [(2, 31, 32, 33), (127, 128, 129), (300, 5, 417)], ids=str)
+# the first three take a warp a bead, the last one the equal runs
+@pytest.mark.parametrize("sizes", [(2, 31, 32, 33), (127, 128, 129), (300, 5, 417), (300, 5, 417) + (151,) * 40],
+                         ids=lambda v: f"{len(v)}x{max(v)}")
 def test_row_sums_against_fp64(sizes):
     from mt_gb300 import engine
     b = batch(sizes, 91)
