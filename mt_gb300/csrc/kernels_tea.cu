@@ -531,9 +531,6 @@ __global__ void k_tea_pack_clear(float4 *pack, int nblocks) {
     pack[k] = make_float4(a, a, b, b);
 }
 
-// Runs of a launch, one CTA each: kTeaRunsPerSlot for every CTA that fits the device, but
-// no item cut into more than about 16 (their sums meet in one CTA).  rare: a
-// launch that mostly finds its gate closed, which should be short then.
 // The same pass for systems too small to fill the GPU, where a pass lasts as long as its
 // chain of waits: a warp a bead, sixteen lanes for the slots of a block and two blocks at once,
 // adds up in registers and by shuffles, so no partial sum goes through memory and
@@ -590,21 +587,31 @@ __global__ void __launch_bounds__(kTeaLaneThreads) k_tea_lanes(KParams P, DevBuf
     }
     if (valid && lane == 0) X.finish(P, B, g, traj, acc, K, feff);
 }
-// Up to these beads and units (32 x 128 pairs) the lanes form is used.  A step of 299 beads 13.9
-// us with k_tea_pass and 10.2 so, 16 x 299 beads 16.8 and 13.3, 1520 beads 18.8 and
-// 17.9, 3300 beads (2704 units) 31.6 and 30.8; but 2 x 3300 beads 46.7 and 50.0,
-// 5600 beads (7700 units) 57.6 and 73.9, 40 x 299 beads (1200 units) 21.7 and 22.3.
-constexpr int kTeaLaneBeads = 6500, kTeaLaneUnits = 2800;
+// Up to these beads and units (32 x 128 pairs) the lanes form is used.  Steps with it and with
+// k_tea_pass: 299 beads 10.2 and 13.9 us, 1520 beads 18.2 and 20.7, 2800 beads (1936 units) 27.1
+// and 28.5, 20 x 299 beads 16.4 and 17.5; but 3300 beads (2704 units) 30.9 and 29.7, 2 x 3300 beads
+// 50 and 41, 40 x 299 beads (1200 units) 22.3 and 21.7.
+constexpr int kTeaLaneBeads = 6500, kTeaLaneUnits = 2000;
+// Runs of a launch, one CTA each: kTeaRunsPerSlot for every CTA that fits the device, but
+// no item cut into more than about 16 (their sums meet in one CTA), or 48 while the
+// runs do not fill the device once (a step of 5600 beads 58 -> 52 us, of 2 x 3300 beads 47 -> 41;
+// of 16 x 1520 beads, which fill it, 56 -> 58).  rare: a
+// launch that mostly finds its gate closed, which should be short then.
 template <class Op>
 static int tea_runs(const KParams &P, bool rare) {
     int dev = 0, sms = 1, occ = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tea_pass<Op>, kTeaThreads, 0);
-    long long slots = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
-    if (!rare) slots *= kTeaRunsPerSlot;
-    const long long least = (P.tea_max_blocks + 15) / 16, runs = (P.tea_units + least - 1) / least;
-    return (int)(runs < slots ? runs : slots);
+    const long long wave = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
+    const long long slots = rare ? wave : wave * kTeaRunsPerSlot;
+    auto runs_of = [&](int pieces) {   // with items in at most this many pieces
+        const long long least = (P.tea_max_blocks + pieces - 1) / pieces;
+        return (P.tea_units + least - 1) / least;
+    };
+    long long runs = runs_of(16);
+    if (runs < wave) runs = std::max(runs, std::min(wave, runs_of(48)));
+    return (int)std::min(runs, slots);
 }
 template <class Op>
 static void tea_launch(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff, const int *gate,
