@@ -40,6 +40,26 @@ def test_small_batches_equal_a_large_one(over, keep):
                                   np.concatenate([k.download_state(forces=True)[1] for k in s.engines]))
 
 
+@pytest.mark.parametrize("keep", [False, True])
+def test_very_large_batch_equals_its_halves(keep):
+    """500 trajectories of 1018 beads and an odd one, above the size from which the step asks ahead."""
+    from mt_gb300 import engine
+    p = synth.default_params(seed=74)
+    a = synth.make_trajectory(18, 784, seed=74, radius=8.12, psi_mode="make_mt", cube=90.0, thermal=0.05)
+    c = synth.make_trajectory(1, 20, seed=75, radius=8.12, psi_mode="make_mt", cube=40.0, thermal=0.05)
+    b = synth.batch_from_trajectories(p, [a] * 250 + [c] + [a] * 250)
+    assert b.nbeads > 500000
+    with engine.Engine(b) as e, engine.ShardedEngine(b, [0, 0]) as s:
+        for k in [e, s]:
+            k.upload_state(b.coords)
+        for k in [e] + s.engines:
+            k.set_keep_forces(keep)
+        e.step(0, 12)
+        s.step(0, 12)
+        assert np.array_equal(e.download_state(), s.download_state())
+        assert np.array_equal(e.download_rng(), s.download_rng())
+
+
 @pytest.mark.parametrize("turns", [3, 150, 170, 4000])
 def test_bending_of_large_angles(turns):
     """Angle differences of many turns, on both sides of the 1000 rad where the sine
