@@ -1,7 +1,9 @@
 // kernels_step.cu - per-bead forces, the fused force + Euler-Maruyama step,
 // energies, and the state <-> Coord conversions.
 //
-// One thread per bead.  A bead's neighbours are read from the current frame
+// One thread per bead (k_step_plain, k_forces), or in small batches four threads
+// by role (k_split), or one CTA per trajectory for a whole list period
+// (k_period_split, k_step_period).  A bead's neighbours are read from the current frame
 // buffer (16 B gathers of precomputed lab-frame site vectors, L2-resident for
 // the batch sizes of interest); the moving bead writes its new state and new
 // site vectors to the other buffer, so forces and integration fuse into one
@@ -359,8 +361,8 @@ __global__ void __launch_bounds__(256, 4) k_step_plain(KParams P, DevBuffers B) 
 }
 
 // ------------------------------------------------------- persistent period
-// A whole run of plain steps between two pair-list rebuilds in one launch:
-// one CTA per trajectory keeps the trajectory's frames (the four planes) and
+// A whole run of plain steps between two pair-list rebuilds in one launch, for
+// trajectories too large for k_period_split: one CTA per trajectory keeps the trajectory's frames (the four planes) and
 // flags in shared memory across the steps, so every neighbour gather of the
 // force loop is a shared-memory load; the pair lists and noise streams stay
 // in global memory (L2).  Each step is a force phase over the CTA's beads, a

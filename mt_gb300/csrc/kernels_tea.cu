@@ -419,7 +419,7 @@ __device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, 
 
 // Runs while gate is null or *gate == run_if.
 template <class Op>
-__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int4 *work, int nwork,
+__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
                                                              float4 *feff, const int *gate, int run_if) {
     chain_wait();
     if (gate && *gate != run_if) return;
@@ -437,9 +437,9 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
         const long long first = B.tea_unit0[item];
         const int nblk = (int)(B.tea_unit0[item + 1] - first);
         const int b0 = (int)(u - first), b1 = (int)min((long long)nblk, u_end - first);
-        const int4 w = work[item];   // trajectory, first bead, end of the trajectory, its first block
+        const int2 w = work[item], span = B.tea_span[item];
         const int traj = w.x, g = w.y + tid;
-        const float4 *pack = B.tea_pack + (size_t)w.w * kTeaBlockF4;
+        const float4 *pack = B.tea_pack + (size_t)span.y * kTeaBlockF4;
         auto issue = [&](int tile) {
             const int q0 = b0 + tile * kTeaTileBlocks, nq = min(kTeaTileBlocks, b1 - q0);
             float4 *dst = s_tile[tile % kTeaStages];
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
             if (k < ntiles) issue(k);
             cp_async_commit();
         }
-        const bool valid = g < w.z;
+        const bool valid = g < span.x;
         const float4 p = valid ? B.frame_in[g] : make_float4(0.f, 0.f, 0.f, 0.f);
         const bool act = __any_sync(0xffffffffu, valid && !(B.flags[g] & kFlagExtra));
         Op X;
@@ -614,7 +614,7 @@ static int tea_runs(const KParams &P, bool rare) {
     return (int)std::min(runs, slots);
 }
 template <class Op>
-static void tea_launch(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff, const int *gate,
+static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
                        int run_if, cudaStream_t s) {
     if (P.nb <= kTeaLaneBeads && P.tea_units <= kTeaLaneUnits) {
         const int beads = kTeaLaneThreads / kTeaLanes;
@@ -630,11 +630,11 @@ void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
 void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s) {
     k_tea_pack_clear<<<(int)(((size_t)nblocks * kTeaBlockF4 + 255) / 256), 256, 0, s>>>(pack, nblocks);
 }
-void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
+void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                           int run_if, cudaStream_t s) {
     tea_launch<EpsOp>(P, B, work, nwork, nullptr, gate, run_if, s);
 }
-void launch_tea_eps(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s) {
+void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
     launch_tea_eps_gated(P, B, work, nwork, nullptr, 0, s);
 }
 void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious, float epsmax, const int *gate,
@@ -644,14 +644,14 @@ void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s) {
     launch_tea_beta_gated(P, B, capricious, epsmax, nullptr, 0, s);
 }
-void launch_tea_step(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s) {
+void launch_tea_step(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s) {
     tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, nullptr, 0, s);
 }
-void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
+void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                            cudaStream_t s) {
     tea_launch<StepOp<false>>(P, B, work, nwork, nullptr, gate, 1, s);
 }
-void launch_tea_feff(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff,
+void launch_tea_feff(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
                      const int *gate, cudaStream_t s) {
     tea_launch<StepOp<true>>(P, B, work, nwork, feff, gate, 0, s);
 }
@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
             const float3 y = ff_proxy(cJ, hJ, m);
             const float2 dx = __fadd2_rn(f2(y.x), nxx), dy = __fadd2_rn(f2(y.y), nxy), dz = __fadd2_rn(f2(y.z), nxz);
             const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-            const float2 rinv = make_float2(rsqrt_hw(fmaxf(r2.x, K.four_a2)), rsqrt_hw(fmaxf(r2.y, K.four_a2)));
+            const float2 rinv = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
             const float2 q2 = __fmul2_rn(rinv, rinv), tq = __fmul2_rn(q2, rinv);
             const float2 cii = __ffma2_rn(vkap, tq, rinv);
             const float2 cr = __fmul2_rn(tq, __ffma2_rn(vn2a2, q2, one));

@@ -522,7 +522,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     e->nwork = (int)work.size();
     // all-pairs TEA kernels: chunks of kTeaChunk beads i, blocks of kTeaBlock
     // beads j, a chunk's units = the blocks of its trajectory
-    std::vector<int4> tea_work;
+    std::vector<int2> tea_work, tea_span;
     std::vector<int> tea_slot(nb), tea_blk0(nt + 1);
     std::vector<long long> tea_unit0{0};
     for (int tr = 0; tr < nt; tr++) {
@@ -531,7 +531,8 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         e->kp.tea_max_blocks = std::max(e->kp.tea_max_blocks, nblk);
         for (int i = 0; i < n; i++) tea_slot[t->offsets[tr] + i] = tea_blk0[tr] * kTeaBlock + i;
         for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) {
-            tea_work.push_back(make_int4(tr, g, t->offsets[tr + 1], tea_blk0[tr]));
+            tea_work.push_back(make_int2(tr, g));
+            tea_span.push_back(make_int2(t->offsets[tr + 1], tea_blk0[tr]));
             tea_unit0.push_back(tea_unit0.back() + nblk);
         }
     }
@@ -541,14 +542,8 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
     const std::vector<int4> list_work = plan_lists(sms, nt, t->offsets, &e->list_parts);
     e->list_nwork = (int)list_work.size();
-    // threads per bead in the near-pair kernel of learned TEA: enough to fill the GPU
-    {
-        // two beads per thread; aim for about two full waves at 64 registers
-        const double target = (double)sms * 2048.0;
-        int sl = 1;
-        while (sl < 8 && (double)nb / 4 * sl < target) sl <<= 1;   // four beads per thread
-        e->kp.tea_slices = sl;
-    }
+    // the tuning's tea_slices as reported before anything sets it (no kernel reads it)
+    for (e->tea_slices = 1; e->tea_slices < 8 && (double)nb / 4 * e->tea_slices < sms * 2048.0;) e->tea_slices <<= 1;
 
 #define ALLOC(ptr, n)                         \
     do {                                      \
@@ -588,6 +583,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     ALLOC(e->stage_i, nb);
     if (p->hdi_on) {
         ALLOC(e->tea_work, e->tea_nwork);
+        ALLOC(e->tea_span, e->tea_nwork);
         ALLOC(e->tea_r, nb);
         ALLOC(e->tea_ci, nb);
         ALLOC(e->tea_eps, nb);
@@ -650,7 +646,8 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     cudaMemsetAsync(e->latc, 0, sizeof(int) * nb, s);
     cudaMemsetAsync(e->force, 0, sizeof(float4) * 2 * nb, s);
     if (p->hdi_on) {
-        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int4) * tea_work.size(), s)) ||
+        if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int2) * tea_work.size(), s)) ||
+            (rc = upload(e->tea_span, tea_span.data(), sizeof(int2) * tea_span.size(), s)) ||
             (rc = upload(e->tea_slot, tea_slot.data(), sizeof(int) * nb, s)) ||
             (rc = upload(e->tea_unit0, tea_unit0.data(), sizeof(long long) * tea_unit0.size(), s))) {
             mtg_destroy(e);
@@ -769,7 +766,7 @@ int mtg_destroy(mtg_engine *e) {
                     e->surr_desc, e->surr_pred, e->surr_stats, e->surr_gate, e->surr_err, e->surr_part,
                     e->tea_ci2, e->feff_a, e->feff_b, e->tea_eps2, e->tea_beta2, e->tea_eps_t2,
                     e->hydro_cand, e->hydro_rank, e->hydro_sums, e->hydro_counts, e->hydro_events,
-                    e->tea_pack, e->tea_slot, e->tea_unit0, e->tea_part, e->tea_cnt};
+                    e->tea_pack, e->tea_span, e->tea_slot, e->tea_unit0, e->tea_part, e->tea_cnt};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (e->stage_host) cudaFreeHost(e->stage_host);
@@ -1094,7 +1091,7 @@ int mtg_get_tuning(mtg_engine *e, mtg_tuning *t) {
     if (!e || !t) return fail(MTG_E_CONFIG, "engine or tuning is NULL");
     t->list_method = e->use_cells ? 2 : 1;
     t->step_block = e->kp.step_block;
-    t->tea_slices = e->kp.tea_slices;
+    t->tea_slices = e->tea_slices;
     t->tea_jparts = e->tea_jparts;
     t->plain_persistent = e->persistent ? 1 : 0;
     return MTG_OK;
@@ -1120,7 +1117,7 @@ int mtg_set_tuning(mtg_engine *e, const mtg_tuning *t) {
     }
     e->persistent = t->plain_persistent != 0;
     e->kp.step_block = t->step_block;
-    e->kp.tea_slices = t->tea_slices;
+    e->tea_slices = t->tea_slices;
     e->tea_jparts = t->tea_jparts;
     destroy_graphs(e);
     return MTG_OK;
@@ -1146,13 +1143,8 @@ int mtg_autotune(mtg_engine *e, long long first_step, int trial_steps, mtg_tunin
     for (int lm : {1, 2}) {
         if (lm == 2 && (!cells_ok || !lists)) continue;
         if (lm == 1 && !lists && !cands.empty()) continue;
-        if (e->p.hdi_on) {
-            // the all-pairs kernels divide their work themselves; threads per bead
-            // matter to the near pairs of the learned mode alone
-            if (e->surr && e->ff_on)
-                for (int sl : {2, 4, 8}) cands.push_back({lm, orig.step_block, sl, orig.tea_jparts, 0});
-            else
-                cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 0});
+        if (e->p.hdi_on) {   // the TEA kernels divide their work themselves
+            cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 0});
         } else {
             for (int bs : {64, 128, 256}) cands.push_back({lm, bs, orig.tea_slices, orig.tea_jparts, 0});
             if (period_fits(e->max_traj_beads)) cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 1});

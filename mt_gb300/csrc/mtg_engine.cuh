@@ -34,7 +34,8 @@ struct mtg_engine {
     int nwork = 0;
     int4 *list_work = nullptr;  // CTAs of the one-launch list rebuild: trajectory, first bead, beads
     int list_nwork = 0, list_parts = 1;
-    int4 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels: trajectory, first bead, its end, its first block
+    int2 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels
+    int2 *tea_span = nullptr;   // their trajectories' ends and first blocks
     int tea_nwork = 0;
     int *work_first = nullptr;
     double *en_partials = nullptr, *en_traj = nullptr, *en_bead = nullptr;
@@ -44,7 +45,7 @@ struct mtg_engine {
     float4 *tea_pack = nullptr, *tea_part = nullptr;   // all-pairs TEA kernels, see DevBuffers
     int *tea_slot = nullptr, *tea_cnt = nullptr;
     long long *tea_unit0 = nullptr;
-    int tea_jparts = 1;            // as set (no effect any more)
+    int tea_slices = 1, tea_jparts = 1;   // of the tuning, as set (no kernel reads them)
     float *stage = nullptr;        // 7*nb floats for host <-> device Coord transfers
     void *stage_host = nullptr;    // pinned mirror of stage
     uint8_t *stage_u8 = nullptr;
@@ -145,6 +146,7 @@ struct mtg_engine {
         b.lat = lat;
         b.err = err;
         b.tea_pack = tea_pack;
+        b.tea_span = tea_span;
         b.tea_slot = tea_slot;
         b.tea_unit0 = tea_unit0;
         b.tea_part = tea_part;

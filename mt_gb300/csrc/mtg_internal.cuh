@@ -60,7 +60,6 @@ struct KParams {
     int maxH, maxLong, maxLat, maxLJ;
     // TEA
     float tea_a, tea_var;
-    int tea_slices;        // threads per bead in the near-pair kernel of learned TEA (1, 2, 4 or 8)
     int tea_max_blocks;    // blocks of kTeaBlock beads of the largest trajectory
     long long tea_units;   // (chunk of kTeaChunk beads) x (block) pairs of the all-pairs kernels
     int chain;             // launch the kernels of a step chained (launch_chained)
@@ -89,6 +88,7 @@ struct DevBuffers {
     double *tea_eps_t;     // [nt]
     // all-pairs kernels (kernels_tea.cu)
     float4 *tea_pack;      // every trajectory's beads in blocks, see tea_pack_bead
+    const int2 *tea_span;  // of each work item: end of its trajectory, first block of it
     const int *tea_slot;   // [nb] slot of each bead in the pack (32 a block)
     const long long *tea_unit0;  // [work items + 1] first unit of each item
     float4 *tea_part;      // partial sums: two slots of kTeaChunk beads per CTA of a launch
@@ -522,16 +522,16 @@ constexpr int kTeaMaxOcc = 12;       // CTAs of the all-pairs kernels per SM at 
 // positions (F and R are zeroed once) into the pack, for epsilon passes outside a TEA step
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s);
 void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s);
-void launch_tea_eps(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s);
+void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s);
-void launch_tea_step(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, cudaStream_t s);
+void launch_tea_step(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 // gated variants: run only while *gate == run_if
-void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
+void launch_tea_eps_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                           int run_if, cudaStream_t s);
 void launch_tea_beta_gated(const KParams &P, const DevBuffers &B, int capricious, float epsmax, const int *gate,
                            int run_if, cudaStream_t s);
 // effective TEA force (no update) into feff, while *gate == 0
-void launch_tea_feff(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, float4 *feff,
+void launch_tea_feff(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff,
                      const int *gate, cudaStream_t s);
 void launch_set_flags(int nb, const uint8_t *extra, const int *gtp, const int *on_tubule, int *flags,
                       cudaStream_t s);
@@ -601,7 +601,7 @@ void launch_ff_far(const KParams &P, const DevBuffers &B, const FFBuffers &F, bo
 void launch_ff_step(const KParams &P, const DevBuffers &B, const FFBuffers &F, bool feff_only, float4 *feff,
                     const int *gate, cudaStream_t s);
 // the exact mobility product + update, only while *gate == 1 (after a fall-back to exact TEA)
-void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int4 *work, int nwork, const int *gate,
+void launch_tea_step_gated(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, const int *gate,
                            cudaStream_t s);
 
 }  // namespace mtg
