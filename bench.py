@@ -258,13 +258,15 @@ def tea_pairs(b) -> int:
     return tot
 
 
-def plain_step_time(kt_ms: dict, launches: dict, period: int):
-    """(kernel, average device ms per MD step) of the plain path's step kernel:
-    the per-step launch, or the persistent launch that covers a whole
+def plain_step_time(kt_ms: dict, launches: dict, period: int, b):
+    """(kernel, average device ms per MD step) of the plain path's step kernel for
+    the batch b: the per-step launch, or the persistent launch that covers a whole
     pair-list period of `period` steps."""
     if launches.get("step_period"):
-        return "k_step_period", kt_ms["step_period"] / (launches["step_period"] * period)
-    return "k_step_plain", kt_ms["step_plain"] / max(1, launches["step_plain"])
+        kernel = "k_period_split" if int(np.diff(b.offsets).max()) <= 192 else "k_step_period"
+        return kernel, kt_ms["step_period"] / (launches["step_period"] * period)
+    kernel = "k_split" if b.nbeads <= 55000 else "k_step_plain"
+    return kernel, kt_ms["step_plain"] / max(1, launches["step_plain"])
 
 
 def ncu_traffic(kernel: str, workload: str):
@@ -469,7 +471,7 @@ def run_gpu(args, spec, dist, cpu_seconds: float = 20.0):
         n_i = (L["lj"][0].astype(np.int64) + L["long"][0] + L["lat"][0] + b.harmonic_count).astype(np.int64)
         act = b.extra == 0
         work = float(np.sum((48 + 64 + 16 + 4 * n_i)[act]))
-        kname, avg_ms = plain_step_time(kt_ms, launches, period)
+        kname, avg_ms = plain_step_time(kt_ms, launches, period, b)
         peak, peak_kind = measured_peaks()
         achieved = work / (avg_ms / 1e3) / 1e9
         roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak,
@@ -483,9 +485,9 @@ def run_gpu(args, spec, dist, cpu_seconds: float = 20.0):
         tf = C.c_double()
         engine.check(engine.load().mtg_measure_fp32_tflops(dist.local, C.byref(tf)))
         achieved = work / (avg_ms / 1e3) / 1e12
-        roof = {"bound": "fp32", "kernel": "k_tea_step", "achieved": achieved, "peak": tf.value,
+        roof = {"bound": "fp32", "kernel": "k_tea_pass", "achieved": achieved, "peak": tf.value,
                 "peak_source": "measured FP32 FMA rate (mtg_measure_fp32_tflops)", "unit": "TFLOP/s",
-                "frac": achieved / tf.value, "traffic": ncu_traffic("k_tea_step", args.workload),
+                "frac": achieved / tf.value, "traffic": ncu_traffic("k_tea_pass", args.workload),
                 "algorithmic_flop_per_launch": work, "avg_launch_ms": avg_ms}
 
     # end to end through the C ABI with pinned host buffers
@@ -584,7 +586,7 @@ def run_long(args, spec, dist):
     L = e.lists()
     n_i = (L["lj"][0].astype(np.int64) + L["long"][0] + L["lat"][0] + b.harmonic_count).astype(np.int64)
     work = float(np.sum((48 + 64 + 16 + 4 * n_i)[b.extra == 0]))
-    kname, avg_ms = plain_step_time(kt_ms, nl, period)
+    kname, avg_ms = plain_step_time(kt_ms, nl, period, b)
     peak, peak_kind = measured_peaks()
     achieved = work / (avg_ms / 1e3) / 1e9
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "peak_source": peak_kind,
@@ -815,7 +817,7 @@ def run_tea_compare(args, spec, dist):
     L, X, S = results["learned"], results["exact"], results["exact_stale_eps"]
     learned_ok = not L["status"]["fell_back"]
     ffs = L["farfield"]
-    roof_exact = fp32_roof(X["kt"], "tea_step", "k_tea_step", 45.0 * tea_pairs(b), "45 FLOP per ordered pair")
+    roof_exact = fp32_roof(X["kt"], "tea_step", "k_tea_pass", 45.0 * tea_pairs(b), "45 FLOP per ordered pair")
     roof_ff = fp32_roof(L["kt"], "ff_near", "k_ff_near", 45.0 * ffs["near_pairs"],
                         "45 FLOP per ordered near pair (the pair loop of k_ff_near; its list walk not counted)")
     out = None
@@ -1008,7 +1010,7 @@ def run_profile_case(name: str):
         else:
             if name == "step_plain":
                 e.set_tuning(2, 256, 1, 1, plain_persistent=0)
-            else:   # whole j ranges: k_tea_step alone, no split tail
+            else:   # k_tea_pass
                 e.set_tuning(2, 128, 4, 1, plain_persistent=0)
             e.step(0, c["steps"])
         out["status"] = "ok"
