@@ -419,9 +419,9 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 //     ascending j; only the site planes that a test needs are then gathered.
 // Bound by instruction issue and, in the walk, by shared-memory bandwidth.
 // 256 x 1520 beads: 203 us for the general path's six launches (the 27-bucket
-// walk ran 7600 instructions a warp, half of them on repeated buckets), 62 us here;
-// 1024 uneven trajectories of up to 3560 beads 775 -> 277 us, 101 lattices of 780 beads
-// 66 -> 22 us, one trajectory of 156 beads 45 (tiles) -> 10 us.
+// walk ran 7600 instructions a warp, half of them on repeated buckets), 61 us here;
+// 1024 uneven trajectories of up to 3560 beads 775 -> 275 us, 101 lattices of 780 beads
+// 66 -> 21 us, one trajectory of 156 beads 45 (tiles) -> 10 us.
 constexpr int kSmemKeys = 32;      // slots for a bead's hits; beads with more than 28 take the slow path below
 constexpr int kSmemBeads = 8192;   // 13 bits of a key
 constexpr unsigned kNoKey = 0x10000u;
@@ -620,10 +620,21 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         return (int)((row_hash(cell_coord(p.y, inv), cell_coord(p.z, inv)) + (uint32_t)cell_coord(p.x, inv)) &
                      (uint32_t)(m - 1));
     };
-    for (int j = t; j < n; j += kListThreads) {
-        const int b = bucket(fr[base + j]);
+    // the first beads of a thread stay in registers until the fill (read again there: 62.4
+    // against 61.1 us for 256 x 1520 beads)
+    constexpr int kKeep = 4;
+    float4 kept[kKeep];
+#pragma unroll
+    for (int k = 0; k < kKeep; k++)
+        if (t + k * kListThreads < n) kept[k] = fr[base + t + k * kListThreads];
+    auto count = [&](float4 p) {
+        const int b = bucket(p);
         atomicAdd(&s_tab[b >> 1], 1u << (16 * (b & 1)));
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; k++)
+        if (t + k * kListThreads < n) count(kept[k]);
+    for (int j = t + kKeep * kListThreads; j < n; j += kListThreads) count(fr[base + j]);
     __syncthreads();
     {   // exclusive scan of the counts, whole words a thread
         const int per = (m / 2 + kListThreads - 1) / kListThreads, lo = min(m / 2, t * per), hi = min(m / 2, lo + per);
@@ -645,13 +656,16 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         }
     }
     __syncthreads();
-    for (int j = t; j < n; j += kListThreads) {
-        float4 p = fr[base + j];
+    auto place = [&](int j, float4 p) {
         const int b = bucket(p), sh = 16 * (b & 1);
         const unsigned slot = (atomicAdd(&s_tab[b >> 1], 1u << sh) >> sh) & 0xffffu;
         p.w = __int_as_float(j);
         s_pos[slot] = p;
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kKeep; k++)
+        if (t + k * kListThreads < n) place(t + k * kListThreads, kept[k]);
+    for (int j = t + kKeep * kListThreads; j < n; j += kListThreads) place(j, fr[base + j]);
     __syncthreads();
 
     // the bead of this thread, and which of the bead's threads it is
