@@ -66,7 +66,7 @@ __device__ __forceinline__ bool group_and(int g, bool v) {
 // Y[n][kOut] = network(normalise(X)) for n rows; err gets kErrTimeout if a
 // wait for the tensor cores runs out.  TRAIN: row i of the batch is sample
 // idx[i] of X (idx may be NULL), and the pre-activations z1..z3 are stored
-// to Z [n][3][kHid] for the backward pass.
+// to Z for the backward pass.
 template <bool TRAIN>
 __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd_tc(const Weights W, const float *X, const int *idx, int n,
                                                                const float *norm, float *Y, float *Z, int *err,
@@ -164,10 +164,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd_tc(const Weights W, 
                     tmem_ld_x32(lane_base + (uint32_t)c0, v);
                     tmem_wait_ld();
                     if (TRAIN && row0 + r < n) {   // pre-activations for the backward pass
-                        float4 *zr = reinterpret_cast<float4 *>(Z + ((size_t)(row0 + r) * 3 + layer) * kHid + c0);
+                        float4 *zr = reinterpret_cast<float4 *>(Z) + (((size_t)tile * 3 + layer) * kHid + c0) / 4 * kTcRows + r;
 #pragma unroll
                         for (int q = 0; q < 8; q++)
-                            zr[q] = make_float4(__uint_as_float(v[4 * q]) + bias[c0 + 4 * q],
+                            zr[q * kTcRows] = make_float4(__uint_as_float(v[4 * q]) + bias[c0 + 4 * q],
                                                 __uint_as_float(v[4 * q + 1]) + bias[c0 + 4 * q + 1],
                                                 __uint_as_float(v[4 * q + 2]) + bias[c0 + 4 * q + 2],
                                                 __uint_as_float(v[4 * q + 3]) + bias[c0 + 4 * q + 3]);

@@ -62,11 +62,14 @@ uint32_t tc_default_spin();
 cudaError_t launch_infer_tc(const Weights &W, const float *X, int n, const float *norm, float *Y, int *err,
                             cudaStream_t s, uint32_t spin = tc_default_spin());
 // Training on the tcgen05 tensor cores: the forward pass with the
-// pre-activations Z [n][3][kHid] (rows of X gathered through idx, may be
-// NULL), and the backward pass (kernels_mlp_train_tc.cu) writing per-CTA
+// pre-activations Z (z_floats(n) floats: [tile of 128 rows][3][kHid / 4][row][4], so that
+// threads with neighbouring rows touch neighbouring words (the forward pass of 4096 rows
+// 23 us with [row][3][kHid], 15 so); rows of X gathered
+// through idx, may be NULL), and the backward pass (kernels_mlp_train_tc.cu) writing per-CTA
 // partial gradients G [backward_parts(n)][kParams] and loss sums.
 cudaError_t launch_forward_tc(const Weights &W, const float *X, const int *idx, int n, const float *norm, float *Y,
                               float *Z, int *err, cudaStream_t s);
+inline size_t z_floats(int n) { return ((size_t)n + 127) / 128 * 128 * 3 * kHid; }
 cudaError_t prepare_backward_tc();
 int backward_parts(int n);
 cudaError_t launch_backward_tc(const Weights &W, const float *X, const int *idx, const float *norm, const float *T,

@@ -519,7 +519,7 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
         for (int k = 0; k < mlp::kOut; k++)
             Tn[(size_t)i * mlp::kOut + k] = (T[(size_t)i * mlp::kOut + k] - s->h_ynorm[k]) / s->h_ynorm[mlp::kOut + k];
     ScratchLease A(s);
-    const size_t nx = (size_t)n * mlp::kIn, ny = (size_t)n * mlp::kOut, nz = (size_t)n * 3 * mlp::kHid,
+    const size_t nx = (size_t)n * mlp::kIn, ny = (size_t)n * mlp::kOut, nz = mlp::z_floats(n),
                  ng = (size_t)parts * mlp::kParams;
     SCK(A.reserve(A.room(nx) + 2 * A.room(ny) + A.room(nz) + A.room(ng) + A.room(mlp::kParams) + A.room(parts)));
     float *dX = A.take(nx), *dT = A.take(ny), *dY = A.take(ny), *dZ = A.take(nz), *dG = A.take(ng),
@@ -604,7 +604,7 @@ int mtg_surrogate_train(mtg_surrogate *s, const float *X, const float *T, int n,
     SCK(cudaMalloc(&S.X, sizeof(float) * (size_t)n * mlp::kIn));
     SCK(cudaMalloc(&S.T, sizeof(float) * (size_t)n * mlp::kOut));
     SCK(cudaMalloc(&S.Y, sizeof(float) * (size_t)batch * mlp::kOut));
-    SCK(cudaMalloc(&S.Z, sizeof(float) * (size_t)batch * 3 * mlp::kHid));
+    SCK(cudaMalloc(&S.Z, sizeof(float) * mlp::z_floats(batch)));
     SCK(cudaMalloc(&S.G, sizeof(float) * (size_t)parts * mlp::kParams));
     SCK(cudaMalloc(&S.L, sizeof(float) * (size_t)parts * nbatches));
     SCK(cudaMalloc(&S.Lsum, sizeof(float) * epochs));
