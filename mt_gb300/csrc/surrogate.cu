@@ -90,14 +90,20 @@ __device__ __forceinline__ void desc_add(float (&s)[10], float rinv, float ux, f
 // one or two cells and walk the same 27-cell neighbourhood, so candidate
 // loads are broadcasts and the loops mostly uniform.  Cells are 20 nm; the
 // candidates of a bucket are visited in ascending bead index.
+// PARTS threads share a bead's cells and add their sums by shuffles: batches too small to fill
+// the GPU last as long as one thread's walk.  Descriptors of 11,040 beads (call with the
+// copy back) 128 us with one thread a bead and 90 with four, 52,800 beads 300 and 273, 105,600 beads
+// 475 and 488; two threads 105, 271 and 483, eight 93, 281 and 514.
+constexpr int kDescParts = 4, kDescSplitBeads = 60000;
+template <int PARTS>
 __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, CellBuffers C, const int2 *work,
                                                        float inv_cell, const float4 *stats, float *desc,
                                                        const int *gate) {
     if (gate && *gate) return;
-    const int2 w = work[blockIdx.x];
+    const int2 w = work[blockIdx.x / PARTS];
     const int traj = w.x, end = B.off[traj + 1];
     const int base = B.off[traj];
-    const int slot = w.y + threadIdx.x;
+    const int slot = w.y + (blockIdx.x % PARTS) * (kTile / PARTS) + threadIdx.x / PARTS, part = threadIdx.x % PARTS;
     __shared__ int s_bk[27][kTile];
     if (slot >= end) return;
     const float4 pi = C.cell_pos[slot];
@@ -126,11 +132,12 @@ __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, 
             for (int v = 0; v < c; v++) seen |= (bk[v] == bk[c]);
             dup |= (seen ? 1u : 0u) << c;
         }
-        int st_next = C.start[bk[0]], ct_next = C.cnt[bk[0]];
-        for (int c = 0; c < 27; c++) {
+        const int b0 = PARTS == 1 ? bk[0] : s_bk[part][threadIdx.x];
+        int st_next = C.start[b0], ct_next = C.cnt[b0];
+        for (int c = part; c < 27; c += PARTS) {
             const int st_c = st_next, ct_c = ct_next;
-            if (c + 1 < 27) {   // the next cell's range is fetched while this one runs
-                const int b = s_bk[c + 1][threadIdx.x];
+            if (c + PARTS < 27) {   // the next cell's range is fetched while this one runs
+                const int b = s_bk[c + PARTS][threadIdx.x];
                 st_next = C.start[b];
                 ct_next = C.cnt[b];
             }
@@ -158,11 +165,23 @@ __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, 
                 }
             }
         }
+        if (PARTS > 1) {
+            const unsigned bead = ((1u << PARTS) - 1u) << (threadIdx.x & 31 & ~(PARTS - 1));
+#pragma unroll
+            for (int o = 1; o < PARTS; o <<= 1)
+#pragma unroll
+                for (int k = 0; k < 10; k++) {
+                    s0[k] += __shfl_xor_sync(bead, s0[k], o);
+                    s1[k] += __shfl_xor_sync(bead, s1[k], o);
+                    s2[k] += __shfl_xor_sync(bead, s2[k], o);
+                }
+        }
         const float4 ts = stats[traj];
         f30 = logf(fmaxf(ts.w, 1.0f));
         const float dx = pi.x - ts.x, dy = pi.y - ts.y, dz = pi.z - ts.z;
         f31 = sqrtf(dx * dx + dy * dy + dz * dz) * 0.01f;
     }
+    if (part > 0) return;
     float4 *o = reinterpret_cast<float4 *>(desc + (size_t)g * kF);
     o[0] = make_float4(s0[0], s0[1], s0[2], s0[3]);
     o[1] = make_float4(s0[4], s0[5], s0[6], s0[7]);
@@ -665,7 +684,10 @@ static void launch_descriptors(mtg_engine *e, const int *gate) {
         k_traj_stats<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_stats);
         inv = bin_beads(e->kp, B, e->cells(), kDescCut, true, e->stream);
     }
-    k_descriptors<<<e->nwork, kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv, e->surr_stats, e->surr_desc, gate);
+    const bool split = e->nb <= kDescSplitBeads;
+    const auto kernel = split ? k_descriptors<kDescParts> : k_descriptors<1>;
+    kernel<<<e->nwork * (split ? kDescParts : 1), kTile, 0, e->stream>>>(e->kp, B, e->cells(), e->work, inv,
+                                                                     e->surr_stats, e->surr_desc, gate);
 }
 
 extern "C" {

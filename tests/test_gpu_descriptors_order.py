@@ -76,6 +76,37 @@ def test_largest_trajectory_equals_the_general_kernels():
     columns(X, descriptors(g)[:16384])
 
 
+def test_large_batch_against_fp64():
+    """400 copies of one trajectory: one thread a bead (the smaller batches have four)."""
+    seed = 1
+    while not clear_of_shells(cloud((151,), seed)):
+        seed += 1
+    one = cloud((151,), seed)
+    b = cloud((151,) * 400, seed)
+    b.coords[:] = np.tile(one.coords, (400, 1))
+    X = descriptors(b)
+    columns(X[:151], M.descriptors(one.coords, one.offsets, one.extra))
+    assert np.array_equal(X, np.tile(X[:151], (400, 1)))
+
+
+@pytest.mark.parametrize("n", [33, 129, 19_500])
+def test_gradient_of_uneven_batches(n):
+    """Batches that end inside a tile, and one with a second tile for some CTAs: the
+    suite's bars for the gradient (see test_gpu_surrogate)."""
+    from mt_gb300 import engine
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, M.IN)).astype(np.float32)
+    T = rng.normal(0.9, 0.3, size=(n, M.OUT)).astype(np.float32)
+    with engine.Surrogate(seed=7) as s:
+        p, nrm = s.params()
+        loss, g = s.loss_grad(X, T)
+    Xn, Tn = M.normalise(X, T, nrm)
+    want, gw = M.loss_grad(p, Xn, Tn, emulate_bf16=True)
+    assert abs(loss - want) / want < 2e-3
+    for a, b in zip((M.OFF_W1, M.OFF_W2, M.OFF_W3, M.OFF_W4, M.OFF_B), (M.OFF_W2, M.OFF_W3, M.OFF_W4, M.OFF_B, M.NPARAMS)):
+        assert np.linalg.norm(g[a:b] - gw[a:b]) <= 2e-2 * np.linalg.norm(gw[a:b])
+
+
 def test_surrogate_scratch():
     """Calls of any order of sizes, past the scratch that is kept, and from two threads
     at once give what a fresh surrogate gives."""
