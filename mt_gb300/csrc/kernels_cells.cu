@@ -600,7 +600,6 @@ __device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &
 template <int PARTS>
 __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int4 *work, int nmax,
                                                                   float inv, ListCuts cut) {
-    chain_wait();
     extern __shared__ float4 s_dyn[];
     const int4 w = work[blockIdx.x];   // trajectory, first bead, number of beads
     const int base = B.off[w.x], n = B.off[w.x + 1] - base, nb = P.nb;
@@ -615,6 +614,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
 
     // the beads in bucket order
     for (int k = t; k < m / 2; k += kListThreads) s_tab[k] = 0;
+    chain_wait();   // no kernel writes the plan that was read so far
     __syncthreads();
     auto bucket = [&](float4 p) {
         return (int)((row_hash(cell_coord(p.y, inv), cell_coord(p.z, inv)) + (uint32_t)cell_coord(p.x, inv)) &

@@ -545,7 +545,7 @@ __device__ __forceinline__ void get_parts(float (*s)[kSplitBeads], int l, Acc &A
 // with the random force of every bead).
 template <bool STEP, bool KEEP_FORCES, bool TEA>
 __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B) {
-    chain_wait();
+    if (!P.early) chain_wait();
     __shared__ float s_part[kParts][kSplitBeads];
     const int role = threadIdx.x >> 5, l = threadIdx.x & 31, g = blockIdx.x * kSplitBeads + l;
     const int nb = P.nb;
@@ -556,10 +556,15 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
     float4 gx, ga, rt;
     Frame Fi;
     Euler E;
+    NbrView V;
+    ListHead H;
+    if (role < 3 && work) {
+        V = {B.frame_in, B.flags, nb, B.base[g]};
+        H = list_head(P, B, g);
+    }
+    if (P.early) chain_wait();   // all above has been there since before the last launch
     if (role < 3) {
         if (work) {
-            const NbrView V = {B.frame_in, B.flags, nb, B.base[g]};
-            const ListHead H = list_head(P, B, g);
             const float4 p0 = B.frame_in[g];
             if (role == 0) {
                 put_axial(s_part, l, axial_force(P, B, V, g, flags, p0, B.frame_in[nb + g], B.frame_in[2 * nb + g].w, H));

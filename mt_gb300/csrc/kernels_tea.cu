@@ -421,8 +421,6 @@ __device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, 
 template <class Op>
 __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
                                                              float4 *feff, const int *gate, int run_if) {
-    chain_wait();
-    if (gate && *gate != run_if) return;
     constexpr int kW = Op::kWords;
     __shared__ float4 s_tile[kTeaStages][kTeaTileBlocks * kW];
     __shared__ int s_last;
@@ -432,6 +430,8 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
     long long u = tea_run_start(U, G, blockIdx.x);
     const long long u_end = tea_run_start(U, G, blockIdx.x + 1);
     int item = tea_find_item(B.tea_unit0, nwork, u);
+    chain_wait();   // no kernel writes the units
+    if (gate && *gate != run_if) return;
     const TeaConst K = tea_const(P.tea_a);
     while (u < u_end) {
         const long long first = B.tea_unit0[item];
@@ -542,14 +542,14 @@ constexpr int kTeaLanes = 32, kTeaLaneThreads = 128;
 template <class Op>
 __global__ void __launch_bounds__(kTeaLaneThreads) k_tea_lanes(KParams P, DevBuffers B, float4 *feff, const int *gate,
                                                                int run_if) {
-    chain_wait();
-    if (gate && *gate != run_if) return;
     constexpr int kGroups = kTeaLanes / kTeaPairSlots;   // blocks taken at once
     const int g = blockIdx.x * (kTeaLaneThreads / kTeaLanes) + threadIdx.x / kTeaLanes, lane = threadIdx.x % kTeaLanes;
     const int t = lane % kTeaPairSlots;
     const bool valid = g < P.nb;
     const int gc = valid ? g : P.nb - 1;
     const int traj = B.traj[gc], base = B.off[traj], n = B.off[traj + 1] - base, slot = B.tea_slot[gc];
+    chain_wait();   // no kernel writes what was read so far
+    if (gate && *gate != run_if) return;
     const float4 p = B.frame_in[gc];
     const TeaConst K = tea_const(P.tea_a);
     Op X;
