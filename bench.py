@@ -265,7 +265,7 @@ def plain_step_time(kt_ms: dict, launches: dict, period: int, b):
     if launches.get("step_period"):
         kernel = "k_period_split" if int(np.diff(b.offsets).max()) <= 192 else "k_step_period"
         return kernel, kt_ms["step_period"] / (launches["step_period"] * period)
-    kernel = "k_split" if b.nbeads <= 55000 else "k_step_plain"
+    kernel = "k_split" if b.nbeads <= 75000 else "k_step_plain"
     return kernel, kt_ms["step_plain"] / max(1, launches["step_plain"])
 
 

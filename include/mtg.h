@@ -428,7 +428,7 @@ int mtg_tea_effective_forces(mtg_engine *e, float *feff_exact, float *feff_ff, f
 /* ---- tuning ------------------------------------------------------------ */
 /* Launch shapes of the engine's kernels.  list_method as
  * mtg_set_list_method (1 tiles, 2 cells); step_block: threads per CTA of the
- * fused plain step of more than 55,000 beads (64, 128, 256); tea_slices (1, 2, 4, 8)
+ * fused plain step of more than 75,000 beads (64, 128, 256); tea_slices (1, 2, 4, 8)
  * and tea_jparts (1, 2, 3, 4): kept for saved tunings, without effect (the TEA
  * kernels divide their work over the GPU themselves); plain_persistent: 1 runs
  * the plain (no-HI) steps between two pair-list rebuilds as one launch with

@@ -417,10 +417,11 @@ __device__ __forceinline__ uint32_t cell_hash(int cx, int cy, int cz) {
 }
 
 // Beads up to which the four-warp form is used.  It wins while its four times as
-// many warps stay within about one and a half fillings of the GPU: a step of one
-// 1520-bead trajectory took 6.8 us with one thread a bead and 4.6 us so, forces
-// of 52,800 beads 11.5 and 11.0 us, but a step of 78,780 beads 12.2 and 14.5 us.
-constexpr int kSplitMaxBeads = 55000;
+// many warps stay within about two fillings of the GPU, and only its launches are chained.
+// 100 steps with lists, one thread a bead and so: 60,800 beads (a third of them in a lattice) 969 and
+// 840 us, 68,640 lattice beads 1396 and 1318, but 78,780 lattice beads 1453 and 1482, 124,800
+// 1800 and 2003.
+constexpr int kSplitMaxBeads = 75000;
 
 // Bucket of cell (cx, cy, cz) = (row_hash(cy, cz) + cx) mod a power of two: the
 // cells of a row along x are neighbouring buckets.

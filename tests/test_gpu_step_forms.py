@@ -12,16 +12,16 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("over", [dict(), dict(barrier=1, is_wall=1, rep_r=20.0)], ids=str)
 @pytest.mark.parametrize("keep", [False, True])
 def test_small_batches_equal_a_large_one(over, keep):
-    """60 trajectories of 1018 and one of 33 beads: above the size of the small form
+    """80 trajectories of 1018 and one of 33 beads: above the size of the small form
     together, below it in three parts."""
     from mt_gb300 import engine
     p = synth.default_params(seed=71, **over)
     a = synth.make_trajectory(18, 784, seed=71, radius=8.12, psi_mode="make_mt", cube=90.0, thermal=0.05)
     c = synth.make_trajectory(1, 20, seed=72, radius=8.12, psi_mode="make_mt", cube=40.0, thermal=0.05)
-    trajs = [a] * 30 + [c] + [a] * 30
+    trajs = [a] * 40 + [c] + [a] * 40
     b = synth.batch_from_trajectories(p, trajs)
     b.extra[5:6000:97] = 1
-    assert b.nbeads > 60000
+    assert b.nbeads > 80000
     with engine.Engine(b) as e, engine.ShardedEngine(b, [0, 0, 0]) as s:
         e.upload_state(b.coords)
         s.upload_state(b.coords)
