@@ -1,5 +1,7 @@
 // kernels_cells.cu - neighbour-list rebuild through a per-trajectory spatial
 // hash (cell list), producing the same lists as the brute-force kernel.
+// k_cell_lists_smem, further down, does it in one launch where the trajectories fit in
+// shared memory; what follows here is the general path.
 //
 // Cells are cubes of edge `reach` (the largest list cutoff, or the 6.6 nm
 // prefilter of the assembly lists), so every partner lies in the 27 cells
