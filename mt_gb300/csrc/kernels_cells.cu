@@ -679,8 +679,9 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     const bool live = !(flags & kFlagExtra);
     const SmemCells C = {s_pos, s_end, n, m, inv};
     // where the bead's own sites are: a bond needs the partner's centre within
-    // 2.5 + 2 nm of one (0.01 nm over the rounding)
-    const float kSite2 = 4.51f * 4.51f;
+    // 2.5 + 2 nm of one (0.01 nm over the rounding of distances, and of a site's coordinates
+    // three units in the last place: beads may be far from the origin)
+    float site_cut = 0.f;
     auto site2 = [](float4 a, float4 q) {   // a coarse test: contracted
         const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
         return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -693,8 +694,8 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         const int jl = __float_as_int(q.w);
         unsigned bits = 0;
         if (P.is_assembly) {
-            bits = (site2(a0, q) < kSite2 ? 1u : 0u) | (site2(a1, q) < kSite2 ? 2u : 0u) |
-                   (site2(a2, q) < kSite2 ? 4u : 0u);
+            bits = (site2(a0, q) < site_cut ? 1u : 0u) | (site2(a1, q) < site_cut ? 2u : 0u) |
+                   (site2(a2, q) < site_cut ? 4u : 0u);
             if (!(r2 < cut.pair) || jl == I.hpart) bits = 0;
         }
         return r2 < cut.lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
@@ -706,6 +707,8 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         const int met = smem_slots(C, p, cut.lj, part * 9 / PARTS, (part + 1) * 9 / PARTS, &s_key[0][t]);
         // the bead's other planes only now: the walk has no registers to spare
         I = list_site(P, p, fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], flags, il, B.harm[g * P.maxH]);
+        const float reach = fmaf(4.0e-7f, fmaxf(fmaxf(fabsf(I.p.x), fabsf(I.p.y)), fabsf(I.p.z)), 4.51f);
+        site_cut = reach * reach;
         a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
         a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
         a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);

@@ -106,3 +106,34 @@ def test_odd_coordinates():
     b.coords[460:465, 1] = np.inf
     b.coords[465:470, 4] = np.nan
     same(b)
+
+
+def far_pairs(points, ends, **over):
+    """One trajectory of pairs of monomers without a partner (points and ends [n, 3]), each with its axis
+    along the pair, so that the longitudinal sites of the two face each other; every pair
+    30 nm from the next along z."""
+    n = 2 * len(points)
+    b = cloud((n,), **over)
+    b.coords[0::2, :3], b.coords[1::2, :3] = points, ends
+    d = (b.coords[1::2, :3].astype(np.float64) - b.coords[0::2, :3])
+    u = -d / np.linalg.norm(d, axis=1)[:, None]
+    b.coords[:, 3] = 0
+    b.coords[:, 4] = np.repeat(np.arccos(u[:, 2]), 2)
+    b.coords[:, 5] = np.repeat(np.arctan2(u[:, 1], u[:, 0]), 2)
+    b.harmonic_count[:] = 0
+    b.harmonic[:] = -1
+    return b
+
+
+@pytest.mark.parametrize("offset", [2.0e5, 9.0e5, 3.9e6])
+def test_sites_far_out(offset):
+    """Bonds near the longest there are, so far out that a site's coordinates keep few digits."""
+    rng = np.random.default_rng(int(offset))
+    n = 1500
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    a = offset * rng.choice([-1.0, 1.0], (n, 3)) + rng.uniform(-50, 50, (n, 3))
+    a[:, 2] += 30.0 * np.arange(n)
+    a = a.astype(np.float32)
+    t = same(far_pairs(a, (a + rng.uniform(6.0, 6.5, (n, 1)) * u).astype(np.float32)))
+    assert t["long"][0].sum() > n / 8
