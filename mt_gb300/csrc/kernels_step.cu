@@ -62,10 +62,18 @@ __device__ __forceinline__ void acc_bend(const KParams &P, Acc &A, float rmon, f
     A.fth = __fmaf_rn(__fmul_rn(sg, P.B_theta), sin_fit(__fmaf_rn(sg, dth, -th0)), A.fth);
 }
 
-// U'(r)/r of a Morse bond plus, with BARR, the Gaussian barrier, from r^2.  r
-// and 1/r come from the hardware reciprocal square root (2e-7 relative, below
-// the rounding of the site vectors that d = site_j - site_i carries).  Sites
-// closer than 1e-15 nm count as touching (no force), as r = 0 does.
+// r and 1/r from r^2 by the hardware reciprocal square root (2e-7 relative, below
+// the rounding of the site vectors that d = site_j - site_i carries).
+// Squares past the largest float count as that one: the exponentials of r are 0 there.
+struct Dist {
+    float r, rinv;
+};
+__device__ __forceinline__ Dist dist_of(float r2) {
+    const float x = fminf(r2, 3.402823466e38f), y = rsqrt_hw(x);
+    return {__fmul_rn(x, y), y};
+}
+// U'(r)/r of a Morse bond.  Squares below the smallest normal float count as touching sites
+// (no force), as r = 0 does.
 __device__ __forceinline__ float dmorse_over_r(float D, float a, float r, float rinv) {
     const float e = expf(__fmul_rn(-a, r));
     return __fmul_rn(__fmul_rn(__fmul_rn(2.0f * a, D), __fmul_rn(__fsub_rn(1.0f, e), e)), rinv);
@@ -73,7 +81,7 @@ __device__ __forceinline__ float dmorse_over_r(float D, float a, float r, float 
 __device__ __forceinline__ float norm2(float3 d) {
     return __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
 }
-constexpr float kTouch2 = 1.0e-30f;
+constexpr float kTouch2 = 1.17549435e-38f;
 
 // Where a bead's neighbours' frames and flags are read: plane k of local bead
 // j at fr[k * stride + base + j], its flags at fl[base + j].  The per-step
@@ -177,10 +185,10 @@ __device__ __forceinline__ Acc axial_force(const KParams &P, const DevBuffers &B
         int gl = flags;   // whose nucleotide sets theta0: the bead's own, or (longitudinal) the
                           // bead's nearer the plus end (:282-283)
         if (!harm) {
-            const float rinv = rsqrt_hw(r2), r = __fmul_rn(r2, rinv);
-            dUdr = dmorse_over_r(P.D_long, P.A_long, r, rinv);
+            const Dist q = dist_of(r2);
+            dUdr = dmorse_over_r(P.D_long, P.A_long, q.r, q.rinv);
             if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
-                dUdr = __fmaf_rn(dbarr(P.a_bl, P.r_bl, P.w_bl, r), rinv, dUdr);
+                dUdr = __fmaf_rn(dbarr(P.a_bl, P.r_bl, P.w_bl, q.r), q.rinv, dUdr);
             if (r2 < kTouch2) dUdr = 0.f;
             if (!(p0.z > rj.z)) gl = fj;
         }
@@ -210,10 +218,11 @@ __device__ __forceinline__ Acc lateral_force(const KParams &P, const DevBuffers 
         const int fj = V.fl[V.base + pj];
         const float3 wi = neg ? l1 : l2;
         const float3 d = site_delta(p0, rj, wi, f3(sj));
-        const float r2 = norm2(d), rinv = rsqrt_hw(r2), r = __fmul_rn(r2, rinv);
-        float dUdr = dmorse_over_r(((flags ^ fj) & kFlagBeta) ? P.D_lat_seam : P.D_lat, P.A_lat, r, rinv);
+        const float r2 = norm2(d);
+        const Dist q = dist_of(r2);
+        float dUdr = dmorse_over_r(((flags ^ fj) & kFlagBeta) ? P.D_lat_seam : P.D_lat, P.A_lat, q.r, q.rinv);
         if (P.barrier && off_tub && (fj & kFlagOnTubule) == 0)
-            dUdr = __fmaf_rn(dbarr(P.a_bt, P.r_bt, P.w_bt, r), rinv, dUdr);
+            dUdr = __fmaf_rn(dbarr(P.a_bt, P.r_bt, P.w_bt, q.r), q.rinv, dUdr);
         if (r2 < kTouch2) dUdr = 0.f;
         acc_pair(A, dUdr, d, wi);
     }

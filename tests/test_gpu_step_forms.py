@@ -123,3 +123,25 @@ def test_persistent_seed_equals_per_step_kernels(sizes, keep):
     for k in ("lj", "long", "lat"):
         assert np.array_equal(l0[k][0], l1[k][0]) and np.array_equal(l0[k][1], l1[k][1])
     assert l0["lj"][0].max() > 1
+
+
+@pytest.mark.parametrize("over", [dict(), dict(barrier=1)], ids=str)
+def test_bonds_past_the_largest_square(over):
+    """A listed partner so far away that the squared distance overflows exerts no force, as one does
+    whose exponential is 0: the other beads' forces are those with the partner at 1e9 nm."""
+    from mt_gb300 import engine
+    b = synth.uniform_batch(synth.default_params(seed=76, **over), 1, 6, 0, seed=76, radius=8.12, psi_mode="make_mt",
+                            thermal=0.05)
+    far, partner = 40, abs(int(b.harmonic[40]))
+    f = []
+    with engine.Engine(b) as e:
+        e.upload_state(b.coords)
+        e.rebuild_pairs()
+        L = e.lists()
+        assert L["lat"][0][far] >= 2
+        for x in (1.0e9, 2.5e19):
+            c = b.coords.copy()
+            c[far, 0] = x
+            e.upload_state(c)
+            f.append(np.delete(e.compute_forces(), (far, partner), 0))
+    assert np.isfinite(f[0]).all() and np.array_equal(f[0], f[1])
