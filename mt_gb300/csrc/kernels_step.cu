@@ -561,11 +561,12 @@ __device__ __forceinline__ void get_parts(float (*s)[kSplitBeads], int l, Acc &A
 // with the random force of every bead).
 template <bool STEP, bool KEEP_FORCES, bool TEA>
 __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B) {
-    if (!P.early) chain_wait();
     __shared__ float s_part[kParts][kSplitBeads];
     const int role = threadIdx.x >> 5, l = threadIdx.x & 31, g = blockIdx.x * kSplitBeads + l;
     const int nb = P.nb;
     const bool valid = g < nb;
+    const int base = valid && role < 3 ? B.base[g] : 0;
+    chain_wait();   // no kernel writes what was read so far
     const int flags = valid ? B.flags[g] : kFlagExtra;
     const bool moving = !(flags & (kFlagExtra | kFlagFixed));
     const bool work = STEP && !KEEP_FORCES ? moving : !(flags & kFlagExtra);
@@ -574,13 +575,10 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(KParams P, DevBuffers B
     Euler E;
     NbrView V;
     ListHead H;
-    if (role < 3 && work) {
-        V = {B.frame_in, B.flags, nb, B.base[g]};
-        H = list_head(P, B, g);
-    }
-    if (P.early) chain_wait();   // all above has been there since before the last launch
     if (role < 3) {
         if (work) {
+            V = {B.frame_in, B.flags, nb, base};
+            H = list_head(P, B, g);
             const float4 p0 = B.frame_in[g];
             if (role == 0) {
                 put_axial(s_part, l, axial_force(P, B, V, g, flags, p0, B.frame_in[nb + g], B.frame_in[2 * nb + g].w, H));

@@ -159,7 +159,6 @@ KParams make_kparams(const mtg_params &p, int nb, int nt, int maxH, int maxLong,
     k.maxLJ = maxLJ;
     k.step_block = 128;
     k.chain = 1;
-    k.early = 0;
     k.tea_a = p.tea_a;
     k.tea_var = sqrtf(2.0f * 0.0019872041f * p.Temp * p.gammaR / p.dt);
     return k;
@@ -282,21 +281,15 @@ void timed_launch(mtg_engine *e, int kind, F &&launch) {
 }
 
 // Enqueues one step of the loop of compute() (src/compute_cuda.cu:1137-1238)
-// minus its host I/O.  follows: the last launch on the stream is of the step
-// before, as enqueued here: it writes neither flags nor lists, and
-// it began its work only when all before it had ended, so the first kernel of this step
-// may read those before its own wait.
-void enqueue_step(mtg_engine *e, long long step, bool allow_rebuild = true, bool follows = false) {
+// minus its host I/O.
+void enqueue_step(mtg_engine *e, long long step, bool allow_rebuild = true) {
     const mtg_params &p = e->p;
-    KParams first = e->kp;
-    first.early = follows;
     if (allow_rebuild && step % p.ljpairsupdatefreq == 0 && (p.lj_on || p.is_assembly)) {
         timed_launch(e, 0, [&] { launch_lists(e); });
         e->lists_valid = true;
-        first.early = 0;
     }
     if (p.hdi_on) {
-        timed_launch(e, 2, [&] { launch_forces(first, e->bufs(), true, e->stream); });
+        timed_launch(e, 2, [&] { launch_forces(e->kp, e->bufs(), true, e->stream); });
         // learned TEA with the far field: proxies of this step's F and R.
         // Without per-kernel timing the inner proxies and M2L run on the
         // second stream beside the network and the near pairs, and join
@@ -347,7 +340,7 @@ void enqueue_step(mtg_engine *e, long long step, bool allow_rebuild = true, bool
             timed_launch(e, 5, [&] { launch_tea_step(e->kp, e->bufs(), e->tea_work, e->tea_nwork, e->stream); });
         }
     } else {
-        timed_launch(e, 1, [&] { launch_step_plain(first, e->bufs(), e->keep_forces, e->stream); });
+        timed_launch(e, 1, [&] { launch_step_plain(e->kp, e->bufs(), e->keep_forces, e->stream); });
     }
     e->cur ^= 1;
 }
@@ -980,10 +973,8 @@ static int enqueue_range(mtg_engine *e, long long first_step, int nsteps) {
         s++;
     }
     if (nsteps > 0) e->lists_fresh = false;
-    bool direct = false;   // the last launch was a step's of this call, outside a graph
     while (s < end) {
         if (use_graphs && s % period == 0 && end - s >= period) {
-            direct = false;
             cudaGraphExec_t &ge = e->graph[e->cur];
             if (!ge) {
                 const int cur0 = e->cur;
@@ -1011,7 +1002,7 @@ static int enqueue_range(mtg_engine *e, long long first_step, int nsteps) {
                             k += run;
                         }
                     } else {
-                        for (long long k = 0; k < period; k++) enqueue_step(e, k, true, k > 0);
+                        for (long long k = 0; k < period; k++) enqueue_step(e, k);
                     }
                     ce = cudaStreamEndCapture(e->stream, &g);
                 }
@@ -1043,8 +1034,7 @@ static int enqueue_range(mtg_engine *e, long long first_step, int nsteps) {
             enqueue_period_run(e, s, (int)run);
             s += run;
         } else {
-            enqueue_step(e, s, true, direct);
-            direct = true;
+            enqueue_step(e, s);
             s++;
         }
     }

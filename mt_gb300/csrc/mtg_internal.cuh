@@ -63,7 +63,6 @@ struct KParams {
     int tea_max_blocks;    // blocks of kTeaBlock beads of the largest trajectory
     long long tea_units;   // (chunk of kTeaChunk beads) x (block) pairs of the all-pairs kernels
     int chain;             // launch the kernels of a step chained (launch_chained)
-    int early;             // the launch before is of the step before: flags and lists may be read ahead of the wait
     int step_block;        // threads per CTA of the fused plain step (64, 128 or 256)
 };
 
@@ -442,10 +441,8 @@ __host__ __device__ inline int row_buckets(int n) {   // at least 2 n
 // launched so calls it before all that depends on another kernel and before it
 // lets its successor start, also where it then has nothing to do: a
 // kernel that ended without it could let its successor overtake its predecessor.
-// Before it a kernel may read what only the engine's creation writes, and, when the launch
-// before is known not to write them (KParams::early), flags and lists: whatever
-// wrote those had ended before that launch passed its own chain_wait (200 steps of one
-// 1520-bead trajectory 899 -> 814 us, 100 steps of 299 beads with TEA 966 -> 907).
+// Before it a kernel reads only what the engine's creation writes (topology, plans of the
+// work): chain_wait is the one point from which other kernels' writes are visible.
 // Batches of the four-warp form only: a launch there costs up to 1 us less (one
 // 1520-bead trajectory, 200 steps, 1.14 -> 1.06 ms), but the waiting CTAs slow a full
 // GPU down (1024 uneven trajectories, 50 steps, 6.85 -> 7.58 ms).

@@ -145,3 +145,32 @@ def test_bonds_past_the_largest_square(over):
             e.upload_state(c)
             f.append(np.delete(e.compute_forces(), (far, partner), 0))
     assert np.isfinite(f[0]).all() and np.array_equal(f[0], f[1])
+
+
+@pytest.mark.parametrize("mode", ["plain", "tea", "learned"])
+def test_chained_launches_equal_unchained(mode):
+    """Small batches launch their kernels chained, except while kernels are timed: 300 steps
+    with 30 rebuilds of lists that change, from graphs and step by step, bit for bit."""
+    from mt_gb300 import engine
+    p = synth.default_params(seed=83, hdi_on=int(mode != "plain"), tea_epsilon_freq=5, viscosity=8.0e3)
+    b = synth.batch_from_trajectories(p, [synth.make_trajectory(*s, seed=83, radius=8.12, psi_mode="make_mt", cube=45.0,
+                                                                thermal=0.05) for s in ((20, 400), (12, 100))])
+    runs = []
+    for timed in (False, True):
+        with engine.Surrogate(seed=5) as net, engine.Engine(b) as e:
+            e.upload_state(b.coords)
+            e.set_kernel_timing(timed)
+            if mode == "learned":
+                e.set_surrogate(net, recheck_every=20, max_err=1.0e9)
+                e.set_tea_farfield(True, 0.85, refresh_every=100)
+            e.rebuild_pairs()
+            before = e.lists()["lj"][0]
+            for first in range(0, 300, 60):
+                e.step(first, 47)
+                e.step(first + 47, 13)
+            runs.append((e.download_state(), e.download_rng(), e.lists()))
+    (x0, r0, l0), (x1, r1, l1) = runs
+    assert np.isfinite(x0).all() and np.array_equal(x0, x1) and np.array_equal(r0, r1)
+    for k in ("lj", "long", "lat"):
+        assert np.array_equal(l0[k][0], l1[k][0]) and np.array_equal(l0[k][1], l1[k][1])
+    assert (before != l0["lj"][0]).any()
