@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <random>
@@ -548,9 +549,11 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     SCK(mlp::launch_forward_tc(s->W, dX, nullptr, n, s->norm, dY, dZ, s->err, s->stream));
     SCK(mlp::launch_backward_tc(s->W, dX, nullptr, s->norm, dT, n, dY, dZ, dG, dL, s->err, s->stream));
     if (grad) SCK(mlp::launch_grad_sum(dG, parts, dSum, s->stream));
+    // the gradient waits here for the error word: the caller's is written by calls that succeed
+    const std::unique_ptr<float[]> G(grad ? new float[mlp::kParams] : nullptr);
     std::vector<float> L(parts);
     int herr = 0;
-    if (grad) SCK(cudaMemcpyAsync(grad, dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));
+    if (grad) SCK(cudaMemcpyAsync(G.get(), dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(L.data(), dL, sizeof(float) * parts, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(&herr, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
@@ -561,6 +564,7 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     double l = 0.0;
     for (float v : L) l += v;
     if (loss) *loss = l / ((double)n * mlp::kOut);
+    if (grad) std::copy_n(G.get(), mlp::kParams, grad);
     return MTG_OK;
 }
 
