@@ -267,10 +267,11 @@ int mtg_download_lists(mtg_engine *e, int *lj_count, int *lj, int *long_count, i
                        int *lat_count, int *lat);
 int mtg_list_capacity(const mtg_engine *e, int *max_long, int *max_lat, int *max_lj);
 /* How the lists are rebuilt; both produce identical lists.  0 = automatic
- * (cell list, except tiles for
- * trajectories of < 512 beads with LJ off or an LJ cutoff below the assembly
- * reach), 1 = brute-force shared-memory tiles over each trajectory (the
- * reference's O(N^2) loops), 2 = per-trajectory spatial-hash cell list (list capacities up to 16 longitudinal / 32 lateral). */
+ * (cell list, except tiles for trajectories of < 512 beads with LJ off or an
+ * LJ cutoff below the assembly reach or above 11 nm), 1 = brute-force
+ * shared-memory tiles over each trajectory (the reference's O(N^2) loops),
+ * 2 = per-trajectory spatial-hash cell list (list capacities up to 16
+ * longitudinal / 32 lateral). */
 int mtg_set_list_method(mtg_engine *e, int method);
 int mtg_get_list_method(mtg_engine *e, int *method);
 

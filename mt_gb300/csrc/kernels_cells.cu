@@ -24,7 +24,7 @@ namespace mtg {
 
 namespace {
 
-constexpr float kPairReach = 6.6f;  // see kPairPrefilter in kernels_lists.cu
+constexpr float kPairReach = 6.6f;  // see kPairPrefilter
 
 __global__ void k_cell_count(KParams P, const float4 *pos, const int *traj, const int *tbase, const int *tmask,
                              float inv_cell, int *key, int *cnt) {
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kTile) k_pairs_from_lj(KParams P, DevBuffers B
 // walk ran 7600 instructions a warp, half of them on repeated buckets), 61 us here;
 // 1024 uneven trajectories of up to 3560 beads 775 -> 275 us, 101 lattices of 780 beads
 // 66 -> 21 us, one trajectory of 156 beads 45 (tiles) -> 10 us.
-constexpr int kSmemKeys = 32;      // slots for a bead's hits; beads with more than 28 take the slow path below
+constexpr int kSmemKeys = 32;      // slots for a bead's hits; beads with more than 28 are walked again, below
 constexpr int kSmemBeads = 8192;   // 13 bits of a key
 constexpr unsigned kNoKey = 0x10000u;
 
@@ -562,13 +562,6 @@ struct ListWriter {
     int nlj, nlo, nla;
     bool overflow;
 };
-__device__ __forceinline__ void lj_append(const KParams &P, const DevBuffers &B, int g, int jl, ListWriter &W) {
-    if (W.nlj < P.maxLJ)
-        B.lj[W.nlj * P.nb + g] = jl;
-    else
-        W.overflow = true;
-    W.nlj++;
-}
 // The site tests of pairs_kernel (src/compute_cuda.cu:527-674) for one key:
 // the planes they need are requested together, then decided as list_bits does.
 struct PairPlanes {
@@ -599,8 +592,97 @@ __device__ __forceinline__ void pair_decide(const KParams &P, const DevBuffers &
     list_append(P, B, g, I, got, jl, W.nlj, W.nlo, W.nla, W.overflow);
 }
 
+// A hit as a key.  A bond needs the partner's centre within 2.5 + 2 nm of one of the bead's own
+// sites (0.01 nm over the rounding of distances, and of a site's coordinates three units in the
+// last place: beads may be far from the origin).
+struct KeyTest {
+    float4 p;             // the bead
+    float3 a0, a1, a2;    // its sites
+    float site, lj, pair; // squared limits
+    int il, hpart;
+    static __device__ __forceinline__ float site2(float3 a, float4 q) {   // a coarse test: contracted
+        const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
+        return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    }
+    __device__ __forceinline__ unsigned key(float4 q) const {
+        const float r2 = dist2_rn(p, q);
+        const int jl = __float_as_int(q.w);
+        unsigned bits = (site2(a0, q) < site ? 1u : 0u) | (site2(a1, q) < site ? 2u : 0u) | (site2(a2, q) < site ? 4u : 0u);
+        if (!(r2 < pair) || jl == hpart) bits = 0;
+        return r2 < lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
+    }
+};
+__device__ __forceinline__ KeyTest key_test(const KParams &P, const ListSite &I, const ListCuts &cut) {
+    const float4 p = I.p;
+    const float reach = fmaf(4.0e-7f, fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)), 4.51f);
+    return {p, make_float3(p.x + I.wi.x, p.y + I.wi.y, p.z + I.wi.z), make_float3(p.x + I.l1.x, p.y + I.l1.y, p.z + I.l1.z),
+            make_float3(p.x + I.l2.x, p.y + I.l2.y, p.z + I.l2.z), P.is_assembly ? reach * reach : 0.f, cut.lj, cut.pair,
+            I.il, I.hpart};
+}
+// The next n keys of a bead's column, ascending, into its lists; before: the last key taken.
+__device__ __forceinline__ void take_keys(const KParams &P, const DevBuffers &B, const ListSite &I, int g, int base,
+                                          float t_site, int n, uint16_t *col, unsigned &before, ListWriter &W) {
+    // the LJ list; the keys with a site test close up in place
+    int np = 0;
+    for (int k = 0; k < n; k++) {
+        const unsigned key = col[k * kListThreads];
+        const bool keep = key != before;   // not found from two rows
+        before = key;
+        if (keep && W.nlj < P.maxLJ) B.lj[W.nlj * P.nb + g] = (int)(key >> 3);
+        W.nlj += keep;
+        col[np * kListThreads] = (uint16_t)key;   // np <= k
+        np += keep && (key & 7u) != 0;
+    }
+    W.overflow = W.overflow || W.nlj > P.maxLJ;
+    for (int k = 0; k < np; k += 2) {   // two partners in flight
+        const unsigned k0 = col[k * kListThreads], k1 = k + 1 < np ? col[(k + 1) * kListThreads] : 0u;
+        const PairPlanes J0 = pair_load(B, P.nb, base + (int)(k0 >> 3), k0 & 7u);
+        const PairPlanes J1 = pair_load(B, P.nb, base + (int)(k1 >> 3), k1 & 7u);
+        pair_decide(P, B, g, I, (int)(k0 >> 3), k0 & 7u, J0, t_site, W);
+        pair_decide(P, B, g, I, (int)(k1 >> 3), k1 & 7u, J1, t_site, W);
+    }
+}
+__device__ __forceinline__ void store_counts(const KParams &P, const DevBuffers &B, int g, const ListWriter &W) {
+    B.ljc[g] = min(W.nlj, P.maxLJ);
+    if (P.is_assembly) {
+        B.lonc[g] = min(W.nlo, P.maxLong);
+        B.latc[g] = min(W.nla, P.maxLat);
+    }
+    if (W.overflow) atomicOr(B.err, kErrOverflow);
+}
+// The lists of a bead with more hits than its slots hold (long cutoffs, dense systems): the
+// smallest keys above the last one taken, kept in order as a walk meets them (a key can come
+// twice), slots after slots.  A call that starts from the bead's index, so that the
+// ordinary path keeps its registers.  256 x 1520 beads with a cutoff of 10, 12, 14 nm: 275, 537,
+// 895 us; 1374, 4175, 8243 with a walk for every entry; 503, 880, 1576 in the general path.
+static __device__ __noinline__ void many_hits(const KParams &P, const DevBuffers &B, SmemCells C, ListCuts cut, int g,
+                                              int il, uint16_t *col) {
+    const int nb = P.nb;
+    const float4 *fr = B.frame_in;
+    const ListSite I =
+        list_site(P, fr[g], fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], B.flags[g], il, B.harm[g * P.maxH]);
+    const KeyTest K = key_test(P, I, cut);
+    ListWriter W = {0, 0, 0, false};
+    unsigned before = kNoKey;
+    int n, last = -1;
+    do {
+        n = 0;
+        smem_candidates(C, K.p, K.lj, [&](int slot) {
+            const unsigned key = K.key(C.pos[slot]);
+            if (key == kNoKey || (int)key <= last || (n == kSmemKeys && key >= col[(kSmemKeys - 1) * kListThreads])) return;
+            int k = n < kSmemKeys ? n++ : kSmemKeys - 1;
+            for (; k > 0 && col[(k - 1) * kListThreads] > key; k--) col[k * kListThreads] = col[(k - 1) * kListThreads];
+            col[k * kListThreads] = (uint16_t)key;
+        });
+        if (n > 0) last = col[(n - 1) * kListThreads];
+        take_keys(P, B, I, g, g - il, cut.site, n, col, before, W);
+    } while (n == kSmemKeys);
+    store_counts(P, B, g, W);
+}
+
 template <int PARTS>
-__global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, DevBuffers B, const int4 *work, int nmax,
+__global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(const __grid_constant__ KParams P,
+                                                                  const __grid_constant__ DevBuffers B, const int4 *work, int nmax,
                                                                   float inv, ListCuts cut) {
     extern __shared__ float4 s_dyn[];
     const int4 w = work[blockIdx.x];   // trajectory, first bead, number of beads
@@ -678,28 +760,9 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     const int flags = valid ? B.flags[g] : kFlagExtra;
     const bool live = !(flags & kFlagExtra);
     const SmemCells C = {s_pos, s_end, n, m, inv};
-    // where the bead's own sites are: a bond needs the partner's centre within
-    // 2.5 + 2 nm of one (0.01 nm over the rounding of distances, and of a site's coordinates
-    // three units in the last place: beads may be far from the origin)
-    float site_cut = 0.f;
-    auto site2 = [](float4 a, float4 q) {   // a coarse test: contracted
-        const float dx = a.x - q.x, dy = a.y - q.y, dz = a.z - q.z;
-        return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    };
     ListSite I;
-    float4 a0, a1, a2;
-    auto make_key = [&](int slot) {
-        const float4 q = s_pos[slot];
-        const float r2 = dist2_rn(I.p, q);
-        const int jl = __float_as_int(q.w);
-        unsigned bits = 0;
-        if (P.is_assembly) {
-            bits = (site2(a0, q) < site_cut ? 1u : 0u) | (site2(a1, q) < site_cut ? 2u : 0u) |
-                   (site2(a2, q) < site_cut ? 4u : 0u);
-            if (!(r2 < cut.pair) || jl == I.hpart) bits = 0;
-        }
-        return r2 < cut.lj && jl != il ? ((unsigned)jl << 3) | bits : kNoKey;
-    };
+    KeyTest K;
+    auto make_key = [&](int slot) { return K.key(s_pos[slot]); };
     int nk = 0;
     bool many = false;
     if (live) {
@@ -707,11 +770,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
         const int met = smem_slots(C, p, cut.lj, part * 9 / PARTS, (part + 1) * 9 / PARTS, &s_key[0][t]);
         // the bead's other planes only now: the walk has no registers to spare
         I = list_site(P, p, fr[nb + g], fr[2 * nb + g], fr[3 * nb + g], flags, il, B.harm[g * P.maxH]);
-        const float reach = fmaf(4.0e-7f, fmaxf(fmaxf(fabsf(I.p.x), fabsf(I.p.y)), fabsf(I.p.z)), 4.51f);
-        site_cut = reach * reach;
-        a0 = make_float4(I.p.x + I.wi.x, I.p.y + I.wi.y, I.p.z + I.wi.z, 0.f);
-        a1 = make_float4(I.p.x + I.l1.x, I.p.y + I.l1.y, I.p.z + I.l1.z, 0.f);
-        a2 = make_float4(I.p.x + I.l2.x, I.p.y + I.l2.y, I.p.z + I.l2.z, 0.f);
+        K = key_test(P, I, cut);
         many = met > kSmemKeys - 4;
         if (!many)
             for (int k = 0; k < met; k++) {
@@ -733,70 +792,33 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(KParams P, 
     if (!valid) return;
     ListWriter W = {0, 0, 0, false};
     if (live) {
-        if (!many) {
-            // one way for the whole warp: a warp with both would run both
-            const unsigned warp = __activemask();
-            if (!__any_sync(warp, nk > 8)) {
-                sort_keys<8>(s_key, nk);
-            } else if (!__any_sync(warp, nk > 16)) {
-                sort_keys<16>(s_key, nk);
-            } else if (!__any_sync(warp, nk > 24)) {
-                sort_keys<24>(s_key, nk);
-            } else {
-                for (int i = 1; i < nk; i++) {
-                    const uint16_t v = s_key[i][t];
-                    int j = i - 1;
-                    while (j >= 0 && s_key[j][t] > v) {
-                        s_key[j + 1][t] = s_key[j][t];
-                        j--;
-                    }
-                    s_key[j + 1][t] = v;
-                }
-            }
-            // the LJ list; the keys with a site test close up in place
-            int np = 0;
-            unsigned before = kNoKey;
-            for (int k = 0; k < nk; k++) {
-                const unsigned key = s_key[k][t];
-                const bool keep = key != before;   // not found from two rows
-                before = key;
-                if (keep && W.nlj < P.maxLJ) B.lj[W.nlj * nb + g] = (int)(key >> 3);
-                W.nlj += keep;
-                s_key[np][t] = (uint16_t)key;   // np <= k
-                np += keep && (key & 7u) != 0;
-            }
-            W.overflow = W.nlj > P.maxLJ;
-            for (int k = 0; k < np; k += 2) {   // two partners in flight
-                const unsigned k0 = s_key[k][t], k1 = k + 1 < np ? s_key[k + 1][t] : 0u;
-                const PairPlanes J0 = pair_load(B, nb, base + (int)(k0 >> 3), k0 & 7u);
-                const PairPlanes J1 = pair_load(B, nb, base + (int)(k1 >> 3), k1 & 7u);
-                pair_decide(P, B, g, I, (int)(k0 >> 3), k0 & 7u, J0, cut.site, W);
-                pair_decide(P, B, g, I, (int)(k1 >> 3), k1 & 7u, J1, cut.site, W);
-            }
+        if (many) {
+            many_hits(P, B, C, cut, g, il, &s_key[0][t]);
+            return;
+        }
+        // one way for the whole warp: a warp with both would run both
+        const unsigned warp = __activemask();
+        if (!__any_sync(warp, nk > 8)) {
+            sort_keys<8>(s_key, nk);
+        } else if (!__any_sync(warp, nk > 16)) {
+            sort_keys<16>(s_key, nk);
+        } else if (!__any_sync(warp, nk > 24)) {
+            sort_keys<24>(s_key, nk);
         } else {
-            // more neighbours than hard spheres of this size allow: the next larger
-            // key is looked up again and again
-            int last = -1;
-            while (true) {
-                unsigned best = 0x7fffffffu;
-                smem_candidates(C, I.p, cut.lj, [&](int slot) {
-                    const unsigned key = make_key(slot);
-                    if (key != kNoKey && (int)key > last) best = min(best, key);
-                });
-                if (best == 0x7fffffffu) break;
-                last = (int)best;
-                lj_append(P, B, g, (int)(best >> 3), W);
-                const PairPlanes J = pair_load(B, nb, base + (int)(best >> 3), best & 7u);
-                pair_decide(P, B, g, I, (int)(best >> 3), best & 7u, J, cut.site, W);
+            for (int i = 1; i < nk; i++) {
+                const uint16_t v = s_key[i][t];
+                int j = i - 1;
+                while (j >= 0 && s_key[j][t] > v) {
+                    s_key[j + 1][t] = s_key[j][t];
+                    j--;
+                }
+                s_key[j + 1][t] = v;
             }
         }
+        unsigned before = kNoKey;
+        take_keys(P, B, I, g, base, cut.site, nk, &s_key[0][t], before, W);
     }
-    B.ljc[g] = min(W.nlj, P.maxLJ);
-    if (P.is_assembly) {
-        B.lonc[g] = min(W.nlo, P.maxLong);
-        B.latc[g] = min(W.nla, P.maxLat);
-    }
-    if (W.overflow) atomicOr(B.err, kErrOverflow);
+    store_counts(P, B, g, W);
 }
 
 // ------------------------------------------------ ordered binning in one CTA

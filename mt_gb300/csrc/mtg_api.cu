@@ -236,6 +236,7 @@ void launch_lists(mtg_engine *e) {
         launch_rebuild(e->kp, e->bufs(), e->work, e->nwork, e->stream);
 }
 
+constexpr float kSmallListCutoff = 11.0f;   // nm
 void choose_list_method(mtg_engine *e) {
     const bool cells_ok = e->kp.maxLong <= kCellMaxLong && e->kp.maxLat <= kCellMaxLat && e->cell_tbase;
     if (e->list_method == 1 || !cells_ok)
@@ -243,9 +244,12 @@ void choose_list_method(mtg_engine *e) {
     else if (e->list_method == 2)
         e->use_cells = true;
     else
-        // the one-launch cell rebuild beats the tiles at every size it takes
-        // (156 beads: 45 against 18 us); the six-launch one from 512 beads on
-        e->use_cells = e->max_traj_beads >= 512 || smem_lists_apply(e->kp, e->max_traj_beads);
+        // The one-launch cell rebuild beats the tiles from 1 to 4096 trajectories of 104 to 516 beads
+        // (one of 156 beads 59 against 16 us, 1024 of 104 beads 65 and 55, 4096 of 156 beads 456 and
+        // 186) until most beads have more hits than its slots hold: 64 x 156 beads with a cutoff of
+        // 11 nm 61 and 36 us, of 12 nm 61 and 88.  The six-launch one beats them from 512 beads on.
+        e->use_cells = e->max_traj_beads >= 512 ||
+                       (smem_lists_apply(e->kp, e->max_traj_beads) && e->kp.ljcut <= kSmallListCutoff);
 }
 
 // Event slot for one timed launch (created outside any stream capture).

@@ -85,6 +85,19 @@ def test_cutoffs(over):
     same(cloud((700, 300), seed=5, **over))
 
 
+@pytest.mark.parametrize("cut", [11.0, 12.0, 17.0, 26.0])
+def test_long_cutoffs(cut):
+    """More hits than a bead's slots, several times as many, and more than the list holds; small
+    trajectories with most beads past the slots take the tiles by themselves."""
+    from mt_gb300 import engine
+    same(synth.uniform_batch(synth.default_params(seed=9, ljpairscutoff=cut), 3, 40, 100, seed=9, radius=8.12,
+                             psi_mode="make_mt", cube=60.0, thermal=0.05))
+    t = same(cloud((450, 150, 3), seed=9, ljpairscutoff=cut))
+    assert t["lj"][0].max() > 32 and t["full"] == (cut > 20)
+    with engine.Engine(cloud((450, 150, 3), seed=9, ljpairscutoff=cut), force_ragged=True) as e:
+        assert e.list_method() == (2 if cut <= 11.0 else 1)
+
+
 def test_lj_without_assembly_lists():
     b = cloud((600, 41), seed=6, is_assembly=0, ljpairscutoff=5.0)
 
