@@ -1150,7 +1150,11 @@ int mtg_autotune(mtg_engine *e, long long first_step, int trial_steps, mtg_tunin
         if (e->p.hdi_on) {   // the TEA kernels divide their work themselves
             cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 0});
         } else {
-            for (int bs : {64, 128, 256}) cands.push_back({lm, bs, orig.tea_slices, orig.tea_jparts, 0});
+            for (int bs : {64, 128, 256}) {
+                if (e->nb <= kSplitMaxBeads) bs = orig.step_block;   // no effect on the four-warp form
+                cands.push_back({lm, bs, orig.tea_slices, orig.tea_jparts, 0});
+                if (e->nb <= kSplitMaxBeads) break;
+            }
             if (period_fits(e->max_traj_beads)) cands.push_back({lm, orig.step_block, orig.tea_slices, orig.tea_jparts, 1});
         }
     }

@@ -174,3 +174,16 @@ def test_chained_launches_equal_unchained(mode):
     for k in ("lj", "long", "lat"):
         assert np.array_equal(l0[k][0], l1[k][0]) and np.array_equal(l0[k][1], l1[k][1])
     assert (before != l0["lj"][0]).any()
+
+
+@pytest.mark.parametrize("block", [64, 256])
+def test_autotune_keeps_a_block_without_effect(block):
+    """step_block has no effect on batches of the four-warp form: its value is kept, not drawn by timing noise."""
+    from mt_gb300 import engine
+    b = synth.uniform_batch(synth.default_params(seed=77), 2, 12, 200, seed=77, radius=8.12, psi_mode="make_mt", cube=60.0)
+    with engine.Engine(b) as e:
+        e.upload_state(b.coords)
+        t = e.tuning()
+        e.set_tuning(**dict(t, step_block=block))
+        res = e.autotune(0, 10)
+        assert res["tuning"]["step_block"] == block and e.tuning()["step_block"] == block
