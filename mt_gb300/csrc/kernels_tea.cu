@@ -3,10 +3,10 @@
 // RPY mobility product fused with the position update; below them the far
 // field of the learned mode.
 //
-// Both O(N^2) passes are one kernel template, k_tea_pass (k_tea_lanes for small
+// Both O(N^2) passes are one kernel template, k_tea_pass (k_tea_small for small
 // systems, which are bound by latency).  They are bound by
 // the FP32 pipe (about 45 FLOP per ordered pair: 24 packed FP32x2 operations
-// for two pairs), so everything else is arranged to stay off its way:
+// for two pairs, each pair visited from both its beads), so everything else is arranged to stay off its way:
 //   * The beads j come from B.tea_pack, where the force kernel of the step has
 //     laid every trajectory out in blocks of 32 beads = 16 pairs in the order the
 //     loop reads them: the two lanes of a packed operation are two beads j, one
@@ -17,14 +17,13 @@
 //   * A CTA of four warps serves 128 beads i, one a thread: 56 registers and nine
 //     CTAs an SM (two beads a thread load half as many words but leave six CTAs:
 //     1.82 against 1.76 ms).
-//   * The work of a launch is the list of units (128 beads i) x (one block of
-//     j), cut into equal contiguous runs, one CTA each, four for every CTA the
-//     GPU holds at once, so the last ones to finish are short whatever the
-//     sizes.  (One each: an SM's schedulers favour their older warps, which leave
-//     the younger ones alone at the end, 1.72 against 1.66 ms.)  A run
-//     that does not hold all units of its 128 beads leaves its partial sums, and the CTA
-//     that comes last (an atomic count; nothing waits) adds them in run order and
-//     finishes the beads, so the result does not depend on the timing.
+//   * A bead's sums are cut by its trajectory alone (tea_fine, mtg_internal.cuh), so they have the
+//     same bits in every batch and in both kernels.  A CTA takes one grain, a whole
+//     node of that tree of sums, for its 128 beads; the grain's size fits the batch
+//     (tea_grain_level).  Of a chunk of several grains each CTA leaves its sums, and the one
+//     that comes last (an atomic count; nothing waits) adds them in the tree's order and
+//     finishes the beads.  (Equal runs of units, cut where k/G of the batch's work is, are
+//     2% faster in the product and 1% slower in the epsilon pass, but a bead's bits then depend on the batch.)
 // The far-field formula runs for every pair; the few overlapping pairs
 // (r <= 2a) are found through a running minimum of r^2 per block; in a block
 // that holds one their distances are taken once more and only they get the near-field formula
@@ -33,9 +32,10 @@
 // the block that holds a bead itself its own pair gets r^2 = 1e30: its term is
 // then far below the rounding of the sums, and the correction skips it.
 // Sums are kept in units of 0.75 a (T' = T / (0.75 a)).
-// Measured (mobility product): 64 x 5600 beads 1.82 -> 1.68 ms (54 TFLOP/s of the measured 80;
-// the FMA pipe is 75% active), 16 x 3300 205 -> 165 us (before: a tile stored twice by
-// every CTA, whole 128-bead items in 3.7 waves or a second kernel for split ones).
+// What the two kernels compute for a bead is written with explicitly rounded operations wherever a product
+// meets a sum, so that both give the same bits.
+// Measured (mobility product): 64 x 5600 beads 1.71 ms (53 TFLOP/s of the measured 80),
+// 16 x 3300 beads 170 us; epsilon pass 1.58 ms and 154 us.
 #include "mtg_internal.cuh"
 
 namespace mtg {
@@ -74,7 +74,7 @@ __device__ __forceinline__ TeaConst tea_const(float a) {
 // near branch (r <= 2a): scaled cii', crr'
 __device__ __forceinline__ void rpy_near(const TeaConst &K, float r2, float rinv, float &cii, float &crr) {
     const float ra = r2 * rinv * K.inv_a;
-    cii = (1.0f - (9.0f / 32.0f) * ra) * K.inv_c075a;
+    cii = __fmaf_rn(-(9.0f / 32.0f), ra, 1.0f) * K.inv_c075a;
     crr = (3.0f / 32.0f) * ra * K.inv_c075a;
 }
 
@@ -88,7 +88,8 @@ __device__ __forceinline__ EpsTerms eps_terms(float dx, float dy, float dz, floa
     const float crq = crr * q;
     const float bc = fmaf(2.0f, cii, crr) * crq;
     const float us = dx + dy + dz;
-    return {bc * dx * dx, bc * dy * dy, bc * dz * dz, cii * cii, fmaf(crq * us, us, 3.0f * cii)};
+    return {__fmul_rn(__fmul_rn(bc, dx), dx), __fmul_rn(__fmul_rn(bc, dy), dy), __fmul_rn(__fmul_rn(bc, dz), dz),
+            __fmul_rn(cii, cii), __fmaf_rn(__fmul_rn(crq, us), us, __fmul_rn(3.0f, cii))};
 }
 
 // Stores the epsilon-pass result of bead g from its scaled sums
@@ -186,39 +187,63 @@ __device__ __forceinline__ float3 tea_pair1(const TeaConst &K, float dx, float d
     return make_float3(fmaf(cii, gx, s * dx), fmaf(cii, gy, s * dy), fmaf(cii, gz, s * dz));
 }
 
+// a / sqrt(1 + beta^2 C): C_i (a = 1) and beta C_i
+__device__ __forceinline__ float tea_norm(float a, float b2, float c) { return a / sqrtf(__fmaf_rn(b2, c, 1.0f)); }
+
+// What the update of bead g starts from; with FEFF its effective force only.
+template <bool FEFF>
+struct TeaBead {
+    float4 ci, F, R, fa;   // fa: ffi, ftheta, fpsi
+    Frame Fr;
+    uint4 s2;
+    int flags;
+    __device__ __forceinline__ void load(const KParams &P, const DevBuffers &B, int g) {
+        const int nb = P.nb;
+        ci = B.tea_ci[g];
+        F = B.force[g];
+        R = B.tea_r[g];
+        if (FEFF) return;
+        fa = B.force[nb + g];
+        flags = B.flags[g];
+        Fr.p0 = B.frame_in[g];
+        Fr.p1 = B.frame_in[nb + g];
+        Fr.p2 = B.frame_in[2 * nb + g];
+        Fr.p3 = B.frame_in[3 * nb + g];
+        s2 = B.seeds[nb + g];
+    }
+};
 // The update of bead g from its scaled mobility sums (sx, sy, sz): back to
 // units of D_ii, plus the bead's own term F_i + C_i o R_i; FEFF stores f_i.
 template <bool FEFF>
-__device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffers &B, int g, float sx, float sy,
-                                                float sz, float b2, const TeaConst &K, float4 *feff) {
+__device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffers &B, int g, TeaBead<FEFF> &b, float sx,
+                                                float sy, float sz, float b2, const TeaConst &K, float4 *feff) {
     const int nb = P.nb;
-    const float4 ci = B.tea_ci[g], Fi = B.force[g], Ri = B.tea_r[g], fa = B.force[nb + g];   // (ffi, ftheta, fpsi)
-    sx = fmaf(K.c075a, sx, Fi.x + Ri.x * (1.0f / sqrtf(1.0f + b2 * ci.x)));
-    sy = fmaf(K.c075a, sy, Fi.y + Ri.y * (1.0f / sqrtf(1.0f + b2 * ci.y)));
-    sz = fmaf(K.c075a, sz, Fi.z + Ri.z * (1.0f / sqrtf(1.0f + b2 * ci.z)));
+    sx = __fmaf_rn(K.c075a, sx, __fmaf_rn(b.R.x, tea_norm(1.0f, b2, b.ci.x), b.F.x));
+    sy = __fmaf_rn(K.c075a, sy, __fmaf_rn(b.R.y, tea_norm(1.0f, b2, b.ci.y), b.F.y));
+    sz = __fmaf_rn(K.c075a, sz, __fmaf_rn(b.R.z, tea_norm(1.0f, b2, b.ci.z), b.F.z));
     if (FEFF) {
         feff[g] = make_float4(sx, sy, sz, 0.f);
         return;
     }
-    const int flags = B.flags[g];
-    Frame Fr;
-    Fr.p0 = B.frame_in[g];
-    Fr.p1 = B.frame_in[nb + g];
-    Fr.p2 = B.frame_in[2 * nb + g];
-    Fr.p3 = B.frame_in[3 * nb + g];
-    uint4 s2 = B.seeds[nb + g];
-    const float4 ga = gauss4(s2);
-    B.seeds[nb + g] = s2;
-    if (!(flags & (kFlagExtra | kFlagFixed))) {
-        const float x = Fr.p0.x + P.kr * sx, y = Fr.p0.y + P.kr * sy, z = Fr.p0.z + P.kr * sz;
-        const float fi = Fr.p0.w + (P.kfi * fa.x + P.nfi * ga.x);
-        const float psi = Fr.p1.w + (P.kfi * fa.z + P.nfi * ga.y);
-        const float th = Fr.p2.w + (P.kth * fa.y + P.varTheta * ga.z);
+    const float4 ga = gauss4(b.s2), fa = b.fa;
+    B.seeds[nb + g] = b.s2;
+    Frame Fr = b.Fr;
+    if (!(b.flags & (kFlagExtra | kFlagFixed))) {
+        const float x = __fmaf_rn(P.kr, sx, Fr.p0.x), y = __fmaf_rn(P.kr, sy, Fr.p0.y), z = __fmaf_rn(P.kr, sz, Fr.p0.z);
+        const float fi = __fadd_rn(Fr.p0.w, __fmaf_rn(P.kfi, fa.x, __fmul_rn(P.nfi, ga.x)));
+        const float psi = __fadd_rn(Fr.p1.w, __fmaf_rn(P.kfi, fa.z, __fmul_rn(P.nfi, ga.y)));
+        const float th = __fadd_rn(Fr.p2.w, __fmaf_rn(P.kth, fa.y, __fmul_rn(P.varTheta, ga.z)));
         Fr = make_frame(P, x, y, z, fi, th, psi);
     }
     store_frame(B.frame_out, nb, g, Fr);
 }
-
+template <bool FEFF>
+__device__ __forceinline__ void tea_bead_update(const KParams &P, const DevBuffers &B, int g, float sx, float sy,
+                                                float sz, float b2, const TeaConst &K, float4 *feff) {
+    TeaBead<FEFF> b;
+    b.load(P, B, g);
+    tea_bead_update<FEFF>(P, B, g, b, sx, sy, sz, b2, K, feff);
+}
 
 // ------------------------------------------------------- the all-pairs pass
 // One block of beads j for the epsilon pass (integrateTea_epsilon_unlisted,
@@ -234,8 +259,9 @@ struct EpsOp {
         nx = f2(-p.x);
         ny = f2(-p.y);
         nz = f2(-p.z);
-        sx = sy = sz = sa = sw = f2(0.f);
+        clear();
     }
+    __device__ __forceinline__ void clear() { sx = sy = sz = sa = sw = f2(0.f); }
     template <bool SELF>
     __device__ __forceinline__ void pair(const TeaConst &K, const float4 *blk, int t, int sp, int se,
                                          float &rm) {
@@ -281,19 +307,23 @@ struct EpsOp {
         float cn, rn;
         rpy_near(K, r2, rinv, cn, rn);
         const EpsTerms n = eps_terms(dx, dy, dz, cn, rn, rinv * rinv);
-        sx.x += n.bx - f.bx;
-        sy.x += n.by - f.by;
-        sz.x += n.bz - f.bz;
-        sa.x += n.a2 - f.a2;
-        sw.x += n.w - f.w;
+        sx.x += __fsub_rn(n.bx, f.bx);
+        sy.x += __fsub_rn(n.by, f.by);
+        sz.x += __fsub_rn(n.bz, f.bz);
+        sa.x += __fsub_rn(n.a2, f.a2);
+        sw.x += __fsub_rn(n.w, f.w);
     }
     __device__ __forceinline__ float4 sum() const {
         const float A = sa.x + sa.y;
         return make_float4(sx.x + sx.y + A, sy.x + sy.y + A, sz.x + sz.y + A, sw.x + sw.y);
     }
-    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, int, float4 acc,
+    struct Bead {
+        int flags;
+        __device__ __forceinline__ void load(const KParams &, const DevBuffers &B, int g) { flags = B.flags[g]; }
+    };
+    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, Bead &b, int, float4 acc,
                                            const TeaConst &K, float4 *) const {
-        eps_store(P, B, g, (B.flags[g] & kFlagExtra) == 0, acc, K);
+        eps_store(P, B, g, (b.flags & kFlagExtra) == 0, acc, K);
     }
 };
 
@@ -316,14 +346,14 @@ struct StepOp {
         if (valid) {
             const float beta = B.tea_beta[traj], b2 = beta * beta;
             const float4 ci = B.tea_ci[g];
-            c = make_float4(beta / sqrtf(1.0f + b2 * ci.x), beta / sqrtf(1.0f + b2 * ci.y),
-                            beta / sqrtf(1.0f + b2 * ci.z), 0.f);
+            c = make_float4(tea_norm(beta, b2, ci.x), tea_norm(beta, b2, ci.y), tea_norm(beta, b2, ci.z), 0.f);
         }
         cbx = f2(c.x);
         cby = f2(c.y);
         cbz = f2(c.z);
-        ax = ay = az = f2(0.f);
+        clear();
     }
+    __device__ __forceinline__ void clear() { ax = ay = az = f2(0.f); }
     template <bool SELF>
     __device__ __forceinline__ void pair(const TeaConst &K, const float4 *blk, int t, int sp, int se,
                                          float &rm) {
@@ -372,74 +402,100 @@ struct StepOp {
     __device__ __forceinline__ float4 sum() const {
         return make_float4(ax.x + ax.y, ay.x + ay.y, az.x + az.y, 0.f);
     }
-    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, int traj, float4 acc,
+    using Bead = TeaBead<FEFF>;
+    __device__ __forceinline__ void finish(const KParams &P, const DevBuffers &B, int g, Bead &b, int traj, float4 acc,
                                            const TeaConst &K, float4 *feff) const {
         const float beta = B.tea_beta[traj];
-        tea_bead_update<FEFF>(P, B, g, acc.x, acc.y, acc.z, beta * beta, K, feff);
+        tea_bead_update<FEFF>(P, B, g, b, acc.x, acc.y, acc.z, beta * beta, K, feff);
     }
 };
 
-// The overlapping beads of a block (own: the bead of this lane is one of it, in
-// slot lane): which they are, then their terms.
+// The overlapping beads of a block (own: the slot of the bead itself, or -1): which they
+// are, then their terms.
 template <class Op>
-__device__ __forceinline__ void tea_near_block(Op &X, const TeaConst &K, const float4 *blk, bool own, int lane) {
+__device__ __forceinline__ void tea_near_block(Op &X, const TeaConst &K, const float4 *blk, int own) {
     unsigned near = 0;
 #pragma unroll 4
     for (int t = 0; t < kTeaPairSlots; t++) {
         const float2 r2 = X.dist2(blk, t);
         near |= (r2.x <= K.four_a2 ? 1u : 0u) << (2 * t) | (r2.y <= K.four_a2 ? 2u : 0u) << (2 * t);
     }
-    if (own) near &= ~(1u << lane);
+    if (own >= 0) near &= ~(1u << own);
     for (; near; near &= near - 1) {
         const int j = __ffs((int)near) - 1;
         X.near(K, blk, j >> 1, j & 1);
     }
 }
 
-// Run k of a launch: units [k U / G, (k + 1) U / G).
-__device__ __forceinline__ long long tea_div(long long a, long long b) {   // 64-bit division only where needed
-    return ((a | b) >> 32) == 0 ? (long long)((unsigned)a / (unsigned)b) : a / b;
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
 }
-__device__ __forceinline__ long long tea_run_start(long long units, int runs, int k) { return tea_div(k * units, runs); }
 
-// The item that holds unit u: the last of unit0[0 .. nwork - 1] that is <= u, by a
-// 32-way search (each round is one dependent load instead of five).
-__device__ __forceinline__ int tea_find_item(const long long *unit0, int nwork, long long u) {
-    const int lane = threadIdx.x & 31;
-    int lo = 0, n = nwork;
-    while (n > 1) {
-        const int step = (n + 31) / 32, k = lo + lane * step;
-        const bool le = lane * step < n && unit0[k] <= u;
-        const int last = 31 - __clz((int)__ballot_sync(0xffffffffu, le));   // lane 0 always is
-        n = min(step, n - last * step);
-        lo += last * step;
+// Adds node v of an item's tree of sums (level lvl, first fine segment lo), of which the segments
+// [s0, s1) of n are in hand: kTeaHold while its right sibling is to come (v is kept in node[lvl]),
+// kTeaCut when its parent is not in hand (v is the sum of the largest node that is, from segment lo),
+// kTeaGroup when v is that of a whole top node.
+enum { kTeaHold, kTeaCut, kTeaGroup };
+__device__ __forceinline__ int tea_carry(float4 &v, int &lo, int lvl, int s0, int s1, int n, float4 *node, int stride) {
+#pragma unroll 1
+    for (; lvl < kTeaLevels; lvl++) {
+        const int plo = lo & ~((2 << lvl) - 1), pend = min(plo + (2 << lvl), n);
+        if (plo < s0 || pend > s1) return kTeaCut;
+        if (lo != plo) {
+            v = add4(node[lvl * stride], v);
+        } else if (lo + (1 << lvl) < n) {
+            node[lvl * stride] = v;
+            return kTeaHold;
+        }   // else there is no right sibling
+        lo = plo;
     }
-    return lo;
+    return kTeaGroup;
 }
 
-// Runs while gate is null or *gate == run_if.
+// The sum of a bead from the slots of its item's grains.  A call, once for an item, so that the
+// pair loop keeps its registers.
+static __device__ __noinline__ float4 tea_collect(const float4 *part, int ng, int level) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int group = level < kTeaLevels ? (1 << kTeaLevels) >> level : 1;   // slots of a top node
+    for (int j = 0; j < ng; j += 8) {   // eight requested at once
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (j + k < ng) v[k] = __ldcg(&part[(j + k) * kTeaI]);
+#pragma unroll
+        for (int h = 1; h < 8; h *= 2)
+#pragma unroll
+            for (int k = 0; k < 8; k += 2 * h)
+                if (h < group && j + k + h < ng) v[k] = add4(v[k], v[k + h]);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k % group == 0 && j + k < ng) acc = add4(acc, v[k]);
+    }
+    return acc;
+}
+
+// One CTA for each grain of the work: 128 beads i and the blocks j of 2^tea_level fine segments
+// (a fixed grid walks over them where a launch mostly finds its gate closed).  Runs
+// while gate is null or *gate == run_if.
 template <class Op>
-__global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffers B, const int2 *work, int nwork,
-                                                             float4 *feff, const int *gate, int run_if) {
+__global__ void __launch_bounds__(kTeaThreads, kTeaOcc) k_tea_pass(KParams P, DevBuffers B, const int2 *work,
+                                                                   int nwork, float4 *feff, const int *gate, int run_if) {
     constexpr int kW = Op::kWords;
     __shared__ float4 s_tile[kTeaStages][kTeaTileBlocks * kW];
+    __shared__ float4 s_node[kTeaLevels + 1][kTeaThreads];   // each thread's own: nodes that wait, the sum
     __shared__ int s_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long U = P.tea_units;
-    const int G = gridDim.x;
-    long long u = tea_run_start(U, G, blockIdx.x);
-    const long long u_end = tea_run_start(U, G, blockIdx.x + 1);
-    int item = tea_find_item(B.tea_unit0, nwork, u);
-    chain_wait();   // no kernel writes the units
+    int2 grain = work[blockIdx.x];   // chunk, first fine segment
+    TeaItem w = B.tea_item[grain.x];
+    chain_wait();   // no kernel writes the grains
     if (gate && *gate != run_if) return;
     const TeaConst K = tea_const(P.tea_a);
-    while (u < u_end) {
-        const long long first = B.tea_unit0[item];
-        const int nblk = (int)(B.tea_unit0[item + 1] - first);
-        const int b0 = (int)(u - first), b1 = (int)min((long long)nblk, u_end - first);
-        const int2 w = work[item], span = B.tea_span[item];
-        const int traj = w.x, g = w.y + tid;
-        const float4 *pack = B.tea_pack + (size_t)span.y * kTeaBlockF4;
+    for (int at = blockIdx.x;;) {
+        const int nblk = (w.end - w.base + kTeaBlock - 1) / kTeaBlock, fine = tea_fine(nblk);
+        const int nfine = (nblk + fine - 1) / fine, s0 = grain.y, s1 = min(nfine, s0 + (1 << P.tea_level));
+        const int b0 = s0 * fine, b1 = min(nblk, s1 * fine);
+        const int g = w.first + tid;
+        const float4 *pack = B.tea_pack + (size_t)w.block * kTeaBlockF4;
         auto issue = [&](int tile) {
             const int q0 = b0 + tile * kTeaTileBlocks, nq = min(kTeaTileBlocks, b1 - q0);
             float4 *dst = s_tile[tile % kTeaStages];
@@ -452,12 +508,16 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
             if (k < ntiles) issue(k);
             cp_async_commit();
         }
-        const bool valid = g < span.x;
+        const bool valid = g < w.end;
         const float4 p = valid ? B.frame_in[g] : make_float4(0.f, 0.f, 0.f, 0.f);
         const bool act = __any_sync(0xffffffffu, valid && !(B.flags[g] & kFlagExtra));
+        const bool split = s1 - s0 < nfine;
+        float4 *node = &s_node[0][tid];
+        node[kTeaLevels * kTeaThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
         Op X;
-        X.start(P, B, traj, p, g, valid);
-        const int self = (w.y - B.off[traj]) / kTeaBlock + warp;   // the block that holds this warp's beads
+        X.start(P, B, w.traj, p, g, valid);
+        const int self = (w.first - w.base) / kTeaBlock + warp;   // the block that holds this warp's beads
+        int left = fine, seg = s0;   // blocks of the fine segment still to come, its index
         for (int tile = 0; tile < ntiles; tile++) {
             cp_async_wait<kTeaStages - 2>();
             __syncthreads();
@@ -476,40 +536,43 @@ __global__ void __launch_bounds__(kTeaThreads, 9) k_tea_pass(KParams P, DevBuffe
 #pragma unroll 8
                     for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
                 }
-                if (rm <= K.four_a2) tea_near_block(X, K, blk, own, lane);
+                if (rm <= K.four_a2) tea_near_block(X, K, blk, own ? lane : -1);
+                if (--left > 0 && q0 + q + 1 < nblk) continue;
+                left = fine;
+                float4 v = X.sum();
+                X.clear();
+                int lo = seg++;
+                if (tea_carry(v, lo, 0, s0, s1, nfine, node, kTeaThreads) != kTeaHold)   // the grain, or a group of the item
+                    node[kTeaLevels * kTeaThreads] = split ? v : add4(node[kTeaLevels * kTeaThreads], v);
             }
         }
-        float4 acc = X.sum();
+        float4 acc = node[kTeaLevels * kTeaThreads];
         bool done = true;
         __syncthreads();   // the tiles are free again (and s_last)
-        if (b0 > 0 || b1 < nblk) {
-            // part of the item: slot 0 of the run for an item begun before it, slot 1 for one it begins
-            B.tea_part[((size_t)blockIdx.x * 2 + (b0 > 0 ? 0 : 1)) * kTeaI + tid] = acc;
-            const int k0 = (int)tea_div((first + 1) * G - 1, U), k1 = (int)tea_div((first + nblk) * G - 1, U);
+        if (split) {
+            float4 *part = B.tea_part + (size_t)w.slot * kTeaI + tid;   // of the item's grains
+            const int ng = (nfine + (1 << P.tea_level) - 1) >> P.tea_level;
+            part[(s0 >> P.tea_level) * kTeaI] = acc;
             __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(&B.tea_cnt[item], 1) == k1 - k0;
+            if (tid == 0) s_last = atomicAdd(&B.tea_cnt[grain.x], 1) == ng - 1;
             __syncthreads();
             done = s_last;
             if (done) {
                 __threadfence();
-                acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = k0; k <= k1; k += 4) {   // four requested at once; run k0 begins the item
-                    float4 q[4];
-#pragma unroll
-                    for (int v = 0; v < 4; v++)
-                        if (k + v <= k1)
-                            q[v] = __ldcg(&B.tea_part[((size_t)(k + v) * 2 + (k + v == k0 ? 1 : 0)) * kTeaI + tid]);
-#pragma unroll
-                    for (int v = 0; v < 4; v++)
-                        if (k + v <= k1) acc = make_float4(acc.x + q[v].x, acc.y + q[v].y, acc.z + q[v].z, acc.w + q[v].w);
-                }
-                if (tid == 0) B.tea_cnt[item] = 0;
+                acc = tea_collect(part, ng, P.tea_level);
+                if (tid == 0) B.tea_cnt[grain.x] = 0;
             }
         }
-        if (done && valid) X.finish(P, B, g, traj, acc, K, feff);
-        u = first + b1;
-        item++;
+        if (done && valid) {
+            typename Op::Bead bead;
+            bead.load(P, B, g);
+            X.finish(P, B, g, bead, w.traj, acc, K, feff);
+        }
+        at += gridDim.x;
+        if (at >= nwork) break;
+        grain = work[at];
+        w = B.tea_item[grain.x];
     }
 }
 
@@ -531,98 +594,120 @@ __global__ void k_tea_pack_clear(float4 *pack, int nblocks) {
     pack[k] = make_float4(a, a, b, b);
 }
 
-// The same pass for systems too small to fill the GPU, where a pass lasts as long as its
-// chain of waits: a warp a bead, sixteen lanes for the slots of a block and two blocks at once,
-// adds up in registers and by shuffles, so no partial sum goes through memory and
-// no CTA waits for another's (in k_tea_pass the fence, the count and the parts of the runs
-// are half of the time there).  The blocks are read straight from L1 and L2.  Overlapping
-// beads are noted in a mask and come after each 32 pairs of blocks, so that the loop
-// has no branch and its loads overlap.
-constexpr int kTeaLanes = 32, kTeaLaneThreads = 128;
+// The same sums for systems too small to fill the GPU, where a pass lasts as long as its
+// chain of waits: a CTA of eight warps serves eight beads, a thread one bead and one fine segment
+// (eight lanes read the same words), the segments meet in shared memory, so
+// no partial sum goes through global memory and no CTA waits for another's.
+// The CTA copies its whole trajectory first, one word further for
+// every block, so that the segments of a warp are in different banks.
+constexpr int kSmallBeads = 8, kSmallThreads = 256, kSmallStride = kTeaBlockF4 + 1;
 template <class Op>
-__global__ void __launch_bounds__(kTeaLaneThreads) k_tea_lanes(KParams P, DevBuffers B, float4 *feff, const int *gate,
-                                                               int run_if) {
-    constexpr int kGroups = kTeaLanes / kTeaPairSlots;   // blocks taken at once
-    const int g = blockIdx.x * (kTeaLaneThreads / kTeaLanes) + threadIdx.x / kTeaLanes, lane = threadIdx.x % kTeaLanes;
-    const int t = lane % kTeaPairSlots;
-    const bool valid = g < P.nb;
-    const int gc = valid ? g : P.nb - 1;
-    const int traj = B.traj[gc], base = B.off[traj], n = B.off[traj + 1] - base, slot = B.tea_slot[gc];
+__global__ void __launch_bounds__(kSmallThreads, 2) k_tea_small(KParams P, DevBuffers B, float4 *feff, const int *gate,
+                                                                int run_if) {
+    __shared__ float4 s_part[kTeaMaxFine][kSmallBeads];
+    extern __shared__ float4 s_pack[];
+    const int l = threadIdx.x % kSmallBeads;
+    const int2 w = B.tea_small[blockIdx.x];   // trajectory, first bead
+    const int traj = w.x, base = B.off[traj], end = B.off[traj + 1], n = end - base, g = w.y + l;
+    const bool valid = g < end;
+    const int gc = valid ? g : end - 1, slot0 = B.tea_slot[base];
     chain_wait();   // no kernel writes what was read so far
     if (gate && *gate != run_if) return;
+    const int nblk = (n + kTeaBlock - 1) / kTeaBlock, fine = tea_fine(nblk), nfine = (nblk + fine - 1) / fine;
+    const float4 *pack = B.tea_pack + (size_t)(slot0 / kTeaBlock) * kTeaBlockF4;
+    for (int q = threadIdx.x / 32; q < nblk; q += kSmallThreads / 32)
+        for (int c = threadIdx.x % 32; c < Op::kWords; c += 32) cp_async16(s_pack + q * kSmallStride + c, pack + q * kTeaBlockF4 + c);
+    cp_async_commit();
     const float4 p = B.frame_in[gc];
     const TeaConst K = tea_const(P.tea_a);
     Op X;
     X.start(P, B, traj, p, gc, valid);
-    const int self = (gc - base) / kTeaBlock, se = slot & 1;
-    const bool mine = (slot % kTeaBlock) >> 1 == t;
-    const float4 *pack = B.tea_pack + (size_t)(slot / kTeaBlock - self) * kTeaBlockF4;
-    const int nblk = (n + kTeaBlock - 1) / kTeaBlock;
-    for (int q0 = lane / kTeaPairSlots; q0 < nblk; q0 += 32 * kGroups) {
-        unsigned near = 0;   // of these blocks, the ones with an overlapping bead in this lane's slot
-        const int nq = min(32, (nblk - q0 + kGroups - 1) / kGroups);
-#pragma unroll 4
-        for (int k = 0; k < nq; k++) {
-            const int q = q0 + k * kGroups;
+    const int self = (gc - base) / kTeaBlock, in = (gc - base) % kTeaBlock;
+    typename Op::Bead bead;
+    if (threadIdx.x < kSmallBeads) bead.load(P, B, gc);   // of the threads that finish the beads
+    cp_async_wait<0>();
+    __syncthreads();
+    for (int f = threadIdx.x / kSmallBeads; f < nfine; f += kSmallThreads / kSmallBeads) {
+        X.clear();
+        const int last = min(nblk, (f + 1) * fine);
+        for (int q = f * fine; q < last; q++) {
+            const float4 *blk = s_pack + q * kSmallStride;
+            const bool own = q == self;
+            const int sp = own ? in >> 1 : -1;
             float rm = 3.4e38f;
-            X.template pair<true>(K, pack + (size_t)q * kTeaBlockF4, t, mine && q == self ? t : -1, se, rm);
-            near |= (rm <= K.four_a2 ? 1u : 0u) << k;
-        }
-        for (; near; near &= near - 1) {
-            const int q = q0 + (__ffs((int)near) - 1) * kGroups;
-            const float4 *blk = pack + (size_t)q * kTeaBlockF4;
-            const bool own = mine && q == self;
-            const float2 r2 = X.dist2(blk, t);
-            if (r2.x <= K.four_a2 && !(own && se == 0)) X.near(K, blk, t, 0);
-            if (r2.y <= K.four_a2 && !(own && se == 1)) X.near(K, blk, t, 1);
-        }
-    }
-    float4 acc = X.sum();
 #pragma unroll
-    for (int o = kTeaLanes / 2; o > 0; o >>= 1) {
-        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
-        acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+            for (int t = 0; t < kTeaPairSlots; t++) X.template pair<true>(K, blk, t, sp, in & 1, rm);
+            if (rm <= K.four_a2) tea_near_block(X, K, blk, own ? in : -1);
+        }
+        s_part[f][l] = X.sum();
     }
-    if (valid && lane == 0) X.finish(P, B, g, traj, acc, K, feff);
+    __syncthreads();
+    // the first warp adds them, a lane a bead and a group of the tree
+    if (threadIdx.x >= 32) return;
+    static_assert(kTeaLevels == 3 && kSmallBeads == 8, "four groups of eight a warp");
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 acc = zero;
+    for (int f0 = 0; f0 < nfine; f0 += 32) {
+        const int f = f0 + threadIdx.x / kSmallBeads * 8, m = nfine - f;
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = k < m ? s_part[f + k][l] : zero;
+#pragma unroll
+        for (int h = 1; h < 8; h *= 2)
+#pragma unroll
+            for (int k = 0; k < 8; k += 2 * h)
+                if (k + h < m) v[k] = add4(v[k], v[k + h]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float4 t = make_float4(__shfl_sync(0xffffffffu, v[0].x, l + 8 * k), __shfl_sync(0xffffffffu, v[0].y, l + 8 * k),
+                                         __shfl_sync(0xffffffffu, v[0].z, l + 8 * k), __shfl_sync(0xffffffffu, v[0].w, l + 8 * k));
+            if (f0 + 8 * k < nfine) acc = add4(acc, t);
+        }
+    }
+    if (threadIdx.x < kSmallBeads && valid) X.finish(P, B, g, bead, traj, acc, K, feff);
 }
-// Up to these beads and units (32 x 128 pairs) the lanes form is used.  Steps with it and with
-// k_tea_pass: 299 beads 10.2 and 13.9 us, 1520 beads 18.2 and 20.7, 2800 beads (1936 units) 27.1
-// and 28.5, 20 x 299 beads 16.4 and 17.5; but 3300 beads (2704 units) 30.9 and 29.7, 2 x 3300 beads
-// 50 and 41, 40 x 299 beads (1200 units) 22.3 and 21.7.
-constexpr int kTeaLaneBeads = 6500, kTeaLaneUnits = 2000;
-// Runs of a launch, one CTA each: kTeaRunsPerSlot for every CTA that fits the device, but
-// no item cut into more than about 16 (their sums meet in one CTA), or 48 while the
-// runs do not fill the device once (a step of 5600 beads 58 -> 52 us, of 2 x 3300 beads 47 -> 41;
-// of 16 x 1520 beads, which fill it, 56 -> 58).  rare: a
-// launch that mostly finds its gate closed, which should be short then.
-template <class Op>
-static int tea_runs(const KParams &P, bool rare) {
-    int dev = 0, sms = 1, occ = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tea_pass<Op>, kTeaThreads, 0);
-    const long long wave = (long long)(occ > 0 ? (occ < kTeaMaxOcc ? occ : kTeaMaxOcc) : 1) * sms;
-    const long long slots = rare ? wave : wave * kTeaRunsPerSlot;
-    auto runs_of = [&](int pieces) {   // with items in at most this many pieces
-        const long long least = (P.tea_max_blocks + pieces - 1) / pieces;
-        return (P.tea_units + least - 1) / least;
-    };
-    long long runs = runs_of(16);
-    if (runs < wave) runs = std::max(runs, std::min(wave, runs_of(48)));
-    return (int)std::min(runs, slots);
+// Up to these CTAs for every SM and blocks of a trajectory the small form is used.  Steps with it and
+// with k_tea_pass: 299 beads 9.4 and 13.5 us, 1520 beads 15.4 and 19.6, 2800 beads (350 CTAs) 28.6 and
+// 29.1, 2 x 1520 beads (380) 22.2 and 23.5; but 3300 beads (104 blocks) 37.6 and 30.5, 4 x 1520 beads
+// (760) 30.2 and 27.5, 20 x 299 beads (760) 20.0 and 18.3.
+constexpr int kTeaSmallCtas = 3, kTeaSmallBlocks = 96;
+int tea_small_prepare() {   // the limit of the largest trajectory: engines share the kernels
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int bytes = kTeaSmallBlocks * kSmallStride * (int)sizeof(float4);
+    return cudaFuncSetAttribute(k_tea_small<EpsOp>, attr, bytes) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_tea_small<StepOp<false>>, attr, bytes) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_tea_small<StepOp<true>>, attr, bytes) == cudaSuccess
+               ? 0
+               : -1;
 }
+int tea_small_beads() { return kSmallBeads; }
+// rare: a launch that mostly finds its gate closed, which should be short then.
 template <class Op>
 static void tea_launch(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, float4 *feff, const int *gate,
                        int run_if, cudaStream_t s) {
-    if (P.nb <= kTeaLaneBeads && P.tea_units <= kTeaLaneUnits) {
-        const int beads = kTeaLaneThreads / kTeaLanes;
-        launch_chained(P, k_tea_lanes<Op>, (P.nb + beads - 1) / beads, kTeaLaneThreads, 0, s, P, B, feff, gate, run_if);
+    if (P.tea_nsmall <= kTeaSmallCtas * (P.tea_wave / kTeaOcc) && P.tea_max_blocks <= kTeaSmallBlocks) {
+        launch_chained(P, k_tea_small<Op>, P.tea_nsmall, kSmallThreads, sizeof(float4) * kSmallStride * P.tea_max_blocks,
+                       s, P, B, feff, gate, run_if);
         return;
     }
-    launch_chained(P, k_tea_pass<Op>, tea_runs<Op>(P, gate && run_if == 1), kTeaThreads, 0, s, P, B, work, nwork, feff,
+    const bool rare = gate && run_if == 1;
+    launch_chained(P, k_tea_pass<Op>, rare ? std::min(nwork, P.tea_wave) : nwork, kTeaThreads, 0, s, P, B, work, nwork, feff,
                    gate, run_if);
+}
+// The grain of a batch: of fine segments, pairs of them, and so on up to whole items the one with the
+// least work a CTA slot plus a quarter of a grain at the end (a CTA alone on an SM is about four times as
+// fast as one of nine), half a block a grain for its start and its partial sums.
+int tea_grain_level(long long units, const long long *ngrains, const int *blocks, int wave) {
+    int best = 0;
+    double least = 1e300;
+    for (int k = 0; k <= kTeaWhole; k++) {
+        const double t = ((double)units + 0.5 * ngrains[k]) / wave + 0.25 * (blocks[k] + 0.5);
+        if (t < least) {
+            least = t;
+            best = k;
+        }
+    }
+    return best;
 }
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s) {
     k_tea_pack<<<(P.nb + 127) / 128, 128, 0, s>>>(P, B);
@@ -1042,7 +1127,7 @@ __global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, D
 #pragma unroll 8
                 for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
             }
-            if (!LISTCORR && rm <= K.four_a2) tea_near_block(X, K, blk, own, lane);
+            if (!LISTCORR && rm <= K.four_a2) tea_near_block(X, K, blk, own ? lane : -1);
         }
         const float4 sum = X.sum();
         const float4 v = make_float4(sum.x + corr.x, sum.y + corr.y, sum.z + corr.z, 0.f);

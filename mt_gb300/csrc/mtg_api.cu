@@ -526,24 +526,39 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     e->nwork = (int)work.size();
     // all-pairs TEA kernels: chunks of kTeaChunk beads i, blocks of kTeaBlock
     // beads j, a chunk's units = the blocks of its trajectory
-    std::vector<int2> tea_work, tea_span;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    std::vector<int2> tea_small;
     std::vector<int> tea_slot(nb), tea_blk0(nt + 1);
-    std::vector<long long> tea_unit0{0};
+    long long ngrains[kTeaWhole + 1] = {};
+    int grain_blocks[kTeaWhole + 1] = {};
     for (int tr = 0; tr < nt; tr++) {
         const int n = t->offsets[tr + 1] - t->offsets[tr], nblk = (n + kTeaBlock - 1) / kTeaBlock;
+        const int chunks = (n + kTeaChunk - 1) / kTeaChunk, nfine = (nblk + tea_fine(nblk) - 1) / tea_fine(nblk);
         tea_blk0[tr + 1] = tea_blk0[tr] + nblk;
         e->kp.tea_max_blocks = std::max(e->kp.tea_max_blocks, nblk);
+        e->kp.tea_units += (long long)chunks * nblk;
+        for (int k = 0; k <= kTeaWhole; k++) {
+            ngrains[k] += (long long)chunks * ((nfine + (1 << k) - 1) >> k);
+            grain_blocks[k] = std::max(grain_blocks[k], std::min(nblk, tea_fine(nblk) << k));
+        }
         for (int i = 0; i < n; i++) tea_slot[t->offsets[tr] + i] = tea_blk0[tr] * kTeaBlock + i;
-        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += kTeaChunk) {
-            tea_work.push_back(make_int2(tr, g));
-            tea_span.push_back(make_int2(t->offsets[tr + 1], tea_blk0[tr]));
-            tea_unit0.push_back(tea_unit0.back() + nblk);
+        for (int g = t->offsets[tr]; g < t->offsets[tr + 1]; g += tea_small_beads()) tea_small.push_back(make_int2(tr, g));
+    }
+    e->kp.tea_wave = kTeaOcc * sms;
+    e->kp.tea_level = tea_grain_level(e->kp.tea_units, ngrains, grain_blocks, e->kp.tea_wave);
+    e->kp.tea_nsmall = (int)tea_small.size();
+    std::vector<TeaItem> tea_item;
+    std::vector<int2> tea_work;
+    for (int tr = 0; tr < nt; tr++) {
+        const int base = t->offsets[tr], end = t->offsets[tr + 1], nblk = tea_blk0[tr + 1] - tea_blk0[tr];
+        for (int g = base; g < end; g += kTeaChunk) {
+            const int slot = (int)tea_work.size(), item = (int)tea_item.size();
+            tea_item.push_back({tr, g, base, end, tea_blk0[tr], slot, {0, 0}});
+            for (int s = 0; s * tea_fine(nblk) < nblk; s += 1 << e->kp.tea_level) tea_work.push_back(make_int2(item, s));
         }
     }
     e->tea_nwork = (int)tea_work.size();
-    e->kp.tea_units = tea_unit0.back();
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
     const std::vector<int4> list_work = plan_lists(sms, nt, t->offsets, &e->list_parts);
     e->list_nwork = (int)list_work.size();
     // the tuning's tea_slices as reported before anything sets it (no kernel reads it)
@@ -587,7 +602,7 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     ALLOC(e->stage_i, nb);
     if (p->hdi_on) {
         ALLOC(e->tea_work, e->tea_nwork);
-        ALLOC(e->tea_span, e->tea_nwork);
+        ALLOC(e->tea_item, tea_item.size());
         ALLOC(e->tea_r, nb);
         ALLOC(e->tea_ci, nb);
         ALLOC(e->tea_eps, nb);
@@ -595,9 +610,9 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         ALLOC(e->tea_eps_t, nt);
         ALLOC(e->tea_pack, (size_t)kTeaBlockF4 * tea_blk0[nt]);
         ALLOC(e->tea_slot, nb);
-        ALLOC(e->tea_unit0, e->tea_nwork + 1);
-        ALLOC(e->tea_part, (size_t)2 * kTeaChunk * std::min<long long>(e->kp.tea_units, (long long)kTeaMaxOcc * kTeaRunsPerSlot * sms));
-        ALLOC(e->tea_cnt, e->tea_nwork);
+        ALLOC(e->tea_small, tea_small.size());
+        ALLOC(e->tea_part, (size_t)kTeaChunk * e->tea_nwork);
+        ALLOC(e->tea_cnt, tea_item.size());
     }
     // spatial-hash tables of the cell-list rebuild
     std::vector<int> tbase(nt + 1, 0), tmask(nt, 0);
@@ -626,9 +641,9 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
         mtg_destroy(e);
         return rc;
     }
-    if (smem_lists_prepare() != 0) {
+    if (smem_lists_prepare() != 0 || tea_small_prepare() != 0) {
         mtg_destroy(e);
-        return fail(MTG_E_CUDA, "the list kernel could not reserve its shared memory");
+        return fail(MTG_E_CUDA, "the list or TEA kernels could not reserve their shared memory");
     }
     choose_list_method(e);
     std::vector<float> zs(nt, 0.f);
@@ -651,13 +666,13 @@ int mtg_create_batch(const mtg_params *p, const mtg_batch_topology *t, mtg_engin
     cudaMemsetAsync(e->force, 0, sizeof(float4) * 2 * nb, s);
     if (p->hdi_on) {
         if ((rc = upload(e->tea_work, tea_work.data(), sizeof(int2) * tea_work.size(), s)) ||
-            (rc = upload(e->tea_span, tea_span.data(), sizeof(int2) * tea_span.size(), s)) ||
-            (rc = upload(e->tea_slot, tea_slot.data(), sizeof(int) * nb, s)) ||
-            (rc = upload(e->tea_unit0, tea_unit0.data(), sizeof(long long) * tea_unit0.size(), s))) {
+            (rc = upload(e->tea_item, tea_item.data(), sizeof(TeaItem) * tea_item.size(), s)) ||
+            (rc = upload(e->tea_small, tea_small.data(), sizeof(int2) * tea_small.size(), s)) ||
+            (rc = upload(e->tea_slot, tea_slot.data(), sizeof(int) * nb, s))) {
             mtg_destroy(e);
             return rc;
         }
-        cudaMemsetAsync(e->tea_cnt, 0, sizeof(int) * e->tea_nwork, s);
+        cudaMemsetAsync(e->tea_cnt, 0, sizeof(int) * tea_item.size(), s);
         launch_tea_pack_clear(e->tea_pack, tea_blk0[nt], s);
         cudaMemsetAsync(e->tea_ci, 0, sizeof(float4) * nb, s);
         cudaMemsetAsync(e->tea_beta, 0, sizeof(float) * nt, s);
@@ -766,11 +781,11 @@ int mtg_destroy(mtg_engine *e) {
                     e->ljc, e->lj, e->lonc, e->lon, e->latc, e->lat, e->err, e->work, e->work_first, e->list_work,
                     e->en_partials, e->en_traj, e->en_bead, e->tea_r, e->tea_ci, e->tea_eps, e->tea_beta,
                     e->tea_eps_t, e->stage, e->stage_u8, e->stage_i, e->cell_tbase, e->cell_tmask,
-                    e->cell_key, e->cell_bead, e->cell_pos, e->cell_cnt, e->cell_start, e->cell_cursor, e->tea_work,
+                    e->cell_key, e->cell_bead, e->cell_pos, e->cell_cnt, e->cell_start, e->cell_cursor, e->tea_work, e->tea_item,
                     e->surr_desc, e->surr_pred, e->surr_stats, e->surr_gate, e->surr_err, e->surr_part,
                     e->tea_ci2, e->feff_a, e->feff_b, e->tea_eps2, e->tea_beta2, e->tea_eps_t2,
                     e->hydro_cand, e->hydro_rank, e->hydro_sums, e->hydro_counts, e->hydro_events,
-                    e->tea_pack, e->tea_span, e->tea_slot, e->tea_unit0, e->tea_part, e->tea_cnt};
+                    e->tea_pack, e->tea_small, e->tea_slot, e->tea_part, e->tea_cnt};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (e->stage_host) cudaFreeHost(e->stage_host);

@@ -34,9 +34,10 @@ struct mtg_engine {
     int nwork = 0;
     int4 *list_work = nullptr;  // CTAs of the one-launch list rebuild: trajectory, first bead, beads
     int list_nwork = 0, list_parts = 1;
-    int2 *tea_work = nullptr;   // chunks of kTeaChunk beads for the TEA kernels
-    int2 *tea_span = nullptr;   // their trajectories' ends and first blocks
+    int2 *tea_work = nullptr;   // all-pairs TEA kernels, see DevBuffers
     int tea_nwork = 0;
+    mtg::TeaItem *tea_item = nullptr;
+    int2 *tea_small = nullptr;
     int *work_first = nullptr;
     double *en_partials = nullptr, *en_traj = nullptr, *en_bead = nullptr;
     float4 *tea_r = nullptr, *tea_ci = nullptr;
@@ -44,7 +45,6 @@ struct mtg_engine {
     double *tea_eps_t = nullptr;
     float4 *tea_pack = nullptr, *tea_part = nullptr;   // all-pairs TEA kernels, see DevBuffers
     int *tea_slot = nullptr, *tea_cnt = nullptr;
-    long long *tea_unit0 = nullptr;
     int tea_slices = 1, tea_jparts = 1;   // of the tuning, as set (no kernel reads them)
     float *stage = nullptr;        // 7*nb floats for host <-> device Coord transfers
     void *stage_host = nullptr;    // pinned mirror of stage
@@ -146,9 +146,9 @@ struct mtg_engine {
         b.lat = lat;
         b.err = err;
         b.tea_pack = tea_pack;
-        b.tea_span = tea_span;
+        b.tea_item = tea_item;
+        b.tea_small = tea_small;
         b.tea_slot = tea_slot;
-        b.tea_unit0 = tea_unit0;
         b.tea_part = tea_part;
         b.tea_cnt = tea_cnt;
         b.tea_r = tea_r;

@@ -62,11 +62,20 @@ struct KParams {
     float tea_a, tea_var;
     int tea_max_blocks;    // blocks of kTeaBlock beads of the largest trajectory
     long long tea_units;   // (chunk of kTeaChunk beads) x (block) pairs of the all-pairs kernels
+    int tea_level;         // the all-pairs kernels' grains are 2^tea_level fine segments of a chunk
+    int tea_wave;          // CTAs of them that the device holds at once
+    int tea_nsmall;        // CTAs of the small form
     int chain;             // launch the kernels of a step chained (launch_chained)
     int step_block;        // threads per CTA of the fused plain step (64, 128 or 256)
 };
 
 // Device buffers of one engine.
+// kTeaChunk beads i of the all-pairs kernels, from `first` on.
+struct __align__(16) TeaItem {
+    int traj, first, base, end;   // its trajectory, and where that begins and ends
+    int block, slot, pad[2];      // the trajectory's first block in the pack; the first of its grains' slots
+};
+
 struct DevBuffers {
     const int *off;        // [nt+1]
     const int *traj;       // [nb]
@@ -88,11 +97,11 @@ struct DevBuffers {
     double *tea_eps_t;     // [nt]
     // all-pairs kernels (kernels_tea.cu)
     float4 *tea_pack;      // every trajectory's beads in blocks, see tea_pack_bead
-    const int2 *tea_span;  // of each work item: end of its trajectory, first block of it
+    const TeaItem *tea_item;   // [chunks]
+    const int2 *tea_small; // CTAs of the small form: trajectory, first bead
     const int *tea_slot;   // [nb] slot of each bead in the pack (32 a block)
-    const long long *tea_unit0;  // [work items + 1] first unit of each item
-    float4 *tea_part;      // partial sums: two slots of kTeaChunk beads per CTA of a launch
-    int *tea_cnt;          // [work items] CTAs of an item that have left their partial sums (0 between launches)
+    float4 *tea_part;      // partial sums: a slot of kTeaChunk beads for every grain of items of several
+    int *tea_cnt;          // [chunks] grains of a chunk that have left their partial sums (0 between launches)
 };
 
 // ------------------------------------------------------------------ RNG
@@ -335,6 +344,13 @@ __device__ __forceinline__ void list_append(const KParams &P, const DevBuffers &
 constexpr int kTeaBlock = 32;
 constexpr int kTeaPairSlots = kTeaBlock / 2;
 constexpr int kTeaBlockF4 = 4 * kTeaPairSlots + kTeaPairSlots / 2;
+// A bead's all-pairs sums are cut by its trajectory alone, so that it gets the same
+// bits in every batch and in every form of the passes: fine segments of tea_fine() blocks, at most
+// kTeaMaxFine, are summed by themselves, then in pairs, pairs of pairs and so on kTeaLevels times
+// (groups of eight), and the groups one after another.
+constexpr int kTeaMaxFine = 48, kTeaLevels = 3;
+constexpr int kTeaWhole = 6;   // the level whose grain is every fine segment
+__host__ __device__ inline int tea_fine(int nblk) { return nblk <= 48 ? 1 : nblk <= 96 ? 2 : 4 * ((nblk + 191) / 192); }
 constexpr float kTeaFarAway = 1.0e18f;     // where extra beads and padding are, with zero F and R
 __device__ __forceinline__ float *tea_pack_at(const DevBuffers &B, int g, int &p, int &odd) {
     const int slot = B.tea_slot[g], l = slot % kTeaBlock;
@@ -518,13 +534,15 @@ void launch_energy(const KParams &P, const DevBuffers &B, double *per_bead, doub
                    const int2 *work, int nwork, cudaStream_t s);
 void launch_energy_totals(const KParams &P, const double *partials, const int *work_first, double *per_traj,
                           int *err, cudaStream_t s);
-// TEA kernels run over their own work list: chunks of kTeaChunk beads.
+// TEA kernels run over their own work list: grains of chunks of kTeaChunk beads (chunk, first fine segment).
 constexpr int kTeaChunk = 128;
 constexpr int kTeaMaxParts = 4;      // largest mtg_tuning::tea_jparts that is accepted
-constexpr int kTeaRunsPerSlot = 4;   // runs of an all-pairs launch for every CTA that fits the device
-constexpr int kTeaMaxOcc = 12;       // CTAs of the all-pairs kernels per SM at most (sizes tea_part)
+constexpr int kTeaOcc = 9;           // CTAs of the all-pairs kernels an SM holds
 // positions (F and R are zeroed once) into the pack, for epsilon passes outside a TEA step
 void launch_tea_pack(const KParams &P, const DevBuffers &B, cudaStream_t s);
+int tea_small_prepare();             // opts the small form into its shared memory (outside captures)
+int tea_small_beads();               // beads of a CTA of the small form
+int tea_grain_level(long long units, const long long *ngrains, const int *blocks, int wave);
 void launch_tea_pack_clear(float4 *pack, int nblocks, cudaStream_t s);
 void launch_tea_eps(const KParams &P, const DevBuffers &B, const int2 *work, int nwork, cudaStream_t s);
 void launch_tea_beta(const KParams &P, const DevBuffers &B, int capricious, float epsmax, cudaStream_t s);

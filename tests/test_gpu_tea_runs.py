@@ -77,3 +77,71 @@ def test_same_bits_every_time(sizes):
     assert np.isfinite(out[0][0]).all()
     for x, c in out[1:]:
         assert np.array_equal(x, out[0][0]) and np.array_equal(c, out[0][1])
+
+
+# (sizes, extra): a CTA a few beads; items held by one run and by several, runs that end one item and begin
+# the next; cuts at fine segments in batches of one and of several waves; cuts at coarse segments
+PRODUCTS = [((299,), False), ((2, 31, 33, 129, 300), True), ((3100,), True), ((1500, 40, 1700, 3000), True),
+            ((130,) * 70 + (2400,), True), ((900, 77) * 45, False), ((1600, 1590) * 60, False)]
+
+
+@pytest.mark.parametrize("sizes,extra", PRODUCTS, ids=lambda v: f"{len(v)}x{max(v)}" if isinstance(v, tuple) else str(v))
+def test_mobility_product_against_fp64(sizes, extra):
+    """Effective forces of the exact product in FP64 from the engine's own F, R, C_i and beta,
+    on both sides of the small form's limits, with overlapping pairs.  Bar: a term carries about a dozen FP32
+    roundings (6e-8 each) and three approximations (1.3e-7), 1.1e-6 of |T||g|, and the sums of
+    at most 64 blocks' terms in one accumulator and 48 segments' sums as much again at most: 4e-6."""
+    from mt_gb300 import engine
+    b = batch(sizes, 93, extra)
+    with engine.Engine(b) as e:
+        e.upload_state(b.coords)
+        e.rebuild_pairs()
+        F = e.compute_forces()[:, :3].astype(np.float64)
+        _, beta, ci, rc = e.tea_update()
+        assert rc in (0, -5)
+        fe, _, R = e.tea_effective_forces(exact=True, farfield=False)
+    check = range(b.ntraj) if b.ntraj < 10 else [0, 1, b.ntraj // 2, b.ntraj - 2, b.ntraj - 1]
+    for t in check:
+        s = slice(int(b.offsets[t]), int(b.offsets[t + 1]))
+        act = b.extra[s] == 0
+        x, f = b.coords[s, :3].astype(np.float64)[act], F[s][act]
+        c = 1.0 / np.sqrt(1.0 + float(beta[t]) ** 2 * ci[s, :3].astype(np.float64)[act])
+        r = R[s, :3].astype(np.float64)[act]
+        got = fe[s, :3].astype(np.float64)[act]
+        for i in range(0, len(x), 500):
+            k = slice(i, min(len(x), i + 500))
+            d = x[None, :, :] - x[k][:, None, :]
+            rr = np.linalg.norm(d, axis=2)
+            rr[np.arange(k.stop - k.start), np.arange(k.start, k.stop)] = 1.0
+            u, ra = d / rr[:, :, None], rr / b.params.tea_a
+            far = ra > 2.0
+            cii = np.where(far, 0.75 / ra * (1 + 2 / (3 * ra * ra)), 1 - 9 * ra / 32)
+            crr = np.where(far, 0.75 / ra * (1 - 2 / (ra * ra)), 3 * ra / 32)
+            for w in (cii, crr):
+                w[np.arange(k.stop - k.start), np.arange(k.start, k.stop)] = 0.0
+            g = f[None, :, :] + float(beta[t]) * c[k][:, None, :] * r[None, :, :]
+            ug = np.einsum("ija,ija->ij", u, g)
+            want = f[k] + c[k] * r[k] + np.einsum("ij,ija->ia", cii, g) + np.einsum("ij,ija->ia", crr * ug, u)
+            size = (np.einsum("ij,ija->ia", np.abs(cii), np.abs(g)) + np.einsum("ij,ija->ia", np.abs(crr)
+                    * np.einsum("ija,ija->ij", np.abs(u), np.abs(g)), np.abs(u)) + np.abs(f[k]) + np.abs(r[k]))
+            assert (np.abs(got[k] - want) <= 4.0e-6 * size).all()
+
+
+@pytest.mark.parametrize("sizes", [(299, 151, 33, 1520), (130,) * 70 + (2400,), (3300,) * 12, (1600, 1590, 40) * 40,
+                                   (5600,) * 30], ids=lambda v: f"{len(v)}x{max(v)}")
+def test_a_trajectory_gets_the_same_bits_in_every_batch(sizes):
+    """A batch on one engine and cut over four, where the whole takes equal runs cut at fine or at coarse
+    segments and the parts others or the small form: state, noise streams and C_i."""
+    from mt_gb300 import engine
+    b = batch(sizes, 94)
+    with engine.Engine(b) as e, engine.ShardedEngine(b, [0] * 4) as s:
+        e.upload_state(b.coords)
+        s.upload_state(b.coords)
+        e.step(0, 3)
+        s.step(0, 3)
+        x = e.download_state()
+        assert np.isfinite(x).all() and np.array_equal(x, s.download_state())
+        assert np.array_equal(e.download_rng(), s.download_rng())
+        whole, parts = e.tea_update(), [k.tea_update() for k in s.engines]
+        for v in range(3):
+            assert np.array_equal(whole[v], np.concatenate([p[v] for p in parts]))
