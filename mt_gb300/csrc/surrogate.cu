@@ -345,7 +345,7 @@ struct mtg_surrogate {
     std::mutex scratch_lock;
     char *scratch = nullptr;
     size_t scratch_bytes = 0;
-    std::vector<float> grad;   // host side of loss_grad's gradient, held with the scratch
+    float *grad = nullptr;         // page-locked host side of loss_grad's gradient, held with the scratch
     uint32_t spin = mlp::tc_default_spin();   // polls of the inference's waits for its MMAs
 };
 
@@ -464,6 +464,7 @@ int mtg_surrogate_destroy(mtg_surrogate *s) {
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     cudaFree(s->scratch);
+    if (s->grad) cudaFreeHost(s->grad);
     cudaFree(s->W.master);
     cudaFree(s->bf);
     cudaFree(s->norm);
@@ -550,10 +551,10 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     SCK(mlp::launch_backward_tc(s->W, dX, nullptr, s->norm, dT, n, dY, dZ, dG, dL, s->err, s->stream));
     if (grad) SCK(mlp::launch_grad_sum(dG, parts, dSum, s->stream));
     // the gradient waits here for the error word: the caller's is written by calls that succeed
-    if (grad) s->grad.resize(mlp::kParams);
+    if (grad && !s->grad) SCK(cudaMallocHost(&s->grad, sizeof(float) * mlp::kParams));
     std::vector<float> L(parts);
     int herr = 0;
-    if (grad) SCK(cudaMemcpyAsync(s->grad.data(), dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));
+    if (grad) SCK(cudaMemcpyAsync(s->grad, dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(L.data(), dL, sizeof(float) * parts, cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaMemcpyAsync(&herr, s->err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
@@ -564,7 +565,7 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     double l = 0.0;
     for (float v : L) l += v;
     if (loss) *loss = l / ((double)n * mlp::kOut);
-    if (grad) std::copy_n(s->grad.data(), mlp::kParams, grad);
+    if (grad) std::copy_n(s->grad, mlp::kParams, grad);
     return MTG_OK;
 }
 

@@ -16,6 +16,7 @@ inline cudaError_t fill(void *p, int v, size_t n, cudaStream_t) { return memset(
 inline cudaError_t ok(...) { return cudaSuccess; }
 }  // namespace fake
 #define cudaMalloc fake::alloc
+#define cudaMallocHost fake::alloc
 #define cudaFree fake::release
 #define cudaMemcpyAsync fake::copy
 #define cudaMemsetAsync fake::fill
