@@ -1022,17 +1022,18 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
 }
 
 // Near pairs.  The near lists of all leaves, one after another, are cut into
-// equal runs, one warp each, as many as the GPU holds at once; a warp goes through the
+// runs of about equal length, one warp each, twice as many as the GPU holds at once; a warp goes through the
 // leaves its run touches, a bead a lane, with the near leaves' beads copied one
 // leaf at a time, two ahead, into its own ring in shared memory: no barrier, no
 // partly filled wave, and equal work for all four schedulers of an SM.  The pair loop
 // is that of the all-pairs pass (StepOp), and like it the kernel is bound by the FP32 pipe.
+// A leaf's list is summed in segments of kFFSeg entries, added in order, and runs begin at the
+// heads of segments, so a bead's sum depends on its leaf alone, not on where the runs of
+// its batch are cut.  A leaf that one run holds goes to FFBuffers::nearsum; of a leaf that several
+// share each segment's sum goes to its slot and k_ff_far adds them.
 // 64 x 5600 beads, 225 M pairs: 256 us with four warps a leaf on 128-bead tiles (2100 of
 // 3950 instructions a warp were not pair arithmetic), 268 us with a whole leaf
-// a warp (a third of the time was the last wave), 233 us so.
-// A leaf that one run holds goes to FFBuffers::nearsum; of a leaf that several
-// share each writes its part (slot 0 of the run for a leaf begun before it, slot 1 for
-// one it begins) and k_ff_far adds them in run order.
+// a warp (a third of the time was the last wave), 242 us so (238 with runs cut at any entry).
 // Overlapping pairs (r <= 2a): with LISTCORR the far-field term of the pair loop is
 // replaced while walking the bead's LJ list once, which holds every pair
 // that close (checked by the launcher), by the run that begins the leaf;
@@ -1040,10 +1041,6 @@ __global__ void __launch_bounds__(32 * kM2LWarps) k_ff_m2l(KParams P, FFBuffers 
 // the all-pairs pass does.
 constexpr int kFFStages = 3;
 static_assert(kFFLeaf == kTeaBlock && kFFPackF4 == kTeaBlockF4, "leaves are blocks of the pair loop");
-// first near entry of run k of F.near_runs
-__device__ __forceinline__ int ff_run_start(const FFBuffers &F, int units, int k) {
-    return (int)((long long)k * units / F.near_runs);
-}
 template <bool LISTCORR>
 __global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, DevBuffers B, FFBuffers F, const int *gate) {
     chain_wait();
@@ -1051,17 +1048,8 @@ __global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, D
     __shared__ float4 s_leaf[kFFWarps][kFFStages][kFFPackF4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, run = blockIdx.x * kFFWarps + warp;
     if (run >= F.near_runs) return;
-    const int units = F.near_start[F.nleaf];
-    const int u0 = ff_run_start(F, units, run), u1 = ff_run_start(F, units, run + 1);
-    if (u0 >= u1) return;
-    int L = 0;   // the leaf whose list holds entry u0 (32-way search)
-    for (int n = F.nleaf; n > 1;) {
-        const int step = (n + 31) / 32;
-        const bool le = lane * step < n && F.near_start[L + lane * step] <= u0;
-        const int last = 31 - __clz((int)__ballot_sync(0xffffffffu, le));
-        n = min(step, n - last * step);
-        L += last * step;
-    }
+    const int u0 = F.near_run[run], u1 = F.near_run[run + 1];   // entries
+    int L = F.run_leaf[run];
     auto issue = [&](int u) {
         if (u < u1) {
             const float4 *src = F.pack + (size_t)F.near[u] * kFFPackF4;
@@ -1111,8 +1099,8 @@ __global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, D
                 }
             }
         }
-        const bool whole = u == e0 && stop == e1;
-        const int slot = u == e0 ? 1 : 0;
+        const int slot = F.near_slot[L];   // of the leaf's first segment, or -1
+        float4 sum = make_float4(corr.x, corr.y, corr.z, 0.f), total = make_float4(0.f, 0.f, 0.f, 0.f);
         for (; u < stop; u++) {
             cp_async_wait<kFFStages - 2>();
             __syncwarp();
@@ -1128,25 +1116,32 @@ __global__ void __launch_bounds__(32 * kFFWarps, kFFCtas) k_ff_near(KParams P, D
                 for (int t = 0; t < kTeaPairSlots; t++) X.template pair<false>(K, blk, t, 0, 0, rm);
             }
             if (!LISTCORR && rm <= K.four_a2) tea_near_block(X, K, blk, own ? lane : -1);
+            if ((u - e0) % kFFSeg < kFFSeg - 1 && u + 1 < e1) continue;
+            sum = add4(X.sum(), sum);   // with the overlapping pairs in the first segment's
+            X.clear();
+            if (slot < 0)
+                total = add4(total, sum);
+            else
+                F.nearpart[(size_t)(slot + (u - e0) / kFFSeg) * kFFLeaf + lane] = sum;
+            sum = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const float4 sum = X.sum();
-        const float4 v = make_float4(sum.x + corr.x, sum.y + corr.y, sum.z + corr.z, 0.f);
-        if (!whole)
-            F.nearpart[((size_t)run * 2 + slot) * kFFLeaf + lane] = v;
-        else if (valid)
-            F.nearsum[s0 + lane] = v;
+        if (slot < 0 && valid) F.nearsum[s0 + lane] = total;
     }
 }
-// The near sum of bead `lane` of leaf L (leaf bead s0 + lane) from its runs.
+// The near sum of bead `lane` of leaf L (leaf bead s0 + lane) from its segments.
 __device__ __forceinline__ float4 ff_near_sum(const FFBuffers &F, int L, int s0, int lane) {
-    const int units = F.near_start[F.nleaf], e0 = F.near_start[L], e1 = F.near_start[L + 1];
-    const int k0 = (int)(((long long)(e0 + 1) * F.near_runs - 1) / units),
-              k1 = (int)(((long long)e1 * F.near_runs - 1) / units);
-    if (k0 == k1) return F.nearsum[s0 + lane];
+    const int slot = F.near_slot[L];
+    if (slot < 0) return F.nearsum[s0 + lane];
+    const int n = (F.near_start[L + 1] - F.near_start[L] + kFFSeg - 1) / kFFSeg;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = k0; k <= k1; k++) {
-        const float4 q = F.nearpart[((size_t)k * 2 + (ff_run_start(F, units, k) > e0 ? 0 : 1)) * kFFLeaf + lane];
-        v = make_float4(v.x + q.x, v.y + q.y, v.z + q.z, 0.f);
+    for (int k = 0; k < n; k += 4) {   // four requested at once
+        float4 q[4];
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+            if (k + h < n) q[h] = F.nearpart[(size_t)(slot + k + h) * kFFLeaf + lane];
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+            if (k + h < n) v = add4(v, q[h]);
     }
     return v;
 }

@@ -574,6 +574,7 @@ constexpr int kFFLeaf = 32;
 constexpr float kFFNode = 0.70710678f;
 constexpr int kFFWarps = 4, kFFCtas = 8;   // warps of a CTA of the near-pair kernel, CTAs an SM
 constexpr int kFFRunsPerSlot = 2;      // runs of the near lists for every warp that fits the device
+constexpr int kFFSeg = 4;              // near entries that are summed by themselves
 constexpr int kFFMaxAnc = 16;          // nodes with far fields on a leaf's path to the root (tree depth bound)
 struct FFBuffers {
     int nleaf, nnode, ntgt, ninner, nrest;
@@ -598,7 +599,10 @@ struct FFBuffers {
     float4 *pack;            // [(nleaf+1)*kFFPackF4] each leaf's beads in the tile layout of the step kernel
                              // (leaf nleaf: padding, far away with zero F and R), written every step by P2M
     int near_runs;           // warps the near lists are divided over
-    float4 *nearpart;        // [2 * near_runs][kFFLeaf] parts of the near sums of leaves that runs share
+    const int *near_run;     // [near_runs + 1] first near entry of each
+    const int *run_leaf;     // [near_runs] the leaf it is of
+    const int *near_slot;    // [nleaf] first slot of nearpart of a leaf that runs share, -1 of others
+    float4 *nearpart;        // [slots][kFFLeaf] segments' sums of the leaves that runs share
     float4 *nearsum;         // [leaf beads] each bead's near-pair sum, in leaf bead order
 };
 // float4 per leaf of FFBuffers::pack, for the bead pairs (2p, 2p+1):

@@ -361,19 +361,36 @@ static int ff_build(mtg_engine *e) {
     if (max_anc > kFFMaxAnc)
         return mtg_internal_fail(MTG_E_CONFIG, "far-field tree deeper than the step kernel's ancestor limit");
     enum { kLeafStart, kLeafBead, kLeafTraj, kNearStart, kNear, kNodeRange, kNodeLeaves, kFarStart, kFar, kTgt,
-           kInner, kAncStart, kAnc, kRest, kParts };
+           kInner, kAncStart, kAnc, kRest, kNearRun, kRunLeaf, kNearSlot, kParts };
+    // runs of the near lists (k_ff_near): kFFRunsPerSlot for each warp the device holds at once, none shorter
+    // than a segment, from the head of the segment that holds entry k U / runs on
+    int sms = 1;
+    FCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
+    const int units = (int)P.near.size();
+    const int near_runs = std::min(std::max(units / kFFSeg, std::min(units, 1)), sms * kFFCtas * kFFWarps * kFFRunsPerSlot);
+    std::vector<int> near_run, run_leaf, near_slot(nleaf, -1);
+    for (int k = 0, L = 0; k < near_runs; k++) {
+        const int at = (int)((long long)k * units / near_runs);
+        while (P.near_start[L + 1] <= at) L++;
+        near_run.push_back(at - (at - P.near_start[L]) % kFFSeg);
+        run_leaf.push_back(L);
+        if (near_run.back() > P.near_start[L]) near_slot[L] = 0;   // shared with the run before
+    }
+    near_run.push_back(units);
+    int near_slots = 0;
+    for (int L = 0; L < nleaf; L++)
+        if (near_slot[L] == 0) {
+            near_slot[L] = near_slots;
+            near_slots += (P.near_start[L + 1] - P.near_start[L] + kFFSeg - 1) / kFFSeg;
+        }
     const std::vector<int> *parts[kParts] = {&P.leaf_start, &P.leaf_bead, &P.leaf_traj, &P.near_start, &P.near,
                                              &P.node_range, &P.node_leaves, &P.far_start, &P.far, &P.tgt, &inner,
-                                             &P.anc_start, &P.anc, &P.rest};
+                                             &P.anc_start, &P.anc, &P.rest, &near_run, &run_leaf, &near_slot};
     size_t nints = 0;
     for (auto *v : parts) nints += v->size() + 1;
     const size_t nn1 = (size_t)std::max(nnode, 1);
-    // runs of the near lists (k_ff_near): two for each warp the device holds at once, or one an entry
-    int sms = 1;
-    FCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
-    const int near_runs = std::min((int)P.near.size(), sms * kFFCtas * kFFWarps * kFFRunsPerSlot);
     const size_t nf4 = (size_t)(2 + 16 + 24) * nn1 + (size_t)kFFPackF4 * (nleaf + 1) + P.leaf_bead.size() +
-                       (size_t)2 * near_runs * kFFLeaf;
+                       (size_t)near_slots * kFFLeaf;
     if (nints > e->ff_ints_cap) {
         if (e->ff_ints) cudaFree(e->ff_ints);
         e->ff_ints = nullptr;
@@ -424,6 +441,9 @@ static int ff_build(mtg_engine *e) {
     F.pack = e->ff_f4 + 42 * nn1;
     F.nearsum = F.pack + (size_t)kFFPackF4 * (nleaf + 1);
     F.near_runs = near_runs;
+    F.near_run = dev[kNearRun];
+    F.run_leaf = dev[kRunLeaf];
+    F.near_slot = dev[kNearSlot];
     F.nearpart = F.nearsum + P.leaf_bead.size();
     e->ff_near_pairs = P.near_pairs;
     e->ff_proxy_pairs = P.proxy_pairs;

@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 from helpers import per_bead_rel, small_system
+from mt_gb300 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -86,7 +87,6 @@ def _trained_surrogate(engine_mod):
 
 def test_learned_mode_with_farfield_runs_and_rechecks(engine_mod):
     s = _trained_surrogate(engine_mod)
-    from mt_gb300 import synth
     p = synth.default_params(seed=52, hdi_on=1, tea_epsilon_freq=5)
     b = synth.uniform_batch(p, 3, 60, 900, seed=52, cube=80.0, thermal=0.05, n_extra_dimers=2)
     e = engine_mod.Engine(b)
@@ -157,3 +157,31 @@ def test_farfield_rejects_bad_arguments(engine_mod):
     with pytest.raises(engine_mod.MtgError, match="theta"):
         e.set_tea_farfield(True, 1.5)
     e.close()
+
+
+@pytest.mark.parametrize("cutoff", [8.0, 5.5])
+def test_a_trajectory_gets_the_same_bits_in_every_batch(engine_mod, cutoff):
+    """Learned TEA of uneven trajectories on one engine, whose near-pair runs fill the GPU, and cut over
+    four whose runs are cut elsewhere: effective forces of the far-field product, states and noise
+    streams; overlapping pairs from the pair list (8 nm) and from the leaves (5.5 nm)."""
+    p = synth.default_params(seed=57, hdi_on=1, tea_epsilon_freq=5, ljpairscutoff=cutoff)
+    trajs = [synth.make_trajectory(pf, free, seed=57 + pf, radius=8.12, psi_mode="make_mt", cube=90.0, thermal=0.05)
+             for pf, free in ((200, 2600), (60, 700), (31, 90), (120, 1500))]
+    b = synth.batch_from_trajectories(p, [trajs[k % 4] for k in range(18)])
+    assert b.nbeads > 36000
+    with engine_mod.Surrogate(seed=5) as net, engine_mod.Engine(b) as e, engine_mod.ShardedEngine(b, [0] * 4) as s:
+        s.upload_state(b.coords)
+        e.upload_state(b.coords)
+        for k in [e] + s.engines:
+            k.set_surrogate(net, recheck_every=0)
+            k.set_tea_farfield(True, 0.85)
+            k.tea_update()
+        whole, parts = e.tea_effective_forces(), [k.tea_effective_forces() for k in s.engines]
+        act = b.extra == 0
+        for v in range(3):
+            assert np.array_equal(whole[v][act], np.concatenate([q[v] for q in parts])[act])
+        e.step(0, 12)
+        s.step(0, 12)
+        x = e.download_state()
+        assert np.isfinite(x).all() and np.array_equal(x, s.download_state())
+        assert np.array_equal(e.download_rng(), s.download_rng())
