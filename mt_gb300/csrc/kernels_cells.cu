@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kListThreads, 2) k_cell_lists_smem(const __gri
 // reproducible) and its place in the ordered copy.  Also the trajectory's centroid
 // and non-extra count.  Before: five launches, the sort with one thread a bucket
 // in global memory; 64 x 5600 beads 138 us, 40 us so.
-constexpr int kOrderThreads = 1024;
+constexpr int kOrderThreads = kStatsThreads;
 constexpr int kOrderBeads = 16384;
 __host__ __device__ inline int order_buckets(int n) {   // the table sizes of CellBuffers
     int m = 32;
@@ -837,52 +837,26 @@ __host__ __device__ inline int order_buckets(int n) {   // the table sizes of Ce
 }
 inline size_t order_bytes(int nmax) { return sizeof(uint16_t) * ((size_t)order_buckets(nmax) + nmax); }
 
-// Sum in two floats (Knuth's two-sum): the accuracy a centroid needs without the FP64
-// pipe, which the additions of a CTA would fill.  A sum that has left the finite numbers is its
-// first float.
-struct Sum2 {
-    float s = 0.f, e = 0.f;
-    __device__ __forceinline__ void add(float x, float xe) {
-        const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
-        e = __fadd_rn(e, __fadd_rn(xe, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z))));
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return isfinite(s) ? (double)s + (double)e : (double)s; }
-};
-
 __global__ void __launch_bounds__(kOrderThreads) k_cell_order(KParams P, DevBuffers B, CellBuffers C, float inv,
                                                               float4 *stats) {
     extern __shared__ unsigned s_tab[];                     // two 16-bit buckets a word, then the indices
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, traj = blockIdx.x;
     const int base = B.off[traj], n = B.off[traj + 1] - base, tb = C.tbase[traj], m = C.tmask[traj] + 1;
     uint16_t *s_end = reinterpret_cast<uint16_t *>(s_tab), *s_idx = s_end + m;
-    __shared__ Sum2 s_sum[kOrderThreads / 32][3];
-    __shared__ unsigned s_warp[kOrderThreads / 32], s_act[kOrderThreads / 32];
+    __shared__ unsigned s_warp[kOrderThreads / 32];
     for (int k = t; k < m / 2; k += kOrderThreads) s_tab[k] = 0;
     __syncthreads();
     auto bucket = [&](float4 p) {
         return (int)(cell_hash(cell_coord(p.x, inv), cell_coord(p.y, inv), cell_coord(p.z, inv)) & (uint32_t)(m - 1));
     };
-    Sum2 c[3];
-    unsigned act = 0;
+    TrajStats S;
     for (int j = t; j < n; j += kOrderThreads) {
         const float4 p = B.frame_in[base + j];
         const int b = bucket(p);
         atomicAdd(&s_tab[b >> 1], 1u << (16 * (b & 1)));
-        if (B.flags[base + j] & kFlagExtra) continue;
-        c[0].add(p.x, 0.f);
-        c[1].add(p.y, 0.f);
-        c[2].add(p.z, 0.f);
-        act++;
+        if (!(B.flags[base + j] & kFlagExtra)) S.add(p);
     }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int d = 0; d < 3; d++)
-            c[d].add(__shfl_xor_sync(0xffffffffu, c[d].s, o), __shfl_xor_sync(0xffffffffu, c[d].e, o));
-    act = __reduce_add_sync(0xffffffffu, act);
-    if (lane == 0) {
-        for (int d = 0; d < 3; d++) s_sum[wid][d] = c[d];
-        s_act[wid] = act;
-    }
+    S.store(stats + traj);
     __syncthreads();
     {   // exclusive scan of the counts, whole words a thread
         const int per = (m / 2 + kOrderThreads - 1) / kOrderThreads, lo = min(m / 2, t * per), hi = min(m / 2, lo + per);
@@ -906,17 +880,6 @@ __global__ void __launch_bounds__(kOrderThreads) k_cell_order(KParams P, DevBuff
             C.cnt[tb + 2 * k + 1] = (int)c1;
             run += c0 + c1;
         }
-    }
-    if (t == 0) {
-        unsigned count = 0;
-        for (int w = 0; w < kOrderThreads / 32; w++) {
-            count += s_act[w];
-            if (w > 0)
-                for (int d = 0; d < 3; d++) c[d].add(s_sum[w][d].s, s_sum[w][d].e);
-        }
-        const double inv_n = count > 0 ? 1.0 / count : 0.0;
-        stats[traj] = make_float4((float)(c[0].value() * inv_n), (float)(c[1].value() * inv_n),
-                                  (float)(c[2].value() * inv_n), (float)count);
     }
     __syncthreads();
     for (int j = t; j < n; j += kOrderThreads) {

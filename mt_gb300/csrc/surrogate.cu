@@ -30,87 +30,72 @@ constexpr float kDescCut = 20.0f;
 constexpr int kF = mlp::kIn;
 
 // centroid and non-extra count of every trajectory: (cx, cy, cz, N')
-__global__ void k_traj_stats(KParams P, DevBuffers B, float4 *stats) {
+__global__ void __launch_bounds__(kStatsThreads) k_traj_stats(KParams P, DevBuffers B, float4 *stats) {
     const int t = blockIdx.x;
     const int base = B.off[t], end = B.off[t + 1];
-    double sx = 0, sy = 0, sz = 0;
-    int cnt = 0;
-    for (int g = base + threadIdx.x; g < end; g += blockDim.x) {
-        if (B.flags[g] & kFlagExtra) continue;
-        const float4 p = B.frame_in[g];
-        sx += p.x;
-        sy += p.y;
-        sz += p.z;
-        cnt++;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, o);
-        sy += __shfl_xor_sync(0xffffffffu, sy, o);
-        sz += __shfl_xor_sync(0xffffffffu, sz, o);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    }
-    __shared__ double s[4][8];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        s[0][wid] = sx;
-        s[1][wid] = sy;
-        s[2][wid] = sz;
-        s[3][wid] = cnt;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0, b = 0, c = 0, n = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-            a += s[0][w];
-            b += s[1][w];
-            c += s[2][w];
-            n += s[3][w];
-        }
-        const double inv = n > 0 ? 1.0 / n : 0.0;
-        stats[t] = make_float4((float)(a * inv), (float)(b * inv), (float)(c * inv), (float)n);
-    }
+    TrajStats S;
+    for (int g = base + threadIdx.x; g < end; g += kStatsThreads)
+        if (!(B.flags[g] & kFlagExtra)) S.add(B.frame_in[g]);
+    S.store(stats + t);
 }
 
-// Shell accumulation of one neighbour: the ten features of its shell.
+// Shell accumulation of one neighbour: the ten features of its shell.  (Explicitly rounded
+// operations: the kernel's forms give the same bits.)
 __device__ __forceinline__ void desc_add(float (&s)[10], float rinv, float ux, float uy, float uz) {
-    const float r2i = rinv * rinv;
+    const float r2i = __fmul_rn(rinv, rinv);
     s[0] += 1.0f;
     s[1] += rinv;
-    s[2] += r2i;
-    s[3] += r2i * rinv;
-    s[4] += ux * ux * rinv;
-    s[5] += uy * uy * rinv;
-    s[6] += uz * uz * rinv;
-    s[7] += ux * uy * rinv;
-    s[8] += ux * uz * rinv;
-    s[9] += uy * uz * rinv;
+    s[2] = __fadd_rn(s[2], r2i);
+    s[3] = __fmaf_rn(r2i, rinv, s[3]);
+    s[4] = __fmaf_rn(__fmul_rn(ux, ux), rinv, s[4]);
+    s[5] = __fmaf_rn(__fmul_rn(uy, uy), rinv, s[5]);
+    s[6] = __fmaf_rn(__fmul_rn(uz, uz), rinv, s[6]);
+    s[7] = __fmaf_rn(__fmul_rn(ux, uy), rinv, s[7]);
+    s[8] = __fmaf_rn(__fmul_rn(ux, uz), rinv, s[8]);
+    s[9] = __fmaf_rn(__fmul_rn(uy, uz), rinv, s[9]);
 }
+__device__ __forceinline__ float norm2(float x, float y, float z) { return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x))); }
 
 // One thread per bead, taken in bucket order: the threads of a warp sit in
 // one or two cells and walk the same 27-cell neighbourhood, so candidate
 // loads are broadcasts and the loops mostly uniform.  Cells are 20 nm; the
 // candidates of a bucket are visited in ascending bead index.
-// PARTS threads share a bead's cells and add their sums by shuffles: batches too small to fill
-// the GPU last as long as one thread's walk.  Descriptors of 11,040 beads (call with the
-// copy back) 128 us with one thread a bead and 90 with four, 52,800 beads 300 and 273, 105,600 beads
-// 475 and 488; two threads 105, 271 and 483, eight 93, 281 and 514.
-constexpr int kDescParts = 4, kDescSplitBeads = 60000;
-template <int PARTS>
-__global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, CellBuffers C, const int2 *work,
+// A bead's sums are those of kDescParts parts of kDescCells cells, added in order.  Batches too small
+// to fill the GPU last as long as one thread's walk, so there THREADS = kDescParts threads share a bead, a
+// part each; otherwise one thread takes the parts one after another: the same bits.  Descriptors, ordered
+// binning and network of 64 x 5600 beads: 437 us so, 475 with four threads a bead, 400 with one sum
+// over all cells (450 without the bound on registers); of eight uneven systems, with the copy back,
+// 90 us with four threads and 128 with one.
+constexpr int kDescParts = 4, kDescCells = 7, kDescSplitBeads = 60000;
+template <int THREADS>
+__global__ void __launch_bounds__(kTile, THREADS == 1 ? 7 : 1) k_descriptors(KParams P, DevBuffers B, CellBuffers C, const int2 *work,
                                                        float inv_cell, const float4 *stats, float *desc,
                                                        const int *gate) {
     if (gate && *gate) return;
-    const int2 w = work[blockIdx.x / PARTS];
+    static_assert(THREADS == 1 || THREADS == kDescParts, "a thread or a part a thread");
+    const int2 w = work[blockIdx.x / THREADS];
     const int traj = w.x, end = B.off[traj + 1];
     const int base = B.off[traj];
-    const int slot = w.y + (blockIdx.x % PARTS) * (kTile / PARTS) + threadIdx.x / PARTS, part = threadIdx.x % PARTS;
+    const int slot = w.y + (blockIdx.x % THREADS) * (kTile / THREADS) + threadIdx.x / THREADS,
+              part = threadIdx.x % THREADS;
     __shared__ int s_bk[27][kTile];
     if (slot >= end) return;
     const float4 pi = C.cell_pos[slot];
     const int word = __float_as_int(pi.w), g = word & kCellIndexMask;
-    float s0[10], s1[10], s2[10];
+    float s0[10], s1[10], s2[10], sum[30];   // of a part; of the parts so far
 #pragma unroll
     for (int k = 0; k < 10; k++) s0[k] = s1[k] = s2[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 30; k++) sum[k] = 0.f;
+    auto flush = [&] {
+#pragma unroll
+        for (int k = 0; k < 10; k++) {
+            sum[k] += s0[k];
+            sum[10 + k] += s1[k];
+            sum[20 + k] += s2[k];
+            s0[k] = s1[k] = s2[k] = 0.f;
+        }
+    };
     float f30 = 0.f, f31 = 0.f;
     if (!(word & kCellExtraBit)) {
         const int cx = cell_coord(pi.x, inv_cell), cy = cell_coord(pi.y, inv_cell), cz = cell_coord(pi.z, inv_cell);
@@ -132,15 +117,16 @@ __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, 
             for (int v = 0; v < c; v++) seen |= (bk[v] == bk[c]);
             dup |= (seen ? 1u : 0u) << c;
         }
-        const int b0 = PARTS == 1 ? bk[0] : s_bk[part][threadIdx.x];
-        int st_next = C.start[b0], ct_next = C.cnt[b0];
-        for (int c = part; c < 27; c += PARTS) {
+        const int c0 = kDescCells * part, c1 = THREADS == 1 ? 27 : min(27, c0 + kDescCells);
+        int st_next = C.start[s_bk[c0][threadIdx.x]], ct_next = C.cnt[s_bk[c0][threadIdx.x]];
+        for (int c = c0; c < c1; c++) {
             const int st_c = st_next, ct_c = ct_next;
-            if (c + PARTS < 27) {   // the next cell's range is fetched while this one runs
-                const int b = s_bk[c + PARTS][threadIdx.x];
+            if (c + 1 < c1) {   // the next cell's range is fetched while this one runs
+                const int b = s_bk[c + 1][threadIdx.x];
                 st_next = C.start[b];
                 ct_next = C.cnt[b];
             }
+            if (THREADS == 1 && c % kDescCells == 0 && c > 0) flush();
             if (((dup >> c) & 1u) || ct_c == 0) continue;
             const int s1e = base + st_c + ct_c;
             for (int s = base + st_c; s < s1e; s += 4) {
@@ -152,7 +138,7 @@ __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, 
                 for (int u = 0; u < 4; u++) {
                     const int wj = __float_as_int(q[u].w);
                     const float ex = q[u].x - pi.x, ey = q[u].y - pi.y, ez = q[u].z - pi.z;
-                    const float r2 = ex * ex + ey * ey + ez * ez;
+                    const float r2 = norm2(ex, ey, ez);
                     if (!(r2 < kDescCut * kDescCut) || !(r2 > 0.f) || (wj & kCellExtraBit) || wj == g) continue;
                     const float rinv = rsqrt_hw(r2), r = r2 * rinv;
                     const float ux = ex * rinv, uy = ey * rinv, uz = ez * rinv;
@@ -165,32 +151,34 @@ __global__ void __launch_bounds__(kTile) k_descriptors(KParams P, DevBuffers B, 
                 }
             }
         }
-        if (PARTS > 1) {
-            const unsigned bead = ((1u << PARTS) - 1u) << (threadIdx.x & 31 & ~(PARTS - 1));
+        if (THREADS > 1) {   // the first thread adds the others' parts to its own
+            const unsigned bead = ((1u << THREADS) - 1u) << (threadIdx.x & 31 & ~(THREADS - 1));
 #pragma unroll
-            for (int o = 1; o < PARTS; o <<= 1)
+            for (int k = 0; k < 10; k++) {
+                float v0 = s0[k], v1 = s1[k], v2 = s2[k];
 #pragma unroll
-                for (int k = 0; k < 10; k++) {
-                    s0[k] += __shfl_xor_sync(bead, s0[k], o);
-                    s1[k] += __shfl_xor_sync(bead, s1[k], o);
-                    s2[k] += __shfl_xor_sync(bead, s2[k], o);
+                for (int o = 1; o < THREADS; o++) {
+                    v0 += __shfl_down_sync(bead, s0[k], o, THREADS);
+                    v1 += __shfl_down_sync(bead, s1[k], o, THREADS);
+                    v2 += __shfl_down_sync(bead, s2[k], o, THREADS);
                 }
+                sum[k] = v0;
+                sum[10 + k] = v1;
+                sum[20 + k] = v2;
+            }
+        } else {
+            flush();
         }
         const float4 ts = stats[traj];
         f30 = logf(fmaxf(ts.w, 1.0f));
         const float dx = pi.x - ts.x, dy = pi.y - ts.y, dz = pi.z - ts.z;
-        f31 = sqrtf(dx * dx + dy * dy + dz * dz) * 0.01f;
+        f31 = sqrtf(norm2(dx, dy, dz)) * 0.01f;
     }
     if (part > 0) return;
     float4 *o = reinterpret_cast<float4 *>(desc + (size_t)g * kF);
-    o[0] = make_float4(s0[0], s0[1], s0[2], s0[3]);
-    o[1] = make_float4(s0[4], s0[5], s0[6], s0[7]);
-    o[2] = make_float4(s0[8], s0[9], s1[0], s1[1]);
-    o[3] = make_float4(s1[2], s1[3], s1[4], s1[5]);
-    o[4] = make_float4(s1[6], s1[7], s1[8], s1[9]);
-    o[5] = make_float4(s2[0], s2[1], s2[2], s2[3]);
-    o[6] = make_float4(s2[4], s2[5], s2[6], s2[7]);
-    o[7] = make_float4(s2[8], s2[9], f30, f31);
+#pragma unroll
+    for (int k = 0; k < 7; k++) o[k] = make_float4(sum[4 * k], sum[4 * k + 1], sum[4 * k + 2], sum[4 * k + 3]);
+    o[7] = make_float4(sum[28], sum[29], f30, f31);
 }
 
 // Exact targets from the current epsilon pass: C_i and beta.
@@ -686,7 +674,7 @@ static void launch_descriptors(mtg_engine *e, const int *gate) {
     if (order_beads_applies(e->max_traj_beads)) {
         inv = order_beads(e->kp, B, e->cells(), kDescCut, e->max_traj_beads, e->surr_stats, e->stream);
     } else {
-        k_traj_stats<<<e->nt, 256, 0, e->stream>>>(e->kp, B, e->surr_stats);
+        k_traj_stats<<<e->nt, kStatsThreads, 0, e->stream>>>(e->kp, B, e->surr_stats);
         inv = bin_beads(e->kp, B, e->cells(), kDescCut, true, e->stream);
     }
     const bool split = e->nb <= kDescSplitBeads;

@@ -133,3 +133,20 @@ def test_surrogate_scratch():
             jobs = [(n, pool.submit(lambda n=n: (s.predict(X[:n]), s.loss_grad(X[:n], T[:n])))) for n in sizes * 3]
             for n, j in jobs:
                 check(j.result(), n)
+
+
+def test_a_trajectory_gets_the_same_bits_in_every_batch():
+    """Descriptors of a batch with one thread a bead and a trajectory past the one-launch ordering, and of
+    its parts with four threads a bead and in one launch."""
+    from mt_gb300 import engine
+    p = synth.default_params(seed=61, hdi_on=1)
+    trajs = [synth.make_trajectory(pf, free, seed=61 + pf, radius=8.12, psi_mode="make_mt", cube=cube, thermal=0.05)
+             for pf, free, cube in ((200, 2600, 120.0), (60, 700, 60.0), (31, 90, 50.0), (120, 1500, 90.0),
+                                    (300, 12600, 260.0))]
+    b = synth.batch_from_trajectories(p, [trajs[k % 4] for k in range(20)] + [trajs[4]])
+    assert b.nbeads > 60000 and np.diff(b.offsets).max() > 16384
+    with engine.Engine(b) as e, engine.ShardedEngine(b, [0] * 3) as s:
+        e.upload_state(b.coords)
+        s.upload_state(b.coords)
+        whole, _ = e.tea_training_data(targets=False)
+        assert np.array_equal(whole, np.concatenate([k.tea_training_data(targets=False)[0] for k in s.engines]))
