@@ -258,14 +258,25 @@ def tea_pairs(b) -> int:
     return tot
 
 
+def engine_constant(name: str) -> int:
+    """An integer constant of the engine's sources (the size limits of its kernels' forms)."""
+    import re
+    src = os.path.join(ROOT, "mt_gb300", "csrc")
+    for f in sorted(os.listdir(src)):
+        m = re.search(rf"constexpr int {name} = (\d+);", open(os.path.join(src, f)).read())
+        if m:
+            return int(m.group(1))
+    raise KeyError(name)
+
+
 def plain_step_time(kt_ms: dict, launches: dict, period: int, b):
     """(kernel, average device ms per MD step) of the plain path's step kernel for
     the batch b: the per-step launch, or the persistent launch that covers a whole
     pair-list period of `period` steps."""
     if launches.get("step_period"):
-        kernel = "k_period_split" if int(np.diff(b.offsets).max()) <= 192 else "k_step_period"
+        kernel = "k_period_split" if int(np.diff(b.offsets).max()) <= engine_constant("kPeriodSplitBeads") else "k_step_period"
         return kernel, kt_ms["step_period"] / (launches["step_period"] * period)
-    kernel = "k_split" if b.nbeads <= 75000 else "k_step_plain"
+    kernel = "k_split" if b.nbeads <= engine_constant("kSplitMaxBeads") else "k_step_plain"
     return kernel, kt_ms["step_plain"] / max(1, launches["step_plain"])
 
 

@@ -324,6 +324,8 @@ __device__ __forceinline__ Frame em_update(const KParams &P, const Frame &Fi, co
 // (250 bytes a bead) do not stay there from step to step: 1024 uneven trajectories
 // of up to 3560 beads 138 -> 134 us a step, 512 x 1520 beads 65.3 -> 64.0; 486,000 beads 42.2
 // and 42.6.
+// kAheadBy: the beads of one CTA of the default block on each of a GB300's SMs (a distance, not a bound: another
+// block or device asks a little earlier or later).
 constexpr int kAheadBeads = 500000, kAheadBy = 152 * 128;
 template <bool KEEP_FORCES, bool AHEAD>
 __global__ void __launch_bounds__(256, 4) k_step_plain(KParams P, DevBuffers B) {

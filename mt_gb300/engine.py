@@ -601,8 +601,10 @@ class ShardedEngine:
     and calls fan out to the engines (concurrently, one host thread each) and
     gather their results in batch order.  No collective and no peer access.
     The noise streams are the ones an engine of the whole batch would draw
-    (mtg_generate_seeds of the whole batch, sliced per group), so the result
-    equals that engine's bit for bit."""
+    (mtg_generate_seeds of the whole batch, sliced per group) and every sum over
+    beads is cut by its trajectory alone, so the result equals that engine's bit
+    for bit, with TEA and in the learned mode too (whose re-check and fall-back judge
+    the beads of each engine by themselves)."""
 
     def __init__(self, batch, devices):
         import concurrent.futures as cf
