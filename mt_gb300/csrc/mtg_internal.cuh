@@ -481,10 +481,11 @@ struct TrajStats {
         __shared__ Sum2 s_sum[kStatsThreads / 32][3];
         __shared__ unsigned s_n[kStatsThreads / 32];
         const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1) {
             for (int d = 0; d < 3; d++)
                 c[d].add(__shfl_xor_sync(0xffffffffu, c[d].s, o), __shfl_xor_sync(0xffffffffu, c[d].e, o));
-        n = __reduce_add_sync(0xffffffffu, n);
+            n += __shfl_xor_sync(0xffffffffu, n, o);
+        }
         if (lane == 0) {
             for (int d = 0; d < 3; d++) s_sum[wid][d] = c[d];
             s_n[wid] = n;
