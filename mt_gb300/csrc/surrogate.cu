@@ -422,6 +422,7 @@ int mtg_surrogate_create(int device, int seed, mtg_surrogate **out) {
     SCK(cudaMalloc(&s->norm, sizeof(s->h_norm)));
     SCK(cudaMalloc(&s->ynorm, sizeof(s->h_ynorm)));
     SCK(cudaMalloc(&s->err, sizeof(int)));
+    SCK(cudaMallocHost(&s->grad, sizeof(float) * mlp::kParams));
     SCK(cudaMemsetAsync(s->err, 0, sizeof(int), s->stream));
     // Glorot-uniform weights, zero biases, identity normalisation
     std::vector<float> h(P, 0.f);
@@ -452,7 +453,7 @@ int mtg_surrogate_destroy(mtg_surrogate *s) {
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
     cudaFree(s->scratch);
-    if (s->grad) cudaFreeHost(s->grad);
+    cudaFreeHost(s->grad);
     cudaFree(s->W.master);
     cudaFree(s->bf);
     cudaFree(s->norm);
@@ -539,7 +540,6 @@ int mtg_surrogate_loss_grad(mtg_surrogate *s, const float *X, const float *T, in
     SCK(mlp::launch_backward_tc(s->W, dX, nullptr, s->norm, dT, n, dY, dZ, dG, dL, s->err, s->stream));
     if (grad) SCK(mlp::launch_grad_sum(dG, parts, dSum, s->stream));
     // the gradient waits here for the error word: the caller's is written by calls that succeed
-    if (grad && !s->grad) SCK(cudaMallocHost(&s->grad, sizeof(float) * mlp::kParams));
     std::vector<float> L(parts);
     int herr = 0;
     if (grad) SCK(cudaMemcpyAsync(s->grad, dSum, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, s->stream));

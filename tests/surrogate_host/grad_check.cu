@@ -49,6 +49,8 @@ int main() {
     static mtg_surrogate s;
     int err = 0;
     s.err = &err;
+    std::vector<float> staging(mlp::kParams);
+    s.grad = staging.data();
     for (float &v : s.h_ynorm) v = 1.0f;
     std::vector<float> X(5 * mlp::kIn, 1.0f), T(5 * mlp::kOut, 1.0f), g(mlp::kParams, -1.0f);
     double loss = -1.0;
