@@ -476,7 +476,7 @@ __device__ __forceinline__ void row_range(const SmemCells &C, int cx, int cy, in
     e = C.end[min(b2, C.m - 1)];
     e2 = b2 >= C.m ? C.end[b2 - C.m] : 0;
 }
-// Calls hit(slot) for every bead of the trajectory in the cells around p that
+// Calls hit(position and index) for every bead of the trajectory in the cells around p that
 // is closer than the root of t2, in no particular order; once for every row whose
 // buckets hold it, so a bead whose own row shares them can come twice.
 template <class F>
@@ -487,13 +487,18 @@ __device__ __forceinline__ void smem_candidates(const SmemCells &C, float4 p, fl
         int s, e, e2;
         row_range(C, cx, cy + r % 3 - 1, cz + r / 3 - 1, s, e, e2);
 #pragma unroll 1
-        for (; s < e || e2 > 0; s++) {
+        for (; s < e || e2 > 0; s += 4) {
             if (s >= e) {
                 s = 0;
                 e = e2;
                 e2 = 0;
             }
-            if (dist2_rn(p, C.pos[s]) < t2) hit(s);
+            float4 q[4];   // four candidates in flight
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = C.pos[min(s + u, e - 1)];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (s + u < e && dist2_rn(p, q[u]) < t2) hit(q[u]);
         }
     }
 }
@@ -653,8 +658,9 @@ __device__ __forceinline__ void store_counts(const KParams &P, const DevBuffers 
 // The lists of a bead with more hits than its slots hold (long cutoffs, dense systems): the
 // smallest keys above the last one taken, kept in order as a walk meets them (a key can come
 // twice), slots after slots.  A call that starts from the bead's index, so that the
-// ordinary path keeps its registers.  256 x 1520 beads with a cutoff of 10, 12, 14 nm: 275, 537,
-// 895 us; 1374, 4175, 8243 with a walk for every entry; 503, 880, 1576 in the general path.
+// ordinary path keeps its registers.  256 x 1520 beads with a cutoff of 10, 12, 14 nm: 254, 508,
+// 832 us; 1374, 4175, 8243 with a walk for every entry; 503, 880, 1576 in the general path (which is
+// ahead in one corner measured: 40 x 8100 beads at 12 nm, up to 68 hits, 1380 against 1260).
 static __device__ __noinline__ void many_hits(const KParams &P, const DevBuffers &B, SmemCells C, ListCuts cut, int g,
                                               int il, uint16_t *col) {
     const int nb = P.nb;
@@ -667,8 +673,8 @@ static __device__ __noinline__ void many_hits(const KParams &P, const DevBuffers
     int n, last = -1;
     do {
         n = 0;
-        smem_candidates(C, K.p, K.lj, [&](int slot) {
-            const unsigned key = K.key(C.pos[slot]);
+        smem_candidates(C, K.p, K.lj, [&](float4 q) {
+            const unsigned key = K.key(q);
             if (key == kNoKey || (int)key <= last || (n == kSmemKeys && key >= col[(kSmemKeys - 1) * kListThreads])) return;
             int k = n < kSmemKeys ? n++ : kSmemKeys - 1;
             for (; k > 0 && col[(k - 1) * kListThreads] > key; k--) col[k * kListThreads] = col[(k - 1) * kListThreads];
