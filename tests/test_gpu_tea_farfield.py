@@ -12,7 +12,6 @@ import numpy as np
 import pytest
 
 from helpers import per_bead_rel, small_system
-from mt_gb300 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -87,6 +86,7 @@ def _trained_surrogate(engine_mod):
 
 def test_learned_mode_with_farfield_runs_and_rechecks(engine_mod):
     s = _trained_surrogate(engine_mod)
+    from mt_gb300 import synth
     p = synth.default_params(seed=52, hdi_on=1, tea_epsilon_freq=5)
     b = synth.uniform_batch(p, 3, 60, 900, seed=52, cube=80.0, thermal=0.05, n_extra_dimers=2)
     e = engine_mod.Engine(b)
@@ -164,6 +164,7 @@ def test_a_trajectory_gets_the_same_bits_in_every_batch(engine_mod, cutoff):
     """Learned TEA of uneven trajectories on one engine, whose near-pair runs fill the GPU, and cut over
     four whose runs are cut elsewhere: effective forces of the far-field product, states and noise
     streams; overlapping pairs from the pair list (8 nm) and from the leaves (5.5 nm)."""
+    from mt_gb300 import synth
     p = synth.default_params(seed=57, hdi_on=1, tea_epsilon_freq=5, ljpairscutoff=cutoff)
     trajs = [synth.make_trajectory(pf, free, seed=57 + pf, radius=8.12, psi_mode="make_mt", cube=90.0, thermal=0.05)
              for pf, free in ((200, 2600), (60, 700), (31, 90), (120, 1500))]
